@@ -1,0 +1,572 @@
+// Greedy-join engine on one thread-block cluster.
+//
+// The same loop as join_engine.cuh (cu/joinEdgeIndel.cu:376-468,
+// cu/joinEdgeBitReverse.cu:404-505), the same joins in the same order, for
+// trees whose slots a cluster of at most 16 CTAs can scan.  The loop is a
+// chain of dependent phases, so what counts is the latency of one phase, not
+// the width of the machine: on 148 CTAs a phase of a 12,000-cell tree took
+// 10.3 us, of which the scan itself was a few hundred nanoseconds and the rest
+// flag barriers through L2, the read of the published table, block-wide
+// argmaxes and about thirty block barriers.  Here
+//  * CTAs exchange their records through distributed shared memory: 16-byte
+//    st.async stores that complete on the receiver's mbarrier, one trip and no
+//    flag, no table read; every wait is bounded;
+//  * a slot's node, maximum and partner live in its CTA's shared memory for
+//    the whole join;
+//  * each CTA publishes the best record of each of four thread groups, after
+//    every phase: the lists are always fresh, so none runs dry.  A rescan phase
+//    publishes them without the rescanned rows, whose new records every CTA
+//    forms itself from the exchanged partial bests;
+//  * one warp takes the decision and broadcasts it through shared memory;
+//  * when half of the slots are dead every CTA squeezes its own range, in the
+//    middle of a join phase; slots never move between CTAs, so a compaction
+//    needs no exchange.
+//
+// A Model supplies the query build, the scores of a CTA's slots and the move
+// of slot data in a compaction.  Rows of new nodes are written by CTA 0 and
+// fenced before its records are sent, so a CTA that has received them reads
+// the row from L2.
+#pragma once
+#include "join_engine.cuh"
+
+namespace casphy {
+namespace joinc {
+
+using joinx::kDead;
+using joinx::kMaxBatch;
+constexpr int kThreads = 512, kWarps = 16;
+constexpr u32 kLists = 4;    // records a CTA publishes per exchange, one per four warps
+constexpr u32 kMaxG = 16;
+constexpr u32 kJoin = 0, kStale = 1;
+
+// One published record: larger ord, then larger inv (smaller node) is better;
+// ord 0 is no record.  slot: rank of the owning CTA << 24 | slot in its range.
+struct alignas(16) Rec {
+    u32 ord, inv, slot, partner;
+};
+
+struct Args {
+    u32 ntip, nnode, G;
+    u32 R;                // slots per CTA at the start
+    const u32* lmOrd;     // ntip slots: maximum, partner and node
+    const u32* lmIdx;
+    const u32* slotNode;
+    u32* nodeSize;
+    u32* rawEdge;
+    int* err;
+    u64 limitNs;
+    unsigned long long* statsOut;  // as joinx::Common
+    unsigned long long* prof;
+    u32 ordNeg1, compactMin, bytesPerPairSite, maxBatch, deathWords, needSizes, keepSizes;
+};
+
+// This CTA's slots [0, n) (capacity cap), in shared memory.
+struct Slots {
+    u32 n, cap;
+    u32* node;
+    u32* ord;
+    u32* idx;
+};
+
+__host__ __device__ inline size_t engine_smem(u32 G, u32 R, u32 deathWords) {
+    const size_t tab = 2 * ((size_t)G * kLists * sizeof(Rec) + (size_t)G * kMaxBatch * sizeof(u64));
+    return (tab + sizeof(u32) * (3 * (size_t)R + joinx::death_words_padded(deathWords)) + 15) & ~size_t(15);
+}
+
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ u32 smem_u32(const void* p) { return static_cast<u32>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ u32 mapa(u32 a, u32 rank) {
+    u32 r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async16(u32 addr, const Rec& r, u32 bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "r"(r.ord), "r"(r.inv), "r"(r.slot), "r"(r.partner), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async8(u32 addr, u64 v, u32 bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_init(u32 bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(u32 bar, u32 bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(u32 bar, u32 parity) {
+    u32 ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0u;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ u32 cluster_rank() {
+    u32 r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// The maximum of the warp's (hi, lo) keys, in every lane.
+__device__ __forceinline__ void warp_max2(u32& hi, u32& lo) {
+    const u32 h = __reduce_max_sync(0xFFFFFFFFu, hi);
+    lo = __reduce_max_sync(0xFFFFFFFFu, hi == h ? lo : 0u);
+    hi = h;
+}
+
+// Best slot of a thread, kept as it walks its slots.
+struct Best {
+    u32 ord, inv, x;
+    __device__ __forceinline__ void init() { ord = inv = x = 0u; }
+    __device__ __forceinline__ void push(u32 o, u32 node, u32 at) {
+        const u32 iv = ~node;
+        if (o > ord || (o == ord && iv > inv)) {
+            ord = o; inv = iv; x = at;
+        }
+    }
+};
+
+// The join loop of one cluster; every CTA of the cluster calls it with its
+// rank.  smem: engine_smem bytes, then the model's.
+template <class M>
+__device__ __forceinline__ void cluster_join(const Args& a, const typename M::Args& m, u32 rank, unsigned char* smem) {
+    const u32 G = a.G;
+    Rec* tab = reinterpret_cast<Rec*>(smem);                       // 2 x G x kLists
+    u64* part = reinterpret_cast<u64*>(tab + 2 * G * kLists);      // 2 x kMaxBatch x G
+    Slots st;
+    st.node = reinterpret_cast<u32*>(part + 2 * G * kMaxBatch);
+    st.ord = st.node + a.R;
+    st.idx = st.ord + a.R;
+    u32* deathBits = st.idx + a.R;
+    typename M::Smem ms;
+    M::carve_smem(a, m, smem + engine_smem(G, a.R, a.deathWords), ms);
+    __shared__ __align__(8) u64 s_bar[2];
+    __shared__ Rec s_wrec[kWarps];
+    __shared__ Rec s_rows[kMaxBatch];   // the rescanned rows
+    __shared__ Rec s_extra[kMaxBatch];  // their new records
+    __shared__ u64 s_red[kMaxBatch][kWarps];
+    __shared__ u32 s_dec[6];            // kind, rescanned rows, j1, slot of j1, j2, failure
+    const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const u32 bar0 = smem_u32(&s_bar[0]);
+
+    joinx::Prof pf;
+    pf.init(a.prof != nullptr && rank == 0);
+    if (tid == 0) {
+        mbar_init(bar0);
+        mbar_init(bar0 + 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (G > 1) mbar_expect(bar0, G * kLists * (u32)sizeof(Rec));  // the first exchange
+    }
+    const u32 lo = min(rank * a.R, a.ntip);
+    st.n = min(lo + a.R, a.ntip) - lo;
+    st.cap = a.R;
+    for (u32 x = tid; x < st.n; x += kThreads) {
+        st.node[x] = a.slotNode[lo + x];
+        st.ord[x] = a.lmOrd[lo + x];
+        st.idx[x] = a.lmIdx[lo + x];
+    }
+    for (u32 i = tid; i < a.deathWords; i += kThreads) deathBits[i] = 0u;
+    if (tid < kMaxBatch * kWarps) (&s_red[0][0])[tid] = 0ull;
+    M::begin(a, m, ms, rank, st);
+    __syncthreads();
+    if (G > 1) cluster_sync();
+
+    // Every group of four warps sends its best record to every CTA.
+    auto send_lists = [&](const Best& b, u32 buf) {
+        u32 hi = b.ord, lw = b.inv;
+        warp_max2(hi, lw);
+        if (hi == 0u) {
+            if (lane == 0) s_wrec[warp] = Rec{0u, 0u, 0u, 0u};
+        } else if (b.ord == hi && b.inv == lw) {
+            s_wrec[warp] = Rec{b.ord, b.inv, (rank << 24) | b.x, st.idx[b.x]};
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");
+        if ((warp & 3) == 0) {
+            const u32 o = lane < 4 ? s_wrec[warp + lane].ord : 0u, v = lane < 4 ? s_wrec[warp + lane].inv : 0u;
+            u32 h2 = o, l2 = v;
+            warp_max2(h2, l2);
+            const u32 w = __ballot_sync(0xFFFFFFFFu, lane < 4 && o == h2 && v == l2);
+            const Rec r = s_wrec[warp + __ffs(w) - 1];
+            Rec* dst = tab + (size_t)buf * G * kLists + rank * kLists + (warp >> 2);
+            if (G == 1) {
+                if (lane == 0) *dst = r;
+            } else if (lane < G) {
+                st_async16(mapa(smem_u32(dst), lane), r, mapa(bar0 + 8 * buf, lane));
+            }
+        }
+    };
+    auto list_best = [&](Best& b) {
+        b.init();
+        for (u32 x = tid; x < st.n; x += kThreads)
+            if (st.node[x] != kDead && st.ord[x] != a.ordNeg1)
+                b.push(st.ord[x], st.node[x], x);
+    };
+
+    const u32 nJoin = a.ntip - 1;
+    u32 k = 0, p = 0, prevQ = 0, S = a.ntip;
+    unsigned long long nStale = 0, nPairs = 0, nComp = 0, algMilli = 0;
+    int fail = 0;
+    {
+        Best b;
+        list_best(b);
+        send_lists(b, 0);
+    }
+    pf.mark(joinx::PROF_COMPACT);
+    for (; k < nJoin; p++) {
+        const u32 buf = p & 1u;
+        if (G == 1) __syncthreads();
+        if (warp == 0) {
+            // the exchange's records, from every CTA
+            u32 bad = 0;
+            if (G > 1) {
+                const u32 bar = bar0 + 8 * buf, parity = (p >> 1) & 1u;
+                if (!mbar_try(bar, parity)) {
+                    const u64 t0 = globaltimer_ns();
+                    while (!mbar_try(bar, parity)) {
+                        if (*(volatile int*)a.err) { bad = 1; break; }
+                        if (globaltimer_ns() - t0 > a.limitNs) {
+                            atomicCAS(a.err, 0, CASPHY_ETIMEOUT);
+                            bad = 1;
+                            break;
+                        }
+                    }
+                }
+                bad = __any_sync(0xFFFFFFFFu, bad);
+            }
+            pf.mark(joinx::PROF_BARRIER);
+            // new records of the rows rescanned in the last phase
+            if (prevQ) {
+                const u32 q = lane >> 2;
+                u64 v = 0ull;
+                if (q < prevQ)
+                    for (u32 r = lane & 3; r < G; r += 4) {
+                        const u64 x = part[((size_t)buf * kMaxBatch + q) * G + r];
+                        v = x > v ? x : v;
+                    }
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    const u64 x = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+                    v = x > v ? x : v;
+                }
+                if (q < prevQ && (lane & 3) == 0) {
+                    const u64 seed = make_key(a.ordNeg1, 0u);
+                    if (v < seed) v = seed;
+                    Rec r = s_rows[q];
+                    const u32 o = key_ord(v);
+                    r.partner = key_node(v);
+                    if (r.slot >> 24 == rank) {
+                        st.ord[r.slot & 0xFFFFFFu] = o;
+                        st.idx[r.slot & 0xFFFFFFu] = r.partner;
+                    }
+                    r.ord = o == a.ordNeg1 ? 0u : o;
+                    if (r.ord == 0u) r.inv = 0u;
+                    s_extra[q] = r;
+                }
+                __syncwarp();
+            }
+            // the decision: the best of up to three records per lane is joined
+            // when its partner lives; else it and the other stale records
+            // above the best live one are rescanned, best first
+            Rec rec[3];
+            bool dead[3];
+            u32 hi = 0, lw = 0;
+#pragma unroll
+            for (u32 j = 0; j < 3; j++) {
+                rec[j] = Rec{0u, 0u, 0u, 0u};
+                if (j < 2) {
+                    if (lane + 32 * j < G * kLists) rec[j] = tab[(size_t)buf * G * kLists + lane + 32 * j];
+                } else if (lane < prevQ) {
+                    rec[j] = s_extra[lane];
+                }
+                if (rec[j].partner >= a.nnode) {
+                    bad = 1;
+                    rec[j].partner = 0u;
+                }
+                dead[j] = rec[j].ord && ((deathBits[rec[j].partner >> 5] >> (rec[j].partner & 31)) & 1u);
+                if (rec[j].ord > hi || (rec[j].ord == hi && rec[j].inv > lw)) {
+                    hi = rec[j].ord;
+                    lw = rec[j].inv;
+                }
+            }
+            const u32 myHi = hi, myLw = lw;
+            warp_max2(hi, lw);
+            u32 nq = 0;
+            bool stale = false;
+#pragma unroll
+            for (u32 j = 0; j < 3; j++) stale |= dead[j] && rec[j].ord == hi && rec[j].inv == lw;
+            if (hi == 0u) bad = bad ? bad : 2u;  // two live rows always have a record
+            if (!__any_sync(0xFFFFFFFFu, stale)) {
+                if (myHi == hi && myLw == lw && hi) {
+#pragma unroll
+                    for (u32 j = 0; j < 3; j++)
+                        if (rec[j].ord == hi && rec[j].inv == lw) {
+                            const u32 j1 = ~lw, j2 = rec[j].partner;
+                            s_dec[2] = j1;
+                            s_dec[3] = rec[j].slot;
+                            s_dec[4] = j2;
+                            if (j1 < a.nnode) {
+                                atomicOr(deathBits + (j1 >> 5), 1u << (j1 & 31));
+                                atomicOr(deathBits + (j2 >> 5), 1u << (j2 & 31));
+                            } else {
+                                bad = 1;
+                            }
+                        }
+                }
+            } else {
+                u32 fk = 0, fi = 0;  // the best record whose partner lives
+#pragma unroll
+                for (u32 j = 0; j < 3; j++)
+                    if (!dead[j] && (rec[j].ord > fk || (rec[j].ord == fk && rec[j].inv > fi))) {
+                        fk = rec[j].ord;
+                        fi = rec[j].inv;
+                    }
+                warp_max2(fk, fi);
+                while (nq < a.maxBatch) {
+#pragma unroll
+                    for (u32 j = 0; j < 3; j++)
+                        if (dead[j] && rec[j].ord == hi && rec[j].inv == lw) {
+                            s_rows[nq] = rec[j];
+                            dead[j] = false;
+                            if ((~lw) >= a.nnode) bad = 1;
+                            // its old record leaves the lists
+                            if (rec[j].slot >> 24 == rank) st.ord[rec[j].slot & 0xFFFFFFu] = a.ordNeg1;
+                        }
+                    nq++;
+                    hi = lw = 0u;
+#pragma unroll
+                    for (u32 j = 0; j < 3; j++)
+                        if (dead[j] && (rec[j].ord > fk || (rec[j].ord == fk && rec[j].inv > fi)) &&
+                            (rec[j].ord > hi || (rec[j].ord == hi && rec[j].inv > lw))) {
+                            hi = rec[j].ord;
+                            lw = rec[j].inv;
+                        }
+                    warp_max2(hi, lw);
+                    if (hi == 0u) break;
+                }
+            }
+            bad = __reduce_max_sync(0xFFFFFFFFu, bad);
+            if (lane == 0) {
+                s_dec[0] = nq ? kStale : kJoin;
+                s_dec[1] = nq;
+                s_dec[5] = bad;
+                if (G > 1) mbar_expect(bar0 + 8 * (buf ^ 1u), G * (kLists * (u32)sizeof(Rec) + nq * (u32)sizeof(u64)));
+            }
+        }
+        __syncthreads();
+        pf.mark(joinx::PROF_DECIDE);
+        const u32 nq = s_dec[1];
+        if (s_dec[5]) {
+            if (s_dec[5] == 2u || G == 1) fail = CASPHY_EINTERNAL;
+            else if (tid == 0) atomicCAS(a.err, 0, CASPHY_EINTERNAL);  // after a timeout the first code stays
+            break;
+        }
+        if (nq) {
+            const u32 nE = M::build_stale(a, m, ms, st, nq, s_rows);
+            pf.mark(joinx::PROF_SELECT);
+            // best (score, node) key of every row over this CTA's live slots
+            // other than its own; one thread calls row(q, ...) per slot
+            u64 bk = 0ull;
+            M::scores(m, ms, st, nq,
+                      [&](u32 q, u32 x, u32 o) {
+                          const u32 node = st.node[x];
+                          if (node == kDead || node == ~s_rows[q].inv) return;
+                          const u64 key = make_key(o, node);
+                          bk = key > bk ? key : bk;
+                      },
+                      [&](u32 q) {  // this warp is done with row q
+                          u32 hi = key_ord(bk), lw = (u32)bk;
+                          warp_max2(hi, lw);
+                          if (lane == 0) s_red[q][warp] = ((u64)hi << 32) | lw;
+                          bk = 0ull;
+                      });
+            pf.mark(joinx::PROF_STALE_SCAN);
+            Best b;
+            list_best(b);
+            send_lists(b, buf ^ 1u);
+            __syncthreads();
+            if (warp < nq) {
+                const u64 v = lane < kWarps ? s_red[warp][lane] : 0ull;
+                u32 hi = key_ord(v), lw = (u32)v;
+                warp_max2(hi, lw);
+                const u64 best = ((u64)hi << 32) | lw;
+                u64* dst = part + ((size_t)(buf ^ 1u) * kMaxBatch + warp) * G + rank;
+                if (G == 1) {
+                    if (lane == 0) *dst = best;
+                } else if (lane < G) {
+                    st_async8(mapa(smem_u32(dst), lane), best, mapa(bar0 + 8 * (buf ^ 1u), lane));
+                }
+                __syncwarp();
+                if (lane < kWarps) s_red[warp][lane] = 0ull;
+            }
+            nStale += nq;
+            nPairs += (unsigned long long)nq * ((a.ntip - k) - 1);
+            algMilli += (unsigned long long)a.bytesPerPairSite * nE * ((a.ntip - k) - 1);
+            prevQ = nq;
+            pf.mark(joinx::PROF_STALE_POST);
+            continue;
+        }
+        // join j1 and j2 into node ntip + k, which takes j1's slot
+        const u32 j1 = s_dec[2], slot1 = s_dec[3], j2 = s_dec[4], newNode = a.ntip + k;
+        u32 sz1 = 0, sz2 = 0;
+        const bool bookkeeper = rank == 0 && tid == kThreads - 1;
+        if (a.needSizes || (a.keepSizes && bookkeeper)) {
+            sz1 = ld_cg_u32(a.nodeSize + j1);
+            sz2 = ld_cg_u32(a.nodeSize + j2);
+        }
+        const u32 own = slot1 >> 24 == rank ? slot1 & 0xFFFFFFu : joinx::kNone;
+        const u32 nE = M::build_join(a, m, ms, st, rank, j1, j2, sz1, sz2, newNode, own);
+        if (bookkeeper) {
+            *reinterpret_cast<uint4*>(a.rawEdge + 4 * (size_t)k) = make_uint4(newNode, j1, newNode, j2);
+            if (a.needSizes || a.keepSizes) a.nodeSize[newNode] = sz1 + sz2;
+        }
+        pf.mark(joinx::PROF_BUILD);
+        Best b;
+        b.init();
+        M::scores(m, ms, st, 1u,
+                  [&](u32, u32 x, u32 o) {
+                      const u32 node = st.node[x];
+                      u32 cur = st.ord[x];
+                      if (node == j1 || node == j2) {
+                          st.node[x] = node == j1 ? newNode : kDead;
+                          st.ord[x] = a.ordNeg1;
+                      } else if (node != kDead) {
+                          if (o > cur) {  // strict improvement
+                              cur = o;
+                              st.ord[x] = o;
+                              st.idx[x] = newNode;
+                          }
+                          if (cur != a.ordNeg1) b.push(cur, node, x);
+                      }
+                  },
+                  [&](u32) {});
+        pf.mark(joinx::PROF_SCAN);
+        nPairs += (a.ntip - k - 1) - 1;
+        algMilli += (unsigned long long)a.bytesPerPairSite * nE * ((a.ntip - k - 1) - 1);
+        k++;
+        const u32 alive = a.ntip - k;
+        if (S >= a.compactMin && 2 * alive < S && k < nJoin) {
+            if (G > 1) cluster_sync();  // the model may read the row CTA 0 has just stored
+            else __syncthreads();
+            // squeeze this CTA's slots, in order: a slot only moves down, and
+            // a chunk is read before any of it is overwritten
+            u32* ranks = M::rank_space(ms);
+            u32 base = 0;
+            for (u32 x0 = 0; x0 < st.n; x0 += kThreads) {
+                const u32 x = x0 + tid;
+                u32 node = kDead, o = 0, i = 0;
+                if (x < st.n) {
+                    node = st.node[x];
+                    o = st.ord[x];
+                    i = st.idx[x];
+                }
+                const u32 live = __ballot_sync(0xFFFFFFFFu, node != kDead);
+                if (lane == 0) s_wrec[warp].ord = __popc(live);
+                __syncthreads();
+                const u32 c = lane < kWarps ? s_wrec[lane].ord : 0u;
+                const u32 before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? c : 0u);
+                const u32 total = __reduce_add_sync(0xFFFFFFFFu, c);
+                const u32 r = base + before + __popc(live & ((1u << lane) - 1u));
+                if (x < st.n) ranks[x] = node != kDead ? r : joinx::kNone;
+                if (node != kDead) {
+                    st.node[r] = node;
+                    st.ord[r] = o;
+                    st.idx[r] = i;
+                }
+                base += total;
+                __syncthreads();
+            }
+            M::compact(a, m, ms, rank, st, base, ranks);
+            st.n = base;
+            __syncthreads();
+            S = alive;
+            nComp++;
+            list_best(b);
+            pf.mark(joinx::PROF_COMPACT);
+        }
+        if (k < nJoin) {  // nothing is sent that nobody waits for
+            // the new node's row, before the records without which no CTA goes on
+            if (rank == 0 && G > 1) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            send_lists(b, buf ^ 1u);
+        }
+        prevQ = 0;
+        pf.mark(joinx::PROF_POST);
+    }
+    if (fail && tid == 0) atomicCAS(a.err, 0, fail);
+    if (rank == 0 && tid == 0) {
+        a.statsOut[0] = nStale;
+        a.statsOut[1] = nPairs;
+        a.statsOut[2] = nComp;
+        a.statsOut[3] = p;
+        a.statsOut[4] = 0;
+        a.statsOut[5] = algMilli / 1000ull;
+    }
+    if (pf.on)
+        for (int i = 0; i < joinx::PROF_N; i++) a.prof[i] = joinx::prof_acc[i];
+    if (G > 1) {
+        // no CTA leaves while another may still write into its shared memory;
+        // after a failure the stores already under way get time to land
+        cluster_sync();
+        if (k < nJoin) {
+            const u64 t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 20000ull) {}
+        }
+        cluster_sync();
+    }
+}
+
+// Host: whether the device can place a cluster of G CTAs of kernel fn.
+inline bool placeable(void* fn, u32 G, size_t smem) {
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(G);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = G;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n >= 1;
+}
+
+// Host: launches `clusters` clusters of G CTAs of kernel fn(args...); *done
+// is false when the device cannot place one (nothing is launched then).
+template <class... K, class... A>
+int launch(void (*fn)(K...), u32 G, u32 clusters, size_t smem, cudaStream_t st, bool* done, const A&... args) {
+    *done = false;
+    if (!placeable((void*)fn, G, smem)) return CASPHY_OK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(G * clusters);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = G;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CASPHY_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, args...));
+    *done = true;
+    return CASPHY_OK;
+}
+
+}  // namespace joinc
+}  // namespace casphy

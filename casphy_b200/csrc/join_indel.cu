@@ -1069,6 +1069,14 @@ struct IndelBits {
     __device__ static void after_compact(const Args&, Smem&, u32, const joinx::Range&) {}
 };
 
+}  // namespace indel
+}  // namespace casphy
+
+#include "join_indel_cluster.cuh"
+
+namespace casphy {
+namespace indel {
+
 // state_out[r] = nodeRow[order[r]] widened to u32
 __global__ void k_gather(const u16* __restrict__ nodeRow, u32 ncol, u32 ncolP, const u32* __restrict__ order,
                          u32 nrows, u32* __restrict__ out) {
@@ -1136,7 +1144,22 @@ static size_t bits_bytes(u32 ntip, u32 ncol, u32 nState) {
     return 2 * (size_t)ncol * nState * Wd * sizeof(u32);
 }
 
-static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nCTA, u32 nChunks, bool useBits) {
+// Trees of at most kClusterTips tips are joined by one cluster.  A phase on a
+// cluster costs about 4 us plus the scan of a sixteenth of the slots, on all
+// SMs about 10 us plus a scan of a 148th: at 65,000 x 1,024 the cluster takes
+// 0.93 s and all SMs 1.10 s, at 12,345 x 777 0.095 s and 0.184 s.
+constexpr u32 kClusterTips = 65536;
+// CTAs of the cluster: 16, fewer when a CTA would have no slot of its own;
+// and the slots of each, a multiple of kBitsAlign.
+static u32 cluster_size(u32 ntip) {
+    u32 G = joinc::kMaxG;
+    while (G > 1 && (G / 2) * kBitsAlign >= ntip) G /= 2;
+    return G;
+}
+static u32 cluster_range(u32 ntip, u32 G) { return ((ntip + G - 1) / G + kBitsAlign - 1) / kBitsAlign * kBitsAlign; }
+
+static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nCTA, u32 nChunks, bool useBits,
+                                bool intPath) {
     const u32 nnode = 2 * ntip - 1, nedge = 2 * ntip - 2;
     // the bitset scan copies 16-byte pieces of bitset rows: slot ranges and
     // row strides are multiples of 128 slots (kBitsAlign)
@@ -1146,11 +1169,14 @@ static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nC
     IndelBuffers l;
     l.Wsel = c.take<u16>(nw ? nw : 1);
     l.nodeRow = c.take<u16>((size_t)nnode * ncolP);
-    l.colT0 = c.take<u16>(useBits ? 0 : (size_t)ncol * Sp);
+    l.colT0 = c.take<u16>(useBits && intPath ? 0 : (size_t)ncol * Sp);  // binary16 initial scan, dense join
     l.colT1 = c.take<u16>(useBits ? 0 : (size_t)ncol * Sp);
     l.bitsWords = useBits ? (size_t)ncol * nState * (Sp / 32) : 0;
-    l.bits0 = c.take<u32>(l.bitsWords);
-    l.bits1 = c.take<u32>(l.bitsWords);
+    // the cluster's layout rounds every CTA's range up
+    const u32 G = cluster_size(ntip);
+    const size_t split = useBits && ntip <= kClusterTips ? (size_t)ncol * nState * (cluster_range(ntip, G) / 32) * G : 0;
+    l.bits0 = c.take<u32>(std::max(l.bitsWords, split));
+    l.bits1 = c.take<u32>(std::max(l.bitsWords, split));
     for (int i = 0; i < 6; i++) l.lm[i] = c.take<u32>(Sp);
     l.node2slot = c.take<u32>(nnode);
     l.nodeDeath = c.take<u32>(nnode);
@@ -1220,6 +1246,75 @@ static int launch_join_fitted(joinx::Common& c, typename M::Args& m, u32* batch,
     return CASPHY_OK;
 }
 
+
+// Cluster and shared memory of an indel join; false when the cluster engine
+// cannot take it.
+template <bool HALF>
+static bool cluster_plan(u32 ntip, u32 ncol, u32 nState, bool unitW, joinc::Args& a,
+                         typename IndelCluster<HALF>::Args& m, size_t* smem) {
+    if (ntip < 2 || ntip > kClusterTips) return false;
+    int smemMax = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return false;
+    const u32 G = cluster_size(ntip);
+    a.ntip = ntip;
+    a.nnode = 2 * ntip - 1;
+    a.G = G;
+    a.R = cluster_range(ntip, G);
+    a.deathWords = (a.nnode + 31) / 32;
+    a.maxBatch = joinx::stale_batch_setting();
+    m.ncol = ncol;
+    m.ncolP = (ncol + 7u) & ~7u;
+    m.nState = nState;
+    m.unitW = unitW ? 1 : 0;
+    m.rows = ncol * nState;
+    const size_t lim = (size_t)smemMax - 6144;  // the kernel's static shared memory
+    // the stage holds at least 32 entries of a CTA's range; then batches of
+    // rescanned rows, then more stage
+    const u32 least = std::max(8192u, 2 * a.R);
+    for (; a.maxBatch >= 1; a.maxBatch--) {
+        m.maxBatch = a.maxBatch;
+        m.stageWords = least;
+        const size_t need = joinc::engine_smem(G, a.R, a.deathWords) + IndelCluster<HALF>::smem_bytes(m, a.R);
+        if (need > lim) continue;
+        m.stageWords += (u32)((std::min(lim, need + 65536) - need) / sizeof(u32)) & ~3u;
+        *smem = joinc::engine_smem(G, a.R, a.deathWords) + IndelCluster<HALF>::smem_bytes(m, a.R);
+        return true;
+    }
+    return false;
+}
+
+// Launches the join on one cluster; *done says whether it could.
+template <bool HALF>
+static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, bool unitW, u32 minSize,
+                                float minRatio, cudaStream_t st, bool* done) {
+    using M = IndelCluster<HALF>;
+    joinc::Args a{};
+    typename M::Args m{};
+    size_t smem = 0;
+    *done = false;
+    if (!cluster_plan<HALF>(ntip, ncol, nState, unitW, a, m, &smem)) return CASPHY_OK;
+    a.lmOrd = L.lm[0]; a.lmIdx = L.lm[1]; a.slotNode = L.lm[2];
+    a.nodeSize = L.nodeSize; a.rawEdge = L.rawEdge; a.err = L.jerr; a.limitNs = 20ull * 1000 * 1000 * 1000;
+    a.statsOut = L.stats;
+    a.prof = getenv("CASPHY_PROFILE") ? L.stats + 8 : nullptr;
+    a.ordNeg1 = ORD_F16_NEG1;
+    a.compactMin = a.G * kBitsAlign + 1;  // a range of one 16-byte piece cannot shrink
+    a.bytesPerPairSite = 125;             // one bit per (candidate, query site)
+    a.needSizes = minSize > 0;            // the minSize / minRatio rule reads node sizes
+    m.minSize = minSize;
+    m.minRatio = minRatio;
+    m.Wsel = L.Wsel;
+    m.nodeRow = L.nodeRow;
+    m.bits[0] = L.bits0;
+    m.bits[1] = L.bits1;
+    if (!joinc::placeable((void*)k_cluster_join<M>, a.G, smem)) return CASPHY_OK;
+    k_split_bits<<<dim3(296, a.G), 256, 0, st>>>(L.bits0, m.rows, (ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32),
+                                                 a.R / 32, L.bits1);
+    return joinc::launch(k_cluster_join<M>, a.G, 1, smem, st, done, a, m);
+}
+
 // Launches prep, initial scan and the persistent join.  Assumes Wsel,
 // tipSize and chunkStart are already on the device; clears everything the
 // kernels expect at zero.  Returns the number of kernels launched.
@@ -1244,17 +1339,18 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
         CASPHY_CUDA_TRY(cudaMemsetAsync(L.bits0, 0, sizeof(u32) * L.bitsWords, st));
         k_build_bits<<<dim3(Sp / 32, (ncol + 31) / 32), dim3(32, 8), 0, st>>>(L.nodeRow, ntip, ncol, ncolP, nState,
                                                                                 Sp / 32, L.bits0);
-    } else {
+    }
+    if (!useBits || !intPath) {
         k_transpose<<<dim3((Sp + 31) / 32, (ncol + 31) / 32), dim3(32, 8), 0, st>>>(L.nodeRow, ntip, ncol, ncolP,
                                                                                       Sp, L.colT0);
     }
     joinx::k_fill_u64<<<(ntip + 255) / 256, 256, 0, st>>>(L.initKey, ntip,
                                                            ((u64)ORD_F16_NEG1 << 32) | 0xFFFFFFFFull);
-    int n = 3;
+    int n = useBits && !intPath ? 4 : 3;
     if (evInit0) CASPHY_CUDA_TRY(cudaEventRecord(evInit0, st));
     InitArgs ia{ntip, ncol, Sp, L.colT0, L.eSC, L.eW, L.eLen, L.chunkStart, nChunks, nTiles, L.tileCounter, L.initKey};
     int perSM = 0;
-    if (useBits) {
+    if (useBits && intPath) {
         InitBitsArgs ib{ntip, ncol, nState, Sp / 32, unitW ? 1 : 0, L.bits0, L.eSC, L.eW, L.eLen, L.chunkStart, nChunks, nTiles,
                         L.tileCounter, L.initKey};
         CASPHY_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_init_bits, kThreads, 0));
@@ -1273,6 +1369,19 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
                                                               L.lm[1], L.lm[2], L.node2slot, L.nodeDeath, L.nodeSize,
                                                               L.tipSize);
     n++;
+    if (useBits) {
+        // one cluster where it can hold the slots; a tree beyond it, or a
+        // device that cannot place the cluster, runs on all SMs
+        bool done = false;
+        const int rc = intPath ? launch_cluster_indel<false>(L, ntip, ncol, nState, unitW, minSize, minRatio, st, &done)
+                               : launch_cluster_indel<true>(L, ntip, ncol, nState, false, minSize, minRatio, st, &done);
+        if (rc) return rc;
+        if (done) {
+            *launches = n + 2;
+            return CASPHY_OK;
+        }
+        if (!intPath) return CASPHY_EINTERNAL;  // the caller asked cluster_plan() before it chose the bitsets
+    }
     joinx::Common c{};
     c.ntip = ntip; c.nnode = nnode; c.nCTA = nCTA; c.align = 8;
     c.lmOrd[0] = L.lm[0]; c.lmIdx[0] = L.lm[1]; c.slotNode[0] = L.lm[2];
@@ -1331,11 +1440,18 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     // allele-bitset scan on the integer path when the two bitset buffers fit
     // a 48 GiB budget (CASPHY_INDEL_SCAN=dense forces the column scan)
     const char* scanEnv = getenv("CASPHY_INDEL_SCAN");
-    bool useBits = intPath && ntip >= 2 && bits_bytes(ntip, ncol, nState) <= (size_t(48) << 30);
+    bool useBits = ntip >= 2 && bits_bytes(ntip, ncol, nState) <= (size_t(48) << 30);
+    if (useBits && !intPath) {  // ordered binary16 sums on the bitsets: the cluster engine only
+        joinc::Args ca{};
+        IndelCluster<true>::Args cm{};
+        size_t cs = 0;
+        useBits = cluster_plan<true>(ntip, ncol, nState, false, ca, cm, &cs) &&
+                  joinc::placeable((void*)k_cluster_join<IndelCluster<true>>, ca.G, cs);
+    }
     if (scanEnv && !strcmp(scanEnv, "dense")) useBits = false;
     lst.scan_path = useBits ? 1u : 0u;
     Carve cv;
-    carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits);
+    carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
     u32* dCodesCopy = cv.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
     u32* dOrder = cv.take<u32>(nrows);
     u32* dState = cv.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
@@ -1344,7 +1460,7 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     if (rc) return rc;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, useBits);
+    const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
     dCodesCopy = c2.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
     dOrder = c2.take<u32>(nrows);
     dState = c2.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
@@ -1619,7 +1735,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev));
     const u32 nChunks = (ntip + kCap - 1) / kCap;
     Carve need;
-    carve_indel(need, ntip, ncol, nState, (u32)nSM, nChunks, false);
+    carve_indel(need, ntip, ncol, nState, (u32)nSM, nChunks, false, false);
     carve_extra(need, ntip, ncol, nState);
     const size_t bytes = need.off + 256;
     if (bytes > kScratchBytes || nChunks > 64) {
@@ -1645,7 +1761,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
     } drain{st};
     Carve c;
     c.base = static_cast<char*>(base);
-    const IndelBuffers L = carve_indel(c, ntip, ncol, nState, (u32)nSM, nChunks, false);
+    const IndelBuffers L = carve_indel(c, ntip, ncol, nState, (u32)nSM, nChunks, false, false);
     const Extra X = carve_extra(c, ntip, ncol, nState);
     const size_t nw = (size_t)nState * ncol;
 
