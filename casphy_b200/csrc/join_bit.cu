@@ -18,7 +18,7 @@
 #include <cstring>
 #include <vector>
 
-#include "join_bit_model.cuh"
+#include "join_bit_cluster.cuh"
 #include "runtime.h"
 
 namespace casphy {
@@ -93,6 +93,50 @@ static int launch_bit_init(const InitArgs& ia, u32 nSM, cudaStream_t st) {
     CASPHY_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_init<PATH>, kThreads, 0));
     k_init<PATH><<<nSM * std::max(perSM, 1), kThreads, 0, st>>>(ia);
     return CASPHY_OK;
+}
+
+// One cluster where its scan of a sixteenth of the matrix is shorter than the
+// phases of the all-SM engine (about 9 us): up to kClusterBytes of columns.
+constexpr size_t kClusterBytes = size_t(8) << 20;
+constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
+
+// Launches the join on one cluster; *done says whether it could.
+template <int PATH>
+static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PATH>::Args& bm, u32 Sp, cudaStream_t st,
+                              bool* done) {
+    using M = BitCluster<PATH>;
+    *done = false;
+    if ((size_t)c.ntip * bm.nbin * sizeof(u32) > kClusterBytes && PATH != PATH_FLOAT) return CASPHY_OK;
+    int smemMax = 0, dev = 0;
+    CASPHY_CUDA_TRY(cudaGetDevice(&dev));
+    CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    joinc::Args a{};
+    a.ntip = c.ntip;
+    a.nnode = c.nnode;
+    a.G = joinc::kMaxG;
+    while (a.G > 1 && (a.G / 2) * kClusterSlots >= c.ntip) a.G /= 2;
+    a.R = ((c.ntip + a.G - 1) / a.G + kClusterSlots - 1) / kClusterSlots * kClusterSlots;
+    // (list entries hold a column offset in 27 bits)
+    if (a.R >= 0xFFFFu || (u64)bm.nbin * Sp >= (1u << 27)) return CASPHY_OK;
+    a.lmOrd = c.lmOrd[0]; a.lmIdx = c.lmIdx[0]; a.slotNode = c.slotNode[0];
+    a.nodeSize = c.nodeSize; a.rawEdge = c.rawEdge; a.err = c.err; a.limitNs = c.limitNs; a.statsOut = c.statsOut;
+    a.prof = c.prof;
+    a.ordNeg1 = c.ordNeg1;
+    a.compactMin = 1024;
+    a.bytesPerPairSite = c.bytesPerPairSite;
+    a.deathWords = (c.nnode + 31) / 32;
+    typename M::Args m{bm.nbin, bm.nbinP, bm.nplanes, bm.ancType, bm.planeMask, bm.wf, bm.nodeSeq, bm.nodeBis,
+                       {bm.colT[0], bm.colT[1]}, Sp, 0, 0};
+    size_t smem = 0;
+    if (!cluster_fit<PATH>(a, m, (size_t)smemMax - 6144, &smem)) return CASPHY_OK;
+    return joinc::launch(k_cluster_join<M>, a.G, 1, smem, st, done, a, m);
+}
+
+template <int PATH>
+static int launch_bit_any(joinx::Common& c, const typename BitModel<PATH>::Args& m, u32 Sp, u32 nCTA, cudaStream_t st) {
+    bool done = false;
+    if (int rc = launch_bit_cluster<PATH>(c, m, Sp, st, &done)) return rc;
+    return done ? CASPHY_OK : launch_bit_join<PATH>(c, m, nCTA, st);
 }
 
 static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_words, const double* weight,
@@ -177,7 +221,7 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
         b.jerr = c.take<int>(1);
         b.tileCounter = c.take<unsigned long long>(1);
         b.chunkStart = c.take<u64>(nChunks + 1);
-        b.stats = c.take<unsigned long long>(8);
+        b.stats = c.take<unsigned long long>(8 + joinx::PROF_N);
         b.tip = c.take<u32>(ntip);
         b.order = c.take<u32>(nrows);
         b.state = c.take<u32>(h_state_out ? (size_t)nrows * nbin : 0);
@@ -249,18 +293,19 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
         c.ordNeg1 = ORD_F32_NEG1; c.compactMin = 4096; c.compactQ8 = 192; c.bytesPerPairSite = 4000;
         c.maxBatch = joinx::stale_batch_setting();
         c.deathWords = (nnode + 31) / 32;
+        c.prof = getenv("CASPHY_PROFILE") ? L.stats + 8 : nullptr;
         if (path == PATH_UNIT) {
             BitModel<PATH_UNIT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                         {L.colT0, L.colT1}};
-            rc = launch_bit_join<PATH_UNIT>(c, m, nCTA, st);
+            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, nCTA, st);
         } else if (path == PATH_PLANES) {
             BitModel<PATH_PLANES>::Args m{nbin, nbinP, nplanes, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                           {L.colT0, L.colT1}};
-            rc = launch_bit_join<PATH_PLANES>(c, m, nCTA, st);
+            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, nCTA, st);
         } else {
             BitModel<PATH_FLOAT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                          {L.colT0, L.colT1}};
-            rc = launch_bit_join<PATH_FLOAT>(c, m, nCTA, st);
+            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, nCTA, st);
         }
         if (rc) return rc;
         launches += 2;
@@ -279,6 +324,11 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
             return jerr;
         }
         joinx::preorder_relabel(ntip, raw.data(), edge_out, order.data());
+        if (getenv("CASPHY_PROFILE")) {
+            unsigned long long prof[joinx::PROF_N] = {0};
+            CASPHY_CUDA_TRY(cudaMemcpy(prof, L.stats + 8, sizeof(prof), cudaMemcpyDeviceToHost));
+            joinx::print_profile(prof);
+        }
     }
     CASPHY_CUDA_TRY(cudaMemcpyAsync(L.order, order.data(), sizeof(u32) * nrows, cudaMemcpyHostToDevice, st));
     u32* sout = d_state_out ? d_state_out : L.state;

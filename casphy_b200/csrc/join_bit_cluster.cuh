@@ -1,0 +1,299 @@
+// Bit-join model for the cluster engine (join_cluster.cuh), for the single
+// join and the batched bootstrap.
+//
+// A CTA keeps the columns of its slots (word w of every slot) in shared
+// memory when they fit, from the start or from the first compaction that makes
+// them fit; until then it reads them from global memory.  Lane = slot, so
+// every read is a row of consecutive words and the query words are broadcast.
+// The warps are shared out among the queries of a rescan batch.
+//  * integer weights: one popcount per (slot, word, plane);
+//  * FLOAT: the query's set bits with their weights as a list in ascending
+//    order, one predicated add each.  (Walking the set bits of every slot's
+//    own intersection, with the weight loaded per bit, took 28 us a scan of a
+//    2,999 x 352 tree.)
+#pragma once
+#include "join_bit_model.cuh"
+#include "join_cluster.cuh"
+
+namespace casphy {
+namespace bitjoin {
+
+template <int PATH>
+struct BitCluster {
+    struct Args {
+        u32 nbin, nbinP, nplanes;
+        int ancType;
+        const u32* planeMask;  // nplanes x nbin
+        const float* wf;       // nbin x 32 (FLOAT)
+        u32* nodeSeq;
+        u32* nodeBis;
+        u32* colT[2];          // nbin x Sp
+        u32 Sp, maxBatch;
+        u32 colWords;          // shared-memory words for resident columns
+    };
+    struct Smem {
+        u32* sq;       // maxBatch x planes x nbinP: (plane-masked) query words
+        uint2* ent;    // FLOAT: maxBatch x nbin * 32 (column offset << 5 | bit, weight), ascending
+        u32* len;      // FLOAT: maxBatch list lengths
+        u32* colS;     // resident columns
+        u16* ranks;
+        const u32* col;
+        u32 stride;
+        u32 next;      // global buffer the next compaction writes
+        u32 rank;
+        u32 par;
+    };
+    __host__ __device__ static u32 planes(const Args& m) { return PATH == PATH_PLANES && m.nplanes ? m.nplanes : 1u; }
+    __host__ static size_t smem_bytes(const Args& m, u32 R) {
+        size_t s = sizeof(u32) * ((size_t)m.maxBatch * planes(m) * m.nbinP + m.colWords) + sizeof(u16) * (size_t)R + 32;
+        if (PATH == PATH_FLOAT)
+            s += (size_t)m.maxBatch * (sizeof(uint2) * m.nbin * 32 + sizeof(u32));
+        return s;
+    }
+    __device__ static void carve_smem(const joinc::Args& a, const Args& m, unsigned char* p, Smem& s) {
+        s.ent = reinterpret_cast<uint2*>(p);
+        s.sq = reinterpret_cast<u32*>(s.ent + (PATH == PATH_FLOAT ? (size_t)m.maxBatch * m.nbin * 32 : 0u));
+        s.colS = s.sq + (size_t)m.maxBatch * planes(m) * m.nbinP;
+        s.len = s.colS + m.colWords;
+        s.ranks = reinterpret_cast<u16*>(s.len + (PATH == PATH_FLOAT ? m.maxBatch : 0u));
+        s.par = 0;
+        (void)a;
+    }
+    __device__ static u16* rank_space(Smem& s) { return s.ranks; }
+    // non-zero (word, plane) entries of the queries being built
+    __device__ static u32* entries(u32 par) {
+        __shared__ u32 s_ne[2];
+        return s_ne + par;
+    }
+    __device__ static void begin(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots& st) {
+        s.rank = rank;
+        s.col = m.colT[0] + (size_t)rank * a.R;
+        s.stride = m.Sp;
+        s.next = 1;
+        if (threadIdx.x < 2) *entries(threadIdx.x) = 0u;
+        if ((size_t)m.nbin * a.R <= m.colWords) {
+            const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            for (u32 w = warp; w < m.nbin; w += joinc::kWarps)
+                for (u32 x = lane; x < st.n; x += 32) s.colS[w * a.R + x] = s.col[(size_t)w * m.Sp + x];
+            s.col = s.colS;
+            s.stride = a.R;
+        }
+    }
+    // Query q's words of one row, this thread's word w (every lane of the warp
+    // calls it; sq = 0 past the row).
+    __device__ static void put(const Args& m, Smem& s, u32 q, u32 w, u32 sq) {
+        const u32 P = planes(m);
+        u32 ne = 0;
+        for (u32 k = 0; k < P; k++) {
+            u32 v = sq;
+            if (PATH == PATH_PLANES && m.nplanes) v &= w < m.nbin ? __ldg(m.planeMask + (size_t)k * m.nbin + w) : 0u;
+            if (w < m.nbinP) s.sq[((size_t)q * P + k) * m.nbinP + w] = v;
+            ne += __popc(__ballot_sync(0xFFFFFFFFu, v != 0u));
+        }
+        if ((threadIdx.x & 31) == 0 && s.rank == 0) atomicAdd(entries(s.par), ne);
+    }
+    // The queries are complete.  FLOAT: their lists, a warp per (query, word),
+    // lane = bit; the bits of the words before place the word's entries.
+    __device__ static u32 finish(const Args& m, Smem& s, u32 nq) {
+        __syncthreads();
+        if (threadIdx.x == 0) *entries(s.par ^ 1u) = 0u;
+        if (PATH == PATH_FLOAT) {
+            const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            for (u32 q = 0; q < nq; q++) {
+                const u32* sq = s.sq + (size_t)q * m.nbinP;
+                for (u32 w = (warp + 16u - (q * m.nbin) % 16u) % 16u; w < m.nbin; w += joinc::kWarps) {
+                    const u32 v = sq[w];
+                    u32 before = 0;
+                    for (u32 i = lane; i < w; i += 32) before += __popc(sq[i]);
+                    before = __reduce_add_sync(0xFFFFFFFFu, before);
+                    if ((v >> lane) & 1u)
+                        s.ent[(size_t)q * m.nbin * 32 + before + __popc(v & ((1u << lane) - 1u))] =
+                            make_uint2((w * s.stride) << 5 | lane, __float_as_uint(__ldg(m.wf + w * 32 + lane)));
+                    if (w == m.nbin - 1 && lane == 0) s.len[q] = before + __popc(v);
+                }
+            }
+            __syncthreads();
+        }
+        return *entries(s.par);
+    }
+    // Warps of one query: all 16 for one, down to two each for eight.
+    __device__ static u32 build_stale(const joinc::Args&, const Args& m, Smem& s, const joinc::Slots&, u32 nq,
+                                      const joinc::Rec* rows) {
+        s.par ^= 1u;
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const u32 lgq = nq <= 1 ? 4u : (nq <= 2 ? 3u : (nq <= 4 ? 2u : 1u));
+        const u32 nwq = 1u << lgq, q = warp >> lgq, wi = warp & (nwq - 1u);
+        if (q < nq) {
+            const u32* src = m.nodeSeq + (size_t)(~rows[q].inv) * m.nbinP;
+            for (u32 w0 = wi * 32; w0 < m.nbinP; w0 += nwq * 32) {
+                const u32 w = w0 + lane;
+                put(m, s, q, w, w < m.nbin ? ld_cg_u32(src + w) : 0u);
+            }
+        }
+        return finish(m, s, nq);
+    }
+    // ancestral rules (updateAncestralKernel / updateAncestralKernel2,
+    // cu/joinEdgeBitReverse.cu:77-113)
+    __device__ static u32 build_join(const joinc::Args&, const Args& m, Smem& s, const joinc::Slots&, u32 rank, u32 j1,
+                                     u32 j2, u32, u32, u32 newNode, u32 own) {
+        s.par ^= 1u;
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        {
+            const size_t r1 = (size_t)j1 * m.nbinP, r2 = (size_t)j2 * m.nbinP, rn = (size_t)newNode * m.nbinP;
+            u32* col = const_cast<u32*>(s.col);
+            for (u32 w0 = warp * 32; w0 < m.nbinP; w0 += joinc::kWarps * 32) {
+                const u32 w = w0 + lane;
+                u32 sq = 0, bs = 0;
+                if (w < m.nbin) {
+                    const u32 s1 = ld_cg_u32(m.nodeSeq + r1 + w), s2 = ld_cg_u32(m.nodeSeq + r2 + w);
+                    const u32 bs1 = ld_cg_u32(m.nodeBis + r1 + w), bs2 = ld_cg_u32(m.nodeBis + r2 + w);
+                    if (m.ancType == 0) {
+                        const u32 diff = s1 ^ s2;
+                        const u32 conflict = diff & (bs1 | bs2);
+                        sq = (s1 | s2) & ~conflict;
+                        bs = (diff & ~(bs1 ^ bs2)) | (bs1 & bs2);
+                    } else {
+                        sq = (s1 & s2) | (bs1 & s2) | (bs2 & s1);
+                        bs = (s1 ^ s2) & ~(bs1 | bs2);
+                    }
+                }
+                if (rank == 0 && w < m.nbinP) {
+                    m.nodeSeq[rn + w] = sq;
+                    m.nodeBis[rn + w] = bs;
+                }
+                if (own != kNone && w < m.nbin) col[(size_t)w * s.stride + own] = sq;
+                put(m, s, 0u, w, sq);
+            }
+        }
+        return finish(m, s, 1u);
+    }
+
+    template <class F, class D>
+    __device__ static void scores(const Args& m, Smem& s, const joinc::Slots& st, u32 nq, F f, D done) {
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const u32 lgq = nq <= 1 ? 4u : (nq <= 2 ? 3u : (nq <= 4 ? 2u : 1u));
+        const u32 nwq = 1u << lgq;
+        const u32 q = warp >> lgq, wi = warp & (nwq - 1u);
+        if (q < nq) {
+            const u32 P = planes(m);
+            const u32* sq = s.sq + (size_t)q * P * m.nbinP;
+            const bool resident = s.col == s.colS;
+            for (u32 x0 = wi * 32; x0 < st.n; x0 += nwq * 32) {
+                const u32 x = x0 + lane, xs = x < st.n ? x : x0;
+                float fa = 0.f;
+                u32 acc = 0;
+                if (PATH == PATH_FLOAT) {
+                    const u32 n = s.len[q];
+                    const uint2* ent = s.ent + (size_t)q * m.nbin * 32;
+                    const u32* c = (resident ? s.colS : s.col) + xs;
+                    auto add = [&](u32 v, uint2 t) {
+                        asm("{\n .reg .pred p;\n .reg .b32 t;\n shf.r.wrap.b32 t, %1, %1, %2;\n and.b32 t, t, 1;\n"
+                            " setp.ne.u32 p, t, 0;\n @p add.rn.f32 %0, %0, %3;\n}"
+                            : "+f"(fa)
+                            : "r"(v), "r"(t.x), "f"(__uint_as_float(t.y)));
+                    };
+                    // only this CTA writes its columns, so plain loads do
+                    u32 e = 0;
+                    for (; e + 7 < n; e += 8) {
+                        uint2 t[8];
+                        u32 v[8];
+#pragma unroll
+                        for (u32 j = 0; j < 8; j++) t[j] = ent[e + j];
+#pragma unroll
+                        for (u32 j = 0; j < 8; j++) v[j] = c[t[j].x >> 5];
+#pragma unroll
+                        for (u32 j = 0; j < 8; j++) add(v[j], t[j]);
+                    }
+                    for (; e < n; e++) add(c[ent[e].x >> 5], ent[e]);
+                } else if (resident) {
+                    const u32* c = s.colS + xs;
+                    if (P == 1) {
+#pragma unroll 8
+                        for (u32 w = 0; w < m.nbin; w++) acc += (u32)__popc(sq[w] & c[w * s.stride]);
+                    } else {
+#pragma unroll 4
+                        for (u32 w = 0; w < m.nbin; w++) {
+                            const u32 v = c[w * s.stride];
+                            for (u32 k = 0; k < P; k++) acc += (u32)__popc(sq[k * m.nbinP + w] & v) << k;
+                        }
+                    }
+                } else {
+                    const u32* c = s.col + xs;
+                    for (u32 w0 = 0; w0 < m.nbin; w0 += 8) {
+                        u32 v[8];
+#pragma unroll
+                        for (u32 j = 0; j < 8; j++) v[j] = w0 + j < m.nbin ? ld_cg_u32(c + (size_t)(w0 + j) * s.stride) : 0u;
+                        for (u32 k = 0; k < P; k++)
+#pragma unroll
+                            for (u32 j = 0; j < 8; j++)
+                                if (w0 + j < m.nbin) acc += (u32)__popc(sq[k * m.nbinP + w0 + j] & v[j]) << k;
+                    }
+                }
+                if (x < st.n) f(q, x, ord_f32(PATH == PATH_FLOAT ? fa : (float)acc));
+            }
+            done(q);
+        }
+        joinx::prof_mark(joinx::PROF_SC_ACC);
+    }
+
+    // Moves the live slots' columns to their new places; n live slots, ranks
+    // by old slot.  In shared memory in place, a warp per column: a slot only
+    // moves down, and 32 are read before any of them is written.
+    __device__ static void compact(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots& st, u32 n,
+                                   const u16* ranks) {
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const bool resident = s.col == s.colS;
+        const u32 Rn = (n + 31u) & ~31u;
+        u32* dst = s.colS;
+        u32 stride = s.stride;
+        if (!resident) {
+            if ((size_t)m.nbin * Rn <= m.colWords) {
+                stride = Rn;
+            } else {
+                dst = (s.next ? m.colT[1] : m.colT[0]) + (size_t)rank * a.R;
+                s.next ^= 1u;
+            }
+        }
+        for (u32 w = warp; w < m.nbin; w += joinc::kWarps) {
+            const u32* src = s.col + (size_t)w * s.stride;
+            for (u32 x0 = 0; x0 < st.n; x0 += 32) {
+                const u32 x = x0 + lane;
+                const u32 r = x < st.n ? ranks[x] : 0xFFFFu;
+                u32 v = 0;
+                if (r != 0xFFFFu) v = resident ? src[x] : ld_cg_u32(src + x);
+                __syncwarp();
+                if (r != 0xFFFFu) dst[(size_t)w * stride + r] = v;
+                __syncwarp();
+            }
+        }
+        s.col = dst;
+        s.stride = stride;
+        __syncthreads();
+    }
+};
+
+template <class M>
+__global__ void __launch_bounds__(joinc::kThreads, 1) k_cluster_join(joinc::Args a, typename M::Args m) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    joinc::cluster_join<M>(a, m, joinc::cluster_rank(), smem);
+}
+
+// Shared memory of a cluster join of a.ntip cells by a.G CTAs (a.R set):
+// batches of rescanned rows first, then resident columns; false when it does
+// not fit.
+template <int PATH>
+inline bool cluster_fit(joinc::Args& a, typename BitCluster<PATH>::Args& m, size_t lim, size_t* smem) {
+    for (a.maxBatch = joinx::stale_batch_setting(); a.maxBatch >= 1; a.maxBatch--) {
+        m.maxBatch = a.maxBatch;
+        m.colWords = 0;
+        const size_t need = joinc::engine_smem(a.G, a.R, a.deathWords) + BitCluster<PATH>::smem_bytes(m, a.R);
+        if (need > lim) continue;
+        m.colWords = (u32)std::min<size_t>((lim - need) / sizeof(u32), (size_t)m.nbin * a.R);
+        *smem = joinc::engine_smem(a.G, a.R, a.deathWords) + BitCluster<PATH>::smem_bytes(m, a.R);
+        return true;
+    }
+    return false;
+}
+
+}  // namespace bitjoin
+}  // namespace casphy

@@ -47,7 +47,7 @@ struct alignas(16) Rec {
 
 struct Args {
     u32 ntip, nnode, G;
-    u32 R;                // slots per CTA at the start
+    u32 R;                // slots per CTA at the start, below 65,535
     const u32* lmOrd;     // ntip slots: maximum, partner and node
     const u32* lmIdx;
     const u32* slotNode;
@@ -456,7 +456,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             else __syncthreads();
             // squeeze this CTA's slots, in order: a slot only moves down, and
             // a chunk is read before any of it is overwritten
-            u32* ranks = M::rank_space(ms);
+            u16* ranks = M::rank_space(ms);
             u32 base = 0;
             for (u32 x0 = 0; x0 < st.n; x0 += kThreads) {
                 const u32 x = x0 + tid;
@@ -473,7 +473,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
                 const u32 before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? c : 0u);
                 const u32 total = __reduce_add_sync(0xFFFFFFFFu, c);
                 const u32 r = base + before + __popc(live & ((1u << lane) - 1u));
-                if (x < st.n) ranks[x] = node != kDead ? r : joinx::kNone;
+                if (x < st.n) ranks[x] = (u16)(node != kDead ? r : 0xFFFFu);
                 if (node != kDead) {
                     st.node[r] = node;
                     st.ord[r] = o;

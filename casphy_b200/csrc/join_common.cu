@@ -1,4 +1,5 @@
 // Kernels and host helpers shared by the indel and bit joins.
+#include <cstdio>
 #include <vector>
 
 #include "join_engine.cuh"
@@ -32,6 +33,14 @@ __global__ void k_slot_init(u32 ntip, u32 Sp, u32 nnode, const unsigned long lon
 __global__ void k_fill_u64(unsigned long long* p, u64 n, u64 v) {
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
+}
+
+void print_profile(const unsigned long long* prof) {
+    static const char* names[PROF_N] = {"barrier", "table", "decide", "build", "scan", "post", "stale_post",
+                                        "compact", "select", "stale_scan", "sc_copy", "sc_acc", "sc_red"};
+    fprintf(stderr, "join-loop sections (CTA 0, ms):");
+    for (int i = 0; i < PROF_N; i++) fprintf(stderr, " %s=%.1f", names[i], prof[i] / 1e6);
+    fprintf(stderr, "\n");
 }
 
 // Pre-order walk of the raw join edges (cu/joinEdgeIndel.cu:488-558): node v's

@@ -840,6 +840,9 @@ __global__ void k_slot_init(u32 ntip, u32 Sp, u32 nnode, const unsigned long lon
                             const u32* tipSize);
 __global__ void k_fill_u64(unsigned long long* p, u64 n, u64 v);
 
+// Prints a join loop's section times (CASPHY_PROFILE).
+void print_profile(const unsigned long long* prof);
+
 // Pre-order walk of the raw join edges (cu/joinEdgeIndel.cu:488-558).
 void preorder_relabel(u32 ntip, const u32* rawEdge, u32* edge_out, u32* order);
 

@@ -1511,12 +1511,7 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
         }
         joinx::preorder_relabel(ntip, raw.data(), edge_out, order.data());
         if (getenv("CASPHY_PROFILE")) {
-            static const char* names[joinx::PROF_N] = {"barrier", "table", "decide", "build", "scan", "post",
-                                                       "stale_post", "compact", "select", "stale_scan",
-                                                       "sc_copy", "sc_acc", "sc_red"};
-            fprintf(stderr, "join-loop sections (CTA 0, ms):");
-            for (int i = 0; i < joinx::PROF_N; i++) fprintf(stderr, " %s=%.1f", names[i], prof[i] / 1e6);
-            fprintf(stderr, "\n");
+            joinx::print_profile(prof);
         }
         for (u32 i = 0; i + 1 < ntip; i++) lst.alg_bytes_init += 2ull * eLenH[i] * (u64)(ntip - 1 - i);
     } else {

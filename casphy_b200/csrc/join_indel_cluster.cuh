@@ -62,7 +62,7 @@ struct IndelCluster {
         s.sums = reinterpret_cast<u16*>(s.eW + (m.unitW ? 0u : (size_t)m.maxBatch * ncolW(m.ncol)));
         s.par = 0;
     }
-    __device__ static u32* rank_space(Smem& s) { return s.stage; }
+    __device__ static u16* rank_space(Smem& s) { return reinterpret_cast<u16*>(s.stage); }
     // A CTA's bitset rows lie together, so that its share of the matrix stays
     // as small as its live slots: k_split_bits has laid them out in bits[1].
     __device__ static void begin(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots&) {
@@ -412,7 +412,7 @@ struct IndelCluster {
     // Rebuilds this CTA's words in the other buffer from the live slots' rows.
     // The engine has moved st.node already; n live slots.
     __device__ static void compact(const joinc::Args&, const Args& m, Smem& s, u32, const joinc::Slots& st, u32 n,
-                                   const u32*) {
+                                   const u16*) {
         const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         u32* B = s.other;
         const u32 pitch = (n + 127u) / 128u * 4u;

@@ -50,3 +50,18 @@ def test_cluster_join_vs_column_scan(gpu_lib, monkeypatch, ncell, nsite, weights
     e0, s0, st0 = gpu_lib.join_indel(codes, ns, w)
     assert st0["scan_path"] == 0
     assert np.array_equal(e1, e0) and np.array_equal(s1, s0)
+
+
+@pytest.mark.parametrize("weights", ["unit", "planes", "float"])
+@pytest.mark.parametrize("ncell,nsite,atype", [
+    (2, 32, 0), (3, 64, 1), (31, 32, 1), (33, 96, 0), (513, 96, 1), (1100, 1056, 0), (2500, 64, 1), (6000, 224, 1)])
+def test_cluster_bit_join_vs_oracle(gpu_lib, weights, ncell, nsite, atype):
+    """Bit rows: one cell to a range and several words per lane; columns that
+    are resident in shared memory at once and only after a compaction."""
+    words = synth.binary_workload(ncell, nsite, 14, 0.04, 0.05, seed=ncell + nsite)
+    rng = np.random.default_rng(ncell)
+    w = {"unit": None, "planes": rng.integers(0, 7, size=nsite).astype(float),
+         "float": rng.uniform(0.01, 3.0, size=nsite)}[weights]
+    e1, s1, _ = gpu_lib.join_bit(words, w, atype)
+    e0, s0, _ = O.join_bit(words, w, atype)
+    assert np.array_equal(e1, e0) and np.array_equal(s1, s0)
