@@ -95,9 +95,12 @@ static int launch_bit_init(const InitArgs& ia, u32 nSM, cudaStream_t st) {
     return CASPHY_OK;
 }
 
-// One cluster where its scan of a sixteenth of the matrix is shorter than the
-// phases of the all-SM engine (about 9 us): up to kClusterBytes of columns.
-constexpr size_t kClusterBytes = size_t(8) << 20;
+// One cluster where every CTA can keep its slots' columns in shared memory
+// from the start: 20,000 x 1,024 takes 3.9 us a phase against 8.6 us on all
+// SMs, but 40,000 x 1,024, whose columns are read through L2 by one GPC,
+// 13.3 us against 8.8 us.  Fractional weights are bound by their ordered adds,
+// and one cluster is the better at every size (30,000 x 1,024: 32 us a phase
+// against 83 us).
 constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 
 // Launches the join on one cluster; *done says whether it could.
@@ -106,7 +109,6 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
                               bool* done) {
     using M = BitCluster<PATH>;
     *done = false;
-    if ((size_t)c.ntip * bm.nbin * sizeof(u32) > kClusterBytes && PATH != PATH_FLOAT) return CASPHY_OK;
     int smemMax = 0, dev = 0;
     CASPHY_CUDA_TRY(cudaGetDevice(&dev));
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -129,6 +131,7 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
                        {bm.colT[0], bm.colT[1]}, Sp, 0, 0};
     size_t smem = 0;
     if (!cluster_fit<PATH>(a, m, (size_t)smemMax - 6144, &smem)) return CASPHY_OK;
+    if (PATH != PATH_FLOAT && m.colWords < (size_t)m.nbin * a.R) return CASPHY_OK;
     return joinc::launch(k_cluster_join<M>, a.G, 1, smem, st, done, a, m);
 }
 

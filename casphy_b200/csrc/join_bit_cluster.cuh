@@ -45,7 +45,8 @@ struct BitCluster {
     };
     __host__ __device__ static u32 planes(const Args& m) { return PATH == PATH_PLANES && m.nplanes ? m.nplanes : 1u; }
     __host__ static size_t smem_bytes(const Args& m, u32 R) {
-        size_t s = sizeof(u32) * ((size_t)m.maxBatch * planes(m) * m.nbinP + m.colWords) + sizeof(u16) * (size_t)R + 32;
+        // (4 words more: the last plane's words are read eight at a time)
+        size_t s = sizeof(u32) * ((size_t)m.maxBatch * planes(m) * m.nbinP + 4 + m.colWords) + sizeof(u16) * (size_t)R + 32;
         if (PATH == PATH_FLOAT)
             s += (size_t)m.maxBatch * (sizeof(uint2) * m.nbin * 32 + sizeof(u32));
         return s;
@@ -53,7 +54,7 @@ struct BitCluster {
     __device__ static void carve_smem(const joinc::Args& a, const Args& m, unsigned char* p, Smem& s) {
         s.ent = reinterpret_cast<uint2*>(p);
         s.sq = reinterpret_cast<u32*>(s.ent + (PATH == PATH_FLOAT ? (size_t)m.maxBatch * m.nbin * 32 : 0u));
-        s.colS = s.sq + (size_t)m.maxBatch * planes(m) * m.nbinP;
+        s.colS = s.sq + (size_t)m.maxBatch * planes(m) * m.nbinP + 4;
         s.len = s.colS + m.colWords;
         s.ranks = reinterpret_cast<u16*>(s.len + (PATH == PATH_FLOAT ? m.maxBatch : 0u));
         s.par = 0;
@@ -168,6 +169,69 @@ struct BitCluster {
         return finish(m, s, 1u);
     }
 
+    // Score of query q (words sq) against the slot whose word w is c[w * stride].
+    template <bool RES>
+    __device__ __forceinline__ static float score(const Args& m, const Smem& s, const u32* c, u32 q, const u32* sq) {
+        const u32 stride = s.stride;
+        if (PATH == PATH_FLOAT) {
+            float fa = 0.f;
+            const u32 n = s.len[q];
+            const uint2* ent = s.ent + (size_t)q * m.nbin * 32;
+            auto add = [&](u32 v, uint2 t) {
+                asm("{\n .reg .pred p;\n .reg .b32 t;\n shf.r.wrap.b32 t, %1, %1, %2;\n and.b32 t, t, 1;\n"
+                    " setp.ne.u32 p, t, 0;\n @p add.rn.f32 %0, %0, %3;\n}"
+                    : "+f"(fa)
+                    : "r"(v), "r"(t.x), "f"(__uint_as_float(t.y)));
+            };
+            // (only this CTA writes its columns, so plain loads do)
+            u32 e = 0;
+            for (; e + 7 < n; e += 8) {
+                uint2 t[8];
+                u32 v[8];
+#pragma unroll
+                for (u32 j = 0; j < 8; j++) t[j] = ent[e + j];
+#pragma unroll
+                for (u32 j = 0; j < 8; j++) v[j] = c[t[j].x >> 5];
+#pragma unroll
+                for (u32 j = 0; j < 8; j++) add(v[j], t[j]);
+            }
+            for (; e < n; e++) add(c[ent[e].x >> 5], ent[e]);
+            return fa;
+        }
+        const u32 P = planes(m);
+        u32 acc = 0;
+        if (P == 1 && RES) {
+#pragma unroll 8
+            for (u32 w = 0; w < m.nbin; w++) acc += (u32)__popc(sq[w] & c[w * stride]);
+            return (float)acc;
+        }
+        // eight words of the slot at a time against every plane's
+        u32 w0 = 0;
+        auto block = [&](const u32 (&v)[8]) {
+            for (u32 k = 0; k < P; k++) {
+                const uint4 a = *reinterpret_cast<const uint4*>(sq + k * m.nbinP + w0);
+                const uint4 b = *reinterpret_cast<const uint4*>(sq + k * m.nbinP + w0 + 4);
+                acc += (u32)(__popc(a.x & v[0]) + __popc(a.y & v[1]) + __popc(a.z & v[2]) + __popc(a.w & v[3]) +
+                             __popc(b.x & v[4]) + __popc(b.y & v[5]) + __popc(b.z & v[6]) + __popc(b.w & v[7]))
+                       << k;
+            }
+        };
+        for (; w0 + 8 <= m.nbin; w0 += 8) {
+            u32 v[8];
+#pragma unroll
+            for (u32 j = 0; j < 8; j++) v[j] = RES ? c[(w0 + j) * stride] : ld_cg_u32(c + (size_t)(w0 + j) * stride);
+            block(v);
+        }
+        if (w0 < m.nbin) {  // words past the row are 0 on the slot's side
+            u32 v[8];
+#pragma unroll
+            for (u32 j = 0; j < 8; j++)
+                v[j] = w0 + j >= m.nbin ? 0u : (RES ? c[(w0 + j) * stride] : ld_cg_u32(c + (size_t)(w0 + j) * stride));
+            block(v);
+        }
+        return (float)acc;
+    }
+
     template <class F, class D>
     __device__ static void scores(const Args& m, Smem& s, const joinc::Slots& st, u32 nq, F f, D done) {
         const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -175,61 +239,13 @@ struct BitCluster {
         const u32 nwq = 1u << lgq;
         const u32 q = warp >> lgq, wi = warp & (nwq - 1u);
         if (q < nq) {
-            const u32 P = planes(m);
-            const u32* sq = s.sq + (size_t)q * P * m.nbinP;
+            const u32* sq = s.sq + (size_t)q * planes(m) * m.nbinP;
             const bool resident = s.col == s.colS;
             for (u32 x0 = wi * 32; x0 < st.n; x0 += nwq * 32) {
                 const u32 x = x0 + lane, xs = x < st.n ? x : x0;
-                float fa = 0.f;
-                u32 acc = 0;
-                if (PATH == PATH_FLOAT) {
-                    const u32 n = s.len[q];
-                    const uint2* ent = s.ent + (size_t)q * m.nbin * 32;
-                    const u32* c = (resident ? s.colS : s.col) + xs;
-                    auto add = [&](u32 v, uint2 t) {
-                        asm("{\n .reg .pred p;\n .reg .b32 t;\n shf.r.wrap.b32 t, %1, %1, %2;\n and.b32 t, t, 1;\n"
-                            " setp.ne.u32 p, t, 0;\n @p add.rn.f32 %0, %0, %3;\n}"
-                            : "+f"(fa)
-                            : "r"(v), "r"(t.x), "f"(__uint_as_float(t.y)));
-                    };
-                    // only this CTA writes its columns, so plain loads do
-                    u32 e = 0;
-                    for (; e + 7 < n; e += 8) {
-                        uint2 t[8];
-                        u32 v[8];
-#pragma unroll
-                        for (u32 j = 0; j < 8; j++) t[j] = ent[e + j];
-#pragma unroll
-                        for (u32 j = 0; j < 8; j++) v[j] = c[t[j].x >> 5];
-#pragma unroll
-                        for (u32 j = 0; j < 8; j++) add(v[j], t[j]);
-                    }
-                    for (; e < n; e++) add(c[ent[e].x >> 5], ent[e]);
-                } else if (resident) {
-                    const u32* c = s.colS + xs;
-                    if (P == 1) {
-#pragma unroll 8
-                        for (u32 w = 0; w < m.nbin; w++) acc += (u32)__popc(sq[w] & c[w * s.stride]);
-                    } else {
-#pragma unroll 4
-                        for (u32 w = 0; w < m.nbin; w++) {
-                            const u32 v = c[w * s.stride];
-                            for (u32 k = 0; k < P; k++) acc += (u32)__popc(sq[k * m.nbinP + w] & v) << k;
-                        }
-                    }
-                } else {
-                    const u32* c = s.col + xs;
-                    for (u32 w0 = 0; w0 < m.nbin; w0 += 8) {
-                        u32 v[8];
-#pragma unroll
-                        for (u32 j = 0; j < 8; j++) v[j] = w0 + j < m.nbin ? ld_cg_u32(c + (size_t)(w0 + j) * s.stride) : 0u;
-                        for (u32 k = 0; k < P; k++)
-#pragma unroll
-                            for (u32 j = 0; j < 8; j++)
-                                if (w0 + j < m.nbin) acc += (u32)__popc(sq[k * m.nbinP + w0 + j] & v[j]) << k;
-                    }
-                }
-                if (x < st.n) f(q, x, ord_f32(PATH == PATH_FLOAT ? fa : (float)acc));
+                // (two calls, so that resident columns are read as shared memory)
+                const float v = resident ? score<true>(m, s, s.colS + xs, q, sq) : score<false>(m, s, s.col + xs, q, sq);
+                if (x < st.n) f(q, x, ord_f32(v));
             }
             done(q);
         }
