@@ -22,16 +22,14 @@
 //     PLANES path).
 //  2. k_bs_init: the initial all-pairs scan of every replicate, tiles of all
 //     replicates drawn from one queue.
-//  3. k_bs_join: persistent and cooperative; each replicate is joined by a
-//     group of G co-resident CTAs running the same join engine as the single
-//     join (G = 1 needs no barrier beyond the block's own).  G comes from a
-//     cost model of the replicate sizes whose constants are fitted to the
-//     per-replicate times of the previous call on the device (the
-//     autotuner): the largest replicates are split until the longest one no
-//     longer outlasts the even share of the work.  Groups run largest first,
-//     so every multi-CTA group forms in the first wave.  Member 0 then lays
-//     out the replicate tree's post-order (heavier child first, so a walk
-//     needs a stack of at most log2(n)+1).
+//  3. k_bs_join: one thread-block cluster per replicate, largest first, running
+//     the cluster join engine.  The cluster size (one for all replicates) comes
+//     from a cost model whose constants are fitted to the per-replicate times of
+//     the previous call on the device (the autotuner): the size with the least
+//     predicted makespan when the replicates are dealt, largest first, to the
+//     clusters that the device holds at once.  CTA 0 then lays out the replicate
+//     tree's post-order (heavier child first, so a walk needs a stack of at most
+//     log2(n)+1).
 //  4. k_bs_transfer: one thread per (full-tree clade X, replicate).  X is the
 //     pre-order tip interval [lo, hi] of the full tree; walking the replicate
 //     tree's post-order with a stack of |X n Y| counts gives, for every
@@ -46,16 +44,17 @@
 #include <cmath>
 #include <cstring>
 #include <numeric>
+#include <queue>
 #include <vector>
 
-#include "join_bit_model.cuh"
+#include "join_bit_cluster.cuh"
 #include "runtime.h"
 
 namespace casphy {
 namespace boot {
 
 using namespace bitjoin;
-using joinx::kDead;
+using Model = BitCluster<PATH_PLANES>;
 
 constexpr u32 kOpInternal = 0x80000000u, kOpRoot = 0x40000000u;
 constexpr u32 kXThreads = 128;  // clades per transfer block
@@ -63,11 +62,11 @@ constexpr u32 kStack = 32;      // post-order stack (heavier child first: <= log
 constexpr u32 kOpChunk = 2048;  // ops staged in shared memory per step
 
 struct Rep {
-    joinx::Common c;
-    BitModel<PATH_PLANES>::Args m;
+    joinc::Args c;
+    Model::Args m;
     InitArgs init;
     u32 off;        // first tip in the concatenated cell list
-    u32 opsOff;     // first op of this replicate
+    u32* colT;
     u32* ops;       // 2n-1 post-order ops
     u32* eW;
     u32* eQ;
@@ -108,7 +107,7 @@ __global__ void k_bs_prep(const Rep* __restrict__ reps, const u32* __restrict__ 
     const u32 cell = cells[warp];
     prep_tip(rows ? rows + (size_t)warp * nbin : words + (size_t)cell * nbin, tip, nbin, R.m.nbinP,
              (R.c.ntip + 7u) & ~7u, R.m.nplanes,
-             R.m.planeMask, R.m.nodeSeq, R.m.nodeBis, R.m.colT[0], R.eW, R.eQ, R.eLen, R.eStride);
+             R.m.planeMask, R.m.nodeSeq, R.m.nodeBis, R.colT, R.eW, R.eQ, R.eLen, R.eStride);
     // initial local maximum: value -1, node ~0 (replaced by the initial scan)
     if ((threadIdx.x & 31) == 0) R.init.initKey[tip] = ((u64)ORD_F32_NEG1 << 32) | 0xFFFFFFFFull;
 }
@@ -138,96 +137,77 @@ __global__ void __launch_bounds__(kThreads) k_bs_init(const Rep* __restrict__ re
     }
 }
 
-// engine slot/node arrays of every replicate: grid (blocks, nrep)
-__global__ void k_bs_slot_init(const Rep* __restrict__ reps) {
-    const Rep& R = reps[blockIdx.y];
-    const joinx::Common& c = R.c;
-    const u32 ntip = c.ntip, Sp = (ntip + 7u) & ~7u, nnode = c.nnode;
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < max(Sp, nnode); i += gridDim.x * blockDim.x) {
-        if (i < Sp) {
-            if (i < ntip) {
-                const u64 k = R.init.initKey[i];
-                c.lmOrd[0][i] = key_ord(k);
-                c.lmIdx[0][i] = key_node(k);
-                c.slotNode[0][i] = i;
-            } else {
-                c.lmOrd[0][i] = c.ordNeg1;
-                c.lmIdx[0][i] = 0;
-                c.slotNode[0][i] = kDead;
-            }
-        }
-        if (i < 16u * c.nCTA) c.flags[i] = 0u;  // barrier epochs of the replicate's group
-        if (i < nnode) {
-            c.node2slot[i] = i < ntip ? i : joinx::kNone;
-            c.nodeDeath[i] = joinx::kNone;
-            c.nodeSize[i] = i < ntip ? 1u : 0u;
-        }
-    }
-}
-
 // Post-order of the replicate tree (raw join edges: node ntip+k has children
 // rawEdge[4k+1], rawEdge[4k+3]; the root is 2ntip-2), heavier child first.
 // Tip ops carry the tip's full-tree pre-order rank; internal ops carry their
-// tip count, the root is flagged.  One thread; offsets in shared memory.
-__device__ void build_ops(const joinx::Common& c, const u32* __restrict__ rankOf, u32* ops, u32* s) {
-    if (threadIdx.x != 0) return;
-    const u32 n = c.ntip;
-    if (n == 1) {
-        ops[0] = rankOf[0];
-        return;
-    }
-    const u32 root = 2 * n - 2;
-    s[root - n] = 0;
-    for (u32 v = root + 1; v-- > n;) {
-        const u32 k = v - n;
-        const u32 base = s[k];
-        const u32 tv = c.nodeSize[v];
-        ops[base + 2 * tv - 2] = kOpInternal | (v == root ? kOpRoot : 0u) | tv;
-        u32 a = c.rawEdge[4 * k + 1], b = c.rawEdge[4 * k + 3];
-        u32 ta = c.nodeSize[a], tb = c.nodeSize[b];
-        if (tb > ta) {
-            const u32 x = a; a = b; b = x;
-            const u32 y = ta; ta = tb; tb = y;
+// tip count, the root is flagged.  Offsets go from parents to children, so one
+// thread walks the nodes from the root down; what it reads of them is staged
+// by the whole block, kOpsStage nodes at a time (read by the walking thread
+// itself, two dependent loads a node, it took about 1 us a node).
+constexpr u32 kOpsStage = 512;
+struct OpsNode {
+    u32 a, b, ta, tb, ra, rb;  // children, their tips and, for tips, their ranks
+};
+__host__ __device__ inline size_t ops_smem(u32 n) { return sizeof(OpsNode) * kOpsStage + sizeof(u32) * (size_t)n; }
+__device__ void build_ops(const joinc::Args& c, const u32* __restrict__ rankOf, u32* ops, unsigned char* smem) {
+    OpsNode* stage = reinterpret_cast<OpsNode*>(smem);
+    u32* s = reinterpret_cast<u32*>(stage + kOpsStage);
+    const u32 n = c.ntip, root = 2 * n - 2;
+    if (threadIdx.x == 0) s[root - n] = 0;
+    for (u32 top = n - 1; top > 0;) {  // nodes n + top - 1 down
+        const u32 m = min(kOpsStage, top);
+        __syncthreads();
+        for (u32 i = threadIdx.x; i < m; i += joinc::kThreads) {
+            const u32 k = top - 1 - i;
+            OpsNode o;
+            o.a = ld_cg_u32(c.rawEdge + 4 * k + 1);
+            o.b = ld_cg_u32(c.rawEdge + 4 * k + 3);
+            o.ta = o.a < n ? 1u : ld_cg_u32(c.nodeSize + o.a);
+            o.tb = o.b < n ? 1u : ld_cg_u32(c.nodeSize + o.b);
+            if (o.tb > o.ta) {
+                const u32 x = o.a; o.a = o.b; o.b = x;
+                const u32 y = o.ta; o.ta = o.tb; o.tb = y;
+            }
+            o.ra = o.a < n ? rankOf[o.a] : 0u;
+            o.rb = o.b < n ? rankOf[o.b] : 0u;
+            stage[i] = o;
         }
-        const u32 sb = base + 2 * ta - 1;
-        if (a < n) ops[base] = rankOf[a];
-        else s[a - n] = base;
-        if (b < n) ops[sb] = rankOf[b];
-        else s[b - n] = sb;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (u32 i = 0; i < m; i++) {
+                const u32 k = top - 1 - i, tv = stage[i].ta + stage[i].tb;
+                const OpsNode o = stage[i];
+                const u32 base = s[k], sb = base + 2 * o.ta - 1;
+                ops[base + 2 * tv - 2] = kOpInternal | (n + k == root ? kOpRoot : 0u) | tv;
+                if (o.a < n) ops[base] = o.ra;
+                else s[o.a - n] = base;
+                if (o.b < n) ops[sb] = o.rb;
+                else s[o.b - n] = sb;
+            }
+        top -= m;
     }
 }
 
-// Work items (replicate, member) in queue order; the members of one
-// replicate are consecutive and multi-CTA replicates come first.
-template <int PATH>
-__global__ void __launch_bounds__(kThreads, 1) k_bs_join(const Rep* __restrict__ reps,
-                                                         const u32* __restrict__ itemRep,
-                                                         const u32* __restrict__ itemMember, u32 nItem,
-                                                         unsigned int* counter, const u32* __restrict__ rankOf) {
+// Cluster i joins replicate order[i].
+__global__ void __launch_bounds__(joinc::kThreads, 1) k_bs_join(const Rep* __restrict__ reps,
+                                                                const u32* __restrict__ order, u32 G,
+                                                                const u32* __restrict__ rankOf) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ u32 s_idx;
-    for (;;) {
-        if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1u);
-        __syncthreads();
-        const u32 idx = s_idx;
-        __syncthreads();
-        if (idx >= nItem) break;
-        const u32 r = itemRep[idx], b = itemMember[idx];
-        const joinx::Common c = reps[r].c;
-        const typename BitModel<PATH>::Args m = reps[r].m;
-        const u64 t0 = globaltimer_ns();
-        if (c.ntip >= 2) joinx::join_run<BitModel<PATH>>(c, m, b, smem);
-        __syncthreads();
-        if (b != 0) continue;
-        int err = 0;
-        if (threadIdx.x == 0) err = *(volatile int*)c.err;
-        if (__syncthreads_or(err)) continue;
-        build_ops(c, rankOf + reps[r].off, reps[r].ops, reinterpret_cast<u32*>(smem));
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            c.statsOut[6] = t0;
-            c.statsOut[7] = globaltimer_ns();
-        }
+    const u32 r = order[blockIdx.x / G], rank = joinc::cluster_rank();
+    const joinc::Args c = reps[r].c;
+    const Model::Args m = reps[r].m;
+    const u64 t0 = globaltimer_ns();
+    joinc::cluster_join<Model>(c, m, rank, smem);
+    __syncthreads();
+    if (rank != 0) return;
+    int err = 0;
+    if (threadIdx.x == 0) err = *(volatile int*)c.err;
+    if (__syncthreads_or(err)) return;
+    build_ops(c, rankOf + reps[r].off, reps[r].ops, smem);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        c.statsOut[6] = t0;
+        c.statsOut[7] = globaltimer_ns();
     }
 }
 
@@ -375,79 +355,51 @@ static int full_tree_intervals(u32 ntip, const u32* edge, std::vector<u32>& Xlo,
 namespace casphy {
 namespace boot {
 
-// Cost of joining one replicate of n cells with G CTAs: its phases times
-// (alpha + beta * n / G + gamma when G > 1) -- a fixed per-phase part, the
-// scan of the slots each CTA owns, and the cross-CTA barrier.  The constants
-// start from a B200 estimate and are refitted on every call from the
-// measured replicate times, per device.
+// Cost of joining one replicate of n cells with a cluster of G CTAs: its
+// phases times (alpha + beta * n / G + gamma when G > 1) -- a fixed per-phase
+// part, the scan of the slots each CTA owns, and the exchange between CTAs.
+// The constants start from a B200 estimate and are refitted on every call from
+// the measured replicate times, per device.
 struct Tune {
     int measured = 0;
-    double alpha = 6.0;        // us per phase
-    double beta = 1.8e-3;      // us per phase per slot of a CTA
-    double gamma = 2.0;        // us per phase for the barrier of a group
-    double phasesPerTip = 1.7;
+    double alpha = 2.2;        // us per phase
+    double beta = 1.0e-3;      // us per phase per slot of a CTA
+    double gamma = 0.6;        // us per phase for the exchange of a cluster
+    double phasesPerTip = 1.5;
 };
 constexpr int kMaxDev = 64;
-constexpr u32 kMaxGroup = 8;
 Tune g_tune[kMaxDev];  // read and written under the device's workspace lock
 
 inline double cost_us(const Tune& T, u32 n, u32 G) {
     return T.phasesPerTip * n * (T.alpha + T.beta * (double)n / G + (G > 1 ? T.gamma : 0.0));
 }
 
-// CTAs per replicate: split the replicate with the longest predicted join
-// while it outlasts the even share of all work over `slots` CTAs and a split
-// still shortens it.
-std::vector<u32> split_groups(const Tune& T, const std::vector<u32>& repN, u32 slots) {
-    const u32 nrep = (u32)repN.size();
-    std::vector<u32> G(nrep, 1);
-    // CASPHY_BS_GROUP=g fixes g CTAs for every replicate of 512 cells or
-    // more while they fit the SMs (the cost model is bypassed)
-    if (const char* env = std::getenv("CASPHY_BS_GROUP")) {
-        const u32 g = std::min<u32>((u32)std::max(1, std::atoi(env)), kMaxGroup);
-        u32 used = 0;
-        for (u32 r = 0; r < nrep; r++)
-            if (g > 1 && repN[r] >= 512 && used + g <= slots) {
-                G[r] = g;
-                used += g;
-            }
-        return G;
+// Predicted time of all replicates, `sorted` by falling size, on `slots`
+// clusters of G CTAs, each taking the next replicate when it is free.
+inline double makespan_us(const Tune& T, const std::vector<u32>& sorted, u32 G, u32 slots) {
+    std::priority_queue<double, std::vector<double>, std::greater<double>> freeAt;
+    for (u32 i = 0; i < slots; i++) freeAt.push(0.0);
+    double end = 0;
+    for (u32 n : sorted) {
+        const double t = freeAt.top() + cost_us(T, n, G);
+        freeAt.pop();
+        freeAt.push(t);
+        end = std::max(end, t);
     }
-    std::vector<double> t(nrep);
-    double W = 0;
-    for (u32 r = 0; r < nrep; r++) {
-        t[r] = cost_us(T, repN[r], 1);
-        W += t[r];
-    }
-    u32 inGroups = 0;
-    for (;;) {
-        u32 rm = 0;
-        for (u32 r = 1; r < nrep; r++)
-            if (t[r] > t[rm]) rm = r;
-        if (t[rm] <= W / slots || G[rm] >= kMaxGroup || repN[rm] < 512) break;
-        const u32 g = G[rm] + 1, extra = G[rm] == 1 ? 2 : 1;
-        const double tn = cost_us(T, repN[rm], g);
-        if (tn >= t[rm] || inGroups + extra > slots) break;
-        W += tn * g - t[rm] * G[rm];
-        inGroups += extra;
-        G[rm] = g;
-        t[rm] = tn;
-    }
-    return G;
+    return end;
 }
 
-// Refit alpha and beta on the single-CTA replicates and gamma on the
-// groups, by least squares of the per-phase time; keeps the previous value
-// of a constant the measurements cannot pin down.
-void refit(Tune& T, const std::vector<u32>& repN, const std::vector<u32>& G, const std::vector<double>& us,
+// Refits alpha and beta (single CTAs) or gamma and beta (clusters) by least
+// squares of the per-phase time over the slots per CTA; keeps the previous
+// value of a constant the measurements cannot pin down.
+void refit(Tune& T, const std::vector<u32>& repN, u32 G, const std::vector<double>& us,
            const std::vector<unsigned long long>& phases) {
     double s1 = 0, sx = 0, sxx = 0, sy = 0, sxy = 0, ptot = 0, ntot = 0;
     for (size_t r = 0; r < repN.size(); r++) {
         if (phases[r] == 0 || us[r] <= 0) continue;
         ptot += (double)phases[r];
         ntot += repN[r];
-        if (G[r] != 1) continue;
-        const double x = repN[r], y = us[r] / (double)phases[r];
+        const double x = (double)repN[r] / G, y = us[r] / (double)phases[r];
         s1 += 1;
         sx += x;
         sxx += x * x;
@@ -459,18 +411,12 @@ void refit(Tune& T, const std::vector<u32>& repN, const std::vector<u32>& G, con
     if (s1 >= 8 && det > 0) {
         const double b = (s1 * sxy - sx * sy) / det, a = (sy - b * sx) / s1;
         if (a > 0 && b > 0) {
-            T.alpha = a;
+            if (G == 1) T.alpha = a;
+            else T.gamma = std::max(0.1, a - T.alpha);
             T.beta = b;
             T.measured = 1;
         }
     }
-    double gs = 0, gn = 0;
-    for (size_t r = 0; r < repN.size(); r++) {
-        if (G[r] == 1 || phases[r] == 0 || us[r] <= 0) continue;
-        gs += us[r] / (double)phases[r] - T.alpha - T.beta * repN[r] / G[r];
-        gn += 1;
-    }
-    if (gn > 0) T.gamma = std::max(0.1, gs / gn);
 }
 
 }  // namespace boot
@@ -558,22 +504,59 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     DeviceScope ds;
     int nSM = 0;
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, ds.dev));
-    // CTAs per replicate from the device's cost model (one join CTA per SM)
+    // CTAs per replicate from the device's cost model (one join CTA per SM):
+    // every size whose shared memory fits the largest replicate
     boot::Tune& tune = boot::g_tune[(ds.dev >= 0 && ds.dev < boot::kMaxDev) ? ds.dev : 0];
     const int tunedBefore = tune.measured;
-    std::vector<u32> Gs = boot::split_groups(tune, repN, (u32)nSM);
-    u32 nItemAll = 0;
-    for (u32 g : Gs) nItemAll += g;
+    int maxSmem = 0;
+    CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ds.dev));
+    const size_t smemLim = (size_t)maxSmem - 6144;  // the kernel's static shared memory
+    auto plan = [&](u32 n, u32 G, joinc::Args& a, Model::Args& m, size_t* smem) {
+        a.ntip = n;
+        a.nnode = 2 * n - 1;
+        a.G = G;
+        a.R = ((n + G - 1) / G + 31u) & ~31u;
+        a.deathWords = (a.nnode + 31) / 32;
+        m.nbin = nbin;
+        m.nbinP = nbinP;
+        m.nplanes = nplanes;
+        return a.R < 0xFFFFu && cluster_fit<PATH_PLANES>(a, m, smemLim, smem);
+    };
+    std::vector<u32> order(nrep), sorted(nrep);
+    std::iota(order.begin(), order.end(), 0u);
+    std::stable_sort(order.begin(), order.end(), [&](u32 a, u32 b) { return repN[a] > repN[b]; });
+    for (u32 r = 0; r < nrep; r++) sorted[r] = repN[order[r]];
+    u32 G = 0, fixedG = 0;
+    if (const char* env = std::getenv("CASPHY_BS_GROUP"))  // a fixed size, at most 8 (the cost model is bypassed)
+        for (fixedG = 1; fixedG < 8 && (int)(2 * fixedG) <= std::atoi(env);) fixedG *= 2;
+    double bestUs = 0;
+    for (u32 g = 1; g <= joinc::kMaxG; g *= 2) {
+        joinc::Args a{};
+        Model::Args m{};
+        size_t sm = 0;
+        if (!plan(nmax, g, a, m, &sm)) continue;
+        sm = std::max(sm, ops_smem(nmax));
+        if (sm > smemLim) continue;
+        const int slots = joinc::placeable((void*)k_bs_join, g, sm);
+        if (slots < 1) continue;
+        const double t = g == fixedG ? 0.0 : makespan_us(tune, sorted, g, (u32)slots);
+        if (G == 0 || t < bestUs) {
+            G = g;
+            bestUs = t;
+        }
+    }
+    if (G == 0) {
+        casphy_set_last_error_msg("bootstrap: replicate too large for one cluster's shared memory");
+        return CASPHY_ERANGE;
+    }
     struct RepBufs {
-        u32 *planeMask, *nodeSeq, *nodeBis, *colT0, *colT1, *lm[6], *node2slot, *nodeDeath, *nodeSize, *rawEdge;
-        u32 *eW, *eQ, *eLen, *pubCnt, *counts, *flags;
+        u32 *planeMask, *nodeSeq, *nodeBis, *colT0, *colT1, *nodeSize, *rawEdge;
+        u32 *eW, *eQ, *eLen;
         unsigned long long* initKey;
-        joinx::BlockRec* pub;
-        u64* partial;
         u64* chunkStart;
         unsigned long long* stats;
     };
-    auto rep_layout = [&](Carve& c, u32 n, u32 G) {
+    auto rep_layout = [&](Carve& c, u32 n) {
         RepBufs b;
         const u32 Sp = (n + 7u) & ~7u, nnode = 2 * n - 1, nChunks = (n + kCap - 1) / kCap;
         b.planeMask = c.take<u32>((size_t)P * nbin);
@@ -581,31 +564,22 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         b.nodeBis = c.take<u32>((size_t)nnode * nbinP);
         b.colT0 = c.take<u32>((size_t)nbin * Sp);
         b.colT1 = c.take<u32>((size_t)nbin * Sp);
-        for (int i = 0; i < 6; i++) b.lm[i] = c.take<u32>(Sp);
-        b.node2slot = c.take<u32>(nnode);
-        b.nodeDeath = c.take<u32>(nnode);
         b.nodeSize = c.take<u32>(nnode);
         b.rawEdge = c.take<u32>((size_t)4 * n);
         b.eW = c.take<u32>((size_t)n * eStride);
         b.eQ = c.take<u32>((size_t)n * eStride);
         b.eLen = c.take<u32>(n);
         b.initKey = c.take<unsigned long long>(n);
-        b.pub = c.take<joinx::BlockRec>(4 * G);
-        b.pubCnt = c.take<u32>(2 * G);
-        b.partial = c.take<u64>((size_t)2 * G * joinx::kMaxBatch);
-        b.counts = c.take<u32>(G);
-        b.flags = c.take<u32>(16 * G);
         b.chunkStart = c.take<u64>(nChunks + 1);
         b.stats = c.take<unsigned long long>(8);
         return b;
     };
     struct Glob {
         Rep* reps;
-        u32 *repOfWarp, *cells, *words, *itemRep, *itemMember, *rankOf, *sortedRank, *ops, *Xlo, *Xhi, *repN, *repOff, *repOpsOff;
+        u32 *repOfWarp, *cells, *words, *order, *rankOf, *sortedRank, *ops, *Xlo, *Xhi, *repN, *repOff, *repOpsOff;
         u32 *ymin, *ysize, *support;
         u64* tileStart;
         unsigned long long* counter;
-        unsigned int* jcounter;
         int* errs;
         int* xerr;
         u32* colIdx;
@@ -617,8 +591,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         g.repOfWarp = c.take<u32>(totalTips);
         g.cells = c.take<u32>(totalTips);
         g.words = c.take<u32>((size_t)ntip * nbin);
-        g.itemRep = c.take<u32>(nItemAll);
-        g.itemMember = c.take<u32>(nItemAll);
+        g.order = c.take<u32>(nrep);
         g.rankOf = c.take<u32>(totalTips);
         g.sortedRank = c.take<u32>(totalTips);
         g.ops = c.take<u32>(repOpsOff[nrep]);
@@ -632,7 +605,6 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         g.support = c.take<u32>(nX);
         g.tileStart = c.take<u64>(nrep + 1);
         g.counter = c.take<unsigned long long>(1);
-        g.jcounter = c.take<unsigned int>(1);
         g.errs = c.take<int>(nrep);
         g.xerr = c.take<int>(1);
         g.colIdx = c.take<u32>(repeat ? (size_t)nrep * nsite : 1);
@@ -641,18 +613,19 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     };
     Carve cv;
     glob_layout(cv);
-    for (u32 r = 0; r < nrep; r++) rep_layout(cv, repN[r], Gs[r]);
+    for (u32 r = 0; r < nrep; r++) rep_layout(cv, repN[r]);
     void* base = nullptr;
     if ((rc = ds.reserve(cv.off + 256, &base))) return rc;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    const Glob G = glob_layout(c2);
+    const Glob gl = glob_layout(c2);
     std::vector<Rep> reps(nrep);
     std::vector<RepBufs> rb(nrep);
     std::vector<u64> tileStart(nrep + 1, 0), chunkAll;
     std::vector<std::vector<u64>> chunkStarts(nrep);
+    size_t smem = ops_smem(nmax);
     for (u32 r = 0; r < nrep; r++) {
-        rb[r] = rep_layout(c2, repN[r], Gs[r]);
+        rb[r] = rep_layout(c2, repN[r]);
         const u32 n = repN[r], Sp = (n + 7u) & ~7u, nChunks = (n + kCap - 1) / kCap;
         auto& cs = chunkStarts[r];
         cs.assign(nChunks + 1, 0);
@@ -663,30 +636,30 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         tileStart[r + 1] = tileStart[r] + cs[nChunks];
         Rep& R = reps[r];
         std::memset(&R, 0, sizeof(Rep));
-        joinx::Common& c = R.c;
         const RepBufs& b = rb[r];
-        c.ntip = n; c.nnode = 2 * n - 1; c.nCTA = Gs[r]; c.align = 8;
-        c.lmOrd[0] = b.lm[0]; c.lmIdx[0] = b.lm[1]; c.slotNode[0] = b.lm[2];
-        c.lmOrd[1] = b.lm[3]; c.lmIdx[1] = b.lm[4]; c.slotNode[1] = b.lm[5];
-        c.node2slot = b.node2slot; c.nodeDeath = b.nodeDeath; c.nodeSize = b.nodeSize; c.rawEdge = b.rawEdge;
-        c.pub = b.pub; c.pubCnt = b.pubCnt; c.partial = b.partial; c.counts = b.counts; c.flags = b.flags;
-        c.err = G.errs + r; c.limitNs = 20ull * 1000 * 1000 * 1000; c.statsOut = b.stats;
-        c.Rmax = ((n + Gs[r] - 1) / Gs[r] + 7u) & ~7u; c.ordNeg1 = ORD_F32_NEG1; c.compactMin = 4096; c.compactQ8 = 192; c.bytesPerPairSite = 4000;
-        c.prof = nullptr;
-        c.maxBatch = joinx::stale_batch_setting();
-        c.deathWords = (2 * n - 1 + 31) / 32;  // joined-node bitmap: 2.5 KB at 10,000 cells
-        c.keepSizes = 1;                         // build_ops lays out clades by node size
-        R.m = BitModel<PATH_PLANES>::Args{nbin, nbinP, nplanes, ancestralType ? 1 : 0, b.planeMask, nullptr,
-                                          b.nodeSeq, b.nodeBis, {b.colT0, b.colT1}};
+        joinc::Args& c = R.c;
+        size_t sm = 0;
+        if (!plan(n, G, c, R.m, &sm)) return CASPHY_EINTERNAL;  // no larger than the largest, which fits
+        smem = std::max(smem, sm);
+        c.initKey = b.initKey;
+        c.nodeSize = b.nodeSize; c.rawEdge = b.rawEdge; c.err = gl.errs + r;
+        c.limitNs = 20ull * 1000 * 1000 * 1000; c.statsOut = b.stats;
+        c.ordNeg1 = ORD_F32_NEG1; c.compactMin = 256; c.bytesPerPairSite = 4000;
+        c.keepSizes = 1;  // build_ops lays out clades by node size
+        R.m.ancType = ancestralType ? 1 : 0;
+        R.m.planeMask = b.planeMask;
+        R.m.nodeSeq = b.nodeSeq; R.m.nodeBis = b.nodeBis;
+        R.m.colT[0] = b.colT0; R.m.colT[1] = b.colT1;
+        R.m.Sp = Sp;
+        R.colT = b.colT0;
         R.init = InitArgs{n, nbin, Sp, eStride, b.colT0, b.eW, b.eQ, b.eLen, nullptr, b.chunkStart, nChunks,
                           cs[nChunks], nullptr, b.initKey};
         R.off = rep_offsets[r];
-        R.opsOff = repOpsOff[r];
-        R.ops = G.ops + repOpsOff[r];
+        R.ops = gl.ops + repOpsOff[r];
         R.eW = b.eW; R.eQ = b.eQ; R.eLen = b.eLen; R.eStride = eStride;
     }
     // host tables: replicate of each tip, ranks, sorted ranks, largest-first order
-    std::vector<u32> repOfWarp(totalTips), rankOf(totalTips), sortedRank(totalTips), order(nrep), repOff(nrep);
+    std::vector<u32> repOfWarp(totalTips), rankOf(totalTips), sortedRank(totalTips), repOff(nrep);
     for (u32 r = 0; r < nrep; r++) {
         repOff[r] = rep_offsets[r];
         for (u32 i = rep_offsets[r]; i < rep_offsets[r + 1]; i++) {
@@ -701,42 +674,6 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
                 return CASPHY_EINVAL;
             }
     }
-    // join items: groups first, then the largest replicates first
-    std::iota(order.begin(), order.end(), 0u);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](u32 a, u32 b) { return Gs[a] != Gs[b] ? Gs[a] > Gs[b] : repN[a] > repN[b]; });
-    std::vector<u32> itemRep, itemMember;
-    u32 maxG = 1, inGroups = 0;
-    for (u32 r : order) {
-        for (u32 b = 0; b < Gs[r]; b++) {
-            itemRep.push_back(r);
-            itemMember.push_back(b);
-        }
-        maxG = std::max(maxG, Gs[r]);
-        if (Gs[r] > 1) inGroups += Gs[r];
-    }
-    const u32 nItem = (u32)itemRep.size();
-    // shared memory of a join CTA: engine + model, or the post-order offsets
-    using M = BitModel<PATH_PLANES>;
-    int maxSmem = 0;
-    CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ds.dev));
-    auto joinSmem = [&] {
-        size_t m = 0;
-        for (u32 r = 0; r < nrep; r++)
-            m = std::max(m, M::engine_smem_bytes(Gs[r], reps[r].c.Rmax, reps[r].c.deathWords) +
-                                M::model_smem_bytes(reps[r].m));
-        return m;
-    };
-    size_t smemJoin = joinSmem();
-    if (smemJoin + 1024 > (size_t)maxSmem) {  // without the joined-node bitmaps (node deaths from global memory)
-        for (u32 r = 0; r < nrep; r++) reps[r].c.deathWords = 0;
-        smemJoin = joinSmem();
-    }
-    const size_t smem = std::max(smemJoin, (size_t)4 * nmax);
-    if (smem + 1024 > (size_t)maxSmem) {
-        casphy_set_last_error_msg("bootstrap: replicate too large for one CTA's shared memory");
-        return CASPHY_ERANGE;
-    }
     cudaStream_t st = 0;
     cudaEvent_t ev[4];
     for (auto& e : ev) CASPHY_CUDA_TRY(cudaEventCreate(&e));
@@ -748,61 +685,45 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         CASPHY_CUDA_TRY(up(b.planeMask, planes.data() + (size_t)r * P * nbin, sizeof(u32) * P * nbin));
         CASPHY_CUDA_TRY(up(b.chunkStart, chunkStarts[r].data(), sizeof(u64) * (nChunks + 1)));
     }
-    CASPHY_CUDA_TRY(up(G.reps, reps.data(), sizeof(Rep) * nrep));
-    CASPHY_CUDA_TRY(up(G.repOfWarp, repOfWarp.data(), 4ull * totalTips));
-    CASPHY_CUDA_TRY(up(G.cells, rep_cells, 4ull * totalTips));
-    CASPHY_CUDA_TRY(up(G.words, words, 4ull * ntip * nbin));
-    CASPHY_CUDA_TRY(up(G.itemRep, itemRep.data(), 4ull * nItem));
-    CASPHY_CUDA_TRY(up(G.itemMember, itemMember.data(), 4ull * nItem));
-    CASPHY_CUDA_TRY(up(G.rankOf, rankOf.data(), 4ull * totalTips));
-    CASPHY_CUDA_TRY(up(G.sortedRank, sortedRank.data(), 4ull * totalTips));
-    CASPHY_CUDA_TRY(up(G.Xlo, Xlo.data(), 4ull * nX));
-    CASPHY_CUDA_TRY(up(G.Xhi, Xhi.data(), 4ull * nX));
-    CASPHY_CUDA_TRY(up(G.repN, repN.data(), 4ull * nrep));
-    CASPHY_CUDA_TRY(up(G.repOff, repOff.data(), 4ull * nrep));
-    CASPHY_CUDA_TRY(up(G.repOpsOff, repOpsOff.data(), 4ull * nrep));
-    CASPHY_CUDA_TRY(up(G.tileStart, tileStart.data(), 8ull * (nrep + 1)));
-    CASPHY_CUDA_TRY(cudaMemsetAsync(G.support, 0, 4ull * nX, st));
-    CASPHY_CUDA_TRY(cudaMemsetAsync(G.counter, 0, sizeof(unsigned long long), st));
-    CASPHY_CUDA_TRY(cudaMemsetAsync(G.jcounter, 0, sizeof(unsigned int), st));
-    CASPHY_CUDA_TRY(cudaMemsetAsync(G.errs, 0, sizeof(int) * nrep, st));
-    CASPHY_CUDA_TRY(cudaMemsetAsync(G.xerr, 0, sizeof(int), st));
-    if (repeat) CASPHY_CUDA_TRY(up(G.colIdx, colIdx.data(), 4ull * nrep * nsite));
+    CASPHY_CUDA_TRY(up(gl.reps, reps.data(), sizeof(Rep) * nrep));
+    CASPHY_CUDA_TRY(up(gl.repOfWarp, repOfWarp.data(), 4ull * totalTips));
+    CASPHY_CUDA_TRY(up(gl.cells, rep_cells, 4ull * totalTips));
+    CASPHY_CUDA_TRY(up(gl.words, words, 4ull * ntip * nbin));
+    CASPHY_CUDA_TRY(up(gl.order, order.data(), 4ull * nrep));
+    CASPHY_CUDA_TRY(up(gl.rankOf, rankOf.data(), 4ull * totalTips));
+    CASPHY_CUDA_TRY(up(gl.sortedRank, sortedRank.data(), 4ull * totalTips));
+    CASPHY_CUDA_TRY(up(gl.Xlo, Xlo.data(), 4ull * nX));
+    CASPHY_CUDA_TRY(up(gl.Xhi, Xhi.data(), 4ull * nX));
+    CASPHY_CUDA_TRY(up(gl.repN, repN.data(), 4ull * nrep));
+    CASPHY_CUDA_TRY(up(gl.repOff, repOff.data(), 4ull * nrep));
+    CASPHY_CUDA_TRY(up(gl.repOpsOff, repOpsOff.data(), 4ull * nrep));
+    CASPHY_CUDA_TRY(up(gl.tileStart, tileStart.data(), 8ull * (nrep + 1)));
+    CASPHY_CUDA_TRY(cudaMemsetAsync(gl.support, 0, 4ull * nX, st));
+    CASPHY_CUDA_TRY(cudaMemsetAsync(gl.counter, 0, sizeof(unsigned long long), st));
+    CASPHY_CUDA_TRY(cudaMemsetAsync(gl.errs, 0, sizeof(int) * nrep, st));
+    CASPHY_CUDA_TRY(cudaMemsetAsync(gl.xerr, 0, sizeof(int), st));
+    if (repeat) CASPHY_CUDA_TRY(up(gl.colIdx, colIdx.data(), 4ull * nrep * nsite));
     int perSM = 0;
     CASPHY_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_bs_init, kThreads, 0));
-    void* joinFn = (void*)k_bs_join<PATH_PLANES>;
-    CASPHY_CUDA_TRY(cudaFuncSetAttribute(joinFn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per = 0;
-    CASPHY_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, joinFn, kThreads, smem));
-    if (per < 1) return CASPHY_ERANGE;
-    const u32 joinGrid = std::min<u32>(nItem, (u32)(nSM * per));
-    if (inGroups > joinGrid) return CASPHY_EINTERNAL;  // a group could not form
-    const Rep* a0 = G.reps;
-    const u32* a1 = G.itemRep;
-    const u32* a2 = G.itemMember;
-    u32 a3 = nItem;
-    unsigned int* a4 = G.jcounter;
-    const u32* a5 = G.rankOf;
-    void* joinArgs[] = {(void*)&a0, (void*)&a1, (void*)&a2, (void*)&a3, (void*)&a4, (void*)&a5};
-    XferArgs xa{nX, nrep, 32u * ((ntip + 31) / 32), G.Xlo, G.Xhi, G.repN, G.repOff, G.repOpsOff, G.sortedRank, G.ops,
-                threshold, G.ymin, G.ysize, G.support, G.xerr};
-    // the whole pass: prep, initial scans, the persistent cooperative join
-    // (every CTA resident, so each group's members run together), transfer
-    const u64 launches = (repeat ? 1 : 0) + 5;
+    // (the planned size may have shrunk to what the replicates need)
+    if (joinc::placeable((void*)k_bs_join, G, smem) < 1) return CASPHY_EINTERNAL;
+    XferArgs xa{nX, nrep, 32u * ((ntip + 31) / 32), gl.Xlo, gl.Xhi, gl.repN, gl.repOff, gl.repOpsOff, gl.sortedRank, gl.ops,
+                threshold, gl.ymin, gl.ysize, gl.support, gl.xerr};
+    // the whole pass: prep, initial scans, the joins, transfer
+    const u64 launches = (repeat ? 1 : 0) + 4;
     auto enqueue = [&](cudaStream_t s) -> cudaError_t {
         cudaError_t e;
         if ((e = cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal)) != cudaSuccess) return e;
         if (repeat)
-            k_bs_gather<<<(totalTips + 7) / 8, 256, 0, s>>>(G.repOfWarp, G.cells, G.words, G.colIdx, nbin, totalTips,
-                                                          G.rrows);
-        k_bs_prep<<<(totalTips + 7) / 8, 256, 0, s>>>(G.reps, G.repOfWarp, G.cells, G.words,
-                                                      repeat ? G.rrows : nullptr, nbin, totalTips);
-        k_bs_init<<<nSM * std::max(perSM, 1), kThreads, 0, s>>>(G.reps, G.tileStart, nrep, G.counter);
-        k_bs_slot_init<<<dim3((2 * nmax + 255) / 256, nrep), 256, 0, s>>>(G.reps);
+            k_bs_gather<<<(totalTips + 7) / 8, 256, 0, s>>>(gl.repOfWarp, gl.cells, gl.words, gl.colIdx, nbin, totalTips,
+                                                          gl.rrows);
+        k_bs_prep<<<(totalTips + 7) / 8, 256, 0, s>>>(gl.reps, gl.repOfWarp, gl.cells, gl.words,
+                                                      repeat ? gl.rrows : nullptr, nbin, totalTips);
+        k_bs_init<<<nSM * std::max(perSM, 1), kThreads, 0, s>>>(gl.reps, gl.tileStart, nrep, gl.counter);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal)) != cudaSuccess) return e;
-        if ((e = cudaLaunchCooperativeKernel(joinFn, dim3(joinGrid), dim3(kThreads), joinArgs, smem, s)) !=
-            cudaSuccess)
+        if ((e = joinc::enqueue(k_bs_join, G, nrep, smem, s, (const Rep*)gl.reps, (const u32*)gl.order, G,
+                                (const u32*)gl.rankOf)) != cudaSuccess)
             return e;
         if ((e = cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal)) != cudaSuccess) return e;
         k_bs_transfer<<<dim3((nX + kXThreads - 1) / kXThreads, nrep), kXThreads, 0, s>>>(xa);
@@ -831,11 +752,11 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     if (!graphed) CASPHY_CUDA_TRY(enqueue(st));
     std::vector<int> errs(nrep);
     int xerr = 0;
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(errs.data(), G.errs, sizeof(int) * nrep, cudaMemcpyDeviceToHost, st));
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(&xerr, G.xerr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(support, G.support, 4ull * nX, cudaMemcpyDeviceToHost, st));
-    if (ymin_out) CASPHY_CUDA_TRY(cudaMemcpyAsync(ymin_out, G.ymin, 4ull * nrep * nX, cudaMemcpyDeviceToHost, st));
-    if (ysize_out) CASPHY_CUDA_TRY(cudaMemcpyAsync(ysize_out, G.ysize, 4ull * nrep * nX, cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(errs.data(), gl.errs, sizeof(int) * nrep, cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(&xerr, gl.xerr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(support, gl.support, 4ull * nX, cudaMemcpyDeviceToHost, st));
+    if (ymin_out) CASPHY_CUDA_TRY(cudaMemcpyAsync(ymin_out, gl.ymin, 4ull * nrep * nX, cudaMemcpyDeviceToHost, st));
+    if (ysize_out) CASPHY_CUDA_TRY(cudaMemcpyAsync(ysize_out, gl.ysize, 4ull * nrep * nX, cudaMemcpyDeviceToHost, st));
     if (rep_raw_edges) {
         size_t o = 0;
         for (u32 r = 0; r < nrep; r++) {
@@ -859,7 +780,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         const unsigned long long t0 = hst[8 * r + 6], t1 = hst[8 * r + 7];
         repUs[r] = t1 > t0 ? (double)(t1 - t0) * 1e-3 : 0.0;
         longest = std::max(longest, repUs[r]);
-        busy += repUs[r] * Gs[r];
+        busy += repUs[r] * G;
     }
     for (u32 r = 0; r < nrep; r++)
         if (errs[r]) {
@@ -871,7 +792,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         casphy_set_last_error_msg("bootstrap: post-order stack overflow");
         return CASPHY_EINTERNAL;
     }
-    boot::refit(tune, repN, Gs, repUs, repPhases);
+    boot::refit(tune, repN, G, repUs, repPhases);
     float tInit = 0, tJoin = 0, tX = 0, tAll = 0;
     cudaEventElapsedTime(&tInit, ev[0], ev[1]);
     cudaEventElapsedTime(&tJoin, ev[1], ev[2]);
@@ -888,7 +809,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         s.total_ms = tAll;
         s.kernel_launches = launches;
         s.join_phases = phases;
-        s.max_ctas_per_rep = maxG;
+        s.max_ctas_per_rep = G;
         s.graph = graphed ? 1u : 0u;
         s.tuned = tunedBefore ? 1u : 0u;
         s.join_longest_ms = longest * 1e-3;

@@ -105,8 +105,8 @@ constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 
 // Launches the join on one cluster; *done says whether it could.
 template <int PATH>
-static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PATH>::Args& bm, u32 Sp, cudaStream_t st,
-                              bool* done) {
+static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PATH>::Args& bm, u32 Sp,
+                              const unsigned long long* initKey, cudaStream_t st, bool* done) {
     using M = BitCluster<PATH>;
     *done = false;
     int smemMax = 0, dev = 0;
@@ -120,7 +120,7 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     a.R = ((c.ntip + a.G - 1) / a.G + kClusterSlots - 1) / kClusterSlots * kClusterSlots;
     // (list entries hold a column offset in 27 bits)
     if (a.R >= 0xFFFFu || (u64)bm.nbin * Sp >= (1u << 27)) return CASPHY_OK;
-    a.lmOrd = c.lmOrd[0]; a.lmIdx = c.lmIdx[0]; a.slotNode = c.slotNode[0];
+    a.initKey = initKey;
     a.nodeSize = c.nodeSize; a.rawEdge = c.rawEdge; a.err = c.err; a.limitNs = c.limitNs; a.statsOut = c.statsOut;
     a.prof = c.prof;
     a.ordNeg1 = c.ordNeg1;
@@ -132,14 +132,19 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     size_t smem = 0;
     if (!cluster_fit<PATH>(a, m, (size_t)smemMax - 6144, &smem)) return CASPHY_OK;
     if (PATH != PATH_FLOAT && m.colWords < (size_t)m.nbin * a.R) return CASPHY_OK;
-    return joinc::launch(k_cluster_join<M>, a.G, 1, smem, st, done, a, m);
+    return joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
 }
 
 template <int PATH>
-static int launch_bit_any(joinx::Common& c, const typename BitModel<PATH>::Args& m, u32 Sp, u32 nCTA, cudaStream_t st) {
+static int launch_bit_any(joinx::Common& c, const typename BitModel<PATH>::Args& m, u32 Sp,
+                          const unsigned long long* initKey, const u32* tipSize, u32 nCTA, cudaStream_t st) {
     bool done = false;
-    if (int rc = launch_bit_cluster<PATH>(c, m, Sp, st, &done)) return rc;
-    return done ? CASPHY_OK : launch_bit_join<PATH>(c, m, nCTA, st);
+    if (int rc = launch_bit_cluster<PATH>(c, m, Sp, initKey, st, &done)) return rc;
+    if (done) return CASPHY_OK;
+    joinx::k_slot_init<<<(std::max(Sp, c.nnode) + 255) / 256, 256, 0, st>>>(
+        c.ntip, Sp, c.nnode, initKey, ORD_F32_NEG1, c.lmOrd[0], c.lmIdx[0], c.slotNode[0], c.node2slot, c.nodeDeath,
+        c.nodeSize, tipSize);
+    return launch_bit_join<PATH>(c, m, nCTA, st);
 }
 
 static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_words, const double* weight,
@@ -282,9 +287,6 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
     }
     CASPHY_CUDA_TRY(cudaEventRecord(ev[2], st));
     if (ntip >= 2) {
-        joinx::k_slot_init<<<(std::max(Sp, nnode) + 255) / 256, 256, 0, st>>>(
-            ntip, Sp, nnode, L.initKey, ORD_F32_NEG1, L.lm[0], L.lm[1], L.lm[2], L.node2slot, L.nodeDeath, L.nodeSize,
-            L.tip);
         joinx::Common c{};
         c.ntip = ntip; c.nnode = nnode; c.nCTA = nCTA; c.align = 8;
         c.lmOrd[0] = L.lm[0]; c.lmIdx[0] = L.lm[1]; c.slotNode[0] = L.lm[2];
@@ -300,15 +302,15 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
         if (path == PATH_UNIT) {
             BitModel<PATH_UNIT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                         {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, nCTA, st);
+            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, L.initKey, L.tip, nCTA, st);
         } else if (path == PATH_PLANES) {
             BitModel<PATH_PLANES>::Args m{nbin, nbinP, nplanes, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                           {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, nCTA, st);
+            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, L.initKey, L.tip, nCTA, st);
         } else {
             BitModel<PATH_FLOAT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                          {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, nCTA, st);
+            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, L.initKey, L.tip, nCTA, st);
         }
         if (rc) return rc;
         launches += 2;

@@ -48,10 +48,9 @@ struct alignas(16) Rec {
 struct Args {
     u32 ntip, nnode, G;
     u32 R;                // slots per CTA at the start, below 65,535
-    const u32* lmOrd;     // ntip slots: maximum, partner and node
-    const u32* lmIdx;
-    const u32* slotNode;
-    u32* nodeSize;
+    const unsigned long long* initKey;  // ntip initial (maximum, partner) keys
+    const u32* tipSize;   // null: all 1
+    u32* nodeSize;        // of the new nodes (needSizes, keepSizes)
     u32* rawEdge;
     int* err;
     u64 limitNs;
@@ -168,9 +167,10 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
     st.n = min(lo + a.R, a.ntip) - lo;
     st.cap = a.R;
     for (u32 x = tid; x < st.n; x += kThreads) {
-        st.node[x] = a.slotNode[lo + x];
-        st.ord[x] = a.lmOrd[lo + x];
-        st.idx[x] = a.lmIdx[lo + x];
+        const u64 key = a.initKey[lo + x];
+        st.node[x] = lo + x;
+        st.ord[x] = key_ord(key);
+        st.idx[x] = key_node(key);
     }
     for (u32 i = tid; i < a.deathWords; i += kThreads) deathBits[i] = 0u;
     if (tid < kMaxBatch * kWarps) (&s_red[0][0])[tid] = 0ull;
@@ -417,8 +417,12 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
         u32 sz1 = 0, sz2 = 0;
         const bool bookkeeper = rank == 0 && tid == kThreads - 1;
         if (a.needSizes || (a.keepSizes && bookkeeper)) {
-            sz1 = ld_cg_u32(a.nodeSize + j1);
-            sz2 = ld_cg_u32(a.nodeSize + j2);
+            auto size_of = [&](u32 j) {
+                if (j >= a.ntip) return ld_cg_u32(a.nodeSize + j);
+                return a.tipSize ? a.tipSize[j] : 1u;
+            };
+            sz1 = size_of(j1);
+            sz2 = size_of(j2);
         }
         const u32 own = slot1 >> 24 == rank ? slot1 & 0xFFFFFFu : joinx::kNone;
         const u32 nE = M::build_join(a, m, ms, st, rank, j1, j2, sz1, sz2, newNode, own);
@@ -521,12 +525,12 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
     }
 }
 
-// Host: whether the device can place a cluster of G CTAs of kernel fn.
-inline bool placeable(void* fn, u32 G, size_t smem) {
+// Host: how many clusters of G CTAs of kernel fn the device can hold at once.
+inline int placeable(void* fn, u32 G, size_t smem) {
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return 0;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(G);
@@ -541,17 +545,14 @@ inline bool placeable(void* fn, u32 G, size_t smem) {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return 0;
     }
-    return n >= 1;
+    return n;
 }
 
-// Host: launches `clusters` clusters of G CTAs of kernel fn(args...); *done
-// is false when the device cannot place one (nothing is launched then).
+// Host: queues `clusters` clusters of G CTAs of kernel fn(args...).
 template <class... K, class... A>
-int launch(void (*fn)(K...), u32 G, u32 clusters, size_t smem, cudaStream_t st, bool* done, const A&... args) {
-    *done = false;
-    if (!placeable((void*)fn, G, smem)) return CASPHY_OK;
+cudaError_t enqueue(void (*fn)(K...), u32 G, u32 clusters, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(G * clusters);
     cfg.blockDim = dim3(kThreads);
@@ -563,7 +564,16 @@ int launch(void (*fn)(K...), u32 G, u32 clusters, size_t smem, cudaStream_t st, 
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CASPHY_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, args...));
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+// Host: one cluster; *done is false when the device cannot place it (nothing
+// is launched then).
+template <class... K, class... A>
+int launch(void (*fn)(K...), u32 G, size_t smem, cudaStream_t st, bool* done, const A&... args) {
+    *done = false;
+    if (!placeable((void*)fn, G, smem)) return CASPHY_OK;
+    CASPHY_CUDA_TRY(enqueue(fn, G, 1, smem, st, args...));
     *done = true;
     return CASPHY_OK;
 }

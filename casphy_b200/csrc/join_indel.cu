@@ -1295,7 +1295,7 @@ static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 n
     size_t smem = 0;
     *done = false;
     if (!cluster_plan<HALF>(ntip, ncol, nState, unitW, a, m, &smem)) return CASPHY_OK;
-    a.lmOrd = L.lm[0]; a.lmIdx = L.lm[1]; a.slotNode = L.lm[2];
+    a.initKey = L.initKey; a.tipSize = L.tipSize;
     a.nodeSize = L.nodeSize; a.rawEdge = L.rawEdge; a.err = L.jerr; a.limitNs = 20ull * 1000 * 1000 * 1000;
     a.statsOut = L.stats;
     a.prof = getenv("CASPHY_PROFILE") ? L.stats + 8 : nullptr;
@@ -1312,7 +1312,7 @@ static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 n
     if (!joinc::placeable((void*)k_cluster_join<M>, a.G, smem)) return CASPHY_OK;
     k_split_bits<<<dim3(296, a.G), 256, 0, st>>>(L.bits0, m.rows, (ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32),
                                                  a.R / 32, L.bits1);
-    return joinc::launch(k_cluster_join<M>, a.G, 1, smem, st, done, a, m);
+    return joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
 }
 
 // Launches prep, initial scan and the persistent join.  Assumes Wsel,
@@ -1364,11 +1364,6 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
     }
     n++;
     if (evInit1) CASPHY_CUDA_TRY(cudaEventRecord(evInit1, st));
-    const u32 initN = std::max(Sp, nnode);  // Sp: slots rounded up to 32
-    joinx::k_slot_init<<<(initN + 255) / 256, 256, 0, st>>>(ntip, Sp, nnode, L.initKey, ORD_F16_NEG1, L.lm[0],
-                                                              L.lm[1], L.lm[2], L.node2slot, L.nodeDeath, L.nodeSize,
-                                                              L.tipSize);
-    n++;
     if (useBits) {
         // one cluster where it can hold the slots; a tree beyond it, or a
         // device that cannot place the cluster, runs on all SMs
@@ -1382,6 +1377,11 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
         }
         if (!intPath) return CASPHY_EINTERNAL;  // the caller asked cluster_plan() before it chose the bitsets
     }
+    const u32 initN = std::max(Sp, nnode);  // Sp: slots rounded up to 32
+    joinx::k_slot_init<<<(initN + 255) / 256, 256, 0, st>>>(ntip, Sp, nnode, L.initKey, ORD_F16_NEG1, L.lm[0],
+                                                              L.lm[1], L.lm[2], L.node2slot, L.nodeDeath, L.nodeSize,
+                                                              L.tipSize);
+    n++;
     joinx::Common c{};
     c.ntip = ntip; c.nnode = nnode; c.nCTA = nCTA; c.align = 8;
     c.lmOrd[0] = L.lm[0]; c.lmIdx[0] = L.lm[1]; c.slotNode[0] = L.lm[2];
