@@ -12,10 +12,18 @@
 //              four bit planes per block of 32 positions (plane j = bit j of
 //              the code), so one block costs popc((q0&c0)|(q1&c1)|(q2&c2)|
 //              (q3&c3)): nine integer operations for 32 positions.
-// Here the whole neighbour relation is produced as a bit matrix in one
-// tiled all-pairs launch (32 query rows per CTA in shared memory x 256
-// candidate rows, one warp ballot per 32 candidates), rows are counted, and
-// a second launch expands the bits into the ascending index lists.
+// Here the whole neighbour relation is produced as a bit matrix, rows are
+// counted, and a second launch expands the bits into the ascending index lists.
+// Both integer scores are shared-bit counts and run on the tensor cores
+// (bitdot.cuh): bit rows as they are, DNA rows as the bits of their four planes,
+// because two unambiguous codes share at most one.  A code of all four bases
+// (N) shares one position with any base but four plane bits with another N, so
+// the positions where both are N are counted once more with weight -3.  Other
+// ambiguity codes anywhere in the matrix (a device word the packing sets) leave
+// the DNA search to k_mask, one popcount per 32 positions.  The relation is
+// symmetric, so a search of all rows computes the tiles on and above the
+// diagonal and writes each result on both sides of it.  20,000 x 2,000 DNA: the
+// relation took 9.3 ms by popcounts of all pairs.
 #include <sys/mman.h>
 
 #include <algorithm>
@@ -23,6 +31,7 @@
 #include <cmath>
 #include <vector>
 
+#include "bitdot.cuh"
 #include "common.cuh"
 #include "runtime.h"
 
@@ -47,17 +56,21 @@ constexpr int kThreads = 256;  // candidates per CTA
 constexpr int kQ = 32;         // query rows per CTA
 enum { SC_UNIT = 0, SC_FLOAT = 1, SC_DNA = 2 };
 
-// rows are column-major: word k of row t at col[k * ld + t]
+// rows are column-major: word k of row t at col[k * ld + t]; DNA blocks of four
+// words lie together (uint4 at [block * ld + t]) and run only in mode 2
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) k_mask(const u32* __restrict__ col, u32 nwords, u32 ld, u32 ntip,
                                                    u32 qBegin, u32 qEnd, const float* __restrict__ wf, float radius,
-                                                   u32 uradius, u32 maskWords, u32* __restrict__ mask) {
+                                                   u32 uradius, u32 maskWords, u32* __restrict__ mask,
+                                                   const u32* __restrict__ dnaMode) {
+    if (MODE == SC_DNA && *dnaMode != 2u) return;
     extern __shared__ __align__(16) u32 qs[];  // kQ x nwords query words (query rows qBegin..qEnd-1)
     const u32 q0 = qBegin + blockIdx.y * kQ;
     const u32 t = blockIdx.x * kThreads + threadIdx.x;
     for (u32 i = threadIdx.x; i < kQ * nwords; i += kThreads) {
         const u32 q = i / nwords, k = i % nwords;
-        qs[q * nwords + k] = q0 + q < qEnd ? col[(size_t)k * ld + q0 + q] : 0u;
+        const size_t at = MODE == SC_DNA ? ((size_t)(k / 4) * ld + q0 + q) * 4 + k % 4 : (size_t)k * ld + q0 + q;
+        qs[q * nwords + k] = q0 + q < qEnd ? col[at] : 0u;
     }
     __syncthreads();
     u32 acc[kQ];
@@ -72,29 +85,23 @@ __global__ void __launch_bounds__(kThreads) k_mask(const u32* __restrict__ col, 
         const uint4* q4 = reinterpret_cast<const uint4*>(qs);
         const u32 nblk = nwords / 4;
         for (u32 b = 0; b < nblk; b++) {
-            const u32 c0 = col[(size_t)(4 * b) * ld + t], c1 = col[(size_t)(4 * b + 1) * ld + t];
-            const u32 c2 = col[(size_t)(4 * b + 2) * ld + t], c3 = col[(size_t)(4 * b + 3) * ld + t];
+            const uint4 c = reinterpret_cast<const uint4*>(col)[(size_t)b * ld + t];
 #pragma unroll
             for (int q = 0; q < kQ; q++) {
                 const uint4 v = q4[q * nblk + b];
-                acc[q] += (u32)__popc((v.x & c0) | (v.y & c1) | (v.z & c2) | (v.w & c3));
+                acc[q] += (u32)__popc((v.x & c.x) | (v.y & c.y) | (v.z & c.z) | (v.w & c.w));
             }
         }
     } else if (t < ntip) {
         for (u32 k = 0; k < nwords; k++) {
             const u32 c = col[(size_t)k * ld + t];
-            if (MODE == SC_UNIT) {
 #pragma unroll
-                for (int q = 0; q < kQ; q++) acc[q] += (u32)__popc(qs[q * nwords + k] & c);
-            } else {
-#pragma unroll
-                for (int q = 0; q < kQ; q++) {
-                    u32 m = qs[q * nwords + k] & c;
-                    while (m) {
-                        const int b = __ffs(m) - 1;
-                        facc[q] += __ldg(wf + k * 32 + b);
-                        m &= m - 1;
-                    }
+            for (int q = 0; q < kQ; q++) {
+                u32 m = qs[q * nwords + k] & c;
+                while (m) {
+                    const int b = __ffs(m) - 1;
+                    facc[q] += __ldg(wf + k * 32 + b);
+                    m &= m - 1;
                 }
             }
         }
@@ -103,8 +110,7 @@ __global__ void __launch_bounds__(kThreads) k_mask(const u32* __restrict__ col, 
 #pragma unroll
     for (int q = 0; q < kQ; q++) {
         bool hit;
-        if (MODE == SC_UNIT) hit = (float)acc[q] >= radius;
-        else if (MODE == SC_DNA) hit = acc[q] >= uradius;
+        if (MODE == SC_DNA) hit = acc[q] >= uradius;
         else hit = facc[q] >= radius;
         hit = hit && t < ntip;
         const u32 bal = __ballot_sync(0xFFFFFFFFu, hit);
@@ -152,12 +158,14 @@ __global__ void k_expand(const u32* __restrict__ mask, u32 ntip, u32 maskWords, 
     }
 }
 
-// fasta2bin bytes -> column-major bit planes: for block b of 32 positions,
-// word 4b+j holds bit j of the low nibble of the code of position 32b+s at
-// bit s (the reference keeps the same low nibbles, packed eight to a word,
-// cu/radiusNeighborDNA.cu:27-53).
+// fasta2bin bytes -> bit planes: for block b of 32 positions, word j of the
+// uint4 at [b * ld + t] holds bit j of the low nibble of the code of position
+// 32b+s at bit s (the reference keeps the same low nibbles, packed eight to a
+// word, cu/radiusNeighborDNA.cu:27-53).  Behind the nblk blocks follow the N
+// positions, 128 to a uint4 (word b % 4 of block nblk + b / 4).  *mode: 1 when
+// some code is N, 2 when some code has two or three bases.
 __global__ void k_pack_dna(const u32* __restrict__ raw, u32 ntip, u32 nbinRaw, u32 nblk, u32 ld,
-                           u32* __restrict__ col) {
+                           u32* __restrict__ col, u32* __restrict__ mode) {
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 b = blockIdx.y;
     if (t >= ntip || b >= nblk) return;
@@ -173,9 +181,57 @@ __global__ void k_pack_dna(const u32* __restrict__ raw, u32 ntip, u32 nbinRaw, u
             for (int j = 0; j < 4; j++) p[j] |= ((code >> j) & 1u) << s;
         }
     }
-#pragma unroll
-    for (int j = 0; j < 4; j++) col[(size_t)(4 * b + j) * ld + t] = p[j];
+    reinterpret_cast<uint4*>(col)[(size_t)b * ld + t] = make_uint4(p[0], p[1], p[2], p[3]);
+    const u32 n = p[0] & p[1] & p[2] & p[3];
+    const u32 two = (p[0] & p[1]) | (p[0] & p[2]) | (p[0] & p[3]) | (p[1] & p[2]) | (p[1] & p[3]) | (p[2] & p[3]);
+    col[((size_t)(nblk + b / 4) * ld + t) * 4 + b % 4] = n;
+    if (b == nblk - 1)
+        for (u32 i = b % 4 + 1; i < 4; i++) col[((size_t)(nblk + b / 4) * ld + t) * 4 + i] = 0u;
+    const u32 m = two & ~n ? 2u : (n ? 1u : 0u);
+    if (m > *(volatile u32*)mode) atomicMax(mode, m);
 }
+
+// Word planes -> 128-bit chunks: uint4 at [c * ld + t] = words 4c .. 4c+3 of row t.
+__global__ void k_pack_bits(const u32* __restrict__ planes, u32 ntip, u32 nwords, uint4* __restrict__ out) {
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (t >= ntip) return;
+    u32 w[4];
+#pragma unroll
+    for (u32 j = 0; j < 4; j++) w[j] = 4 * c + j < nwords ? planes[(size_t)(4 * c + j) * ntip + t] : 0u;
+    out[(size_t)c * ntip + t] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Epilogue of the shared-bit counts: hits (count >= the threshold) of the
+// tile's rows as mask words and, when every pair is computed once, of its
+// columns too.
+struct RadiusTile {
+    struct Params {
+        int least8;  // eight times the least count that is a hit
+        u32 maskWords, mirror;
+        u32* mask;   // rowsA rows (all rows when mirrored)
+    };
+    __device__ static void tile(const bitdot::Args& a, const Params& p, u32 m0, u32 n0, u32 taddr, unsigned char*) {
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wr = warp & 3u;
+        const u32 q = m0 + 32 * wr + lane, qword = m0 / 32 + wr;
+        const bool qok = q < a.rowsA;
+        for (u32 cb = warp >> 2; cb < bitdot::kN / 32; cb += bitdot::kThreads / 128) {
+            u32 r[32];
+            bitdot::load32(taddr + (32 * wr << 16) + cb * 32, r);
+            const u32 n = n0 + cb * 32, cols = n < a.rowsB ? min(a.rowsB - n, 32u) : 0u;
+            u32 word = 0, col = 0;
+#pragma unroll
+            for (u32 j = 0; j < 32; j++) {
+                const bool hit = (int)r[j] >= p.least8;
+                word |= (u32)hit << j;
+                const u32 b = __ballot_sync(0xFFFFFFFFu, hit && qok);
+                if (lane == j) col = b;
+            }
+            if (cols < 32u) word &= (1u << cols) - 1u;
+            if (qok && cols) p.mask[(size_t)q * p.maskWords + n / 32] = word;
+            if (p.mirror && lane < cols && qword < p.maskWords) p.mask[(size_t)(n + lane) * p.maskWords + qword] = col;
+        }
+    }
+};
 
 // tryRadius: counts[r] = #{t < ntip : score(q_r, t) >= radius}; bit rows
 // with radius <= 0 also count the idle threads of the last 128-thread block
@@ -189,11 +245,10 @@ __global__ void k_try(const u32* __restrict__ col, u32 nwords, u32 ld, u32 ntip,
     bool hit = false;
     if (t < ntip && MODE == SC_DNA) {
         u32 acc = 0;
+        const uint4* c4 = reinterpret_cast<const uint4*>(col);
         for (u32 b = 0; b < nwords / 4; b++) {
-            u32 x = 0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) x |= col[(size_t)(4 * b + j) * ld + q] & col[(size_t)(4 * b + j) * ld + t];
-            acc += (u32)__popc(x);
+            const uint4 x = c4[(size_t)b * ld + q], y = c4[(size_t)b * ld + t];
+            acc += (u32)__popc((x.x & y.x) | (x.y & y.y) | (x.z & y.z) | (x.w & y.w));
         }
         hit = acc >= uradius;
     } else if (t < ntip) {
@@ -234,16 +289,21 @@ struct RadiusInput {
     u32 uradius;
 };
 
-// Uploads rows column-major (ld = ntip); returns the device pointer.
-static int upload_rows(const RadiusInput& in, Carve& c, u32** col, float** wf, cudaStream_t st) {
-    *col = c.take<u32>((size_t)in.nwords * in.ntip);
+// Words of the device rows: DNA rows carry their N positions behind the planes.
+static size_t row_words(const RadiusInput& in) { return in.dna ? in.nwords + 4 * ((in.nwords / 4 + 3) / 4) : in.nwords; }
+
+// Uploads the rows (ld = ntip); mode: the word k_pack_dna sets.
+static int upload_rows(const RadiusInput& in, Carve& c, u32** col, float** wf, u32** mode, cudaStream_t st) {
+    *col = c.take<u32>(row_words(in) * in.ntip);
     *wf = c.take<float>(in.wf.size() ? in.wf.size() : 1);
+    *mode = c.take<u32>(2);  // [1]: error of a device-side wait
+    CASPHY_CUDA_TRY(cudaMemsetAsync(*mode, 0, 2 * sizeof(u32), st));
     if (in.dna) {
         u32* raw = c.take<u32>((size_t)in.ntip * in.nbinRaw);
         CASPHY_CUDA_TRY(cudaMemcpyAsync(raw, in.hostRaw, sizeof(u32) * (size_t)in.ntip * in.nbinRaw,
                                         cudaMemcpyHostToDevice, st));
         k_pack_dna<<<dim3((in.ntip + 255) / 256, in.nwords / 4), 256, 0, st>>>(raw, in.ntip, in.nbinRaw, in.nwords / 4,
-                                                                               in.ntip, *col);
+                                                                               in.ntip, *col, *mode);
     } else {
         CASPHY_CUDA_TRY(cudaMemcpyAsync(*col, in.hostWordPlane, sizeof(u32) * (size_t)in.nwords * in.ntip,
                                         cudaMemcpyHostToDevice, st));
@@ -308,7 +368,8 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     DeviceScope ds;
     cudaStream_t st = 0;
     auto lay = [&](Carve& c) {
-        struct B { u32* mask; u32* counts; u64* off; } b;
+        struct B { uint4* chunks; u32* mask; u32* counts; u64* off; } b;
+        b.chunks = c.take<uint4>(in.mode == SC_UNIT ? (size_t)((in.nwords + 3) / 4) * ntip : 0);
         b.mask = c.take<u32>((size_t)nq * maskWords);
         b.counts = c.take<u32>(nq);
         b.off = c.take<u64>(nq);
@@ -318,8 +379,10 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     Carve cv;
     u32* dcol;
     float* dwf;
-    cv.take<u32>((size_t)in.nwords * ntip);
+    u32* dmode;
+    cv.take<u32>(row_words(in) * ntip);
     cv.take<float>(in.wf.size() ? in.wf.size() : 1);
+    cv.take<u32>(2);
     if (in.dna) cv.take<u32>((size_t)ntip * in.nbinRaw);
     lay(cv);
     const size_t base0 = cv.off;
@@ -328,26 +391,58 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     if (rc) return rc;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    rc = upload_rows(in, c2, &dcol, &dwf, st);
+    rc = upload_rows(in, c2, &dcol, &dwf, &dmode, st);
     if (rc) return rc;
     auto L = lay(c2);
     dim3 grid((ntip + kThreads - 1) / kThreads, (nq + kQ - 1) / kQ);
-    void* fn = in.mode == SC_UNIT ? (void*)k_mask<SC_UNIT> : in.mode == SC_DNA ? (void*)k_mask<SC_DNA>
-                                                                                  : (void*)k_mask<SC_FLOAT>;
-    CASPHY_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (in.mode == SC_UNIT)
-        k_mask<SC_UNIT><<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius, in.uradius,
-                                                       maskWords, L.mask);
-    else if (in.mode == SC_DNA)
-        k_mask<SC_DNA><<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius, in.uradius,
-                                                      maskWords, L.mask);
-    else
+    if (in.mode != SC_UNIT) {
+        void* fn = in.mode == SC_DNA ? (void*)k_mask<SC_DNA> : (void*)k_mask<SC_FLOAT>;
+        CASPHY_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
+    if (in.mode == SC_FLOAT) {
         k_mask<SC_FLOAT><<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius, in.uradius,
-                                                        maskWords, L.mask);
+                                                        maskWords, L.mask, nullptr);
+    } else {
+        const u32 nchunk = (in.nwords + 3) / 4;
+        const bool upper = nq == ntip;
+        bitdot::Args a{};
+        a.A = a.B = in.dna ? reinterpret_cast<const uint4*>(dcol) : L.chunks;
+        a.ldA = a.ldB = ntip;
+        a.a0 = row0;
+        a.rowsA = nq;
+        a.rowsB = ntip;
+        a.chunks = in.dna ? (u32)(row_words(in) / 4) : nchunk;
+        a.negFrom = nchunk;
+        a.upper = upper ? 1u : 0u;
+        a.tilesN = bitdot::tiles_n(ntip);
+        a.mode = in.dna ? dmode : nullptr;
+        a.err = reinterpret_cast<int*>(dmode + 1);
+        // (counts stay far below 2^24: the least hit as an integer)
+        const u32 least = in.dna ? in.uradius : (in.radius <= 0.f ? 0u : (u32)std::min(in.radius, 268435455.f));
+        RadiusTile::Params p{(int)(8u * std::min(least, 0x0FFFFFFFu)), maskWords, upper ? 1u : 0u, L.mask};
+        const u64 nt = bitdot::tiles(nq, ntip, upper);
+        if (nt > 0x7FFFFFFFull) {
+            casphy_set_last_error_msg("radius: too many rows");
+            return CASPHY_ERANGE;
+        }
+        if (!in.dna) k_pack_bits<<<dim3((ntip + 255) / 256, nchunk), 256, 0, st>>>(dcol, ntip, in.nwords, L.chunks);
+        CASPHY_CUDA_TRY(cudaFuncSetAttribute((void*)bitdot::k_bitdot<RadiusTile>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitdot::kSmemBytes));
+        bitdot::k_bitdot<RadiusTile><<<(u32)nt, bitdot::kThreads, bitdot::kSmemBytes, st>>>(a, p);
+        if (in.dna)
+            k_mask<SC_DNA><<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius,
+                                                          in.uradius, maskWords, L.mask, dmode);
+    }
     k_count<<<(nq + 7) / 8, 256, 0, st>>>(L.mask, nq, maskWords, L.counts);
     CASPHY_CUDA_TRY(cudaGetLastError());
     CASPHY_CUDA_TRY(cudaMemcpyAsync(counts, L.counts, sizeof(u32) * nq, cudaMemcpyDeviceToHost, st));
+    int werr = 0;
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(&werr, dmode + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+    if (werr) {
+        casphy_set_last_error_msg("radius: a device-side wait timed out");
+        return werr;
+    }
     std::vector<u64> off(nq);
     u64 tot = 0;
     for (u32 i = 0; i < nq; i++) {
@@ -383,8 +478,9 @@ static int try_impl(RadiusInput& in, u32 nrep, const u32* qidx, u32* counts) {
     DeviceScope ds;
     cudaStream_t st = 0;
     Carve cv;
-    cv.take<u32>((size_t)in.nwords * in.ntip);
+    cv.take<u32>(row_words(in) * in.ntip);
     cv.take<float>(in.wf.size() ? in.wf.size() : 1);
+    cv.take<u32>(2);
     if (in.dna) cv.take<u32>((size_t)in.ntip * in.nbinRaw);
     cv.take<u32>(nrep);
     cv.take<u32>(nrep);
@@ -395,7 +491,8 @@ static int try_impl(RadiusInput& in, u32 nrep, const u32* qidx, u32* counts) {
     c2.base = static_cast<char*>(base);
     u32* dcol;
     float* dwf;
-    rc = upload_rows(in, c2, &dcol, &dwf, st);
+    u32* dmode;
+    rc = upload_rows(in, c2, &dcol, &dwf, &dmode, st);
     if (rc) return rc;
     u32* dq = c2.take<u32>(nrep);
     u32* dc = c2.take<u32>(nrep);

@@ -10,95 +10,112 @@
 // changes the result only when rows carry bits past ntip, and it is kept
 // exactly.  Sizes are min(k, ntip - k), k = popcount of the row (:107-121).
 //
-// One launch tiles 32 x rows (lanes) by 64 y rows (8 warps x one group of
-// 8), streams 32-word chunks of both tiles through shared memory, and keeps
-// the 8 distances per thread in registers; x minima are reduced across the
-// warps, y minima across aligned 8-lane segments, then merged with atomicMin.
+// d = |x| + |y| - 2 |x n y|, so the distances of a 128 x 256 tile of pairs are
+// one tensor-core contraction (bitdot.cuh) and the row popcounts; the tile's
+// epilogue forms the grouped minima from them (groups of 8 columns in a thread,
+// groups of 8 rows by shuffles), one atomicMin per row and column of the tile.
+// 9,998 x 9,998 rows of 313 words: popcounts of the XORed words took 7 ms.
 #include <vector>
 
+#include "bitdot.cuh"
 #include "common.cuh"
 #include "runtime.h"
 
 namespace casphy {
 namespace tdis {
 
-constexpr u32 kTX = 32, kTY = 64, kChunk = 32;
-
-__global__ void __launch_bounds__(256) k_cross(const u32* __restrict__ X, const u32* __restrict__ Y, u32 nx, u32 ny,
-                                               u32 ncol, u32 ntip, u32* __restrict__ xmin, u32* __restrict__ ymin) {
-    __shared__ u32 xs[kTX][kChunk + 1];
-    __shared__ u32 ys[kTY][kChunk];
-    __shared__ u32 red[8][kTX];
-    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const u32 x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY;
-    u32 d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (u32 k0 = 0; k0 < ncol; k0 += kChunk) {
-        const u32 kn = min(kChunk, ncol - k0);
-        for (u32 i = threadIdx.x; i < kTX * kChunk; i += 256) {
-            const u32 r = i / kChunk, k = i % kChunk;
-            xs[r][k] = (x0 + r < nx && k < kn) ? X[(size_t)(x0 + r) * ncol + k0 + k] : 0u;
+struct TransferTile {
+    struct Params {
+        u32 full, pad;  // 32 ncol, and the bits past ntip
+        const u32* cx;  // popcounts of the rows
+        const u32* cy;
+        u32* xmin;
+        u32* ymin;
+    };
+    // x rows are the tile's rows, y rows its columns
+    __device__ static void tile(const bitdot::Args& a, const Params& p, u32 m0, u32 n0, u32 taddr, unsigned char* smem) {
+        u32* s_cy = reinterpret_cast<u32*>(smem);  // kN
+        u32* s_y = s_cy + bitdot::kN;              // kN
+        u32* s_x = s_y + bitdot::kN;               // kM
+        const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp & 3u;
+        if (tid < bitdot::kN) {
+            s_cy[tid] = n0 + tid < a.rowsB ? p.cy[n0 + tid] : 0u;
+            s_y[tid] = 0xFFFFFFFFu;
         }
-        for (u32 i = threadIdx.x; i < kTY * kChunk; i += 256) {
-            const u32 r = i / kChunk, k = i % kChunk;
-            ys[r][k] = (y0 + r < ny && k < kn) ? Y[(size_t)(y0 + r) * ncol + k0 + k] : 0u;
-        }
+        if (tid < bitdot::kM) s_x[tid] = 0xFFFFFFFFu;
         __syncthreads();
-        for (u32 k = 0; k < kn; k++) {
-            const u32 xv = xs[lane][k];
+        const u32 x = m0 + 32 * wr + lane;
+        const bool xok = x < a.rowsA, gok = (x & ~7u) < a.rowsA;
+        const u32 mc = xok ? p.cx[x] : 0u;
+        u32 xm = 0xFFFFFFFFu;
+        for (u32 cb = warp >> 2; cb < bitdot::kN / 32; cb += bitdot::kThreads / 128) {
+            u32 r[32], keep = 0xFFFFFFFFu;
+            bitdot::load32(taddr + (32 * wr << 16) + cb * 32, r);
+            const u32 n = n0 + cb * 32;
 #pragma unroll
-            for (int i = 0; i < 8; i++) d[i] += (u32)__popc(xv ^ ys[w * 8 + i][k]);
-        }
-        __syncthreads();
-    }
-    const u32 full = 32u * ncol, pad = 32u * ncol - ntip;
-    const bool xok = x0 + lane < nx;
-    // x side: this thread's 8 y rows are one aligned group
-    {
-        u32 A = full, B = full;
+            for (u32 g = 0; g < 4; g++) {
+                u32 A = p.full, B = p.full;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            if (y0 + w * 8 + i < ny) {
-                A = min(A, d[i]);
-                B = min(B, full - d[i]);
+                for (u32 i = 0; i < 8; i++) {
+                    const u32 j = 8 * g + i;
+                    const u32 d = mc + s_cy[cb * 32 + j] - (r[j] >> 2);  // the accumulator is 8 |x n y|
+                    if (n + j < a.rowsB) {
+                        A = min(A, d);
+                        B = min(B, p.full - d);
+                    }
+                    u32 ya = xok ? d : p.full, yb = xok ? p.full - d : p.full;
+#pragma unroll
+                    for (u32 o = 1; o < 8; o <<= 1) {
+                        ya = min(ya, __shfl_xor_sync(0xFFFFFFFFu, ya, o));
+                        yb = min(yb, __shfl_xor_sync(0xFFFFFFFFu, yb, o));
+                    }
+                    u32 v = gok ? min(ya, yb - p.pad) : 0xFFFFFFFFu;
+                    v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, 8));
+                    v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, 16));
+                    if (lane == j) keep = v;
+                }
+                if (n + 8 * g < a.rowsB) xm = min(xm, min(A, B - p.pad));
             }
+            if (n + lane < a.rowsB) atomicMin(s_y + cb * 32 + lane, keep);
         }
-        const u32 t2 = B - pad;
-        red[w][lane] = A > t2 ? t2 : A;
+        if (xok) atomicMin(s_x + 32 * wr + lane, xm);
         __syncthreads();
-        if (w == 0 && xok) {
-            u32 v = red[0][lane];
-            for (int g = 1; g < 8; g++)
-                if (y0 + g * 8 < ny) v = min(v, red[g][lane]);
-            atomicMin(xmin + x0 + lane, v);
-        }
+        if (tid < bitdot::kN && n0 + tid < a.rowsB) atomicMin(p.ymin + n0 + tid, s_y[tid]);
+        if (tid < bitdot::kM && m0 + tid < a.rowsA) atomicMin(p.xmin + m0 + tid, s_x[tid]);
     }
-    // y side: aligned groups of 8 lanes are groups of 8 x rows
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        u32 A = xok ? d[i] : full;
-        u32 B = xok ? full - d[i] : full;
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            A = min(A, __shfl_xor_sync(0xFFFFFFFFu, A, o));
-            B = min(B, __shfl_xor_sync(0xFFFFFFFFu, B, o));
-        }
-        const u32 y = y0 + w * 8 + i;
-        if ((lane & 7) == 0 && y < ny && x0 + lane < nx) {
-            const u32 t2 = B - pad;
-            atomicMin(ymin + y, A > t2 ? t2 : A);
-        }
-    }
-}
+};
 
-__global__ void k_sizes(const u32* __restrict__ M, u32 n, u32 ncol, u32 ntip, u32* __restrict__ size) {
-    const u32 r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    const u32 lane = threadIdx.x & 31;
-    if (r >= n) return;
-    u32 c = 0;
-    for (u32 k = lane; k < ncol; k += 32) c += (u32)__popc(M[(size_t)r * ncol + k]);
+// Rows of ncol words -> 128-bit chunks, uint4 at [c * n + row], and the rows'
+// popcounts and sizes: a block takes 32 rows, a warp four of them at a time.
+__global__ void __launch_bounds__(256) k_pack_rows(const u32* __restrict__ M, u32 n, u32 ncol, u32 ntip, uint4* __restrict__ out,
+                                                   u32* __restrict__ pop, u32* __restrict__ size) {
+    __shared__ u32 t[32][33];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * 32;
+    u32 cnt[4] = {0u, 0u, 0u, 0u};  // rows r0 + warp + 8 i
+    for (u32 k0 = 0; k0 < ncol; k0 += 32) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-    if (lane == 0) size[r] = c > ntip - c ? ntip - c : c;
+        for (u32 i = 0; i < 4; i++) {
+            const u32 r = r0 + warp + 8 * i, k = k0 + lane;
+            const u32 v = r < n && k < ncol ? M[(size_t)r * ncol + k] : 0u;
+            t[warp + 8 * i][lane] = v;
+            cnt[i] += (u32)__popc(v);
+        }
+        __syncthreads();
+        // warp w: chunk w of the eight, lane = row
+        const u32 c = k0 / 4 + warp;
+        if (4 * c < ncol && r0 + lane < n)
+            out[(size_t)c * n + r0 + lane] =
+                make_uint4(t[lane][4 * warp], t[lane][4 * warp + 1], t[lane][4 * warp + 2], t[lane][4 * warp + 3]);
+        __syncthreads();
+    }
+#pragma unroll
+    for (u32 i = 0; i < 4; i++) {
+        const u32 c = __reduce_add_sync(0xFFFFFFFFu, cnt[i]), r = r0 + warp + 8 * i;
+        if (lane == 0 && r < n) {
+            pop[r] = c;
+            size[r] = c > ntip - c ? ntip - c : c;
+        }
+    }
 }
 
 __global__ void k_fill_u32(u32* p, u32 n, u32 v) {
@@ -108,16 +125,55 @@ __global__ void k_fill_u32(u32* p, u32 n, u32 v) {
 
 }  // namespace tdis
 
-int transfer_dis_device(u32 ny, u32 nx, u32 ncol, u32 ntip, const u32* dY, const u32* dX, u32* dYmin, u32* dYsize,
-                        u32* dXmin, u32* dXsize, cudaStream_t st) {
+// Device scratch of transfer_dis_device.
+struct TransferScratch {
+    uint4 *cy, *cx;  // chunks
+    u32 *py, *px;    // popcounts
+    int* err;
+};
+static TransferScratch carve_scratch(Carve& c, u32 ny, u32 nx, u32 ncol) {
+    const size_t chunks = (ncol + 3) / 4;
+    TransferScratch s;
+    s.cy = c.take<uint4>(chunks * ny);
+    s.cx = c.take<uint4>(chunks * nx);
+    s.py = c.take<u32>(ny);
+    s.px = c.take<u32>(nx);
+    s.err = c.take<int>(1);
+    return s;
+}
+
+static int transfer_dis_device(u32 ny, u32 nx, u32 ncol, u32 ntip, const u32* dY, const u32* dX, u32* dYmin,
+                               u32* dYsize, u32* dXmin, u32* dXsize, const TransferScratch& s, cudaStream_t st) {
     using namespace tdis;
     const u32 full = 32u * ncol;
-    if (ny) k_fill_u32<<<(ny + 255) / 256, 256, 0, st>>>(dYmin, ny, full);
-    if (nx) k_fill_u32<<<(nx + 255) / 256, 256, 0, st>>>(dXmin, nx, full);
-    if (nx && ny) k_cross<<<dim3((nx + kTX - 1) / kTX, (ny + kTY - 1) / kTY), 256, 0, st>>>(dX, dY, nx, ny, ncol, ntip,
-                                                                                           dXmin, dYmin);
-    if (ny) k_sizes<<<(ny + 7) / 8, 256, 0, st>>>(dY, ny, ncol, ntip, dYsize);
-    if (nx) k_sizes<<<(nx + 7) / 8, 256, 0, st>>>(dX, nx, ncol, ntip, dXsize);
+    CASPHY_CUDA_TRY(cudaMemsetAsync(s.err, 0, sizeof(int), st));
+    if (ny) {
+        k_fill_u32<<<(ny + 255) / 256, 256, 0, st>>>(dYmin, ny, full);
+        k_pack_rows<<<(ny + 31) / 32, 256, 0, st>>>(dY, ny, ncol, ntip, s.cy, s.py, dYsize);
+    }
+    if (nx) {
+        k_fill_u32<<<(nx + 255) / 256, 256, 0, st>>>(dXmin, nx, full);
+        k_pack_rows<<<(nx + 31) / 32, 256, 0, st>>>(dX, nx, ncol, ntip, s.cx, s.px, dXsize);
+    }
+    if (nx && ny) {
+        bitdot::Args a{};
+        a.A = s.cx;
+        a.B = s.cy;
+        a.ldA = a.rowsA = nx;
+        a.ldB = a.rowsB = ny;
+        a.chunks = a.negFrom = (ncol + 3) / 4;
+        a.tilesN = bitdot::tiles_n(ny);
+        a.err = s.err;
+        const u64 nt = bitdot::tiles(nx, ny, false);
+        if (nt > 0x7FFFFFFFull) {
+            casphy_set_last_error_msg("transfer: too many rows");
+            return CASPHY_ERANGE;
+        }
+        CASPHY_CUDA_TRY(cudaFuncSetAttribute((void*)bitdot::k_bitdot<TransferTile>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitdot::kSmemBytes));
+        bitdot::k_bitdot<TransferTile><<<(u32)nt, bitdot::kThreads, bitdot::kSmemBytes, st>>>(
+            a, TransferTile::Params{full, full - ntip, s.px, s.py, dXmin, dYmin});
+    }
     CASPHY_CUDA_TRY(cudaGetLastError());
     return CASPHY_OK;
 }
@@ -134,13 +190,14 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     DeviceScope ds;
     cudaStream_t st = 0;
     auto lay = [&](Carve& c) {
-        struct B { u32* y; u32* x; u32* ymin; u32* ysize; u32* xmin; u32* xsize; } b;
+        struct B { u32* y; u32* x; u32* ymin; u32* ysize; u32* xmin; u32* xsize; TransferScratch s; } b;
         b.y = c.take<u32>((size_t)nrow_y * ncol);
         b.x = c.take<u32>((size_t)nrow_x * ncol);
         b.ymin = c.take<u32>(nrow_y);
         b.ysize = c.take<u32>(nrow_y);
         b.xmin = c.take<u32>(nrow_x);
         b.xsize = c.take<u32>(nrow_x);
+        b.s = carve_scratch(c, nrow_y, nrow_x, ncol);
         return b;
     };
     Carve cv;
@@ -153,8 +210,10 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     auto L = lay(c2);
     if (nrow_y) CASPHY_CUDA_TRY(cudaMemcpyAsync(L.y, y, sizeof(u32) * (size_t)nrow_y * ncol, cudaMemcpyHostToDevice, st));
     if (nrow_x) CASPHY_CUDA_TRY(cudaMemcpyAsync(L.x, x, sizeof(u32) * (size_t)nrow_x * ncol, cudaMemcpyHostToDevice, st));
-    rc = transfer_dis_device(nrow_y, nrow_x, ncol, ntip, L.y, L.x, L.ymin, L.ysize, L.xmin, L.xsize, st);
+    rc = transfer_dis_device(nrow_y, nrow_x, ncol, ntip, L.y, L.x, L.ymin, L.ysize, L.xmin, L.xsize, L.s, st);
     if (rc) return rc;
+    int werr = 0;
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(&werr, L.s.err, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (nrow_y) {
         CASPHY_CUDA_TRY(cudaMemcpyAsync(ymin, L.ymin, sizeof(u32) * nrow_y, cudaMemcpyDeviceToHost, st));
         CASPHY_CUDA_TRY(cudaMemcpyAsync(ysize, L.ysize, sizeof(u32) * nrow_y, cudaMemcpyDeviceToHost, st));
@@ -164,5 +223,6 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
         CASPHY_CUDA_TRY(cudaMemcpyAsync(xsize, L.xsize, sizeof(u32) * nrow_x, cudaMemcpyDeviceToHost, st));
     }
     CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
-    return CASPHY_OK;
+    if (werr) casphy_set_last_error_msg("transfer: a device-side wait timed out");
+    return werr;
 }
