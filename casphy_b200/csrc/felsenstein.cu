@@ -389,6 +389,55 @@ __global__ void k_pmat_irr(const double* __restrict__ t, u32 nedge, double rate,
     if (e < nedge) p[e] = make_float2((float)exp(-rate * t[e]), (float)(-expm1(-rate * t[e])));
 }
 
+// Allele counts of the tips per site (count: nsite x qstride, zeroed) and the
+// check of the codes (*bad set when one is beyond nallele + 1).  A block takes
+// 32 sites of kCountRows tips, a warp a row at a time, lane = site; counts go
+// through shared memory when the 32 sites' counters fit there.  On the host
+// this was one strided read of the codes per (site, tip), 5 ms of a 4,099 x
+// 500 call.
+constexpr u32 kCountRows = 256;
+__global__ void __launch_bounds__(256) k_allele_counts(const u32* __restrict__ codes, u32 ntip, u32 nsite, u32 nallele,
+                                                       u32 qstride, u32 useShared, u32* __restrict__ count, int* bad) {
+    extern __shared__ u32 hist[];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.x * 32 + lane;
+    const u32 r0 = blockIdx.y * kCountRows, r1 = min(r0 + kCountRows, ntip);
+    if (useShared) {
+        for (u32 i = threadIdx.x; i < 32 * qstride; i += 256) hist[i] = 0u;
+        __syncthreads();
+    }
+    bool wrong = false;
+    if (s < nsite)
+        for (u32 r = r0 + warp; r < r1; r += 8) {
+            const u32 c = codes[(size_t)r * nsite + s];
+            if (c > nallele + 1) wrong = true;
+            else if (c >= 2) {
+                if (useShared) atomicAdd(hist + lane * qstride + c - 1, 1u);
+                else if (count) atomicAdd(count + (size_t)s * qstride + c - 1, 1u);
+            }
+        }
+    if (wrong) *bad = 1;
+    if (!useShared || !count) return;
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < 32 * qstride; i += 256) {
+        const u32 at = blockIdx.x * 32 + i / qstride;
+        if (at < nsite && hist[i]) atomicAdd(count + (size_t)at * qstride + i % qstride, hist[i]);
+    }
+}
+// q = count / total per site, binary64 rounded to binary32; equal shares where
+// no tip has an allele.  A warp per site.
+__global__ void __launch_bounds__(256) k_allele_freq(const u32* __restrict__ count, u32 nsite, u32 qstride,
+                                                     float* __restrict__ q) {
+    const u32 lane = threadIdx.x & 31, s = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (s >= nsite) return;
+    u32 t = 0;
+    for (u32 a = 1 + lane; a < qstride; a += 32) t += count[(size_t)s * qstride + a];
+    t = __reduce_add_sync(0xFFFFFFFFu, t);
+    for (u32 a = lane; a < qstride; a += 32)
+        q[(size_t)s * qstride + a] = a == 0 ? 0.f
+                                     : t    ? (float)((double)count[(size_t)s * qstride + a] / (double)t)
+                                            : (float)(1.0 / (qstride - 1));
+}
+
 // One (node, site) of the inside pass once its children's partials are in.
 __device__ __forceinline__ void inside_irr_site(const IrrBuf& B, const Chunk& C, u32 vi, float2 pa, float2 pb, u32 s,
                                                 float4 la, float4 lb) {
@@ -982,22 +1031,30 @@ struct FelProblem {
         if (launches) *launches = n;
     }
 
-    int capture() {
-        for (int k = 0; k < 2; k++) {
-            cudaGraph_t g;
-            CASPHY_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            enqueue(k == 0, k == 0 ? &launchesFull : &launchesLL);
-            CASPHY_CUDA_TRY(cudaStreamEndCapture(st, &g));
-            if (launchErr != cudaSuccess) {
-                cudaGraphDestroy(g);
-                CASPHY_CUDA_TRY(launchErr);
-            }
-            cudaGraphExec_t ex;
-            const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+    // The graph of one kind of evaluation, captured when it is first wanted.
+    int capture(bool withGrad) {
+        cudaGraphExec_t& ex = withGrad ? gFull : gLL;
+        if (ex) return CASPHY_OK;
+        cudaGraph_t g;
+        CASPHY_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        enqueue(withGrad, withGrad ? &launchesFull : &launchesLL);
+        CASPHY_CUDA_TRY(cudaStreamEndCapture(st, &g));
+        if (launchErr != cudaSuccess) {
             cudaGraphDestroy(g);
-            CASPHY_CUDA_TRY(e);
-            (k == 0 ? gFull : gLL) = ex;
+            CASPHY_CUDA_TRY(launchErr);
         }
+        const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) ex = nullptr;
+        CASPHY_CUDA_TRY(e);
+        return CASPHY_OK;
+    }
+    // One evaluation without a graph, for a problem that is evaluated once (the
+    // capture and instantiation cost more than its launches).
+    int eval_once(bool withGrad, double* llOut) {
+        enqueue(withGrad, nullptr);
+        CASPHY_CUDA_TRY(launchErr);
+        CASPHY_CUDA_TRY(cudaMemcpyAsync(llOut, ll, sizeof(double), cudaMemcpyDeviceToHost, st));
         return CASPHY_OK;
     }
 
@@ -1005,6 +1062,7 @@ struct FelProblem {
     // eval_launch() queues the graph and the read of log L into *llOut,
     // eval_done() (after the stream is synchronised) adds its graph time
     int eval_launch(bool withGrad, double* llOut) {
+        if (int rc = capture(withGrad)) return rc;
         CASPHY_CUDA_TRY(cudaEventRecord(g0, st));
         CASPHY_CUDA_TRY(cudaGraphLaunch(withGrad ? gFull : gLL, st));
         CASPHY_CUDA_TRY(cudaEventRecord(g1, st));
@@ -1070,11 +1128,6 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
             casphy_set_last_error_msg("felsenstein: irreversible model needs rate > 0 and 1 <= nallele <= 32752");
             return CASPHY_EINVAL;
         }
-        for (size_t i = 0; i < (size_t)ntip * nsite; i++)
-            if (codes[i] > model->nallele + 1) {
-                casphy_set_last_error_msg("felsenstein: tip code beyond nallele + 1");
-                return CASPHY_ERANGE;
-            }
     }
     F.rate = model->rate;
     const u32 nint = F.th.nint;
@@ -1099,6 +1152,8 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         u32 *kidA, *kidB, *edgeA, *edgeB, *inO, *outO, *codes, *flags, *inEB, *outEB;
         uint4 *inInfo, *outInfo;
         double *t, *w, *grad, *gpart, *part, *ll;
+        u32* alleleCount;
+        int* badCode;
         double *x, *g, *d, *xn, *S, *Y, *rho, *gam, *sc, *lpart;
         float *P, *dP, *q;
         float2* p;
@@ -1142,6 +1197,8 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         b.dP = c.take<float>(isH ? 16 * (size_t)nedge : 0);
         b.p = c.take<float2>(isH ? 0 : nedge);
         b.q = c.take<float>(isH ? 0 : (size_t)nsite * qstride);
+        b.alleleCount = c.take<u32>(isH || model->allele_freq ? 0 : (size_t)nsite * qstride);
+        b.badCode = c.take<int>(1);
         b.L = c.take<float4>((size_t)nint * F.W);
         b.U = c.take<float4>((size_t)nint * F.W);
         b.E = c.take<int>(isH ? (size_t)nint * F.W : 0);
@@ -1190,26 +1247,34 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
     CASPHY_CUDA_TRY(up(L.w, wv.data(), 8ull * nsite));
     CASPHY_CUDA_TRY(cudaMemsetAsync(L.err, 0, sizeof(int), st));
     std::vector<float> q;
+    int bad = 0;
     if (!isH) {
-        // allele frequencies per site: given, or the tips' allele counts
-        q.assign((size_t)nsite * qstride, 0.f);
-        std::vector<double> cnt(qstride);
-        for (u32 s = 0; s < nsite; s++) {
-            std::fill(cnt.begin(), cnt.end(), 0.0);
-            if (model->allele_freq) {
-                for (u32 a = 1; a < qstride; a++) cnt[a] = std::max(0.0, model->allele_freq[(size_t)s * qstride + a]);
-            } else {
-                for (u32 i = 0; i < ntip; i++) {
-                    const u32 c = codes[(size_t)i * nsite + s];
-                    if (c >= 2) cnt[c - 1] += 1;
+        // the codes are checked, and the allele frequencies taken from the tips'
+        // counts, on the device; given frequencies are normalised here
+        const bool given = model->allele_freq != nullptr;
+        const u32 useShared = !given && 32u * qstride * sizeof(u32) <= 48 * 1024 ? 1u : 0u;
+        CASPHY_CUDA_TRY(cudaMemsetAsync(L.badCode, 0, sizeof(int), st));
+        if (!given) CASPHY_CUDA_TRY(cudaMemsetAsync(L.alleleCount, 0, 4ull * nsite * qstride, st));
+        k_allele_counts<<<dim3((nsite + 31) / 32, (ntip + kCountRows - 1) / kCountRows), 256,
+                          useShared ? 32u * qstride * sizeof(u32) : 0u, st>>>(
+            L.codes, ntip, nsite, model->nallele, qstride, useShared, given ? nullptr : L.alleleCount, L.badCode);
+        if (!given) k_allele_freq<<<(nsite + 7) / 8, 256, 0, st>>>(L.alleleCount, nsite, qstride, L.q);
+        CASPHY_CUDA_TRY(cudaGetLastError());
+        CASPHY_CUDA_TRY(cudaMemcpyAsync(&bad, L.badCode, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (given) {
+            q.assign((size_t)nsite * qstride, 0.f);
+            std::vector<double> cnt(qstride);
+            for (u32 s = 0; s < nsite; s++) {
+                double tot = 0;
+                for (u32 a = 1; a < qstride; a++) {
+                    cnt[a] = std::max(0.0, model->allele_freq[(size_t)s * qstride + a]);
+                    tot += cnt[a];
                 }
+                for (u32 a = 1; a < qstride; a++)
+                    q[(size_t)s * qstride + a] = tot > 0 ? (float)(cnt[a] / tot) : (float)(1.0 / (qstride - 1));
             }
-            double tot = 0;
-            for (u32 a = 1; a < qstride; a++) tot += cnt[a];
-            for (u32 a = 1; a < qstride; a++)
-                q[(size_t)s * qstride + a] = tot > 0 ? (float)(cnt[a] / tot) : (float)(1.0 / (qstride - 1));
+            CASPHY_CUDA_TRY(up(L.q, q.data(), 4 * q.size()));
         }
-        CASPHY_CUDA_TRY(up(L.q, q.data(), 4 * q.size()));
     }
     F.T = Tree{ntip, L.kidA, L.kidB, L.edgeA, L.edgeB, L.inO, L.outO, L.inInfo, L.inEB, L.outInfo, L.outEB};
     F.t = L.t;
@@ -1225,10 +1290,12 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
     F.p = L.p;
     F.lb = Lb{nedge, nCTA, Mr, L.x, L.g, L.d, L.xn, L.t, L.grad, L.S, L.Y, L.rho, L.gam, L.sc, L.lpart,
               L.flags, L.err, 5ull * 1000 * 1000 * 1000, 1e-8, 10.0};
-    rc = F.capture();
-    if (rc) return rc;
     // host staging buffers (wv, q) must outlive the copies
     CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+    if (bad) {
+        casphy_set_last_error_msg("felsenstein: tip code beyond nallele + 1");
+        return CASPHY_ERANGE;
+    }
     return CASPHY_OK;
 }
 
@@ -1292,12 +1359,10 @@ extern "C" int casphy_felsenstein_loglik(uint32_t ntip, uint32_t nedge, const ui
     FelProblem F;
     rc = setup_problem(F, ds, ntip, nedge, edge, brlen, nsite, tip_codes, site_weights, model, 0);
     if (rc) return rc;
-    rc = F.eval(grad != nullptr, loglik);
+    rc = F.eval_once(grad != nullptr, loglik);
     if (rc) return rc;
-    if (grad) {
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(grad, F.grad, sizeof(double) * nedge, cudaMemcpyDeviceToHost, F.st));
-        CASPHY_CUDA_TRY(cudaStreamSynchronize(F.st));
-    }
+    if (grad) CASPHY_CUDA_TRY(cudaMemcpyAsync(grad, F.grad, sizeof(double) * nedge, cudaMemcpyDeviceToHost, F.st));
+    CASPHY_CUDA_TRY(cudaStreamSynchronize(F.st));
     return CASPHY_OK;
 }
 
