@@ -46,6 +46,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "runtime.h"
 
@@ -270,6 +271,29 @@ __global__ void __launch_bounds__(kSites) k_loglik_hky(u32 root, Tree T, HkyBuf 
     if (threadIdx.x == 0) part[C.blk0 + blockIdx.x] = v;
 }
 
+// One (node, site) of the outside pass: both children's site terms in gs and
+// their outside vectors stored.  M: P - I of both child edges, then their dP.
+__device__ __forceinline__ void outside_hky_site(const Tree& T, const HkyBuf& B, const Chunk& C, const float* M, u32 ca,
+                                                 u32 cb, u32 s, bool ok, float4 u, float4 la, float4 lb, float ws,
+                                                 float (&gs)[2]) {
+    const float4 ma = pmatvec(M, la), mb = pmatvec(M + 16, lb);
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+        const u32 c = side ? cb : ca;
+        const float4 msib = side ? ma : mb;
+        const float4 lc = side ? lb : la;
+        const float4 mc = side ? mb : ma;
+        const float4 r = make_float4(u.x * msib.x, u.y * msib.y, u.z * msib.z, u.w * msib.w);
+        const float4 dm = matvec(M + 32 + 16 * side, lc);
+        gs[side] = ok ? ws * (dot4(r, dm) / dot4(r, mc)) : 0.f;
+        if (ok && c >= T.ntip) {
+            float4 uc = pvecmat(r, M + 16 * side);
+            renorm4(uc);
+            B.U[(size_t)(c - T.ntip) * C.W + s] = uc;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kSites / 2, 10) k_outside_hky(u32 root, Tree T, HkyBuf B, Chunk C, u32 off, Hky m,
                                                         const double* __restrict__ w, double* gpart) {
     pdl_wait();
@@ -300,34 +324,17 @@ __global__ void __launch_bounds__(kSites / 2, 10) k_outside_hky(u32 root, Tree T
         lb[j] = child_hky(T, B, C, cb, ssj[j], &e);
     }
     __syncthreads();
-    float gs[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [side][j]
+    float gs[2][2];  // [j][side]
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        const float4 ma = pmatvec(sm, la[j]), mb = pmatvec(sm + 16, lb[j]);
-        const float ws = okj[j] ? (float)w[C.s0 + sj[j]] : 0.f;
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-            const u32 c = side ? cb : ca;
-            const float4 msib = side ? ma : mb;
-            const float4 lc = side ? lb[j] : la[j];
-            const float4 mc = side ? mb : ma;
-            const float4 r = make_float4(u[j].x * msib.x, u[j].y * msib.y, u[j].z * msib.z, u[j].w * msib.w);
-            const float4 dm = matvec(sm + 32 + 16 * side, lc);
-            gs[side][j] = okj[j] ? ws * (dot4(r, dm) / dot4(r, mc)) : 0.f;
-            if (okj[j] && c >= T.ntip) {
-                float4 uc = pvecmat(r, sm + 16 * side);
-                renorm4(uc);
-                B.U[(size_t)(c - T.ntip) * C.W + sj[j]] = uc;
-            }
-        }
-    }
+    for (int j = 0; j < 2; j++)
+        outside_hky_site(T, B, C, sm, ca, cb, sj[j], okj[j], u[j], la[j], lb[j], okj[j] ? (float)w[C.s0 + sj[j]] : 0.f, gs[j]);
     // site terms in binary32 within the block, grouped as 32-site warps in
     // site order (warp w of half j holds sites 128 j + 32 w ..); blocks are
     // added in binary64
     __shared__ float2 red8[kSites / 32];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-        float a = gs[0][j], b = gs[1][j];
+        float a = gs[j][0], b = gs[j][1];
         for (int o = 16; o > 0; o >>= 1) {
             a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
             b += __shfl_xor_sync(0xFFFFFFFFu, b, o);
@@ -507,13 +514,10 @@ __global__ void __launch_bounds__(kSites) k_loglik_irr(u32 root, Tree T, IrrBuf 
     if (threadIdx.x == 0) part[C.blk0 + blockIdx.x] = v;
 }
 
-__global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf B, Chunk C, u32 off,
-                                                        const double* __restrict__ w, double* gpart) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ float2 red[kSites / 32];
-    const u32 s = blockIdx.x * kSites + threadIdx.x;
-    const uint4 nf = T.outInfo[off + blockIdx.y];
+// One (node, site) of the outside pass: both children's site terms in gsum and
+// their outside vectors stored.
+__device__ __forceinline__ void outside_irr_site(u32 root, const Tree& T, const IrrBuf& B, const Chunk& C, uint4 nf,
+                                                 u32 edB, u32 s, const double* __restrict__ w, float (&gsum)[2]) {
     const u32 v = nf.x, vi = v - T.ntip;
     const bool ok = s < C.w;
     const u32 ss = ok ? s : 0, gs = C.s0 + ss;
@@ -527,7 +531,7 @@ __global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf
         aY = __float_as_int(u.w);
     }
     const u32 kids[2] = {nf.y, nf.z};
-    const u32 eds[2] = {nf.w, T.outEdgeB[off + blockIdx.y]};
+    const u32 eds[2] = {nf.w, edB};
     float4 l[2];
     float m0[2], qs[2];
     float2 pp[2];
@@ -539,7 +543,6 @@ __global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf
         m0[i] = l[i].x + pp[i].y * (qs[i] - l[i].x);
     }
     const float ws = ok ? (float)w[gs] : 0.f;
-    float gsum[2];
 #pragma unroll
     for (int c = 0; c < 2; c++) {
         const int sb = 1 - c;
@@ -582,12 +585,132 @@ __global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf
             B.U[(size_t)(kids[c] - T.ntip) * C.W + s] = make_float4(u0, x, y, __int_as_float(aR));
         }
     }
+}
+
+__global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf B, Chunk C, u32 off,
+                                                        const double* __restrict__ w, double* gpart) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float2 red[kSites / 32];
+    const u32 s = blockIdx.x * kSites + threadIdx.x;
+    const uint4 nf = T.outInfo[off + blockIdx.y];
+    const u32 eds[2] = {nf.w, T.outEdgeB[off + blockIdx.y]};
+    float gsum[2];
+    outside_irr_site(root, T, B, C, nf, eds[1], s, w, gsum);
     // site terms in binary32 within the block; blocks are added in binary64
     const float2 g = block_sum2f(gsum[0], gsum[1], red);
     if (threadIdx.x == 0) {
         gpart[(size_t)eds[0] * C.nblkTot + C.blk0 + blockIdx.x] = g.x;
         gpart[(size_t)eds[1] * C.nblkTot + C.blk0 + blockIdx.x] = g.y;
     }
+}
+
+// ------------------------------------------------------- narrow levels ---
+// The levels near the root have few nodes, and a launch each costs more than
+// their work (about 4 us against 1 us).  Sites are independent, so one CTA
+// takes 32 sites through all narrow levels, a warp per node, with a block
+// barrier between levels; what it reads of a level's nodes was written by
+// itself (or, for the first level, by the launches before).  The arithmetic per
+// (node, site) is the wide kernels'.  The gradient's site terms are summed over
+// 32 sites here, as in a warp of the wide kernels, and k_sum_grad adds the eight
+// sums of a 256-site block in the same order, so every bit is the same.
+constexpr u32 kNarrow = 64;      // nodes of a narrow level, at most
+constexpr u32 kTopWarps = 16;
+constexpr u32 kMaxTop = 128;     // narrow levels of one launch
+
+struct TopLevels {
+    u32 n;
+    u32 off[kMaxTop + 1];
+};
+
+template <class Buf, class F>
+__device__ __forceinline__ void walk_levels(const TopLevels& lv, F node) {
+    for (u32 l = 0; l < lv.n; l++) {
+        for (u32 i = lv.off[l] + (threadIdx.x >> 5); i < lv.off[l + 1]; i += kTopWarps) node(i);
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(32 * kTopWarps) k_inside_top_hky(Tree T, HkyBuf B, Chunk C, TopLevels lv) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 s = blockIdx.x * 32 + (threadIdx.x & 31), ss = s < C.w ? s : 0u;
+    walk_levels<HkyBuf>(lv, [&](u32 i) {
+        const uint4 nf = T.inInfo[i];
+        int ea, eb;
+        const float4 la = child_hky(T, B, C, nf.y, ss, &ea), lb = child_hky(T, B, C, nf.z, ss, &eb);
+        if (s < C.w) inside_hky_site(B, C, nf.x - T.ntip, nf.w, T.inEdgeB[i], s, la, ea, lb, eb);
+    });
+}
+
+__global__ void __launch_bounds__(32 * kTopWarps) k_inside_top_irr(Tree T, IrrBuf B, Chunk C, TopLevels lv) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 s = blockIdx.x * 32 + (threadIdx.x & 31), ss = s < C.w ? s : 0u;
+    walk_levels<IrrBuf>(lv, [&](u32 i) {
+        const uint4 nf = T.inInfo[i];
+        const float2 pa = B.p[nf.w], pb = B.p[T.inEdgeB[i]];
+        const float4 la = child_irr(T, B, C, nf.y, ss), lb = child_irr(T, B, C, nf.z, ss);
+        if (s < C.w) inside_irr_site(B, C, nf.x - T.ntip, pa, pb, s, la, lb);
+    });
+}
+
+// Sum over the warp's 32 sites, as the wide kernels' first step.
+__device__ __forceinline__ void warp_terms(float (&g)[2], const Chunk& C, u32 eA, u32 eB, u32 nsite32,
+                                           float* __restrict__ gw) {
+    float a = g[0], b = g[1];
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+        b += __shfl_xor_sync(0xFFFFFFFFu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        gw[(size_t)eA * nsite32 + C.s0 / 32 + blockIdx.x] = a;
+        gw[(size_t)eB * nsite32 + C.s0 / 32 + blockIdx.x] = b;
+    }
+}
+
+__global__ void __launch_bounds__(32 * kTopWarps) k_outside_top_hky(u32 root, Tree T, HkyBuf B, Chunk C, TopLevels lv,
+                                                                    Hky m, const double* __restrict__ w, u32 nsite32,
+                                                                    float* __restrict__ gw) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float sm[kTopWarps][64];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u32 s = blockIdx.x * 32 + lane, ss = s < C.w ? s : 0u;
+    const bool ok = s < C.w;
+    const float ws = ok ? (float)w[C.s0 + s] : 0.f;
+    walk_levels<HkyBuf>(lv, [&](u32 i) {
+        const uint4 nf = T.outInfo[i];
+        const u32 eA = nf.w, eB = T.outEdgeB[i];
+        float* M = sm[warp];
+        __syncwarp();
+        M[lane] = __ldg(B.P + 16 * (lane < 16 ? eA : eB) + (lane & 15));
+        M[32 + lane] = __ldg(B.dP + 16 * (lane < 16 ? eA : eB) + (lane & 15));
+        __syncwarp();
+        float4 u;
+        if (nf.x == root) u = make_float4((float)m.pi[0], (float)m.pi[1], (float)m.pi[2], (float)m.pi[3]);
+        else u = B.U[(size_t)(nf.x - T.ntip) * C.W + ss];
+        int e;
+        const float4 la = child_hky(T, B, C, nf.y, ss, &e), lb = child_hky(T, B, C, nf.z, ss, &e);
+        float g[2];
+        outside_hky_site(T, B, C, M, nf.y, nf.z, s, ok, u, la, lb, ws, g);
+        warp_terms(g, C, eA, eB, nsite32, gw);
+    });
+}
+
+__global__ void __launch_bounds__(32 * kTopWarps) k_outside_top_irr(u32 root, Tree T, IrrBuf B, Chunk C, TopLevels lv,
+                                                                    const double* __restrict__ w, u32 nsite32,
+                                                                    float* __restrict__ gw) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 s = blockIdx.x * 32 + (threadIdx.x & 31);
+    walk_levels<IrrBuf>(lv, [&](u32 i) {
+        const uint4 nf = T.outInfo[i];
+        const u32 eB = T.outEdgeB[i];
+        float g[2];
+        outside_irr_site(root, T, B, C, nf, eB, s, w, g);
+        warp_terms(g, C, nf.w, eB, nsite32, gw);
+    });
 }
 
 // ------------------------------------------------ fixed-order reductions ---
@@ -605,13 +728,25 @@ __global__ void k_sum_ll(const double* __restrict__ part, u32 n, double* out) {
     if (threadIdx.x == 0) *out = v;
 }
 
-__global__ void k_sum_grad(const double* __restrict__ gpart, u32 nedge, u32 nblk, double* __restrict__ grad) {
+// Edges of narrow levels (top) have a sum per 32 sites, the others per 256.
+__global__ void k_sum_grad(const double* __restrict__ gpart, const float* __restrict__ gw,
+                           const unsigned char* __restrict__ top, u32 nedge, u32 nblk, u32 nsite32,
+                           double* __restrict__ grad) {
     pdl_wait();
     pdl_trigger();
     const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nedge) return;
     double v = 0;
-    for (u32 b = 0; b < nblk; b++) v += gpart[(size_t)e * nblk + b];
+    if (top[e]) {
+        const float* g = gw + (size_t)e * nsite32;
+        for (u32 b = 0; b < nblk; b++) {
+            float t = 0.f;
+            for (u32 i = 8 * b; i < min(8 * b + 8, nsite32); i++) t += g[i];
+            v += (double)t;
+        }
+    } else {
+        for (u32 b = 0; b < nblk; b++) v += gpart[(size_t)e * nblk + b];
+    }
     grad[e] = v;
 }
 
@@ -748,6 +883,195 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_accept(Lb a, u32 slot) {
     }
 }
 
+// The same steps on one cluster of kLbCluster CTAs, for problems of at most one
+// element a thread of the grid kernels (n <= 512 nCTA): the direction alone, or
+// an accept, the direction and the trial point in one launch.  The grid kernels
+// spend their time in reductions behind a flag barrier of all SMs, 17 of about
+// 6 us a step, for vectors of a few KB; a cluster exchanges the partial sums
+// through distributed shared memory in under 1 us.  The sums keep the grid
+// kernels' grouping (CTA r sums the 512-element blocks r, r + 16, ... that
+// their CTAs would, and the blocks are added in order), so every bit is the
+// same.  V: blocks per CTA.
+constexpr u32 kLbCluster = 16;
+constexpr u32 kLbMaxBlocks = 160;
+enum { LB_ACCEPT = 1, LB_DIR = 2, LB_TRIAL = 4 };
+
+struct LbExchange {
+    u32 rank, nv, epoch, bar;
+    double* part;  // 2 x kLbMaxBlocks x 3
+    double (*red)[3][kLbThreads / 32];
+};
+
+// K sums (the last of them a maximum when MAX), in all threads of all CTAs.
+template <int V, int K, bool MAX>
+__device__ __forceinline__ void cluster_reduce(const Lb& a, LbExchange& x, const double (&v)[V][K], double (&out)[K]) {
+    const u32 tid = threadIdx.x, buf = x.epoch & 1u, bar = x.bar + 8 * buf;
+    if (tid == 0) clu::mbar_expect(bar, x.nv * K * 8u);
+#pragma unroll
+    for (int j = 0; j < V; j++)
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            double s = v[j][k];
+            for (int o = 16; o > 0; o >>= 1) {
+                const double y = __shfl_xor_sync(0xFFFFFFFFu, s, o);
+                s = MAX && k == K - 1 ? fmax(s, y) : s + y;
+            }
+            if ((tid & 31) == 0) x.red[j][k][tid >> 5] = s;
+        }
+    __syncthreads();
+    if (tid < V * K) {
+        const u32 j = tid / K, k = tid % K, b = x.rank + kLbCluster * j;
+        if (b < x.nv) {
+            double s = 0.0;
+            for (u32 i = 0; i < kLbThreads / 32; i++)
+                s = MAX && k == K - 1 ? fmax(s, x.red[j][k][i]) : s + x.red[j][k][i];
+            const u32 to = clu::smem_u32(x.part + (buf * kLbMaxBlocks + b) * 3 + k);
+            for (u32 r = 0; r < kLbCluster; r++)
+                clu::st_async8(clu::mapa(to, r), (u64)__double_as_longlong(s), clu::mapa(bar, r));
+        }
+    }
+    clu::mbar_wait(bar, (x.epoch >> 1) & 1u, a.err, a.limitNs);  // on failure the host drops the step
+#pragma unroll
+    for (int k = 0; k < K; k++) out[k] = 0.0;
+    for (u32 b = 0; b < x.nv; b++)
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const double y = x.part[(buf * kLbMaxBlocks + b) * 3 + k];
+            out[k] = MAX && k == K - 1 ? fmax(out[k], y) : out[k] + y;
+        }
+    x.epoch++;
+}
+
+template <int V>
+__global__ void __launch_bounds__(kLbThreads) k_lb_cluster(Lb a, u32 what, u32 slot, u32 first, u32 count, double step) {
+    __shared__ double part[2 * kLbMaxBlocks * 3];
+    __shared__ double red[V][3][kLbThreads / 32];
+    __shared__ __align__(8) u64 bars[2];
+    __shared__ double alpha[kMaxHist];
+    LbExchange x{clu::cluster_rank(), (a.n + kLbThreads - 1) / kLbThreads, 0u, clu::smem_u32(&bars[0]), part, red};
+    if (threadIdx.x == 0) {
+        clu::mbar_init(x.bar);
+        clu::mbar_init(x.bar + 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    clu::cluster_sync();
+    u32 at[V];
+    bool ok[V];
+    double g[V], d[V];
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+        at[j] = (x.rank + kLbCluster * j) * kLbThreads + threadIdx.x;
+        ok[j] = at[j] < a.n;
+        if (!ok[j]) at[j] = 0u;
+        g[j] = ok[j] ? a.g[at[j]] : 0.0;
+        d[j] = 0.0;
+    }
+    const bool writer = x.rank == 0 && threadIdx.x == 0;
+    double rhoNew = 0.0, gamNew = 1.0;
+    if (what & LB_ACCEPT) {
+        double v[V][3], o[3];
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            v[j][0] = v[j][1] = v[j][2] = 0.0;
+            if (!ok[j]) continue;
+            const u32 i = at[j];
+            const double gn = -a.grad[i] * a.t[i];
+            const double s = a.xn[i] - a.x[i], y = gn - g[j];
+            a.S[(size_t)slot * a.n + i] = s;
+            a.Y[(size_t)slot * a.n + i] = y;
+            v[j][0] += s * y;
+            v[j][1] += y * y;
+            v[j][2] += gn * gn;
+            a.x[i] = a.xn[i];
+            a.g[i] = gn;
+            g[j] = gn;
+        }
+        cluster_reduce<V, 3, false>(a, x, v, o);
+        rhoNew = o[0] != 0.0 ? 1.0 / o[0] : 0.0;
+        gamNew = o[1] > 0.0 ? o[0] / o[1] : 1.0;
+        if (writer) {
+            a.sc[SC_SY] = o[0];
+            a.sc[SC_YY] = o[1];
+            a.sc[SC_GG] = o[2];
+            a.rho[slot] = rhoNew;
+            a.gam[slot] = gamNew;
+        }
+    }
+    if (what & LB_DIR) {
+        const bool fresh = (what & LB_ACCEPT) != 0;  // rho and gamma of `slot` are this launch's
+#pragma unroll
+        for (int j = 0; j < V; j++) d[j] = g[j];
+        double v[V][1], o[1];
+        for (int k = (int)count - 1; k >= 0; k--) {
+            const u32 r = (first + (u32)k) % a.Mr;
+            const double* s = a.S + (size_t)r * a.n;
+            const double* y = a.Y + (size_t)r * a.n;
+            double yv[V];
+#pragma unroll
+            for (int j = 0; j < V; j++) {
+                v[j][0] = 0.0;
+                yv[j] = ok[j] ? y[at[j]] : 0.0;
+                if (ok[j]) v[j][0] += s[at[j]] * d[j];
+            }
+            cluster_reduce<V, 1, false>(a, x, v, o);
+            const double al = (fresh && r == slot ? rhoNew : a.rho[r]) * o[0];
+            if (threadIdx.x == 0) alpha[k] = al;
+#pragma unroll
+            for (int j = 0; j < V; j++) d[j] -= al * yv[j];
+        }
+        __syncthreads();
+        if (count > 0) {
+            const u32 r = (first + count - 1) % a.Mr;
+            const double gm = fresh && r == slot ? gamNew : a.gam[r];
+#pragma unroll
+            for (int j = 0; j < V; j++) d[j] *= gm;
+        }
+        for (u32 k = 0; k < count; k++) {
+            const u32 r = (first + k) % a.Mr;
+            const double* s = a.S + (size_t)r * a.n;
+            const double* y = a.Y + (size_t)r * a.n;
+            double sv[V];
+#pragma unroll
+            for (int j = 0; j < V; j++) {
+                v[j][0] = 0.0;
+                sv[j] = ok[j] ? s[at[j]] : 0.0;
+                if (ok[j]) v[j][0] += y[at[j]] * d[j];
+            }
+            cluster_reduce<V, 1, false>(a, x, v, o);
+            const double c = alpha[k] - (fresh && r == slot ? rhoNew : a.rho[r]) * o[0];
+#pragma unroll
+            for (int j = 0; j < V; j++) d[j] += c * sv[j];
+        }
+        double w[V][2], o2[2];
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            w[j][0] = w[j][1] = 0.0;
+            d[j] = -d[j];
+            if (!ok[j]) continue;
+            a.d[at[j]] = d[j];
+            w[j][0] += g[j] * d[j];
+            w[j][1] = fmax(w[j][1], fabs(d[j]));
+        }
+        cluster_reduce<V, 2, true>(a, x, w, o2);
+        if (writer) {
+            a.sc[SC_GD] = o2[0];
+            a.sc[SC_DMAX] = o2[1];
+        }
+    }
+    if (what & LB_TRIAL) {
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            if (!ok[j]) continue;
+            const u32 i = at[j];
+            const double xn = a.x[i] + step * d[j];
+            a.xn[i] = xn;
+            a.t[i] = fmin(fmax(exp(xn), a.tmin), a.tmax);
+        }
+    }
+    clu::cluster_sync();  // no CTA leaves while another's sums are under way to it
+}
+
 __global__ void k_lb_trial(Lb a, double step) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
@@ -780,6 +1104,10 @@ struct FelTreeHost {
     u32 ntip = 0, nn = 0, nint = 0, nedge = 0, root = 0;
     std::vector<u32> kidA, kidB, edgeA, edgeB, inOrder, outOrder;
     std::vector<u32> inOff, outOff;  // level offsets
+    // narrow levels, walked in one launch: inside levels from inTop on, outside
+    // levels before outTop
+    u32 inTop = 0, outTop = 0;
+    std::vector<unsigned char> topEdge;  // edges whose gradient those levels form
 };
 
 static int build_tree(u32 ntip, u32 nedge, const u32* edge, FelTreeHost& T) {
@@ -874,6 +1202,15 @@ static int build_tree(u32 ntip, u32 nedge, const u32* edge, FelTreeHost& T) {
         T.outOrder.insert(T.outOrder.end(), byD[d].begin(), byD[d].end());
         T.outOff.push_back((u32)T.outOrder.size());
     }
+    const u32 nin = (u32)T.inOff.size() - 1, nout = (u32)T.outOff.size() - 1;
+    T.inTop = nin;
+    while (T.inTop > 0 && nin - T.inTop < kMaxTop && T.inOff[T.inTop] - T.inOff[T.inTop - 1] <= kNarrow) T.inTop--;
+    while (T.outTop < nout && T.outTop < kMaxTop && T.outOff[T.outTop + 1] - T.outOff[T.outTop] <= kNarrow) T.outTop++;
+    T.topEdge.assign(nedge, 0);
+    for (u32 i = 0; i < T.outOff[T.outTop]; i++) {
+        const u32 v = T.outOrder[i] - ntip;
+        T.topEdge[T.edgeA[v]] = T.topEdge[T.edgeB[v]] = 1;
+    }
     return CASPHY_OK;
 }
 
@@ -948,11 +1285,14 @@ struct FelProblem {
     Hky hky{};
     double rate = 1.0;
     double *t = nullptr, *w = nullptr, *grad = nullptr, *gpart = nullptr, *part = nullptr, *ll = nullptr;
+    float* gw = nullptr;  // narrow levels' gradient terms, per edge and 32 sites
+    const unsigned char* top = nullptr;
     HkyBuf hb{};
     IrrBuf ib{};
     float *P = nullptr, *dP = nullptr;
     float2* p = nullptr;
     Lb lb{};
+    int lbCluster = -1;  // whether the L-BFGS steps run on a cluster (-1: not asked yet)
     cudaGraphExec_t gFull = nullptr, gLL = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1004,17 +1344,36 @@ struct FelProblem {
             C.blk0 = C.s0 / kSites;
             C.nblkTot = nblkTot;
             const u32 nb = (C.w + kSites - 1) / kSites;
-            for (size_t lv = 0; lv + 1 < th.inOff.size(); lv++) {
+            const u32 nb32 = (C.w + 31) / 32, nsite32 = (nsite + 31) / 32;
+            for (size_t lv = 0; lv < th.inTop; lv++) {
                 const dim3 grid(nb, th.inOff[lv + 1] - th.inOff[lv]);
                 if (model == CASPHY_MODEL_HKY85) lp(k_inside_hky, grid, kSites / 2, T, hb, C, th.inOff[lv]);
                 else lp(k_inside_irr, grid, kSites / 2, T, ib, C, th.inOff[lv]);
+                n++;
+            }
+            if (th.inTop + 1 < th.inOff.size()) {
+                TopLevels lv;
+                lv.n = (u32)th.inOff.size() - 1 - th.inTop;
+                for (u32 l = 0; l <= lv.n; l++) lv.off[l] = th.inOff[th.inTop + l];
+                if (model == CASPHY_MODEL_HKY85) lp(k_inside_top_hky, dim3(nb32), 32 * kTopWarps, T, hb, C, lv);
+                else lp(k_inside_top_irr, dim3(nb32), 32 * kTopWarps, T, ib, C, lv);
                 n++;
             }
             if (model == CASPHY_MODEL_HKY85) lp(k_loglik_hky, dim3(nb), kSites, th.root, T, hb, C, hky, (const double*)w, part);
             else lp(k_loglik_irr, dim3(nb), kSites, th.root, T, ib, C, (const double*)w, part);
             n++;
             if (!withGrad) continue;
-            for (size_t lv = 0; lv + 1 < th.outOff.size(); lv++) {
+            if (th.outTop > 0) {
+                TopLevels lv;
+                lv.n = th.outTop;
+                for (u32 l = 0; l <= lv.n; l++) lv.off[l] = th.outOff[l];
+                if (model == CASPHY_MODEL_HKY85)
+                    lp(k_outside_top_hky, dim3(nb32), 32 * kTopWarps, th.root, T, hb, C, lv, hky, (const double*)w, nsite32,
+                       gw);
+                else lp(k_outside_top_irr, dim3(nb32), 32 * kTopWarps, th.root, T, ib, C, lv, (const double*)w, nsite32, gw);
+                n++;
+            }
+            for (size_t lv = th.outTop; lv + 1 < th.outOff.size(); lv++) {
                 const dim3 grid(nb, th.outOff[lv + 1] - th.outOff[lv]);
                 if (model == CASPHY_MODEL_HKY85)
                     lp(k_outside_hky, grid, kSites / 2, th.root, T, hb, C, th.outOff[lv], hky, (const double*)w, gpart);
@@ -1025,7 +1384,8 @@ struct FelProblem {
         lp(k_sum_ll, dim3(1), 256, (const double*)part, nblkTot, ll);
         n++;
         if (withGrad) {
-            lp(k_sum_grad, dim3((ne + 255) / 256), 256, (const double*)gpart, ne, nblkTot, grad);
+            lp(k_sum_grad, dim3((ne + 255) / 256), 256, (const double*)gpart, (const float*)gw, top, ne, nblkTot,
+               (nsite + 31) / 32, grad);
             n++;
         }
         if (launches) *launches = n;
@@ -1154,6 +1514,8 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         double *t, *w, *grad, *gpart, *part, *ll;
         u32* alleleCount;
         int* badCode;
+        float* gw;
+        unsigned char* top;
         double *x, *g, *d, *xn, *S, *Y, *rho, *gam, *sc, *lpart;
         float *P, *dP, *q;
         float2* p;
@@ -1199,6 +1561,8 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         b.q = c.take<float>(isH ? 0 : (size_t)nsite * qstride);
         b.alleleCount = c.take<u32>(isH || model->allele_freq ? 0 : (size_t)nsite * qstride);
         b.badCode = c.take<int>(1);
+        b.gw = c.take<float>((size_t)nedge * ((nsite + 31) / 32));
+        b.top = c.take<unsigned char>(nedge);
         b.L = c.take<float4>((size_t)nint * F.W);
         b.U = c.take<float4>((size_t)nint * F.W);
         b.E = c.take<int>(isH ? (size_t)nint * F.W : 0);
@@ -1240,6 +1604,7 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
     CASPHY_CUDA_TRY(up(L.outInfo, outInfo.data(), sizeof(uint4) * nint));
     CASPHY_CUDA_TRY(up(L.inEB, inEB.data(), 4ull * nint));
     CASPHY_CUDA_TRY(up(L.outEB, outEB.data(), 4ull * nint));
+    CASPHY_CUDA_TRY(up(L.top, F.th.topEdge.data(), nedge));
     CASPHY_CUDA_TRY(up(L.codes, codes, 4ull * ntip * nsite));
     CASPHY_CUDA_TRY(up(L.t, brlen, 8ull * nedge));
     std::vector<double> wv(nsite, 1.0);
@@ -1283,6 +1648,8 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
     F.gpart = L.gpart;
     F.part = L.part;
     F.ll = L.ll;
+    F.gw = L.gw;
+    F.top = L.top;
     F.hb = HkyBuf{L.codes, L.L, L.E, L.U, L.P, L.dP};
     F.ib = IrrBuf{L.codes, L.L, L.U, L.p, L.q, qstride, (float)model->rate};
     F.P = L.P;
@@ -1302,6 +1669,36 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
 static int lb_coop(FelProblem& F, const void* fn, void** args) {
     CASPHY_CUDA_TRY(cudaMemsetAsync(F.lb.flags, 0, sizeof(u32) * 16 * F.lb.nCTA, F.st));
     CASPHY_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(F.lb.nCTA), dim3(kLbThreads), args, 0, F.st));
+    return CASPHY_OK;
+}
+
+// The accept (into ring slot `slot`), the direction over `count` pairs from
+// `first` and the trial point at `step`, as `what` asks: one cluster launch
+// where the problem fits it, else the grid kernels.
+static int lb_step(FelProblem& F, u32 what, u32 slot, u32 first, u32 count, double step) {
+    Lb& a = F.lb;
+    const u32 V = (a.n + kLbThreads * kLbCluster - 1) / (kLbThreads * kLbCluster);
+    if (F.lbCluster < 0) {
+        const bool fits = a.n <= a.nCTA * kLbThreads && a.nCTA <= kLbMaxBlocks && V <= 10;
+        const void* fn = V <= 1 ? (const void*)k_lb_cluster<1> : V <= 2 ? (const void*)k_lb_cluster<2>
+                         : V <= 5 ? (const void*)k_lb_cluster<5> : (const void*)k_lb_cluster<10>;
+        F.lbCluster = fits && clu::placeable(const_cast<void*>(fn), kLbCluster, 0) > 0 ? 1 : 0;
+    }
+    if (F.lbCluster) {
+        auto run = [&](auto fn) { return clu::enqueue(fn, kLbCluster, 1, 0, F.st, a, what, slot, first, count, step); };
+        CASPHY_CUDA_TRY(V <= 1 ? run(k_lb_cluster<1>) : V <= 2 ? run(k_lb_cluster<2>) : V <= 5 ? run(k_lb_cluster<5>)
+                                                                                      : run(k_lb_cluster<10>));
+        return CASPHY_OK;
+    }
+    if (what & LB_ACCEPT) {
+        void* args[] = {&a, &slot};
+        if (int rc = lb_coop(F, (const void*)k_lb_accept, args)) return rc;
+    }
+    if (what & LB_DIR) {
+        void* args[] = {&a, &first, &count};
+        if (int rc = lb_coop(F, (const void*)k_lb_dir, args)) return rc;
+    }
+    if (what & LB_TRIAL) k_lb_trial<<<(a.n + 255) / 256, 256, 0, F.st>>>(a, step);
     return CASPHY_OK;
 }
 
@@ -1412,8 +1809,7 @@ extern "C" int casphy_felsenstein_optimize(uint32_t ntip, uint32_t nedge, const 
             u32 cnt = count;
             double sc[2] = {0, 0};
             for (int attempt = 0; attempt < 2; attempt++) {
-                void* args[] = {&a, &first, &cnt};
-                if ((rc = lb_coop(F, (const void*)k_lb_dir, args))) return rc;
+                if ((rc = lb_step(F, LB_DIR, 0, first, cnt, 0.0))) return rc;
                 if ((rc = lb_read(F, a.sc + SC_GD, sc, 2))) return rc;
                 if (sc[0] < 0 || cnt == 0) break;
                 cnt = 0;  // not a descent direction: restart from steepest descent
@@ -1454,14 +1850,10 @@ extern "C" int casphy_felsenstein_optimize(uint32_t ntip, uint32_t nedge, const 
         const double rel = std::fabs(f - fn) / std::max(std::fabs(f), 1e-300);
         const u32 quietNext = rel <= rel_tol ? quiet + 1 : 0;
         u32 slot = (first + count) % a.Mr;
-        void* args[] = {&a, &slot};
-        if ((rc = lb_coop(F, (const void*)k_lb_accept, args))) return rc;
         double sy = 0;
         if (adj && quietNext < kQuiet && it + 1 < max_iter) {
             u32 cntN = count < M ? count + 1 : count, firstN = count < M ? first : (first + 1) % a.Mr;
-            void* dargs[] = {&a, &firstN, &cntN};
-            if ((rc = lb_coop(F, (const void*)k_lb_dir, dargs))) return rc;
-            k_lb_trial<<<nb, 256, 0, F.st>>>(a, 1.0);
+            if ((rc = lb_step(F, LB_ACCEPT | LB_DIR | LB_TRIAL, slot, firstN, cntN, 1.0))) return rc;
             if ((rc = F.eval_launch(adj, &specLl))) return rc;
             double sc3[3] = {0, 0, 0};  // g.d, max|d| of the direction; s.y of the accept
             if ((rc = lb_read(F, a.sc + SC_GD, sc3, 3))) return rc;
@@ -1472,6 +1864,7 @@ extern "C" int casphy_felsenstein_optimize(uint32_t ntip, uint32_t nedge, const 
             specDmax = sc3[SC_DMAX - SC_GD];
             spec = sy > 1e-12 && specGd < 0;
         } else {
+            if ((rc = lb_step(F, LB_ACCEPT, slot, 0, 0, 0.0))) return rc;
             if ((rc = lb_read(F, a.sc + SC_SY, &sy, 1))) return rc;
         }
         st.iterations++;

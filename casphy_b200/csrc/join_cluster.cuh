@@ -27,16 +27,17 @@
 // fenced before its records are sent, so a CTA that has received them reads
 // the row from L2.
 #pragma once
+#include "cluster.cuh"
 #include "join_engine.cuh"
 
 namespace casphy {
 namespace joinc {
 
+using namespace clu;
 using joinx::kDead;
 using joinx::kMaxBatch;
-constexpr int kThreads = 512, kWarps = 16;
+constexpr int kThreads = clu::kThreads, kWarps = kThreads / 32;
 constexpr u32 kLists = 4;    // records a CTA publishes per exchange, one per four warps
-constexpr u32 kMaxG = 16;
 constexpr u32 kJoin = 0, kStale = 1;
 
 // One published record: larger ord, then larger inv (smaller node) is better;
@@ -74,45 +75,6 @@ __host__ __device__ inline size_t engine_smem(u32 G, u32 R, u32 deathWords) {
 
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ u32 smem_u32(const void* p) { return static_cast<u32>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ u32 mapa(u32 a, u32 rank) {
-    u32 r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_async16(u32 addr, const Rec& r, u32 bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
-                 "r"(r.ord), "r"(r.inv), "r"(r.slot), "r"(r.partner), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void st_async8(u32 addr, u64 v, u32 bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_init(u32 bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(u32 bar, u32 bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(u32 bar, u32 parity) {
-    u32 ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0u;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ u32 cluster_rank() {
-    u32 r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // The maximum of the warp's (hi, lo) keys, in every lane.
 __device__ __forceinline__ void warp_max2(u32& hi, u32& lo) {
     const u32 h = __reduce_max_sync(0xFFFFFFFFu, hi);
@@ -198,7 +160,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             if (G == 1) {
                 if (lane == 0) *dst = r;
             } else if (lane < G) {
-                st_async16(mapa(smem_u32(dst), lane), r, mapa(bar0 + 8 * buf, lane));
+                st_async16(mapa(smem_u32(dst), lane), make_uint4(r.ord, r.inv, r.slot, r.partner), mapa(bar0 + 8 * buf, lane));
             }
         }
     };
@@ -226,18 +188,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             // the exchange's records, from every CTA
             u32 bad = 0;
             if (G > 1) {
-                const u32 bar = bar0 + 8 * buf, parity = (p >> 1) & 1u;
-                if (!mbar_try(bar, parity)) {
-                    const u64 t0 = globaltimer_ns();
-                    while (!mbar_try(bar, parity)) {
-                        if (*(volatile int*)a.err) { bad = 1; break; }
-                        if (globaltimer_ns() - t0 > a.limitNs) {
-                            atomicCAS(a.err, 0, CASPHY_ETIMEOUT);
-                            bad = 1;
-                            break;
-                        }
-                    }
-                }
+                bad = mbar_wait(bar0 + 8 * buf, (p >> 1) & 1u, a.err, a.limitNs) ? 0u : 1u;
                 bad = __any_sync(0xFFFFFFFFu, bad);
             }
             pf.mark(joinx::PROF_BARRIER);
@@ -523,59 +474,6 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
         }
         cluster_sync();
     }
-}
-
-// Host: how many clusters of G CTAs of kernel fn the device can hold at once.
-inline int placeable(void* fn, u32 G, size_t smem) {
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(G);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = G;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
-}
-
-// Host: queues `clusters` clusters of G CTAs of kernel fn(args...).
-template <class... K, class... A>
-cudaError_t enqueue(void (*fn)(K...), u32 G, u32 clusters, size_t smem, cudaStream_t st, const A&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(G * clusters);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = G;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, args...);
-}
-
-// Host: one cluster; *done is false when the device cannot place it (nothing
-// is launched then).
-template <class... K, class... A>
-int launch(void (*fn)(K...), u32 G, size_t smem, cudaStream_t st, bool* done, const A&... args) {
-    *done = false;
-    if (!placeable((void*)fn, G, smem)) return CASPHY_OK;
-    CASPHY_CUDA_TRY(enqueue(fn, G, 1, smem, st, args...));
-    *done = true;
-    return CASPHY_OK;
 }
 
 }  // namespace joinc
