@@ -9,8 +9,8 @@
 // integer; the per-site log likelihood and its sum are binary64.
 //
 // Inside pass: internal nodes grouped by height, one launch per height, one
-// thread per (node, site).  Outside pass: internal nodes grouped by depth,
-// one launch per depth; for each child edge c of node p it forms
+// thread per (node, site).  Outside pass: the same groups of internal nodes,
+// one launch per height, highest first; for each child edge c of node p it forms
 // R = U_p * M_sibling and the site term w_s (R . dM_c/dt) / (R . M_c) of
 // d log L / d t_c, then passes U_c = R P_c down.  Both ratios are invariant
 // to the scale of R, so outside vectors are renormalised freely.  Site terms
@@ -66,7 +66,7 @@ struct Tree {
     const u32* edgeA;
     const u32* edgeB;
     const u32* inOrder;   // internal nodes by height
-    const u32* outOrder;  // internal nodes by depth
+    const u32* outOrder;  // internal nodes by falling height
     const uint4* inInfo;  // per position of inOrder: {node, kidA, kidB, edgeA}
     const u32* inEdgeB;   // per position of inOrder: edgeB
     const uint4* outInfo; // per position of outOrder
@@ -127,29 +127,32 @@ struct Hky {
     double pi[4];
 };
 
+// Four threads per edge, a row of P and dP each.
 __global__ void k_pmat_hky(const double* __restrict__ t, u32 nedge, Hky m, float* __restrict__ P,
                            float* __restrict__ dP) {
     pdl_wait();
     pdl_trigger();
-    const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 x = blockIdx.x * blockDim.x + threadIdx.x, e = x / 4, i = x % 4;
     if (e >= nedge) return;
     double ex[4], dx[4];
     for (int k = 0; k < 4; k++) {
         ex[k] = exp(m.lam[k] * t[e]);
         dx[k] = m.lam[k] * ex[k];
     }
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) {
-            double a = 0, b = 0;
-            for (int k = 0; k < 4; k++) {
-                a += m.V[i * 4 + k] * ex[k] * m.Vi[k * 4 + j];
-                b += m.V[i * 4 + k] * dx[k] * m.Vi[k * 4 + j];
-            }
-            // store P - I: O(t) entries with full relative precision, so the
-            // binary32 rounding is not one shared error across all sites
-            P[e * 16 + i * 4 + j] = (float)(i == j ? a - 1.0 : fmax(a, 0.0));
-            dP[e * 16 + i * 4 + j] = (float)b;
+    double V[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) V[k] = i == 0 ? m.V[k] : i == 1 ? m.V[4 + k] : i == 2 ? m.V[8 + k] : m.V[12 + k];
+    for (int j = 0; j < 4; j++) {
+        double a = 0, b = 0;
+        for (int k = 0; k < 4; k++) {
+            a += V[k] * ex[k] * m.Vi[k * 4 + j];
+            b += V[k] * dx[k] * m.Vi[k * 4 + j];
         }
+        // store P - I: O(t) entries with full relative precision, so the
+        // binary32 rounding is not one shared error across all sites
+        P[e * 16 + i * 4 + j] = (float)((int)i == j ? a - 1.0 : fmax(a, 0.0));
+        dP[e * 16 + i * 4 + j] = (float)b;
+    }
 }
 
 __device__ __forceinline__ float4 tip_hky(u32 code) {
@@ -623,10 +626,37 @@ struct TopLevels {
     u32 off[kMaxTop + 1];
 };
 
-template <class Buf, class F>
-__device__ __forceinline__ void walk_levels(const TopLevels& lv, F node) {
+// Walks the levels; node(i, nf, edgeB, ok) is called for two positions at a
+// time, so that the loads of both are in flight together, in two steps: load
+// (issue) and use.  A level's node records are brought to shared memory while
+// the level before is computed.
+template <class L, class U>
+__device__ __forceinline__ void walk_levels(const TopLevels& lv, const uint4* __restrict__ info,
+                                            const u32* __restrict__ edgeB, L load, U use) {
+    __shared__ uint4 s_info[2][kNarrow];
+    __shared__ u32 s_eb[2][kNarrow];
+    auto fetch = [&](u32 l) {
+        if (l < lv.n && threadIdx.x < lv.off[l + 1] - lv.off[l]) {
+            s_info[l & 1u][threadIdx.x] = info[lv.off[l] + threadIdx.x];
+            s_eb[l & 1u][threadIdx.x] = edgeB[lv.off[l] + threadIdx.x];
+        }
+    };
+    const u32 warp = threadIdx.x >> 5;
+    fetch(0);
+    __syncthreads();
     for (u32 l = 0; l < lv.n; l++) {
-        for (u32 i = lv.off[l] + (threadIdx.x >> 5); i < lv.off[l + 1]; i += kTopWarps) node(i);
+        const u32 cnt = lv.off[l + 1] - lv.off[l];
+        fetch(l + 1);
+        for (u32 i = warp; i < cnt; i += 2 * kTopWarps) {
+            const bool two = i + kTopWarps < cnt;
+            const u32 k = two ? i + kTopWarps : i;
+            const uint4 n0 = s_info[l & 1u][i], n1 = s_info[l & 1u][k];
+            const u32 e0 = s_eb[l & 1u][i], e1 = s_eb[l & 1u][k];
+            auto a = load(n0, e0, 0u);
+            auto b = load(n1, e1, 1u);
+            use(n0, e0, 0u, a);
+            if (two) use(n1, e1, 1u, b);
+        }
         __syncthreads();
     }
 }
@@ -634,25 +664,40 @@ __device__ __forceinline__ void walk_levels(const TopLevels& lv, F node) {
 __global__ void __launch_bounds__(32 * kTopWarps) k_inside_top_hky(Tree T, HkyBuf B, Chunk C, TopLevels lv) {
     pdl_wait();
     pdl_trigger();
-    const u32 s = blockIdx.x * 32 + (threadIdx.x & 31), ss = s < C.w ? s : 0u;
-    walk_levels<HkyBuf>(lv, [&](u32 i) {
-        const uint4 nf = T.inInfo[i];
+    struct In {
+        float4 la, lb;
         int ea, eb;
-        const float4 la = child_hky(T, B, C, nf.y, ss, &ea), lb = child_hky(T, B, C, nf.z, ss, &eb);
-        if (s < C.w) inside_hky_site(B, C, nf.x - T.ntip, nf.w, T.inEdgeB[i], s, la, ea, lb, eb);
-    });
+    };
+    const u32 s = blockIdx.x * 32 + (threadIdx.x & 31), ss = s < C.w ? s : 0u;
+    walk_levels(
+        lv, T.inInfo, T.inEdgeB,
+        [&](uint4 nf, u32, u32) {
+            In x;
+            x.la = child_hky(T, B, C, nf.y, ss, &x.ea);
+            x.lb = child_hky(T, B, C, nf.z, ss, &x.eb);
+            return x;
+        },
+        [&](uint4 nf, u32 eB, u32, const In& x) {
+            if (s < C.w) inside_hky_site(B, C, nf.x - T.ntip, nf.w, eB, s, x.la, x.ea, x.lb, x.eb);
+        });
 }
 
 __global__ void __launch_bounds__(32 * kTopWarps) k_inside_top_irr(Tree T, IrrBuf B, Chunk C, TopLevels lv) {
     pdl_wait();
     pdl_trigger();
+    struct In {
+        float4 la, lb;
+        float2 pa, pb;
+    };
     const u32 s = blockIdx.x * 32 + (threadIdx.x & 31), ss = s < C.w ? s : 0u;
-    walk_levels<IrrBuf>(lv, [&](u32 i) {
-        const uint4 nf = T.inInfo[i];
-        const float2 pa = B.p[nf.w], pb = B.p[T.inEdgeB[i]];
-        const float4 la = child_irr(T, B, C, nf.y, ss), lb = child_irr(T, B, C, nf.z, ss);
-        if (s < C.w) inside_irr_site(B, C, nf.x - T.ntip, pa, pb, s, la, lb);
-    });
+    walk_levels(
+        lv, T.inInfo, T.inEdgeB,
+        [&](uint4 nf, u32 eB, u32) {
+            return In{child_irr(T, B, C, nf.y, ss), child_irr(T, B, C, nf.z, ss), B.p[nf.w], B.p[eB]};
+        },
+        [&](uint4 nf, u32, u32, const In& x) {
+            if (s < C.w) inside_irr_site(B, C, nf.x - T.ntip, x.pa, x.pb, s, x.la, x.lb);
+        });
 }
 
 // Sum over the warp's 32 sites, as the wide kernels' first step.
@@ -674,28 +719,36 @@ __global__ void __launch_bounds__(32 * kTopWarps) k_outside_top_hky(u32 root, Tr
                                                                     float* __restrict__ gw) {
     pdl_wait();
     pdl_trigger();
-    __shared__ float sm[kTopWarps][64];
+    __shared__ float sm[kTopWarps][2][64];
+    struct In {
+        float4 u, la, lb;
+    };
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u32 s = blockIdx.x * 32 + lane, ss = s < C.w ? s : 0u;
     const bool ok = s < C.w;
     const float ws = ok ? (float)w[C.s0 + s] : 0.f;
-    walk_levels<HkyBuf>(lv, [&](u32 i) {
-        const uint4 nf = T.outInfo[i];
-        const u32 eA = nf.w, eB = T.outEdgeB[i];
-        float* M = sm[warp];
-        __syncwarp();
-        M[lane] = __ldg(B.P + 16 * (lane < 16 ? eA : eB) + (lane & 15));
-        M[32 + lane] = __ldg(B.dP + 16 * (lane < 16 ? eA : eB) + (lane & 15));
-        __syncwarp();
-        float4 u;
-        if (nf.x == root) u = make_float4((float)m.pi[0], (float)m.pi[1], (float)m.pi[2], (float)m.pi[3]);
-        else u = B.U[(size_t)(nf.x - T.ntip) * C.W + ss];
-        int e;
-        const float4 la = child_hky(T, B, C, nf.y, ss, &e), lb = child_hky(T, B, C, nf.z, ss, &e);
-        float g[2];
-        outside_hky_site(T, B, C, M, nf.y, nf.z, s, ok, u, la, lb, ws, g);
-        warp_terms(g, C, eA, eB, nsite32, gw);
-    });
+    walk_levels(
+        lv, T.outInfo, T.outEdgeB,
+        [&](uint4 nf, u32 eB, u32 h) {
+            In x;
+            if (nf.x == root) x.u = make_float4((float)m.pi[0], (float)m.pi[1], (float)m.pi[2], (float)m.pi[3]);
+            else x.u = B.U[(size_t)(nf.x - T.ntip) * C.W + ss];
+            int e;
+            x.la = child_hky(T, B, C, nf.y, ss, &e);
+            x.lb = child_hky(T, B, C, nf.z, ss, &e);
+            const u32 ed = 16 * (lane < 16 ? nf.w : eB) + (lane & 15);
+            const float p = __ldg(B.P + ed), dp = __ldg(B.dP + ed);
+            __syncwarp();
+            sm[warp][h][lane] = p;
+            sm[warp][h][32 + lane] = dp;
+            __syncwarp();
+            return x;
+        },
+        [&](uint4 nf, u32 eB, u32 h, const In& x) {
+            float g[2];
+            outside_hky_site(T, B, C, sm[warp][h], nf.y, nf.z, s, ok, x.u, x.la, x.lb, ws, g);
+            warp_terms(g, C, nf.w, eB, nsite32, gw);
+        });
 }
 
 __global__ void __launch_bounds__(32 * kTopWarps) k_outside_top_irr(u32 root, Tree T, IrrBuf B, Chunk C, TopLevels lv,
@@ -703,14 +756,15 @@ __global__ void __launch_bounds__(32 * kTopWarps) k_outside_top_irr(u32 root, Tr
                                                                     float* __restrict__ gw) {
     pdl_wait();
     pdl_trigger();
+    struct In {};
     const u32 s = blockIdx.x * 32 + (threadIdx.x & 31);
-    walk_levels<IrrBuf>(lv, [&](u32 i) {
-        const uint4 nf = T.outInfo[i];
-        const u32 eB = T.outEdgeB[i];
-        float g[2];
-        outside_irr_site(root, T, B, C, nf, eB, s, w, g);
-        warp_terms(g, C, nf.w, eB, nsite32, gw);
-    });
+    walk_levels(
+        lv, T.outInfo, T.outEdgeB, [&](uint4, u32, u32) { return In{}; },
+        [&](uint4 nf, u32 eB, u32, const In&) {
+            float g[2];
+            outside_irr_site(root, T, B, C, nf, eB, s, w, g);
+            warp_terms(g, C, nf.w, eB, nsite32, gw);
+        });
 }
 
 // ------------------------------------------------ fixed-order reductions ---
@@ -728,31 +782,39 @@ __global__ void k_sum_ll(const double* __restrict__ part, u32 n, double* out) {
     if (threadIdx.x == 0) *out = v;
 }
 
-// Edges of narrow levels (top) have a sum per 32 sites, the others per 256.
-__global__ void k_sum_grad(const double* __restrict__ gpart, const float* __restrict__ gw,
-                           const unsigned char* __restrict__ top, u32 nedge, u32 nblk, u32 nsite32,
-                           double* __restrict__ grad) {
+// Edges of narrow levels (top) have a sum per 32 sites, the others per 256.  A
+// warp per edge loads 32 terms at once and every lane adds them in order.
+__global__ void __launch_bounds__(256) k_sum_grad(const double* __restrict__ gpart, const float* __restrict__ gw,
+                                                  const unsigned char* __restrict__ top, u32 nedge, u32 nblk,
+                                                  u32 nsite32, double* __restrict__ grad) {
     pdl_wait();
     pdl_trigger();
-    const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 e = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (e >= nedge) return;
     double v = 0;
     if (top[e]) {
-        const float* g = gw + (size_t)e * nsite32;
-        for (u32 b = 0; b < nblk; b++) {
-            float t = 0.f;
-            for (u32 i = 8 * b; i < min(8 * b + 8, nsite32); i++) t += g[i];
-            v += (double)t;
+        for (u32 i0 = 0; i0 < nsite32; i0 += 32) {
+            const float x = i0 + lane < nsite32 ? gw[(size_t)e * nsite32 + i0 + lane] : 0.f;
+            for (u32 b = 0; b < 4 && i0 + 8 * b < nsite32; b++) {
+                float t = 0.f;
+#pragma unroll
+                for (u32 i = 0; i < 8; i++) t += __shfl_sync(0xFFFFFFFFu, x, 8 * b + i);
+                v += (double)t;
+            }
         }
     } else {
-        for (u32 b = 0; b < nblk; b++) v += gpart[(size_t)e * nblk + b];
+        for (u32 b0 = 0; b0 < nblk; b0 += 32) {
+            const double x = b0 + lane < nblk ? gpart[(size_t)e * nblk + b0 + lane] : 0.0;
+            const u32 m = min(32u, nblk - b0);
+            for (u32 b = 0; b < m; b++) v += __shfl_sync(0xFFFFFFFFu, x, b);
+        }
     }
-    grad[e] = v;
+    if (lane == 0) grad[e] = v;
 }
 
 // ----------------------------------------------------------- L-BFGS ----
 
-enum { SC_GD = 0, SC_DMAX = 1, SC_SY = 2, SC_YY = 3, SC_GG = 4, SC_N = 8 };
+enum { SC_GD = 0, SC_DMAX = 1, SC_SY = 2, SC_YY = 3, SC_GG = 4, SC_LL = 5, SC_ERR = 6, SC_N = 8 };
 
 struct Lb {
     u32 n, nCTA, Mr;  // Mr: ring slots (history + one spare)
@@ -1002,46 +1064,65 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_cluster(Lb a, u32 what, u32 s
         const bool fresh = (what & LB_ACCEPT) != 0;  // rho and gamma of `slot` are this launch's
 #pragma unroll
         for (int j = 0; j < V; j++) d[j] = g[j];
-        double v[V][1], o[1];
-        for (int k = (int)count - 1; k >= 0; k--) {
-            const u32 r = (first + (u32)k) % a.Mr;
-            const double* s = a.S + (size_t)r * a.n;
-            const double* y = a.Y + (size_t)r * a.n;
-            double yv[V];
+        // the pairs' vectors and 1 / s.y are loaded one pair ahead, so that no
+        // load waits behind a reduction
+        double v[V][1], o[1], sv[V], yv[V], sn[V], yn[V];
+        double rho = 0.0, rhoN = 0.0;
+        auto fetch = [&](u32 k) {
+            const u32 r = (first + k) % a.Mr;
+            rhoN = fresh && r == slot ? rhoNew : a.rho[r];
 #pragma unroll
             for (int j = 0; j < V; j++) {
-                v[j][0] = 0.0;
-                yv[j] = ok[j] ? y[at[j]] : 0.0;
-                if (ok[j]) v[j][0] += s[at[j]] * d[j];
+                sn[j] = ok[j] ? a.S[(size_t)r * a.n + at[j]] : 0.0;
+                yn[j] = ok[j] ? a.Y[(size_t)r * a.n + at[j]] : 0.0;
             }
-            cluster_reduce<V, 1, false>(a, x, v, o);
-            const double al = (fresh && r == slot ? rhoNew : a.rho[r]) * o[0];
-            if (threadIdx.x == 0) alpha[k] = al;
+        };
+        auto take = [&] {
+            rho = rhoN;
 #pragma unroll
-            for (int j = 0; j < V; j++) d[j] -= al * yv[j];
-        }
-        __syncthreads();
+            for (int j = 0; j < V; j++) {
+                sv[j] = sn[j];
+                yv[j] = yn[j];
+            }
+        };
+        double gm = 1.0;
         if (count > 0) {
             const u32 r = (first + count - 1) % a.Mr;
-            const double gm = fresh && r == slot ? gamNew : a.gam[r];
-#pragma unroll
-            for (int j = 0; j < V; j++) d[j] *= gm;
+            gm = fresh && r == slot ? gamNew : a.gam[r];
+            fetch(count - 1);
         }
-        for (u32 k = 0; k < count; k++) {
-            const u32 r = (first + k) % a.Mr;
-            const double* s = a.S + (size_t)r * a.n;
-            const double* y = a.Y + (size_t)r * a.n;
-            double sv[V];
+        for (int k = (int)count - 1; k >= 0; k--) {
+            take();
+            fetch(k > 0 ? (u32)k - 1u : 0u);  // (the second loop starts with pair 0)
 #pragma unroll
             for (int j = 0; j < V; j++) {
                 v[j][0] = 0.0;
-                sv[j] = ok[j] ? s[at[j]] : 0.0;
-                if (ok[j]) v[j][0] += y[at[j]] * d[j];
+                if (ok[j]) v[j][0] += sv[j] * d[j];
             }
             cluster_reduce<V, 1, false>(a, x, v, o);
-            const double c = alpha[k] - (fresh && r == slot ? rhoNew : a.rho[r]) * o[0];
+            const double al = rho * o[0];
+            if (threadIdx.x == 0) alpha[k] = al;
 #pragma unroll
-            for (int j = 0; j < V; j++) d[j] += c * sv[j];
+            for (int j = 0; j < V; j++)
+                if (ok[j]) d[j] -= al * yv[j];
+        }
+        __syncthreads();
+        if (count > 0)
+#pragma unroll
+            for (int j = 0; j < V; j++) d[j] *= gm;
+        for (u32 k = 0; k < count; k++) {
+            take();
+            if (k + 1 < count) fetch(k + 1);
+#pragma unroll
+            for (int j = 0; j < V; j++) {
+                v[j][0] = 0.0;
+                if (ok[j]) v[j][0] += yv[j] * d[j];
+            }
+            cluster_reduce<V, 1, false>(a, x, v, o);
+            const double c = alpha[k] - rho * o[0];
+#pragma unroll
+            for (int j = 0; j < V; j++)
+                if (ok[j]) d[j] += c * sv[j];
         }
         double w[V][2], o2[2];
 #pragma unroll
@@ -1160,7 +1241,7 @@ static int build_tree(u32 ntip, u32 nedge, const u32* edge, FelTreeHost& T) {
             return CASPHY_EINVAL;
         }
     // heights and depths without recursion (parents before children)
-    std::vector<u32> order, height(nn, 0), depth(nn, 0);
+    std::vector<u32> order, height(nn, 0);
     order.reserve(nn);
     std::vector<u32> stack{T.root};
     while (!stack.empty()) {
@@ -1169,7 +1250,6 @@ static int build_tree(u32 ntip, u32 nedge, const u32* edge, FelTreeHost& T) {
         order.push_back(v);
         if (v >= ntip) {
             const u32 a = T.kidA[v - ntip], b = T.kidB[v - ntip];
-            depth[a] = depth[b] = depth[v] + 1;
             stack.push_back(a);
             stack.push_back(b);
         }
@@ -1179,27 +1259,24 @@ static int build_tree(u32 ntip, u32 nedge, const u32* edge, FelTreeHost& T) {
         casphy_set_last_error_msg("felsenstein: the edges do not form one tree");
         return CASPHY_EINVAL;
     }
-    u32 H = 0, D = 0;
+    u32 H = 0;
     for (auto it = order.rbegin(); it != order.rend(); ++it) {
         const u32 v = *it;
         if (v >= ntip) height[v] = 1 + std::max(height[T.kidA[v - ntip]], height[T.kidB[v - ntip]]);
         H = std::max(H, height[v]);
-        D = std::max(D, depth[v]);
     }
-    std::vector<std::vector<u32>> byH(H + 1), byD(D + 1);
-    for (u32 v = ntip; v < nn; v++) {
-        byH[height[v]].push_back(v);
-        byD[depth[v]].push_back(v);
-    }
+    std::vector<std::vector<u32>> byH(H + 1);
+    for (u32 v = ntip; v < nn; v++) byH[height[v]].push_back(v);
     T.inOff.assign(1, 0);
     for (u32 h = 1; h <= H; h++) {
         T.inOrder.insert(T.inOrder.end(), byH[h].begin(), byH[h].end());
         T.inOff.push_back((u32)T.inOrder.size());
     }
+    // the outside pass walks the same levels downwards (a parent is higher than
+    // its children); by depth the wide levels lay between narrow ones
     T.outOff.assign(1, 0);
-    for (u32 d = 0; d <= D; d++) {
-        if (byD[d].empty()) continue;
-        T.outOrder.insert(T.outOrder.end(), byD[d].begin(), byD[d].end());
+    for (u32 h = H; h >= 1; h--) {
+        T.outOrder.insert(T.outOrder.end(), byH[h].begin(), byH[h].end());
         T.outOff.push_back((u32)T.outOrder.size());
     }
     const u32 nin = (u32)T.inOff.size() - 1, nout = (u32)T.outOff.size() - 1;
@@ -1332,7 +1409,7 @@ struct FelProblem {
     void enqueue(bool withGrad, u64* launches) {
         u64 n = 0;
         const u32 ne = th.nedge;
-        if (model == CASPHY_MODEL_HKY85) lp(k_pmat_hky, dim3((ne + 127) / 128), 128, (const double*)t, ne, hky, P, dP);
+        if (model == CASPHY_MODEL_HKY85) lp(k_pmat_hky, dim3((ne + 31) / 32), 128, (const double*)t, ne, hky, P, dP);
         else lp(k_pmat_irr, dim3((ne + 127) / 128), 128, (const double*)t, ne, rate, p);
         n++;
         for (u32 c = 0; c < nchunk; c++) {
@@ -1384,7 +1461,7 @@ struct FelProblem {
         lp(k_sum_ll, dim3(1), 256, (const double*)part, nblkTot, ll);
         n++;
         if (withGrad) {
-            lp(k_sum_grad, dim3((ne + 255) / 256), 256, (const double*)gpart, (const float*)gw, top, ne, nblkTot,
+            lp(k_sum_grad, dim3((ne + 7) / 8), 256, (const double*)gpart, (const float*)gw, top, ne, nblkTot,
                (nsite + 31) / 32, grad);
             n++;
         }
@@ -1419,14 +1496,25 @@ struct FelProblem {
     }
 
     // log L (and d log L / d t in `grad`) at the branch lengths in `t`:
-    // eval_launch() queues the graph and the read of log L into *llOut,
-    // eval_done() (after the stream is synchronised) adds its graph time
-    int eval_launch(bool withGrad, double* llOut) {
+    // eval_launch() queues the graph, read() brings the scalars (log L among
+    // them) to sc with one copy and one synchronisation, eval_done() adds the
+    // graph's time
+    int eval_launch(bool withGrad) {
         if (int rc = capture(withGrad)) return rc;
         CASPHY_CUDA_TRY(cudaEventRecord(g0, st));
         CASPHY_CUDA_TRY(cudaGraphLaunch(withGrad ? gFull : gLL, st));
         CASPHY_CUDA_TRY(cudaEventRecord(g1, st));
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(llOut, ll, sizeof(double), cudaMemcpyDeviceToHost, st));
+        return CASPHY_OK;
+    }
+    int read() {
+        CASPHY_CUDA_TRY(cudaMemcpyAsync(sc, lb.sc, sizeof(sc), cudaMemcpyDeviceToHost, st));
+        CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+        int err;
+        std::memcpy(&err, sc + SC_ERR, sizeof(err));
+        if (err) {
+            casphy_set_last_error_msg("felsenstein: a grid barrier of the L-BFGS step timed out");
+            return CASPHY_ETIMEOUT;
+        }
         return CASPHY_OK;
     }
     void eval_done() {
@@ -1434,11 +1522,13 @@ struct FelProblem {
         if (cudaEventElapsedTime(&ms, g0, g1) == cudaSuccess) graphMs += ms;
     }
     int eval(bool withGrad, double* llOut) {
-        if (int rc = eval_launch(withGrad, llOut)) return rc;
-        CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+        if (int rc = eval_launch(withGrad)) return rc;
+        if (int rc = read()) return rc;
+        *llOut = sc[SC_LL];
         eval_done();
         return CASPHY_OK;
     }
+    double sc[SC_N] = {0};
     cudaEvent_t g0 = nullptr, g1 = nullptr;
     double graphMs = 0;
 };
@@ -1538,13 +1628,11 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         b.outEB = c.take<u32>(nint);
         b.codes = c.take<u32>((size_t)ntip * nsite);
         b.flags = c.take<u32>(16 * nCTA);
-        b.err = c.take<int>(1);
         b.t = c.take<double>(nedge);
         b.w = c.take<double>(nsite);
         b.grad = c.take<double>(nedge);
         b.gpart = c.take<double>((size_t)nedge * F.nblkTot);
         b.part = c.take<double>(F.nblkTot);
-        b.ll = c.take<double>(1);
         b.x = c.take<double>(nv);
         b.g = c.take<double>(nv);
         b.d = c.take<double>(nv);
@@ -1553,7 +1641,9 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         b.Y = c.take<double>(Mr * nv);
         b.rho = c.take<double>(Mr);
         b.gam = c.take<double>(Mr);
-        b.sc = c.take<double>(SC_N);
+        b.sc = c.take<double>(SC_N);  // read back together: scalars, log L, barrier error
+        b.err = reinterpret_cast<int*>(b.sc + SC_ERR);
+        b.ll = b.sc + SC_LL;
         b.lpart = c.take<double>(8 * (size_t)nCTA);
         b.P = c.take<float>(isH ? 16 * (size_t)nedge : 0);
         b.dP = c.take<float>(isH ? 16 * (size_t)nedge : 0);
@@ -1702,20 +1792,6 @@ static int lb_step(FelProblem& F, u32 what, u32 slot, u32 first, u32 count, doub
     return CASPHY_OK;
 }
 
-// Reads `n` doubles from the device scalars at `src` together with the grid
-// barrier's error flag, with one synchronisation.
-static int lb_read(FelProblem& F, const double* src, double* dst, size_t n) {
-    int err = 0;
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(&err, F.lb.err, sizeof(int), cudaMemcpyDeviceToHost, F.st));
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(dst, src, sizeof(double) * n, cudaMemcpyDeviceToHost, F.st));
-    CASPHY_CUDA_TRY(cudaStreamSynchronize(F.st));
-    if (err) {
-        casphy_set_last_error_msg("felsenstein: a grid barrier of the L-BFGS step timed out");
-        return CASPHY_ETIMEOUT;
-    }
-    return CASPHY_OK;
-}
-
 // Per-edge central differences of log L into F.grad (as d log L / d t).
 // The step is taken in x = log t: t e^{+-h} with h = 1e-3, large enough that
 // the binary32 rounding of the partials (about 1e-7 of |log L|) stays well
@@ -1807,17 +1883,16 @@ extern "C" int casphy_felsenstein_optimize(uint32_t ntip, uint32_t nedge, const 
         double gd = specGd, dmax = specDmax;
         if (!spec) {
             u32 cnt = count;
-            double sc[2] = {0, 0};
             for (int attempt = 0; attempt < 2; attempt++) {
                 if ((rc = lb_step(F, LB_DIR, 0, first, cnt, 0.0))) return rc;
-                if ((rc = lb_read(F, a.sc + SC_GD, sc, 2))) return rc;
-                if (sc[0] < 0 || cnt == 0) break;
+                if ((rc = F.read())) return rc;
+                if (F.sc[SC_GD] < 0 || cnt == 0) break;
                 cnt = 0;  // not a descent direction: restart from steepest descent
             }
             if (cnt == 0 && count != 0) first = (first + count) % a.Mr;
             count = cnt;
-            gd = sc[0];
-            dmax = sc[1];
+            gd = F.sc[SC_GD];
+            dmax = F.sc[SC_DMAX];
             if (!(gd < 0)) break;  // stationary
         }
         double step = count == 0 ? std::min(1.0, 1.0 / std::max(dmax, 1e-12)) : 1.0;
@@ -1854,18 +1929,19 @@ extern "C" int casphy_felsenstein_optimize(uint32_t ntip, uint32_t nedge, const 
         if (adj && quietNext < kQuiet && it + 1 < max_iter) {
             u32 cntN = count < M ? count + 1 : count, firstN = count < M ? first : (first + 1) % a.Mr;
             if ((rc = lb_step(F, LB_ACCEPT | LB_DIR | LB_TRIAL, slot, firstN, cntN, 1.0))) return rc;
-            if ((rc = F.eval_launch(adj, &specLl))) return rc;
-            double sc3[3] = {0, 0, 0};  // g.d, max|d| of the direction; s.y of the accept
-            if ((rc = lb_read(F, a.sc + SC_GD, sc3, 3))) return rc;
+            if ((rc = F.eval_launch(adj))) return rc;
+            if ((rc = F.read())) return rc;
             F.eval_done();
             st.evaluations++;
-            sy = sc3[SC_SY - SC_GD];
-            specGd = sc3[SC_GD - SC_GD];
-            specDmax = sc3[SC_DMAX - SC_GD];
+            specLl = F.sc[SC_LL];
+            sy = F.sc[SC_SY];
+            specGd = F.sc[SC_GD];
+            specDmax = F.sc[SC_DMAX];
             spec = sy > 1e-12 && specGd < 0;
         } else {
             if ((rc = lb_step(F, LB_ACCEPT, slot, 0, 0, 0.0))) return rc;
-            if ((rc = lb_read(F, a.sc + SC_SY, &sy, 1))) return rc;
+            if ((rc = F.read())) return rc;
+            sy = F.sc[SC_SY];
         }
         st.iterations++;
         if (sy > 1e-12) {
