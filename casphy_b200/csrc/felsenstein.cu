@@ -1695,7 +1695,7 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
     CASPHY_CUDA_TRY(up(L.inEB, inEB.data(), 4ull * nint));
     CASPHY_CUDA_TRY(up(L.outEB, outEB.data(), 4ull * nint));
     CASPHY_CUDA_TRY(up(L.top, F.th.topEdge.data(), nedge));
-    CASPHY_CUDA_TRY(up(L.codes, codes, 4ull * ntip * nsite));
+    if ((rc = Staged::to_device(ds, L.codes, codes, 4ull * ntip * nsite, st))) return rc;
     CASPHY_CUDA_TRY(up(L.t, brlen, 8ull * nedge));
     std::vector<double> wv(nsite, 1.0);
     if (weights) wv.assign(weights, weights + nsite);

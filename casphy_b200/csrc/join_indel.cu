@@ -1470,8 +1470,7 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     CASPHY_CUDA_TRY(cudaEventRecord(ev[0], st));
     const u32* codes = d_codes;
     if (h_codes) {
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(dCodesCopy, h_codes, sizeof(u32) * (size_t)ntip * ncol,
-                                        cudaMemcpyHostToDevice, st));
+        if ((rc = Staged::to_device(ds, dCodesCopy, h_codes, sizeof(u32) * (size_t)ntip * ncol, st))) return rc;
         codes = dCodesCopy;
     }
     std::vector<u64> chunkStart(nChunks + 1);
@@ -1529,9 +1528,7 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     u32* sout = d_state_out ? d_state_out : dState;
     k_gather<<<nrows, 256, 0, st>>>(L.nodeRow, ncol, (ncol + 7u) & ~7u, dOrder, nrows, sout);
     launches++;
-    if (h_state_out)
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(h_state_out, sout, sizeof(u32) * (size_t)nrows * ncol, cudaMemcpyDeviceToHost,
-                                        st));
+    if (h_state_out && (rc = Staged::to_host(ds, h_state_out, sout, sizeof(u32) * (size_t)nrows * ncol, st))) return rc;
     CASPHY_CUDA_TRY(cudaEventRecord(ev[4], st));
     CASPHY_CUDA_TRY(cudaEventSynchronize(ev[4]));
     float t12 = 0, t23 = 0, t04 = 0;

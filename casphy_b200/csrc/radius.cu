@@ -293,20 +293,19 @@ struct RadiusInput {
 static size_t row_words(const RadiusInput& in) { return in.dna ? in.nwords + 4 * ((in.nwords / 4 + 3) / 4) : in.nwords; }
 
 // Uploads the rows (ld = ntip); mode: the word k_pack_dna sets.
-static int upload_rows(const RadiusInput& in, Carve& c, u32** col, float** wf, u32** mode, cudaStream_t st) {
+static int upload_rows(DeviceScope& ds, const RadiusInput& in, Carve& c, u32** col, float** wf, u32** mode, cudaStream_t st) {
     *col = c.take<u32>(row_words(in) * in.ntip);
     *wf = c.take<float>(in.wf.size() ? in.wf.size() : 1);
     *mode = c.take<u32>(2);  // [1]: error of a device-side wait
     CASPHY_CUDA_TRY(cudaMemsetAsync(*mode, 0, 2 * sizeof(u32), st));
     if (in.dna) {
         u32* raw = c.take<u32>((size_t)in.ntip * in.nbinRaw);
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(raw, in.hostRaw, sizeof(u32) * (size_t)in.ntip * in.nbinRaw,
-                                        cudaMemcpyHostToDevice, st));
+        if (int rc = Staged::to_device(ds, raw, in.hostRaw, sizeof(u32) * (size_t)in.ntip * in.nbinRaw, st)) return rc;
         k_pack_dna<<<dim3((in.ntip + 255) / 256, in.nwords / 4), 256, 0, st>>>(raw, in.ntip, in.nbinRaw, in.nwords / 4,
                                                                                in.ntip, *col, *mode);
     } else {
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(*col, in.hostWordPlane, sizeof(u32) * (size_t)in.nwords * in.ntip,
-                                        cudaMemcpyHostToDevice, st));
+        if (int rc = Staged::to_device(ds, *col, in.hostWordPlane, sizeof(u32) * (size_t)in.nwords * in.ntip, st))
+            return rc;
     }
     if (in.wf.size())
         CASPHY_CUDA_TRY(cudaMemcpyAsync(*wf, in.wf.data(), sizeof(float) * in.wf.size(), cudaMemcpyHostToDevice, st));
@@ -391,7 +390,7 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     if (rc) return rc;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    rc = upload_rows(in, c2, &dcol, &dwf, &dmode, st);
+    rc = upload_rows(ds, in, c2, &dcol, &dwf, &dmode, st);
     if (rc) return rc;
     auto L = lay(c2);
     dim3 grid((ntip + kThreads - 1) / kThreads, (nq + kQ - 1) / kQ);
@@ -465,7 +464,7 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     CASPHY_CUDA_TRY(cudaMemcpyAsync(L.off, off.data(), sizeof(u64) * nq, cudaMemcpyHostToDevice, st));
     k_expand<<<(nq + 7) / 8, 256, 0, st>>>(L.mask, nq, maskWords, L.off, didx);
     CASPHY_CUDA_TRY(cudaGetLastError());
-    if (tot) CASPHY_CUDA_TRY(cudaMemcpyAsync(idx, didx, sizeof(u32) * tot, cudaMemcpyDeviceToHost, st));
+    if (tot && (rc = Staged::to_host(ds, idx, didx, sizeof(u32) * tot, st))) return rc;
     CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
     return CASPHY_OK;
 }
@@ -492,7 +491,7 @@ static int try_impl(RadiusInput& in, u32 nrep, const u32* qidx, u32* counts) {
     u32* dcol;
     float* dwf;
     u32* dmode;
-    rc = upload_rows(in, c2, &dcol, &dwf, &dmode, st);
+    rc = upload_rows(ds, in, c2, &dcol, &dwf, &dmode, st);
     if (rc) return rc;
     u32* dq = c2.take<u32>(nrep);
     u32* dc = c2.take<u32>(nrep);

@@ -20,6 +20,16 @@ struct DeviceScope {
     int reserve_aux(size_t bytes, void** out);
 };
 
+// Copies of large pageable host buffers: kCopyMin bytes and more go through
+// pinned slots of the device's arena, filled or emptied by several host
+// threads (the driver's own staging copies on one).  to_device returns when
+// every copy is queued on the stream and src has been read; to_host when dst
+// has been written, after all work queued on the stream before.
+struct Staged {
+    static int to_device(DeviceScope& ds, void* dst, const void* src, size_t bytes, void* stream);
+    static int to_host(DeviceScope& ds, void* dst, const void* src, size_t bytes, void* stream);
+};
+
 struct Carve {
     size_t off = 0;
     char* base = nullptr;

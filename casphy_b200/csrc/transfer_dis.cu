@@ -208,8 +208,8 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     Carve c2;
     c2.base = static_cast<char*>(base);
     auto L = lay(c2);
-    if (nrow_y) CASPHY_CUDA_TRY(cudaMemcpyAsync(L.y, y, sizeof(u32) * (size_t)nrow_y * ncol, cudaMemcpyHostToDevice, st));
-    if (nrow_x) CASPHY_CUDA_TRY(cudaMemcpyAsync(L.x, x, sizeof(u32) * (size_t)nrow_x * ncol, cudaMemcpyHostToDevice, st));
+    if (nrow_y && (rc = Staged::to_device(ds, L.y, y, sizeof(u32) * (size_t)nrow_y * ncol, st))) return rc;
+    if (nrow_x && (rc = Staged::to_device(ds, L.x, x, sizeof(u32) * (size_t)nrow_x * ncol, st))) return rc;
     rc = transfer_dis_device(nrow_y, nrow_x, ncol, ntip, L.y, L.x, L.ymin, L.ysize, L.xmin, L.xsize, L.s, st);
     if (rc) return rc;
     int werr = 0;
