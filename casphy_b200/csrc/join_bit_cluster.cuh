@@ -20,6 +20,7 @@ namespace bitjoin {
 
 template <int PATH>
 struct BitCluster {
+    static constexpr bool kNarrow = false;  // binary32 scores
     struct Args {
         u32 nbin, nbinP, nplanes;
         int ancType;
@@ -42,6 +43,7 @@ struct BitCluster {
         u32 next;      // global buffer the next compaction writes
         u32 rank;
         u32 par;
+        bool prof;     // section times are taken
     };
     __host__ __device__ static u32 planes(const Args& m) { return PATH == PATH_PLANES && m.nplanes ? m.nplanes : 1u; }
     __host__ static size_t smem_bytes(const Args& m, u32 R) {
@@ -183,19 +185,46 @@ struct BitCluster {
                     : "+f"(fa)
                     : "r"(v), "r"(t.x), "f"(__uint_as_float(t.y)));
             };
-            // (only this CTA writes its columns, so plain loads do)
+            // eight entries at a time, the next eight loaded before these are
+            // added (only this CTA writes its columns, so plain loads do)
             u32 e = 0;
-            for (; e + 7 < n; e += 8) {
+            if (n > 7) {
                 uint2 t[8];
                 u32 v[8];
 #pragma unroll
-                for (u32 j = 0; j < 8; j++) t[j] = ent[e + j];
+                for (u32 j = 0; j < 8; j++) {
+                    t[j] = ent[j];
+                    v[j] = c[t[j].x >> 5];
+                }
+                for (; e + 15 < n; e += 8) {
+                    uint2 nt[8];
+                    u32 nv[8];
 #pragma unroll
-                for (u32 j = 0; j < 8; j++) v[j] = c[t[j].x >> 5];
+                    for (u32 j = 0; j < 8; j++) nt[j] = ent[e + 8 + j];
+#pragma unroll
+                    for (u32 j = 0; j < 8; j++) nv[j] = c[nt[j].x >> 5];
+#pragma unroll
+                    for (u32 j = 0; j < 8; j++) add(v[j], t[j]);
+#pragma unroll
+                    for (u32 j = 0; j < 8; j++) {
+                        t[j] = nt[j];
+                        v[j] = nv[j];
+                    }
+                }
+#pragma unroll
+                for (u32 j = 0; j < 8; j++) add(v[j], t[j]);
+                e += 8;
+            }
+            if (e < n) {  // the rest as one batch; past the end, words of 0
+                uint2 t[8];
+                u32 v[8];
+#pragma unroll
+                for (u32 j = 0; j < 8; j++) t[j] = e + j < n ? ent[e + j] : make_uint2(0u, 0u);
+#pragma unroll
+                for (u32 j = 0; j < 8; j++) v[j] = e + j < n ? c[t[j].x >> 5] : 0u;
 #pragma unroll
                 for (u32 j = 0; j < 8; j++) add(v[j], t[j]);
             }
-            for (; e < n; e++) add(c[ent[e].x >> 5], ent[e]);
             return fa;
         }
         const u32 P = planes(m);
@@ -249,7 +278,7 @@ struct BitCluster {
             }
             done(q);
         }
-        joinx::prof_mark(joinx::PROF_SC_ACC);
+        if (s.prof) joinx::prof_mark(joinx::PROF_SC_ACC);
     }
 
     // Moves the live slots' columns to their new places; n live slots, ranks

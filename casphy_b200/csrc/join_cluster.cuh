@@ -38,7 +38,6 @@ using joinx::kDead;
 using joinx::kMaxBatch;
 constexpr int kThreads = clu::kThreads, kWarps = kThreads / 32;
 constexpr u32 kLists = 4;    // records a CTA publishes per exchange, one per four warps
-constexpr u32 kJoin = 0, kStale = 1;
 
 // One published record: larger ord, then larger inv (smaller node) is better;
 // ord 0 is no record.  slot: rank of the owning CTA << 24 | slot in its range.
@@ -75,8 +74,20 @@ __host__ __device__ inline size_t engine_smem(u32 G, u32 R, u32 deathWords) {
 
 // ---------------------------------------------------------------------------
 
-// The maximum of the warp's (hi, lo) keys, in every lane.
+// The maximum of the warp's (ord, inv) keys, in every lane.  NARROW: the
+// scores are non-negative binary16 and the nodes below 2^17, so the key fits 32
+// bits (ord's top bit is set in every record) and one reduction (about 90
+// clocks) finds it instead of two.
+constexpr u32 kNarrowNodes = 1u << 17;
+template <bool NARROW>
 __device__ __forceinline__ void warp_max2(u32& hi, u32& lo) {
+    if (NARROW) {
+        constexpr u32 base = 0xFFFFFFFFu - (kNarrowNodes - 1u);  // inv of the largest node
+        const u32 k = __reduce_max_sync(0xFFFFFFFFu, hi ? ((hi & 0x7FFFu) << 17) | (lo - base) : 0u);
+        hi = k ? 0x8000u | (k >> 17) : 0u;
+        lo = k ? base + (k & (kNarrowNodes - 1u)) : 0u;
+        return;
+    }
     const u32 h = __reduce_max_sync(0xFFFFFFFFu, hi);
     lo = __reduce_max_sync(0xFFFFFFFFu, hi == h ? lo : 0u);
     hi = h;
@@ -108,12 +119,13 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
     u32* deathBits = st.idx + a.R;
     typename M::Smem ms;
     M::carve_smem(a, m, smem + engine_smem(G, a.R, a.deathWords), ms);
+    ms.prof = a.prof != nullptr && rank == 0;
     __shared__ __align__(8) u64 s_bar[2];
     __shared__ Rec s_wrec[kWarps];
     __shared__ Rec s_rows[kMaxBatch];   // the rescanned rows
     __shared__ Rec s_extra[kMaxBatch];  // their new records
     __shared__ u64 s_red[kMaxBatch][kWarps];
-    __shared__ u32 s_dec[6];            // kind, rescanned rows, j1, slot of j1, j2, failure
+    __shared__ u32 s_dec[6];            // -, rescanned rows, j1, slot of j1, j2, failure
     const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const u32 bar0 = smem_u32(&s_bar[0]);
 
@@ -143,7 +155,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
     // Every group of four warps sends its best record to every CTA.
     auto send_lists = [&](const Best& b, u32 buf) {
         u32 hi = b.ord, lw = b.inv;
-        warp_max2(hi, lw);
+        warp_max2<M::kNarrow>(hi, lw);
         if (hi == 0u) {
             if (lane == 0) s_wrec[warp] = Rec{0u, 0u, 0u, 0u};
         } else if (b.ord == hi && b.inv == lw) {
@@ -153,7 +165,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
         if ((warp & 3) == 0) {
             const u32 o = lane < 4 ? s_wrec[warp + lane].ord : 0u, v = lane < 4 ? s_wrec[warp + lane].inv : 0u;
             u32 h2 = o, l2 = v;
-            warp_max2(h2, l2);
+            warp_max2<M::kNarrow>(h2, l2);
             const u32 w = __ballot_sync(0xFFFFFFFFu, lane < 4 && o == h2 && v == l2);
             const Rec r = s_wrec[warp + __ffs(w) - 1];
             Rec* dst = tab + (size_t)buf * G * kLists + rank * kLists + (warp >> 2);
@@ -225,60 +237,53 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             // the decision: the best of up to three records per lane is joined
             // when its partner lives; else it and the other stale records
             // above the best live one are rescanned, best first
+            const u32 nList = G * kLists;
+            const Rec* T = tab + (size_t)buf * nList;
             Rec rec[3];
-            bool dead[3];
-            u32 hi = 0, lw = 0;
-#pragma unroll
-            for (u32 j = 0; j < 3; j++) {
-                rec[j] = Rec{0u, 0u, 0u, 0u};
-                if (j < 2) {
-                    if (lane + 32 * j < G * kLists) rec[j] = tab[(size_t)buf * G * kLists + lane + 32 * j];
-                } else if (lane < prevQ) {
-                    rec[j] = s_extra[lane];
-                }
-                if (rec[j].partner >= a.nnode) {
-                    bad = 1;
-                    rec[j].partner = 0u;
-                }
-                dead[j] = rec[j].ord && ((deathBits[rec[j].partner >> 5] >> (rec[j].partner & 31)) & 1u);
-                if (rec[j].ord > hi || (rec[j].ord == hi && rec[j].inv > lw)) {
-                    hi = rec[j].ord;
-                    lw = rec[j].inv;
-                }
+            rec[0] = lane < nList ? T[lane] : Rec{0u, 0u, 0u, 0u};
+            rec[1] = lane + 32 < nList ? T[lane + 32] : Rec{0u, 0u, 0u, 0u};
+            rec[2] = lane < prevQ ? s_extra[lane] : Rec{0u, 0u, 0u, 0u};
+            auto better = [](const Rec& r, u32 ord, u32 inv) { return r.ord > ord || (r.ord == ord && r.inv > inv); };
+            auto is_dead = [&](const Rec& r) {
+                return r.ord && r.partner < a.nnode && ((deathBits[r.partner >> 5] >> (r.partner & 31)) & 1u);
+            };
+            u32 top = better(rec[1], rec[0].ord, rec[0].inv) ? 1u : 0u;
+            Rec mine = top ? rec[1] : rec[0];
+            if (prevQ && better(rec[2], mine.ord, mine.inv)) {
+                mine = rec[2];
+                top = 2u;
             }
-            const u32 myHi = hi, myLw = lw;
-            warp_max2(hi, lw);
-            u32 nq = 0;
-            bool stale = false;
-#pragma unroll
-            for (u32 j = 0; j < 3; j++) stale |= dead[j] && rec[j].ord == hi && rec[j].inv == lw;
+            u32 hi = mine.ord, lw = mine.inv, nq = 0;
+            warp_max2<M::kNarrow>(hi, lw);
+            const bool winner = hi && mine.ord == hi && mine.inv == lw;
+            if (winner) {
+                if ((~lw) >= a.nnode || mine.partner >= a.nnode) bad = 1;
+            }
             if (hi == 0u) bad = bad ? bad : 2u;  // two live rows always have a record
+            bool stale = winner && is_dead(mine);
             if (!__any_sync(0xFFFFFFFFu, stale)) {
-                if (myHi == hi && myLw == lw && hi) {
-#pragma unroll
-                    for (u32 j = 0; j < 3; j++)
-                        if (rec[j].ord == hi && rec[j].inv == lw) {
-                            const u32 j1 = ~lw, j2 = rec[j].partner;
-                            s_dec[2] = j1;
-                            s_dec[3] = rec[j].slot;
-                            s_dec[4] = j2;
-                            if (j1 < a.nnode) {
-                                atomicOr(deathBits + (j1 >> 5), 1u << (j1 & 31));
-                                atomicOr(deathBits + (j2 >> 5), 1u << (j2 & 31));
-                            } else {
-                                bad = 1;
-                            }
-                        }
+                if (winner) {
+                    const u32 j1 = ~lw, j2 = mine.partner;
+                    s_dec[2] = j1;
+                    s_dec[3] = mine.slot;
+                    s_dec[4] = j2;
+                    if (!bad) {
+                        atomicOr(deathBits + (j1 >> 5), 1u << (j1 & 31));
+                        atomicOr(deathBits + (j2 >> 5), 1u << (j2 & 31));
+                    }
                 }
             } else {
+                bool dead[3];
                 u32 fk = 0, fi = 0;  // the best record whose partner lives
 #pragma unroll
-                for (u32 j = 0; j < 3; j++)
-                    if (!dead[j] && (rec[j].ord > fk || (rec[j].ord == fk && rec[j].inv > fi))) {
+                for (u32 j = 0; j < 3; j++) {
+                    dead[j] = is_dead(rec[j]);
+                    if (!dead[j] && better(rec[j], fk, fi)) {
                         fk = rec[j].ord;
                         fi = rec[j].inv;
                     }
-                warp_max2(fk, fi);
+                }
+                warp_max2<M::kNarrow>(fk, fi);
                 while (nq < a.maxBatch) {
 #pragma unroll
                     for (u32 j = 0; j < 3; j++)
@@ -293,20 +298,18 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
                     hi = lw = 0u;
 #pragma unroll
                     for (u32 j = 0; j < 3; j++)
-                        if (dead[j] && (rec[j].ord > fk || (rec[j].ord == fk && rec[j].inv > fi)) &&
-                            (rec[j].ord > hi || (rec[j].ord == hi && rec[j].inv > lw))) {
+                        if (dead[j] && better(rec[j], fk, fi) && better(rec[j], hi, lw)) {
                             hi = rec[j].ord;
                             lw = rec[j].inv;
                         }
-                    warp_max2(hi, lw);
+                    warp_max2<M::kNarrow>(hi, lw);
                     if (hi == 0u) break;
                 }
             }
-            bad = __reduce_max_sync(0xFFFFFFFFu, bad);
+            const u32 badAny = __any_sync(0xFFFFFFFFu, bad == 1u) ? 1u : bad;
             if (lane == 0) {
-                s_dec[0] = nq ? kStale : kJoin;
                 s_dec[1] = nq;
-                s_dec[5] = bad;
+                s_dec[5] = badAny;
                 if (G > 1) mbar_expect(bar0 + 8 * (buf ^ 1u), G * (kLists * (u32)sizeof(Rec) + nq * (u32)sizeof(u64)));
             }
         }
@@ -333,7 +336,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
                       },
                       [&](u32 q) {  // this warp is done with row q
                           u32 hi = key_ord(bk), lw = (u32)bk;
-                          warp_max2(hi, lw);
+                          warp_max2<M::kNarrow>(hi, lw);
                           if (lane == 0) s_red[q][warp] = ((u64)hi << 32) | lw;
                           bk = 0ull;
                       });
@@ -345,7 +348,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             if (warp < nq) {
                 const u64 v = lane < kWarps ? s_red[warp][lane] : 0ull;
                 u32 hi = key_ord(v), lw = (u32)v;
-                warp_max2(hi, lw);
+                warp_max2<M::kNarrow>(hi, lw);
                 const u64 best = ((u64)hi << 32) | lw;
                 u64* dst = part + ((size_t)(buf ^ 1u) * kMaxBatch + warp) * G + rank;
                 if (G == 1) {

@@ -1148,7 +1148,8 @@ static size_t bits_bytes(u32 ntip, u32 ncol, u32 nState) {
 // cluster costs about 4 us plus the scan of a sixteenth of the slots, on all
 // SMs about 10 us plus a scan of a 148th: at 65,000 x 1,024 the cluster takes
 // 0.93 s and all SMs 1.10 s, at 12,345 x 777 0.095 s and 0.184 s.
-constexpr u32 kClusterTips = 65536;
+constexpr u32 kClusterTips = 65536;  // (the engine's narrow keys: nodes below 2^17)
+static_assert(2 * kClusterTips <= joinc::kNarrowNodes, "narrow keys");
 // CTAs of the cluster: 16, fewer when a CTA would have no slot of its own;
 // and the slots of each, a multiple of kBitsAlign.
 static u32 cluster_size(u32 ntip) {

@@ -10,8 +10,8 @@
 //    are summed by shuffles.  No warp needs another's sums, so nothing but the
 //    copies is waited for.  (Warps that split the entries instead, with a tree
 //    over their counters in shared memory, took 2.9 us a phase for the tree.)
-//  * HALF: lane = slot, the entries in ascending site order, one predicated
-//    add each.  The bit test replaces the column scan's compare of 16-bit
+//  * HALF: a lane takes two slots and the entries in ascending site order, one
+//    paired binary16 add each.  The bit test replaces the column scan's compare of 16-bit
 //    codes, and the copies are issued by all threads, where the column scan
 //    had one thread in flight per eight slots (27 slots a CTA at 4,000 cells)
 //    and spent 6.5 us a scan.
@@ -22,8 +22,11 @@
 namespace casphy {
 namespace indel {
 
+constexpr u32 kOneCopyWords = 4096;
+
 template <bool HALF>
 struct IndelCluster {
+    static constexpr bool kNarrow = true;  // non-negative binary16 scores; cluster_plan bounds the nodes
     struct Args {
         u32 ncol, ncolP, nState, minSize;
         float minRatio;
@@ -39,11 +42,12 @@ struct IndelCluster {
         u32* eRow;    // maxBatch x ncolW: bitset row of every entry
         u32* eW;      // maxBatch x ncolW: weights (unless all are 1); HALF: in both halves of a word
         u32* stage;   // stageWords
-        u16* sums;    // HALF: maxBatch x R running sums
+        u32* sums;    // HALF: maxBatch x R / 2 pairs of running sums
         u32* B;       // this CTA's bitset rows, `pitch` words each
         u32* other;   // the same in the other buffer
         u32 pitch;
         u32 par;      // parity of the entry counters
+        bool prof;    // section times are taken
     };
     // entry counters of the current and the next query build
     __device__ static u32* counts(u32 par) {
@@ -59,7 +63,7 @@ struct IndelCluster {
         s.stage = reinterpret_cast<u32*>(p);
         s.eRow = s.stage + m.stageWords;
         s.eW = s.eRow + (size_t)m.maxBatch * ncolW(m.ncol);
-        s.sums = reinterpret_cast<u16*>(s.eW + (m.unitW ? 0u : (size_t)m.maxBatch * ncolW(m.ncol)));
+        s.sums = s.eW + (m.unitW ? 0u : (size_t)m.maxBatch * ncolW(m.ncol));
         s.par = 0;
     }
     __device__ static u16* rank_space(Smem& s) { return reinterpret_cast<u16*>(s.stage); }
@@ -217,20 +221,29 @@ struct IndelCluster {
     template <class F>
     __device__ static void rounds(const Args& m, Smem& s, u32 nq, u32 total, u32 per, u32 wb, u32 wst, u32 pitch, F add) {
         for (u32 r0 = 0; r0 < total; r0 += per) {
-            const u32 r1 = min(total, r0 + per), rm = min(r1, r0 + (((r1 - r0) / 2 + 7u) & ~7u));
+            const u32 r1 = min(total, r0 + per);
+            // (a few KB arrive together: halves would only add a barrier)
+            const bool halves = (r1 - r0) * wst > kOneCopyWords;
+            const u32 rm = halves ? min(r1, r0 + (((r1 - r0) / 2 + 7u) & ~7u)) : r1;
             copy_range(m, s, nq, r0, r0, rm, wb, wst, pitch);
             cp_async_commit();
-            copy_range(m, s, nq, r0, rm, r1, wb, wst, pitch);
-            cp_async_commit();
-            cp_async_wait_group<1>();
+            if (halves) {
+                copy_range(m, s, nq, r0, rm, r1, wb, wst, pitch);
+                cp_async_commit();
+                cp_async_wait_group<1>();
+            } else {
+                cp_async_wait_group<0>();
+            }
             __syncthreads();
-            joinx::prof_mark(joinx::PROF_SC_COPY);
+            if (s.prof) joinx::prof_mark(joinx::PROF_SC_COPY);
             add(r0, r0, rm);
-            cp_async_wait_group<0>();
-            __syncthreads();
-            add(r0, rm, r1);
+            if (halves) {
+                cp_async_wait_group<0>();
+                __syncthreads();
+                add(r0, rm, r1);
+            }
             if (r1 < total) __syncthreads();  // the next round overwrites the stage
-            joinx::prof_mark(joinx::PROF_SC_ACC);
+            if (s.prof) joinx::prof_mark(joinx::PROF_SC_ACC);
         }
     }
 
@@ -303,12 +316,18 @@ struct IndelCluster {
             }
         }
         constexpr int F = N + 5 < kPlanes ? N + 5 : kPlanes;
-        for (u32 j = 0; j < words; j++) {
-            u32 v = 0;
+        // two words at a time, so that their chains of shuffles overlap
+        for (u32 j = 0; j < words; j += 2) {
+            u32 v = 0, w = 0;
+            const u32 j1 = j + 1 < words ? j + 1 : j;
 #pragma unroll
-            for (int k = 0; k < F; k++) v |= ((__shfl_sync(0xFFFFFFFFu, c[k], j) >> lane) & 1u) << k;
+            for (int k = 0; k < F; k++) {
+                v |= ((__shfl_sync(0xFFFFFFFFu, c[k], j) >> lane) & 1u) << k;
+                w |= ((__shfl_sync(0xFFFFFFFFu, c[k], j1) >> lane) & 1u) << k;
+            }
             const u32 x = (w0 + j) * 32 + lane;
             if (x < st.n) f(q, x, ord_f16((u16)half_bits_of_int(v)));
+            if (j1 != j && x + 32 < st.n) f(q, x + 32, ord_f16((u16)half_bits_of_int(w)));
         }
     }
 
@@ -329,44 +348,87 @@ struct IndelCluster {
         const u32 myN = q < nq ? cnt[q] : 0u;
         const u32* wl = s.eW + (size_t)(q < nq ? q : 0u) * ncolW(m.ncol);
         if constexpr (HALF) {
-            u16* sums = s.sums + (size_t)(q < nq ? q : 0u) * st.cap;
+            // two words a warp, so a lane adds the two slots of its bit as a
+            // pair: one 8-byte load of the words and a quarter of a 16-byte load
+            // of the weights serve both (with a load of either per word and
+            // entry, the shared-memory loads set the time: 1.8 us a phase at 120
+            // entries of 8 words)
+            u32* sums = s.sums + (size_t)(q < nq ? q : 0u) * (st.cap / 2);
             const u32 per = total * W4 <= m.stageWords ? max(total, 1u) : m.stageWords / W4 & ~7u;
+            const u32 pairs = (Wc + 1u) / 2u;
             auto walk = [&](u32 r0, u32 a, u32 b) {
                 const u32 lo = max(a, myOff), hi = min(b, myOff + myN);
                 if (q >= nq || lo >= hi) return;
-                for (u32 wd = wi; wd < Wc; wd += nwq) {
-                    const u32 x = wd * 32 + lane, bit = 1u << lane;
-                    u32 h = lo > myOff ? sums[x] : 0u;
-                    const u32* col = s.stage + wd;
-                    u32 e = lo - r0;
-                    auto step = [&](u32 v, u32 wt) {
-                        asm("{\n .reg .pred p;\n .reg .b32 t;\n and.b32 t, %1, %2;\n setp.ne.u32 p, t, 0;\n"
-                            " @p add.rn.f16x2 %0, %0, %3;\n}"
-                            : "+r"(h)
-                            : "r"(v), "r"(bit), "r"(wt));
+                for (u32 pr = wi; pr < pairs; pr += nwq) {
+                    u32 h = lo > myOff ? sums[pr * 32 + lane] : 0u;
+                    const u32* col = s.stage + 2 * pr;
+                    // adding +0 leaves a sum of non-negative weights as it is
+                    auto step = [&](uint2 v, u32 wt) {
+                        const u32 bits = __byte_perm(v.x >> lane, v.y >> lane, 0x5410u) & 0x00010001u;
+                        const u32 w = wt & (bits * 0xFFFFu);
+                        asm("add.rn.f16x2 %0, %0, %1;" : "+r"(h) : "r"(w));
                     };
-                    for (; e + 7 < hi - r0; e += 8) {
-                        u32 v[8], wt[8];
+                    const u32 end = hi - r0;
+                    u32 e = lo - r0;
+                    const u32* w = wl + (lo - myOff);  // entry e's weight, advanced with e
+                    if (((lo - myOff) & 3u) == 0u) {
+                        // the next eight entries are loaded before these are added
+                        uint2 v[8], nv[8];
+                        uint4 w0, w1, nw0, nw1;
+                        auto load = [&](u32 at, const u32* wp, uint2 (&x)[8], uint4& a0, uint4& a1) {
 #pragma unroll
-                        for (u32 j = 0; j < 8; j++) v[j] = col[(e + j) * W4];
-#pragma unroll
-                        for (u32 j = 0; j < 8; j++) wt[j] = wl[e + j + r0 - myOff];
-#pragma unroll
-                        for (u32 j = 0; j < 8; j++) step(v[j], wt[j]);
+                            for (u32 k = 0; k < 8; k++) x[k] = *reinterpret_cast<const uint2*>(col + (at + k) * W4);
+                            a0 = reinterpret_cast<const uint4*>(wp)[0];
+                            a1 = reinterpret_cast<const uint4*>(wp)[1];
+                        };
+                        auto add = [&](const uint2 (&x)[8], const uint4& a0, const uint4& a1) {
+                            step(x[0], a0.x);
+                            step(x[1], a0.y);
+                            step(x[2], a0.z);
+                            step(x[3], a0.w);
+                            step(x[4], a1.x);
+                            step(x[5], a1.y);
+                            step(x[6], a1.z);
+                            step(x[7], a1.w);
+                        };
+                        if (e + 7 < end) {
+                            load(e, w, v, w0, w1);
+                            for (; e + 23 < end; e += 16, w += 16) {
+                                load(e + 8, w + 8, nv, nw0, nw1);
+                                add(v, w0, w1);
+                                load(e + 16, w + 16, v, w0, w1);
+                                add(nv, nw0, nw1);
+                            }
+                            add(v, w0, w1);
+                            e += 8;
+                            w += 8;
+                        }
                     }
-                    for (; e < hi - r0; e++) step(col[e * W4], wl[e + r0 - myOff]);
-                    sums[x] = (u16)h;
+                    for (; e < end; e += 8, w += 8) {  // words past the end 0
+                        uint2 v[8];
+                        u32 wt[8];
+#pragma unroll
+                        for (u32 k = 0; k < 8; k++) {
+                            v[k] = e + k < end ? *reinterpret_cast<const uint2*>(col + (e + k) * W4) : make_uint2(0u, 0u);
+                            wt[k] = e + k < end ? w[k] : 0u;
+                        }
+#pragma unroll
+                        for (u32 k = 0; k < 8; k++) step(v[k], wt[k]);
+                    }
+                    sums[pr * 32 + lane] = h;
                 }
             };
             if (Wc) rounds(m, s, nq, total, per, 0u, W4, W4, walk);
             // the same lanes that formed the sums read them
             if (q < nq) {
-                for (u32 wd = wi; wd < Wc; wd += nwq) {
-                    const u32 x = wd * 32 + lane;
-                    if (x < st.n) f(q, x, ord_f16(myN ? sums[x] : (u16)0));
+                for (u32 pr = wi; pr < pairs; pr += nwq) {
+                    const u32 x = pr * 64 + lane, h = myN ? sums[pr * 32 + lane] : 0u;
+                    if (x < st.n) f(q, x, ord_f16((u16)h));
+                    if (x + 32 < st.n) f(q, x + 32, ord_f16((u16)(h >> 16)));
                 }
                 done(q);
             }
+            if (s.prof) joinx::prof_mark(joinx::PROF_SC_RED);
         } else {
         for (u32 wb = 0; wb < Wc; wb += 32u * nwq) {
             const u32 wp = min(Wc - wb, 32u * nwq), wst = min(W4 - wb, 32u * nwq);  // words of this pass, staged
@@ -406,7 +468,7 @@ struct IndelCluster {
         }
         if (q < nq) done(q);
         }
-        joinx::prof_mark(joinx::PROF_SC_RED);
+        if (s.prof) joinx::prof_mark(joinx::PROF_SC_RED);
     }
 
     // Rebuilds this CTA's words in the other buffer from the live slots' rows.
