@@ -1279,7 +1279,7 @@ static bool cluster_plan(u32 ntip, u32 ncol, u32 nState, bool unitW, joinc::Args
         m.stageWords = least;
         const size_t need = joinc::engine_smem(G, a.R, a.deathWords) + IndelCluster<HALF>::smem_bytes(m, a.R);
         if (need > lim) continue;
-        m.stageWords += (u32)((std::min(lim, need + 65536) - need) / sizeof(u32)) & ~3u;
+        m.stageWords += (u32)((lim - need) / sizeof(u32)) & ~3u;
         *smem = joinc::engine_smem(G, a.R, a.deathWords) + IndelCluster<HALF>::smem_bytes(m, a.R);
         return true;
     }
@@ -1301,7 +1301,8 @@ static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 n
     a.statsOut = L.stats;
     a.prof = getenv("CASPHY_PROFILE") ? L.stats + 8 : nullptr;
     a.ordNeg1 = ORD_F16_NEG1;
-    a.compactMin = a.G * kBitsAlign + 1;  // a range of one 16-byte piece cannot shrink
+    // a range of one 16-byte piece cannot shrink; resident codes can
+    a.compactMin = M::resident_pitch(m, a.R) ? 512u : a.G * kBitsAlign + 1;
     a.bytesPerPairSite = 125;             // one bit per (candidate, query site)
     a.needSizes = minSize > 0;            // the minSize / minRatio rule reads node sizes
     m.minSize = minSize;
@@ -1311,7 +1312,8 @@ static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 n
     m.bits[0] = L.bits0;
     m.bits[1] = L.bits1;
     if (!joinc::placeable((void*)k_cluster_join<M>, a.G, smem)) return CASPHY_OK;
-    k_split_bits<<<dim3(296, a.G), 256, 0, st>>>(L.bits0, m.rows, (ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32),
+    if (!M::resident_pitch(m, a.R))  // (else no CTA reads them)
+        k_split_bits<<<dim3(296, a.G), 256, 0, st>>>(L.bits0, m.rows, (ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32),
                                                  a.R / 32, L.bits1);
     return joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
 }

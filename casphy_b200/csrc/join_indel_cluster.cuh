@@ -15,6 +15,13 @@
 //    codes, and the copies are issued by all threads, where the column scan
 //    had one thread in flight per eight slots (27 slots a CTA at 4,000 cells)
 //    and spent 6.5 us a scan.
+// When a CTA's slots are few (from the start or after a compaction) their codes
+// fit shared memory as bytes, [site][slot], and nothing is copied: a thread
+// compares four slots (HALF: a lane two) with the query's code at a time.  A
+// phase of a 1,024 x 256 tree spent 1.5 of its 4 us on the copies and on folding
+// the bit-sliced counts of many lanes; loops measured with bitsets and with codes:
+// 1,024 x 256 unit 5.78 and 4.94 ms, 1,000 x 300 fractional 5.73 and 4.92 us a
+// join, 4,000 x 500 fractional 27.5 and 24.9 ms.
 // Included by join_indel.cu after the bit-sliced adders.
 #pragma once
 #include "join_cluster.cuh"
@@ -23,6 +30,11 @@ namespace casphy {
 namespace indel {
 
 constexpr u32 kOneCopyWords = 4096;
+constexpr u32 kResidentWords = 384;  // resident codes: words of four slots, at most
+// ... and, for the integer sums, (slot, site) pairs: comparing bytes costs more
+// than adding bits once a phase is not all latency (2,000 x 256 on 16 CTAs, 32,000
+// pairs: 5.1 us a join resident, 5.9 with bitsets; 8,000 x 500, 250,000: 7.8 and 6.8)
+constexpr u32 kResidentUnits = 80000;
 
 template <bool HALF>
 struct IndelCluster {
@@ -39,13 +51,15 @@ struct IndelCluster {
         u32 stageWords;
     };
     struct Smem {
-        u32* eRow;    // maxBatch x ncolW: bitset row of every entry
+        u32* eRow;    // maxBatch x ncolW: bitset row of every entry, or its codes' offset << 8 | code
         u32* eW;      // maxBatch x ncolW: weights (unless all are 1); HALF: in both halves of a word
         u32* stage;   // stageWords
         u32* sums;    // HALF: maxBatch x R / 2 pairs of running sums
+        u32* slab;    // else: 12 planes of 32 words per warp
         u32* B;       // this CTA's bitset rows, `pitch` words each
         u32* other;   // the same in the other buffer
         u32 pitch;
+        u32 rp;       // bytes per site of the resident codes, 0 when there are none
         u32 par;      // parity of the entry counters
         bool prof;    // section times are taken
     };
@@ -57,23 +71,49 @@ struct IndelCluster {
     __host__ __device__ static u32 ncolW(u32 ncol) { return (ncol + 7u) & ~7u; }
     __host__ static size_t smem_bytes(const Args& m, u32 R) {
         return sizeof(u32) * ((size_t)m.maxBatch * ncolW(m.ncol) * (m.unitW ? 1 : 2) + m.stageWords) +
-               (HALF ? sizeof(u16) * (size_t)m.maxBatch * R : 0) + 16;
+               (HALF ? sizeof(u16) * (size_t)m.maxBatch * R : sizeof(u32) * joinc::kWarps * 32 * 12) + 16;
     }
     __device__ static void carve_smem(const joinc::Args&, const Args& m, unsigned char* p, Smem& s) {
         s.stage = reinterpret_cast<u32*>(p);
         s.eRow = s.stage + m.stageWords;
         s.eW = s.eRow + (size_t)m.maxBatch * ncolW(m.ncol);
         s.sums = s.eW + (m.unitW ? 0u : (size_t)m.maxBatch * ncolW(m.ncol));
+        s.slab = s.sums;
         s.par = 0;
     }
     __device__ static u16* rank_space(Smem& s) { return reinterpret_cast<u16*>(s.stage); }
+    // Bytes per site of n slots' resident codes: an odd number of words, so that
+    // a slot's column spreads over the banks; 0 when they do not fit (the codes
+    // a byte, the stage, the partial sums in the slab).
+    __host__ __device__ static u32 resident_pitch(const Args& m, u32 n) {
+        const u32 nw = (n + 3u) / 4u, rp = (nw | 1u) * 4u;
+        return m.nState <= 253u && nw <= kResidentWords && (HALF || (size_t)n * m.ncol <= kResidentUnits) &&
+                       (size_t)m.ncol * rp <= sizeof(u32) * (size_t)m.stageWords
+                   ? rp
+                   : 0u;
+    }
+    // The resident codes of the first n slots from their nodes' rows.
+    __device__ static void load_codes(const Args& m, Smem& s, const joinc::Slots& st, u32 n) {
+        unsigned char* c8 = reinterpret_cast<unsigned char*>(s.stage);
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (u32 x = warp; x < ((n + 3u) & ~3u); x += joinc::kWarps) {
+            const u16* row = m.nodeRow + (size_t)(x < n ? st.node[x] : 0u) * m.ncolP;
+            for (u32 i = 2 * lane; i < m.ncol; i += 64) {
+                const u32 c = x < n ? ld_cg_u32(reinterpret_cast<const u32*>(row + i)) : 0u;
+                c8[i * s.rp + x] = (unsigned char)c;
+                if (i + 1 < m.ncol) c8[(i + 1) * s.rp + x] = (unsigned char)(c >> 16);
+            }
+        }
+    }
     // A CTA's bitset rows lie together, so that its share of the matrix stays
     // as small as its live slots: k_split_bits has laid them out in bits[1].
-    __device__ static void begin(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots&) {
+    __device__ static void begin(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots& st) {
         const size_t region = (size_t)rank * m.rows * (a.R / 32);
         s.B = m.bits[1] + region;
         s.other = m.bits[0] + region;
         s.pitch = a.R / 32;
+        s.rp = resident_pitch(m, st.n);
+        if (s.rp) load_codes(m, s, st, st.n);
         if (threadIdx.x < joinx::kMaxBatch) counts(0)[threadIdx.x] = counts(1)[threadIdx.x] = 0u;
     }
 
@@ -84,7 +124,7 @@ struct IndelCluster {
         const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
         __shared__ u32 s_wc[joinx::kMaxBatch][joinc::kWarps];
         auto put = [&](u32 q, u32 pos, u32 st, u32 code) {
-            s.eRow[(size_t)q * ncolW(m.ncol) + pos] = st * m.nState + code - 2u;
+            s.eRow[(size_t)q * ncolW(m.ncol) + pos] = s.rp ? (st * s.rp) << 8 | code : st * m.nState + code - 2u;
             if (!m.unitW)
                 s.eW[(size_t)q * ncolW(m.ncol) + pos] = m.Wsel[(size_t)(code - 2u) * m.ncol + st] * (HALF ? 0x10001u : 1u);
         };
@@ -175,6 +215,11 @@ struct IndelCluster {
                     for (u32 h = 0; h < 2; h++) {
                         const u32 o = (x >> (16 * h)) & 0xFFFFu, n = (c[0] >> (16 * h)) & 0xFFFFu;
                         if (o == n) continue;
+                        if (s.rp) {
+                            if (site + h < m.ncol)
+                                reinterpret_cast<unsigned char*>(s.stage)[(site + h) * s.rp + own] = (unsigned char)n;
+                            continue;
+                        }
                         const size_t row = (size_t)(site + h) * m.nState;
                         if (o > 1u) atomicAnd(s.B + (row + o - 2u) * s.pitch + word, ~bit);
                         if (n > 1u) atomicOr(s.B + (row + n - 2u) * s.pitch + word, bit);
@@ -300,7 +345,8 @@ struct IndelCluster {
     // The lanes' counts (N planes) of one word summed into all of them, then
     // f(query, slot, score) for the warp's words, lane = slot.
     template <int N, class FN>
-    __device__ static void emit(u32 (&c)[kPlanes], u32 wpw, u32 q, u32 w0, u32 words, const joinc::Slots& st, FN f) {
+    __device__ static void emit(u32 (&c)[kPlanes], u32* slab, u32 wpw, u32 q, u32 w0, u32 words, const joinc::Slots& st,
+                                FN f) {
         const u32 lane = threadIdx.x & 31;
         if (wpw <= 16u) {
             fold<N>(c, 16u);
@@ -315,24 +361,191 @@ struct IndelCluster {
                 }
             }
         }
+        // a word's planes go through shared memory: three 16-byte broadcasts
+        // where a shuffle per plane was ten
         constexpr int F = N + 5 < kPlanes ? N + 5 : kPlanes;
-        // two words at a time, so that their chains of shuffles overlap
-        for (u32 j = 0; j < words; j += 2) {
-            u32 v = 0, w = 0;
-            const u32 j1 = j + 1 < words ? j + 1 : j;
+        constexpr int V = (F + 3) / 4;
+        if (lane < wpw) {
 #pragma unroll
-            for (int k = 0; k < F; k++) {
-                v |= ((__shfl_sync(0xFFFFFFFFu, c[k], j) >> lane) & 1u) << k;
-                w |= ((__shfl_sync(0xFFFFFFFFu, c[k], j1) >> lane) & 1u) << k;
+            for (int k = 0; k < V; k++)
+                reinterpret_cast<uint4*>(slab)[lane * 3 + k] = make_uint4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
+        }
+        __syncwarp();
+        for (u32 j = 0; j < words; j++) {
+            u32 v = 0;
+#pragma unroll
+            for (int k = 0; k < V; k++) {
+                const uint4 p = reinterpret_cast<const uint4*>(slab)[j * 3 + k];
+                v |= ((p.x >> lane) & 1u) << (4 * k) | ((p.y >> lane) & 1u) << (4 * k + 1) |
+                     ((p.z >> lane) & 1u) << (4 * k + 2) | ((p.w >> lane) & 1u) << (4 * k + 3);
             }
             const u32 x = (w0 + j) * 32 + lane;
             if (x < st.n) f(q, x, ord_f16((u16)half_bits_of_int(v)));
-            if (j1 != j && x + 32 < st.n) f(q, x + 32, ord_f16((u16)half_bits_of_int(w)));
         }
+        __syncwarp();
+    }
+
+    // Bytes of x equal to the code repeated in q4, as bit 7 of each byte.
+    __device__ __forceinline__ static u32 equal_bytes(u32 x, u32 q4) {
+        const u32 t = x ^ q4;
+        return ~(((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t);
+    }
+    // The scores from resident codes.
+    template <class F, class D>
+    __device__ static void scores_resident(const Args& m, Smem& s, const joinc::Slots& st, u32 nq, F f, D done) {
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const u32 lgq = nq <= 1 ? 4u : (nq <= 2 ? 3u : (nq <= 4 ? 2u : 1u));
+        const u32 nwq = 1u << lgq, q = warp >> lgq, wi = warp & (nwq - 1u);
+        const u32 nE = q < nq ? counts(s.par)[q] : 0u;
+        const unsigned char* c8 = reinterpret_cast<const unsigned char*>(s.stage);
+        const u32* list = s.eRow + (size_t)(q < nq ? q : 0u) * ncolW(m.ncol);
+        const u32* wl = s.eW + (size_t)(q < nq ? q : 0u) * ncolW(m.ncol);
+        if constexpr (HALF) {
+            // a lane adds two neighbouring slots as a pair, the entries in order
+            if (q < nq) {
+                for (u32 x0 = 64 * wi; x0 < st.n; x0 += 64 * nwq) {
+                    const u32 x = x0 + 2 * lane;
+                    const unsigned char* c = c8 + (x < st.n ? x : x0);
+                    u32 h = 0;
+                    auto step = [&](u32 v, u32 en, u32 wt) {
+                        const u32 eq = equal_bytes(v, __byte_perm(en, 0u, 0x4400u));
+                        u32 mask;  // the two bytes' top bits over a half each
+                        asm("prmt.b32 %0, %1, %1, 0x9988;" : "=r"(mask) : "r"(eq));
+                        asm("add.rn.f16x2 %0, %0, %1;" : "+r"(h) : "r"(wt & mask));
+                    };
+                    u32 e = 0;
+                    uint4 en[2], wt[2], ne[2], nw[2];
+                    u32 v[8], nv[8];
+                    auto load_list = [&](u32 at, uint4 (&a)[2], uint4 (&b)[2]) {
+                        a[0] = *reinterpret_cast<const uint4*>(list + at);
+                        a[1] = *reinterpret_cast<const uint4*>(list + at + 4);
+                        b[0] = *reinterpret_cast<const uint4*>(wl + at);
+                        b[1] = *reinterpret_cast<const uint4*>(wl + at + 4);
+                    };
+                    auto load_codes8 = [&](const uint4 (&a)[2], u32 (&to)[8]) {
+                        const u32 o[8] = {a[0].x, a[0].y, a[0].z, a[0].w, a[1].x, a[1].y, a[1].z, a[1].w};
+#pragma unroll
+                        for (u32 k = 0; k < 8; k++) to[k] = *reinterpret_cast<const u16*>(c + (o[k] >> 8));
+                    };
+                    auto add8 = [&](const uint4 (&a)[2], const uint4 (&b)[2], const u32 (&x8)[8]) {
+                        step(x8[0], a[0].x, b[0].x);
+                        step(x8[1], a[0].y, b[0].y);
+                        step(x8[2], a[0].z, b[0].z);
+                        step(x8[3], a[0].w, b[0].w);
+                        step(x8[4], a[1].x, b[1].x);
+                        step(x8[5], a[1].y, b[1].y);
+                        step(x8[6], a[1].z, b[1].z);
+                        step(x8[7], a[1].w, b[1].w);
+                    };
+                    if (nE >= 8) {
+                        load_list(0, en, wt);
+                        load_codes8(en, v);
+                        for (; e + 23 < nE; e += 16) {  // the next eight are loaded before these are added
+                            load_list(e + 8, ne, nw);
+                            load_codes8(ne, nv);
+                            add8(en, wt, v);
+                            load_list(e + 16, en, wt);
+                            load_codes8(en, v);
+                            add8(ne, nw, nv);
+                        }
+                        add8(en, wt, v);
+                        e += 8;
+                    }
+                    for (; e < nE; e += 8) {  // the rest; past the end a weight of 0
+                        u32 o[8], w8[8];
+#pragma unroll
+                        for (u32 k = 0; k < 8; k++) {
+                            o[k] = e + k < nE ? list[e + k] : 0u;
+                            w8[k] = e + k < nE ? wl[e + k] : 0u;
+                        }
+#pragma unroll
+                        for (u32 k = 0; k < 8; k++) v[k] = *reinterpret_cast<const u16*>(c + (o[k] >> 8));
+#pragma unroll
+                        for (u32 k = 0; k < 8; k++) step(v[k], o[k], w8[k]);
+                    }
+                    if (x < st.n) f(q, x, ord_f16((u16)h));
+                    if (x + 1 < st.n) f(q, x + 1, ord_f16((u16)(h >> 16)));
+                }
+                done(q);
+            }
+        } else {
+            // lanes: words of four slots, lanes that share one when a warp has
+            // more than the words; warps: 32-word chunks, then shares of the
+            // entries.  Counts in 16 bits, bytes 0 and 2 of a word in one half
+            // of the pair, 1 and 3 in the other.
+            const u32 nw = (st.n + 3u) / 4u, chunks = (nw + 31u) / 32u;
+            const u32 lgw = nw > 16u ? 5u : (nw > 8u ? 4u : (nw > 4u ? 3u : 2u));
+            const u32 t = lane & ((1u << lgw) - 1u), sub = lane >> lgw;
+            // warps that share a chunk's entries: a power of two, so that nothing
+            // is divided
+            const u32 lgc = chunks <= 1u ? 0u : 32u - __clz(chunks - 1u);
+            const u32 lgg = lgc < lgq ? lgq - lgc : 0u, wg = 1u << lgg;
+            const u32 NG = wg << (5u - lgw);
+            u32* part = s.slab;
+            if (q < nq) {
+                const u32 g = wi & (wg - 1u);
+                for (u32 ch = wi >> lgg; ch < chunks; ch += nwq >> lgg) {
+                    const u32 word = 32 * ch + t;
+                    u32 lo = 0, hi = 0;
+                    if (word < nw) {
+                        const unsigned char* c = c8 + 4 * word;
+                        // eight entries at a time; past the end code 255, which
+                        // no cell has
+                        for (u32 b = g + wg * sub; b < nE; b += 8 * NG) {
+                            u32 en[8], x[8], acc = 0;
+#pragma unroll
+                            for (u32 k = 0; k < 8; k++) en[k] = b + k * NG < nE ? list[b + k * NG] : 255u;
+#pragma unroll
+                            for (u32 k = 0; k < 8; k++) x[k] = *reinterpret_cast<const u32*>(c + (en[k] >> 8));
+                            if (m.unitW) {
+#pragma unroll
+                                for (u32 k = 0; k < 8; k++)
+                                    acc += (equal_bytes(x[k], __byte_perm(en[k], 0u, 0x0000u)) >> 7) & 0x01010101u;
+                                lo += acc & 0x00FF00FFu;
+                                hi += (acc >> 8) & 0x00FF00FFu;
+                            } else {
+#pragma unroll
+                                for (u32 k = 0; k < 8; k++) {
+                                    const u32 w = b + k * NG < nE ? wl[b + k * NG] : 0u;
+                                    const u32 eq = equal_bytes(x[k], __byte_perm(en[k], 0u, 0x0000u)) >> 7;
+                                    lo += (eq & 0x00010001u) * w;
+                                    hi += ((eq >> 8) & 0x00010001u) * w;
+                                }
+                            }
+                        }
+                    }
+                    for (u32 o = 1u << lgw; o < 32u; o <<= 1) {
+                        lo += __shfl_xor_sync(0xFFFFFFFFu, lo, o);
+                        hi += __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+                    }
+                    if (sub == 0 && word < nw)
+                        reinterpret_cast<uint2*>(part)[((size_t)q * wg + g) * nw + word] = make_uint2(lo, hi);
+                }
+            }
+            __syncthreads();
+            if (q < nq) {
+                const u16* p16 = reinterpret_cast<const u16*>(part) + (size_t)q * wg * nw * 4;
+                for (u32 x = 32 * wi + lane; x - lane < st.n; x += 32 * nwq) {
+                    if (x < st.n) {
+                        const u32 at = (x & ~3u) | ((x & 1u) << 1) | ((x >> 1) & 1u);
+                        u32 v = 0;
+#pragma unroll 8
+                        for (u32 g = 0; g < wg; g++) v += p16[(size_t)g * nw * 4 + at];
+                        f(q, x, ord_f16((u16)half_bits_of_int(v)));
+                    }
+                }
+                done(q);
+            }
+        }
+        if (s.prof) joinx::prof_mark(joinx::PROF_SC_RED);
     }
 
     template <class F, class D>
     __device__ static void scores(const Args& m, Smem& s, const joinc::Slots& st, u32 nq, F f, D done) {
+        if (s.rp) {
+            scores_resident(m, s, st, nq, f, done);
+            return;
+        }
         const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const u32 lgq = nq <= 1 ? 4u : (nq <= 2 ? 3u : (nq <= 4 ? 2u : 1u));
         const u32 nwq = 1u << lgq;  // warps per query
@@ -459,11 +672,12 @@ struct IndelCluster {
                     for (u32 e = lo - r0 + g; e < hi - r0; e += NG) vadd(c, stage[e * pitch], wl[e + r0 - myOff]);
                 }
             });
+            u32* slab = s.slab + warp * 32 * 12;
             const u32 mine = q < nq && wi * wpw < wp ? min(wpw, wp - wi * wpw) : 0u;
-            if (m.unitW && mostLane <= 7u) emit<3>(c, wpw, q, wb + wi * wpw, mine, st, f);
-            else if (m.unitW && mostLane <= 31u) emit<5>(c, wpw, q, wb + wi * wpw, mine, st, f);
-            else if (m.unitW && mostLane <= 127u) emit<7>(c, wpw, q, wb + wi * wpw, mine, st, f);
-            else emit<kPlanes>(c, wpw, q, wb + wi * wpw, mine, st, f);
+            if (m.unitW && mostLane <= 7u) emit<3>(c, slab, wpw, q, wb + wi * wpw, mine, st, f);
+            else if (m.unitW && mostLane <= 31u) emit<5>(c, slab, wpw, q, wb + wi * wpw, mine, st, f);
+            else if (m.unitW && mostLane <= 127u) emit<7>(c, slab, wpw, q, wb + wi * wpw, mine, st, f);
+            else emit<kPlanes>(c, slab, wpw, q, wb + wi * wpw, mine, st, f);
             if (wb + 32u * nwq < Wc) __syncthreads();
         }
         if (q < nq) done(q);
@@ -476,6 +690,12 @@ struct IndelCluster {
     __device__ static void compact(const joinc::Args&, const Args& m, Smem& s, u32, const joinc::Slots& st, u32 n,
                                    const u16*) {
         const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        s.rp = resident_pitch(m, n);
+        if (s.rp) {
+            load_codes(m, s, st, n);
+            __syncthreads();
+            return;
+        }
         u32* B = s.other;
         const u32 pitch = (n + 127u) / 128u * 4u;
         const size_t pieces = (size_t)m.rows * pitch / 4;

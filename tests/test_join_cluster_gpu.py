@@ -22,7 +22,7 @@ def _case(ncell, nsite, nallele, weights, seed):
 
 @pytest.mark.parametrize("weights", ["unit", "integer", "half"])
 @pytest.mark.parametrize("ncell,nsite,nallele", [
-    (2, 1, 2), (3, 5, 3), (33, 7, 4), (128, 31, 9), (129, 64, 9), (257, 1030, 30), (1025, 40, 8), (2049, 33, 12),
+    (2, 1, 2), (3, 5, 3), (33, 7, 4), (128, 31, 9), (129, 64, 9), (257, 1030, 30), (1025, 40, 8), (2049, 33, 12), (700, 90, 300), (1600, 260, 200),
     (4400, 12, 5)])
 def test_cluster_join_vs_oracle(gpu_lib, weights, ncell, nsite, nallele):
     codes, ns, w = _case(ncell, nsite, nallele, weights, seed=ncell + nsite)
