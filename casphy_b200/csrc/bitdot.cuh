@@ -125,21 +125,25 @@ __device__ __forceinline__ void upper_tile(u32 t, u32 tilesN, u32& mb, u32& nb) 
 
 // One tile per CTA.  E::tile(p, m0, n0, taddr) reads the accumulators (eight
 // times the counts; lane l of warp w holds row 32 (w % 4) + l) and is called by
-// all warps of the CTA.
+// all warps of the CTA.  With E::kBatched the grid covers the tiles of many
+// matrices: E::pick(a, p, block) fills in the rows of this block's and returns
+// the tile's index there.
 template <class E>
 __global__ void __launch_bounds__(kThreads, 2) k_bitdot(Args a, typename E::Params p) {
     extern __shared__ __align__(128) unsigned char stage[];
     __shared__ __align__(8) u64 s_bar[2];
     __shared__ u32 s_tmem;
     const u32 tid = threadIdx.x, warp = tid >> 5;
+    u32 index = blockIdx.x;
+    if constexpr (E::kBatched) index = E::pick(a, p, index);
     const u32 mode = a.mode ? *a.mode : 1u;
     if (mode > 1u) return;
     const u32 chunks = mode ? a.chunks : a.negFrom;
     u32 mb, nb;
-    if (a.upper) upper_tile(blockIdx.x, a.tilesN, mb, nb);
+    if (a.upper) upper_tile(index, a.tilesN, mb, nb);
     else {
-        mb = blockIdx.x / a.tilesN;
-        nb = blockIdx.x % a.tilesN;
+        mb = index / a.tilesN;
+        nb = index % a.tilesN;
     }
     const u32 m0 = mb * kM, n0 = nb * kN;
     if (m0 >= a.rowsA) return;  // (an odd number of row tiles)

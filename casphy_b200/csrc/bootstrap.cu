@@ -11,6 +11,9 @@
 // (cal.abs, R/bootstrap_functions.R:190-219).
 //
 // Here all replicates run in one pass:
+//  0. k_bs_ranks: one block per replicate looks up its cells' places in the
+//     full tree and sorts them (they are distinct: a bitmap and its running
+//     counts).
 //  1. k_bs_prep: one warp per (replicate, tip) gathers the tip's row of the
 //     full matrix and builds the replicate's slot matrix and query entries.
 //     When every replicate's weights sum to at most the site count (a
@@ -20,7 +23,9 @@
 //     one entry per word instead of one per (word, weight bit plane).
 //     Otherwise the weights are integer bit planes (the single join's
 //     PLANES path).
-//  2. k_bs_init: the initial all-pairs scan of every replicate, tiles of all
+//  2. The initial all-pairs scan of every replicate.  Unit weights (repeated
+//     columns): shared-bit counts on the tensor cores, all replicates' tiles in
+//     one grid (InitTile).  Bit planes: k_bs_init, popcounts, tiles of all
 //     replicates drawn from one queue.
 //  3. k_bs_join: one thread-block cluster per replicate, largest first, running
 //     the cluster join engine.  The cluster size (one for all replicates) comes
@@ -47,6 +52,7 @@
 #include <queue>
 #include <vector>
 
+#include "bitdot.cuh"
 #include "join_bit_cluster.cuh"
 #include "runtime.h"
 
@@ -72,7 +78,59 @@ struct Rep {
     u32* eQ;
     u32* eLen;
     u32 eStride;
+    uint4* chunks;  // unit weights: the rows as [128-bit chunk][tip], else null
 };
+
+// Places of the replicates' cells in the full tree's tip order, as listed and
+// sorted.  Block r is replicate r; a window of kRankWords words of the bitmap is
+// in shared memory at a time.  (64 replicates of 1,667 to 5,000 cells took a
+// host thread 9.5 ms to sort; this takes 12 us.)
+constexpr u32 kRankThreads = 512, kRankWords = 8192;
+__global__ void __launch_bounds__(kRankThreads) k_bs_ranks(const u32* __restrict__ repOff, const u32* __restrict__ repN,
+                                                           const u32* __restrict__ cells,
+                                                           const u32* __restrict__ rank, u32 ntip, u32* repOfWarp,
+                                                           u32* rankOf, u32* sortedRank, int* twice) {
+    __shared__ u32 s_bits[kRankWords];
+    __shared__ u32 s_warp[kRankThreads / 32];
+    const u32 r = blockIdx.x, off = repOff[r], n = repN[r];
+    const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (u32 i = tid; i < n; i += kRankThreads) {
+        repOfWarp[off + i] = r;
+        rankOf[off + i] = rank[cells[off + i]];
+    }
+    u32 done = 0;
+    for (u32 lo = 0; lo < ntip; lo += 32 * kRankWords) {
+        const u32 words = (min(ntip - lo, 32 * kRankWords) + 31u) / 32u;
+        for (u32 w = tid; w < words; w += kRankThreads) s_bits[w] = 0u;
+        __syncthreads();
+        for (u32 i = tid; i < n; i += kRankThreads) {  // (each thread reads what it wrote)
+            const u32 x = rankOf[off + i] - lo;
+            if (x < 32 * words && (atomicOr(&s_bits[x / 32], 1u << (x & 31u)) >> (x & 31u) & 1u)) *twice = 1;
+        }
+        __syncthreads();
+        const u32 per = (words + kRankThreads - 1) / kRankThreads;
+        const u32 w0 = min(tid * per, words), w1 = min(w0 + per, words);
+        u32 mine = 0;
+        for (u32 w = w0; w < w1; w++) mine += (u32)__popc(s_bits[w]);
+        u32 scan = mine;
+        for (u32 o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xFFFFFFFFu, scan, o);
+            if (lane >= o) scan += y;
+        }
+        if (lane == 31) s_warp[warp] = scan;
+        __syncthreads();
+        u32 before = done, total = 0;
+        for (u32 k = 0; k < kRankThreads / 32; k++) {
+            if (k < warp) before += s_warp[k];
+            total += s_warp[k];
+        }
+        u32 pos = off + before + scan - mine;
+        for (u32 w = w0; w < w1; w++)
+            for (u32 b = s_bits[w]; b; b &= b - 1u) sortedRank[pos++] = lo + 32 * w + (u32)__ffs(b) - 1u;
+        done += total;
+        __syncthreads();  // the next window clears the bitmap
+    }
+}
 
 // Resampled rows: bit b of word j of (replicate r, tip) is the full row's
 // bit colIdx[r][32j+b] (kNone pads).  One warp per (replicate, tip).
@@ -110,9 +168,75 @@ __global__ void k_bs_prep(const Rep* __restrict__ reps, const u32* __restrict__ 
              R.m.planeMask, R.m.nodeSeq, R.m.nodeBis, R.colT, R.eW, R.eQ, R.eLen, R.eStride);
     // initial local maximum: value -1, node ~0 (replaced by the initial scan)
     if ((threadIdx.x & 31) == 0) R.init.initKey[tip] = ((u64)ORD_F32_NEG1 << 32) | 0xFFFFFFFFull;
+    if (R.chunks) {
+        const u32* row = rows + (size_t)warp * nbin;
+        u32* c = reinterpret_cast<u32*>(R.chunks + tip);
+        for (u32 w = threadIdx.x & 31; w < R.m.nbinP; w += 32)
+            c[(size_t)(w / 4) * R.c.ntip * 4 + (w & 3u)] = w < nbin ? row[w] : 0u;
+    }
 }
 
-// initial scan: tiles of all replicates from one queue
+// Initial scan of unit-weight replicates from the shared-bit counts: every
+// row's best column above it, ties to the smaller.  A thread owns a row and a
+// third of the tile's columns; one 64-bit maximum per thread and tile goes to
+// memory.  (64 replicates of 1,667 to 5,000 cells x 512 sites: popcounts took
+// 5.8 ms, this takes 0.37 ms.)
+struct InitTile {
+    static constexpr bool kBatched = true;
+    struct Params {
+        const Rep* reps;
+        const u64* tileStart;  // replicate r's tiles from tileStart[r]
+        u32 nrep;
+        u64 first;             // tile of block 0
+        unsigned long long* key;
+    };
+    __device__ static u32 pick(bitdot::Args& a, Params& p, u32 block) {
+        const u64 t = p.first + block;
+        u32 lo = 0, hi = p.nrep;  // tileStart[lo] <= t < tileStart[hi]
+        while (hi - lo > 1) {
+            const u32 mid = (lo + hi) / 2;
+            if (p.tileStart[mid] <= t) lo = mid;
+            else hi = mid;
+        }
+        const Rep& R = p.reps[lo];
+        a.A = a.B = R.chunks;
+        a.ldA = a.ldB = a.rowsA = a.rowsB = R.c.ntip;
+        a.tilesN = (R.c.ntip + bitdot::kN - 1) / bitdot::kN;
+        p.key = R.init.initKey;
+        return (u32)(t - p.tileStart[lo]);
+    }
+    __device__ static void tile(const bitdot::Args& a, const Params& p, u32 m0, u32 n0, u32 taddr, unsigned char*) {
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wr = warp & 3u;
+        const u32 q = m0 + 32 * wr + lane;
+        int best = -1;
+        u32 at = 0;
+        for (u32 cb = warp >> 2; cb < bitdot::kN / 32; cb += bitdot::kThreads / 128) {
+            const u32 n = n0 + cb * 32;
+            if (n >= a.rowsB || n + 31 <= m0 + 32 * wr) continue;  // no column above any of the warp's rows
+            u32 r[32];
+            bitdot::load32(taddr + (32 * wr << 16) + cb * 32, r);
+            if (n > m0 + 32 * wr + 31 && n + 32 <= a.rowsB) {
+#pragma unroll
+                for (u32 j = 0; j < 32; j++)
+                    if ((int)r[j] > best) {
+                        best = (int)r[j];
+                        at = n + j;
+                    }
+            } else {
+#pragma unroll
+                for (u32 j = 0; j < 32; j++)
+                    if ((int)r[j] > best && n + j > q && n + j < a.rowsB) {
+                        best = (int)r[j];
+                        at = n + j;
+                    }
+            }
+        }
+        if (best >= 0 && q < a.rowsA)
+            atomicMax(p.key + q, (unsigned long long)make_key(ord_f32((float)(best / 8)), at));
+    }
+};
+
+// initial scan with bit planes: tiles of all replicates from one queue
 __global__ void __launch_bounds__(kThreads) k_bs_init(const Rep* __restrict__ reps, const u64* __restrict__ tileStart,
                                                       u32 nrep, unsigned long long* counter) {
     __shared__ unsigned long long s_tile[2];
@@ -191,9 +315,11 @@ __device__ void build_ops(const joinc::Args& c, const u32* __restrict__ rankOf, 
 // Cluster i joins replicate order[i].
 __global__ void __launch_bounds__(joinc::kThreads, 1) k_bs_join(const Rep* __restrict__ reps,
                                                                 const u32* __restrict__ order, u32 G,
-                                                                const u32* __restrict__ rankOf) {
+                                                                const u32* __restrict__ rankOf,
+                                                                const int* __restrict__ initErr) {
     extern __shared__ __align__(16) unsigned char smem[];
     const u32 r = order[blockIdx.x / G], rank = joinc::cluster_rank();
+    if (*initErr) return;  // (an earlier kernel's: the same for all)
     const joinc::Args c = reps[r].c;
     const Model::Args m = reps[r].m;
     const u64 t0 = globaltimer_ns();
@@ -552,12 +678,12 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     struct RepBufs {
         u32 *planeMask, *nodeSeq, *nodeBis, *colT0, *colT1, *nodeSize, *rawEdge;
         u32 *eW, *eQ, *eLen;
+        uint4* chunks;
         unsigned long long* initKey;
         u64* chunkStart;
-        unsigned long long* stats;
     };
     auto rep_layout = [&](Carve& c, u32 n) {
-        RepBufs b;
+        RepBufs b{};
         const u32 Sp = (n + 7u) & ~7u, nnode = 2 * n - 1, nChunks = (n + kCap - 1) / kCap;
         b.planeMask = c.take<u32>((size_t)P * nbin);
         b.nodeSeq = c.take<u32>((size_t)nnode * nbinP);
@@ -566,12 +692,15 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         b.colT1 = c.take<u32>((size_t)nbin * Sp);
         b.nodeSize = c.take<u32>(nnode);
         b.rawEdge = c.take<u32>((size_t)4 * n);
-        b.eW = c.take<u32>((size_t)n * eStride);
-        b.eQ = c.take<u32>((size_t)n * eStride);
-        b.eLen = c.take<u32>(n);
+        if (repeat) {
+            b.chunks = c.take<uint4>((size_t)n * (nbinP / 4));
+        } else {
+            b.eW = c.take<u32>((size_t)n * eStride);
+            b.eQ = c.take<u32>((size_t)n * eStride);
+            b.eLen = c.take<u32>(n);
+            b.chunkStart = c.take<u64>(nChunks + 1);
+        }
         b.initKey = c.take<unsigned long long>(n);
-        b.chunkStart = c.take<u64>(nChunks + 1);
-        b.stats = c.take<unsigned long long>(8);
         return b;
     };
     struct Glob {
@@ -580,8 +709,10 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         u32 *ymin, *ysize, *support;
         u64* tileStart;
         unsigned long long* counter;
+        unsigned long long* stats;
+        u32* rank;
         int* errs;
-        int* xerr;
+        int* xerr;  // post-order stack, a cell listed twice, initial scan
         u32* colIdx;
         u32* rrows;
     };
@@ -606,7 +737,9 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         g.tileStart = c.take<u64>(nrep + 1);
         g.counter = c.take<unsigned long long>(1);
         g.errs = c.take<int>(nrep);
-        g.xerr = c.take<int>(1);
+        g.xerr = c.take<int>(3);
+        g.stats = c.take<unsigned long long>((size_t)8 * nrep);
+        g.rank = c.take<u32>(ntip);
         g.colIdx = c.take<u32>(repeat ? (size_t)nrep * nsite : 1);
         g.rrows = c.take<u32>(repeat ? (size_t)totalTips * nbin : 1);
         return g;
@@ -633,7 +766,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
             const u64 end = std::min<u64>((u64)(k + 1) * kCap, n);
             cs[k + 1] = cs[k] + (end >= 1 ? end - 1 : 0);
         }
-        tileStart[r + 1] = tileStart[r] + cs[nChunks];
+        tileStart[r + 1] = tileStart[r] + (repeat ? bitdot::tiles(n, n, true) : cs[nChunks]);
         Rep& R = reps[r];
         std::memset(&R, 0, sizeof(Rep));
         const RepBufs& b = rb[r];
@@ -643,7 +776,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         smem = std::max(smem, sm);
         c.initKey = b.initKey;
         c.nodeSize = b.nodeSize; c.rawEdge = b.rawEdge; c.err = gl.errs + r;
-        c.limitNs = 20ull * 1000 * 1000 * 1000; c.statsOut = b.stats;
+        c.limitNs = 20ull * 1000 * 1000 * 1000; c.statsOut = gl.stats + (size_t)8 * r;
         c.ordNeg1 = ORD_F32_NEG1; c.compactMin = 256; c.bytesPerPairSite = 4000;
         c.keepSizes = 1;  // build_ops lays out clades by node size
         R.m.ancType = ancestralType ? 1 : 0;
@@ -657,52 +790,48 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         R.off = rep_offsets[r];
         R.ops = gl.ops + repOpsOff[r];
         R.eW = b.eW; R.eQ = b.eQ; R.eLen = b.eLen; R.eStride = eStride;
-    }
-    // host tables: replicate of each tip, ranks, sorted ranks, largest-first order
-    std::vector<u32> repOfWarp(totalTips), rankOf(totalTips), sortedRank(totalTips), repOff(nrep);
-    for (u32 r = 0; r < nrep; r++) {
-        repOff[r] = rep_offsets[r];
-        for (u32 i = rep_offsets[r]; i < rep_offsets[r + 1]; i++) {
-            repOfWarp[i] = r;
-            rankOf[i] = rank[rep_cells[i]];
-        }
-        std::copy(rankOf.begin() + rep_offsets[r], rankOf.begin() + rep_offsets[r + 1], sortedRank.begin() + rep_offsets[r]);
-        std::sort(sortedRank.begin() + rep_offsets[r], sortedRank.begin() + rep_offsets[r + 1]);
-        for (u32 i = rep_offsets[r] + 1; i < rep_offsets[r + 1]; i++)
-            if (sortedRank[i] == sortedRank[i - 1]) {
-                casphy_set_last_error_msg("bootstrap: a replicate lists a cell twice");
-                return CASPHY_EINVAL;
-            }
+        R.chunks = b.chunks;
     }
     cudaStream_t st = 0;
     cudaEvent_t ev[4];
     for (auto& e : ev) CASPHY_CUDA_TRY(cudaEventCreate(&e));
     auto up = [&](void* d, const void* h, size_t n) { return cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, st); };
     // per-replicate plane masks and tile tables
-    for (u32 r = 0; r < nrep; r++) {
+    for (u32 r = 0; r < nrep && !repeat; r++) {
         const RepBufs& b = rb[r];
         const u32 nChunks = (u32)chunkStarts[r].size() - 1;
         CASPHY_CUDA_TRY(up(b.planeMask, planes.data() + (size_t)r * P * nbin, sizeof(u32) * P * nbin));
         CASPHY_CUDA_TRY(up(b.chunkStart, chunkStarts[r].data(), sizeof(u64) * (nChunks + 1)));
     }
     CASPHY_CUDA_TRY(up(gl.reps, reps.data(), sizeof(Rep) * nrep));
-    CASPHY_CUDA_TRY(up(gl.repOfWarp, repOfWarp.data(), 4ull * totalTips));
     CASPHY_CUDA_TRY(up(gl.cells, rep_cells, 4ull * totalTips));
     CASPHY_CUDA_TRY(up(gl.words, words, 4ull * ntip * nbin));
     CASPHY_CUDA_TRY(up(gl.order, order.data(), 4ull * nrep));
-    CASPHY_CUDA_TRY(up(gl.rankOf, rankOf.data(), 4ull * totalTips));
-    CASPHY_CUDA_TRY(up(gl.sortedRank, sortedRank.data(), 4ull * totalTips));
+    CASPHY_CUDA_TRY(up(gl.rank, rank.data(), 4ull * ntip));
     CASPHY_CUDA_TRY(up(gl.Xlo, Xlo.data(), 4ull * nX));
     CASPHY_CUDA_TRY(up(gl.Xhi, Xhi.data(), 4ull * nX));
     CASPHY_CUDA_TRY(up(gl.repN, repN.data(), 4ull * nrep));
-    CASPHY_CUDA_TRY(up(gl.repOff, repOff.data(), 4ull * nrep));
+    CASPHY_CUDA_TRY(up(gl.repOff, rep_offsets, 4ull * nrep));
     CASPHY_CUDA_TRY(up(gl.repOpsOff, repOpsOff.data(), 4ull * nrep));
     CASPHY_CUDA_TRY(up(gl.tileStart, tileStart.data(), 8ull * (nrep + 1)));
     CASPHY_CUDA_TRY(cudaMemsetAsync(gl.support, 0, 4ull * nX, st));
     CASPHY_CUDA_TRY(cudaMemsetAsync(gl.counter, 0, sizeof(unsigned long long), st));
     CASPHY_CUDA_TRY(cudaMemsetAsync(gl.errs, 0, sizeof(int) * nrep, st));
-    CASPHY_CUDA_TRY(cudaMemsetAsync(gl.xerr, 0, sizeof(int), st));
+    CASPHY_CUDA_TRY(cudaMemsetAsync(gl.xerr, 0, 3 * sizeof(int), st));
     if (repeat) CASPHY_CUDA_TRY(up(gl.colIdx, colIdx.data(), 4ull * nrep * nsite));
+    k_bs_ranks<<<nrep, kRankThreads, 0, st>>>(gl.repOff, gl.repN, gl.cells, gl.rank, ntip, gl.repOfWarp, gl.rankOf,
+                                              gl.sortedRank, gl.xerr + 1);
+    CASPHY_CUDA_TRY(cudaGetLastError());
+    int twice = 0;
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(&twice, gl.xerr + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+    if (twice) {
+        for (auto& e : ev) cudaEventDestroy(e);
+        casphy_set_last_error_msg("bootstrap: a replicate lists a cell twice");
+        return CASPHY_EINVAL;
+    }
+    CASPHY_CUDA_TRY(cudaFuncSetAttribute((void*)bitdot::k_bitdot<InitTile>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)bitdot::kSmemBytes));
     int perSM = 0;
     CASPHY_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_bs_init, kThreads, 0));
     // (the planned size may have shrunk to what the replicates need)
@@ -710,7 +839,9 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     XferArgs xa{nX, nrep, 32u * ((ntip + 31) / 32), gl.Xlo, gl.Xhi, gl.repN, gl.repOff, gl.repOpsOff, gl.sortedRank, gl.ops,
                 threshold, gl.ymin, gl.ysize, gl.support, gl.xerr};
     // the whole pass: prep, initial scans, the joins, transfer
-    const u64 launches = (repeat ? 1 : 0) + 4;
+    constexpr u64 kGrid = 1ull << 30;  // tiles per launch
+    const u64 nTile = tileStart[nrep];
+    const u64 launches = 4 + (repeat ? 1 + (nTile + kGrid - 1) / kGrid : 1);
     auto enqueue = [&](cudaStream_t s) -> cudaError_t {
         cudaError_t e;
         if ((e = cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal)) != cudaSuccess) return e;
@@ -719,11 +850,21 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
                                                           gl.rrows);
         k_bs_prep<<<(totalTips + 7) / 8, 256, 0, s>>>(gl.reps, gl.repOfWarp, gl.cells, gl.words,
                                                       repeat ? gl.rrows : nullptr, nbin, totalTips);
-        k_bs_init<<<nSM * std::max(perSM, 1), kThreads, 0, s>>>(gl.reps, gl.tileStart, nrep, gl.counter);
+        if (repeat) {
+            bitdot::Args a{};
+            a.chunks = a.negFrom = nbinP / 4;
+            a.upper = 1;
+            a.err = gl.xerr + 2;
+            for (u64 t = 0; t < nTile; t += kGrid)
+                bitdot::k_bitdot<InitTile><<<(u32)std::min(kGrid, nTile - t), bitdot::kThreads, bitdot::kSmemBytes, s>>>(
+                    a, InitTile::Params{gl.reps, gl.tileStart, nrep, t, nullptr});
+        } else {
+            k_bs_init<<<nSM * std::max(perSM, 1), kThreads, 0, s>>>(gl.reps, gl.tileStart, nrep, gl.counter);
+        }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal)) != cudaSuccess) return e;
         if ((e = joinc::enqueue(k_bs_join, G, nrep, smem, s, (const Rep*)gl.reps, (const u32*)gl.order, G,
-                                (const u32*)gl.rankOf)) != cudaSuccess)
+                                (const u32*)gl.rankOf, (const int*)(gl.xerr + 2))) != cudaSuccess)
             return e;
         if ((e = cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal)) != cudaSuccess) return e;
         k_bs_transfer<<<dim3((nX + kXThreads - 1) / kXThreads, nrep), kXThreads, 0, s>>>(xa);
@@ -731,7 +872,6 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         return cudaEventRecordWithFlags(ev[3], s, cudaEventRecordExternal);
     };
     // run it as one captured CUDA graph; launch directly if capture fails
-    CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
     bool graphed = false;
     {
         cudaStream_t cs = nullptr;
@@ -751,9 +891,9 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     }
     if (!graphed) CASPHY_CUDA_TRY(enqueue(st));
     std::vector<int> errs(nrep);
-    int xerr = 0;
+    int xerr[3] = {0, 0, 0};
     CASPHY_CUDA_TRY(cudaMemcpyAsync(errs.data(), gl.errs, sizeof(int) * nrep, cudaMemcpyDeviceToHost, st));
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(&xerr, gl.xerr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(xerr, gl.xerr, sizeof(xerr), cudaMemcpyDeviceToHost, st));
     CASPHY_CUDA_TRY(cudaMemcpyAsync(support, gl.support, 4ull * nX, cudaMemcpyDeviceToHost, st));
     if (ymin_out) CASPHY_CUDA_TRY(cudaMemcpyAsync(ymin_out, gl.ymin, 4ull * nrep * nX, cudaMemcpyDeviceToHost, st));
     if (ysize_out) CASPHY_CUDA_TRY(cudaMemcpyAsync(ysize_out, gl.ysize, 4ull * nrep * nX, cudaMemcpyDeviceToHost, st));
@@ -766,9 +906,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         }
     }
     std::vector<unsigned long long> hst((size_t)8 * nrep);
-    for (u32 r = 0; r < nrep; r++)
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(hst.data() + 8 * r, rb[r].stats, sizeof(unsigned long long) * 8,
-                                        cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaMemcpyAsync(hst.data(), gl.stats, sizeof(unsigned long long) * hst.size(), cudaMemcpyDeviceToHost, st));
     CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
     unsigned long long phases = 0;
     std::vector<double> repUs(nrep, 0.0);
@@ -782,13 +920,17 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         longest = std::max(longest, repUs[r]);
         busy += repUs[r] * G;
     }
+    if (xerr[2]) {
+        casphy_set_last_error_msg("bootstrap: a device-side wait timed out");
+        return xerr[2];
+    }
     for (u32 r = 0; r < nrep; r++)
         if (errs[r]) {
             casphy_set_last_error_msg(errs[r] == CASPHY_ETIMEOUT ? "bootstrap: a replicate join timed out"
                                                                   : "bootstrap: a replicate join failed");
             return errs[r];
         }
-    if (xerr) {
+    if (xerr[0]) {
         casphy_set_last_error_msg("bootstrap: post-order stack overflow");
         return CASPHY_EINTERNAL;
     }

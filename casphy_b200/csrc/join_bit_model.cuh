@@ -271,7 +271,8 @@ struct BitModel {
 };
 
 // One warp prepares tip `tip` from its row `src`: node rows (seq = input,
-// bistate = 0), its column of the slot matrix and its query entries.
+// bistate = 0), its column of the slot matrix and its query entries (none when
+// eW is null).
 __device__ __forceinline__ void prep_tip(const u32* __restrict__ src, u32 tip, u32 nbin, u32 nbinP, u32 Sp,
                                          u32 nplanes, const u32* __restrict__ planeMask, u32* nodeSeq, u32* nodeBis,
                                          u32* colT, u32* eW, u32* eQ, u32* eLen, u32 eStride) {
@@ -286,6 +287,7 @@ __device__ __forceinline__ void prep_tip(const u32* __restrict__ src, u32 tip, u
             nodeBis[(size_t)tip * nbinP + w] = 0u;
         }
         if (w < nbin) colT[(size_t)w * Sp + tip] = v;
+        if (!eW) continue;
         for (u32 k = 0; k < P; k++) {
             const u32 m = nplanes ? (v & (w < nbin ? planeMask[(size_t)k * nbin + w] : 0u)) : v;
             const u32 bal = __ballot_sync(0xFFFFFFFFu, m != 0u);
@@ -297,7 +299,7 @@ __device__ __forceinline__ void prep_tip(const u32* __restrict__ src, u32 tip, u
             n += __popc(bal);
         }
     }
-    if (lane == 0) eLen[tip] = n;
+    if (lane == 0 && eW) eLen[tip] = n;
 }
 
 // Entries of one tip are ordered by plane inside each 32-word block; the

@@ -205,6 +205,7 @@ __global__ void k_pack_bits(const u32* __restrict__ planes, u32 ntip, u32 nwords
 // tile's rows as mask words and, when every pair is computed once, of its
 // columns too.
 struct RadiusTile {
+    static constexpr bool kBatched = false;
     struct Params {
         int least8;  // eight times the least count that is a hit
         u32 maskWords, mirror;

@@ -25,6 +25,7 @@ namespace casphy {
 namespace tdis {
 
 struct TransferTile {
+    static constexpr bool kBatched = false;
     struct Params {
         u32 full, pad;  // 32 ncol, and the bits past ntip
         const u32* cx;  // popcounts of the rows
