@@ -778,6 +778,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         c.nodeSize = b.nodeSize; c.rawEdge = b.rawEdge; c.err = gl.errs + r;
         c.limitNs = 20ull * 1000 * 1000 * 1000; c.statsOut = gl.stats + (size_t)8 * r;
         c.ordNeg1 = ORD_F32_NEG1; c.compactMin = 256; c.bytesPerPairSite = 4000;
+        R.m.compactAt = 12;  // a few CTAs per tree, many slots each: 8 took 31.8 ms where this takes 31.0
         c.keepSizes = 1;  // build_ops lays out clades by node size
         R.m.ancType = ancestralType ? 1 : 0;
         R.m.planeMask = b.planeMask;

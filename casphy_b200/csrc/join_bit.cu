@@ -128,7 +128,7 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     a.bytesPerPairSite = c.bytesPerPairSite;
     a.deathWords = (c.nnode + 31) / 32;
     typename M::Args m{bm.nbin, bm.nbinP, bm.nplanes, bm.ancType, bm.planeMask, bm.wf, bm.nodeSeq, bm.nodeBis,
-                       {bm.colT[0], bm.colT[1]}, Sp, 0, 0};
+                       {bm.colT[0], bm.colT[1]}, Sp, 0, 0, 8};
     size_t smem = 0;
     if (!cluster_fit<PATH>(a, m, (size_t)smemMax - 6144, &smem)) return CASPHY_OK;
     if (PATH != PATH_FLOAT && m.colWords < (size_t)m.nbin * a.R) return CASPHY_OK;

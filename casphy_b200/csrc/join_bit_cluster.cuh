@@ -31,6 +31,7 @@ struct BitCluster {
         u32* colT[2];          // nbin x Sp
         u32 Sp, maxBatch;
         u32 colWords;          // shared-memory words for resident columns
+        u32 compactAt;         // sixteenths of the slots still live at a compaction
     };
     struct Smem {
         u32* sq;       // maxBatch x planes x nbinP: (plane-masked) query words
@@ -281,6 +282,7 @@ struct BitCluster {
         if (s.prof) joinx::prof_mark(joinx::PROF_SC_ACC);
     }
 
+    __device__ static u32 compact_at(const Args& m, u32) { return m.compactAt; }
     // Moves the live slots' columns to their new places; n live slots, ranks
     // by old slot.  In shared memory in place, a warp per column: a slot only
     // moves down, and 32 are read before any of them is written.

@@ -409,7 +409,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
         algMilli += (unsigned long long)a.bytesPerPairSite * nE * ((a.ntip - k - 1) - 1);
         k++;
         const u32 alive = a.ntip - k;
-        if (S >= a.compactMin && 2 * alive < S && k < nJoin) {
+        if (S >= a.compactMin && 16 * alive < M::compact_at(m, S) * S && k < nJoin) {
             if (G > 1) cluster_sync();  // the model may read the row CTA 0 has just stored
             else __syncthreads();
             // squeeze this CTA's slots, in order: a slot only moves down, and

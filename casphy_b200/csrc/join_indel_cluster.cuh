@@ -685,6 +685,12 @@ struct IndelCluster {
         if (s.prof) joinx::prof_mark(joinx::PROF_SC_RED);
     }
 
+    // Sixteenths of the slots that are still live when the dead are squeezed
+    // out; the same for all CTAs (so nothing of this CTA's slots goes in).
+    // Scans of fewer dead slots pay for clearing all bitset rows, unless there
+    // are many rows a slot: 40,000 x 1,024 x 256 alleles 464 ms at 8 and 433 at
+    // 12, 8,000 x 500 x 64 55.0 and 52.8, but 12,345 x 777 x 256 99.7 and 101.2.
+    __device__ static u32 compact_at(const Args& m, u32 S) { return m.rows <= 8u * S ? 12u : 8u; }
     // Rebuilds this CTA's words in the other buffer from the live slots' rows.
     // The engine has moved st.node already; n live slots.
     __device__ static void compact(const joinc::Args&, const Args& m, Smem& s, u32, const joinc::Slots& st, u32 n,
