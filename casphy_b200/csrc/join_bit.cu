@@ -10,6 +10,8 @@
 //    sites whose weight has bit k, score = sum_k 2^k popcount(q & mask_k & c).
 //  * FLOAT (anything else): per candidate, the matching bits are visited in
 //    ascending order and added in binary32, as the reference does.
+// Trees whose slots' columns fit the shared memory of one thread-block cluster
+// are joined there (join_bit_cluster.cuh), larger ones on all SMs.
 // Node state is the (seq, bistate) pair of cu/joinEdgeBitReverse.cu:77-113;
 // rows are output as seq & ~bistate (:115-121).  Candidate rows live
 // column-major by slot (word w of slots c..c+3 is one 16-byte load).

@@ -1,4 +1,5 @@
-// Persistent greedy-join engine shared by the indel and bit joins.
+// Persistent greedy-join engine of the indel and bit joins on all SMs, for trees
+// that one cluster cannot hold (smaller ones: join_cluster.cuh).
 //
 // The reference joins (cu/joinEdgeIndel.cu:376-468, cu/joinEdgeBitReverse.cu:
 // 404-505) repeat: take the global best local maximum (larger value, then
@@ -73,7 +74,6 @@ struct Common {
     u32 maxBatch;         // stale rows per rescan phase, 1..kMaxBatch
     u32 deathWords;       // words of the per-CTA shared-memory bitmap of joined nodes (0: none)
     u32 needSizes;        // the model's join reads the two node sizes (minSize > 0)
-    u32 keepSizes;        // the caller reads nodeSize of new nodes after the loop (bootstrap clade layout)
     u32 preSlots;         // a join's scan prefetches its slots' node, maximum and partner into shared memory
     unsigned long long* prof;  // nullable: CTA 0 section times (ns), see PROF_*
 };
@@ -503,21 +503,14 @@ __device__ __forceinline__ void join_run(const Common& a, const typename M::Args
         const u32 j1 = key_node(g.key), c1 = g.slot, j2 = g.partner;
         if (c1 >= rg.S || j1 >= a.nnode || j2 >= a.nnode) { fail = CASPHY_EINTERNAL; break; }
         // With the joined-node bitmap and no size rule, the decision needs no
-        // load: the partner's slot (and, for callers that read the new node's
-        // size, the two node sizes) is loaded by thread 0 and first used after
-        // the query build, which hides its latency.
+        // load: the partner's slot is loaded by thread 0 and first used after the
+        // query build, which hides its latency.
         const bool quick = a.deathWords && !a.needSizes;
         bool stale;
-        u32 c2 = 0, s1 = 0, s2 = 0, c2pending = 0, s1pending = 0, s2pending = 0;
+        u32 c2 = 0, s1 = 0, s2 = 0, c2pending = 0;
         if (quick) {
             stale = (deathBits[j2 >> 5] >> (j2 & 31)) & 1u;
-            if (!stale && threadIdx.x == 0) {
-                c2pending = ld_cg_u32(a.node2slot + j2);
-                if (a.keepSizes) {
-                    s1pending = ld_cg_u32(a.nodeSize + j1);
-                    s2pending = ld_cg_u32(a.nodeSize + j2);
-                }
-            }
+            if (!stale && threadIdx.x == 0) c2pending = ld_cg_u32(a.node2slot + j2);
         } else {
             if (threadIdx.x == 0) {
                 s_val[0] = ld_cg_u32(a.nodeDeath + j2);
@@ -650,8 +643,8 @@ __device__ __forceinline__ void join_run(const Common& a, const typename M::Args
         if (quick) {
             if (threadIdx.x == 0) {
                 s_val[1] = c2pending;
-                s_val[2] = s1pending;
-                s_val[3] = s2pending;
+                s_val[2] = 0u;
+                s_val[3] = 0u;
             }
             __syncthreads();
             c2 = s_val[1];

@@ -18,11 +18,10 @@
 //    launch over (candidate chunk, query) tiles in chunk-major order: a 4096-
 //    candidate chunk stays in L2 while every earlier query streams it, and the
 //    per-query best is merged with a 64-bit atomicMax on (score, ~node) keys.
-//  * The join loop (cu/joinEdgeIndel.cu:376-468) runs in the persistent join
-//    engine (join_engine.cuh) with the IndelDense model below: every CTA
-//    merges the two children itself, builds the query site list in shared
-//    memory and scores its own slots.  Dead slots are squeezed out of the
-//    column matrix whenever fewer than 3/4 of the slots are alive.
+//  * The join loop (cu/joinEdgeIndel.cu:376-468) runs on one thread-block
+//    cluster (join_cluster.cuh) for trees it can hold and in the engine of all
+//    SMs (join_engine.cuh) beyond: every CTA merges the two children itself,
+//    builds the query site list in shared memory and scores its own slots.
 //  * Pre-order relabelling (cu/joinEdgeIndel.cu:488-558) walks the 2(N-1)
 //    raw edges on the host in O(N) and gathers the state rows on device.
 #include <algorithm>

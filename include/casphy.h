@@ -47,13 +47,14 @@ typedef struct {
     uint64_t compactions;        /* slot-matrix compactions */
     uint64_t kernel_launches;    /* kernels launched by this call */
     uint32_t int_path;           /* 1: exact integer accumulation was used */
-    uint32_t scan_path;          /* indel: 0 column-major codes, 1 allele bitsets */
+    uint32_t scan_path;          /* indel: 0 column-major codes, 1 allele bitsets
+                                    (fractional weights: on one cluster only) */
     double init_scan_ms;         /* device time, initial all-pairs scan */
     double join_loop_ms;         /* device time, persistent join loop */
     double total_ms;             /* device time of the whole call */
     uint64_t alg_bytes_init;     /* algorithmic bytes of the initial scan */
     uint64_t alg_bytes_join;     /* algorithmic bytes of the join-loop scans */
-    uint64_t phases;             /* grid-wide phases of the join loop */
+    uint64_t phases;             /* phases of the join loop */
     uint64_t refreshes;          /* republish phases (exhausted per-CTA lists) */
 } casphy_join_stats;
 
@@ -215,8 +216,8 @@ typedef struct {
                                    including a speculated unit step that the
                                    accept then discards */
     uint32_t site_chunks;
-    uint32_t levels_inside;     /* tree height (inside launches per chunk) */
-    uint32_t levels_outside;    /* depth levels (outside launches per chunk) */
+    uint32_t levels_inside;     /* tree height (narrow levels share a launch) */
+    uint32_t levels_outside;    /* the same levels, downwards */
     uint32_t reserved;
     double loglik_start, loglik_end;
     double seconds;             /* device time of the whole optimisation */
@@ -344,17 +345,17 @@ int casphy_ancestral_char(uint32_t ntip, uint32_t nnode, uint32_t nsite, const i
  *   rep_raw_edges optional: per replicate, 2*(n_r-1) raw join edges (parent,
  *                child) in join order over the replicate's tip ids
  * Each replicate tree is the tree joinEdgeBitReverse builds from its rows and
- * weights (the same engine as casphy_join_bit).  The CTAs joining each
- * replicate come from a cost model refitted after every call on the device;
- * the environment variable CASPHY_BS_GROUP=g fixes g of them (at most 8) for
- * every replicate of 512 cells or more instead.
+ * weights (the same engine as casphy_join_bit).  Every replicate is joined by
+ * one thread-block cluster; the clusters' size, the same for all, comes from a
+ * cost model refitted after every call on the device, or from the environment
+ * variable CASPHY_BS_GROUP=g: the largest power of two up to g and 8.
  */
 typedef struct {
     uint32_t nrep, nclade;
     double prep_ms, join_ms, transfer_ms, total_ms;  /* device times */
     uint64_t kernel_launches;
     uint64_t join_phases;                            /* summed over replicates */
-    uint32_t max_ctas_per_rep;                       /* CTAs the largest replicate's join used */
+    uint32_t max_ctas_per_rep;                       /* CTAs of a replicate's cluster */
     uint32_t tuned;                                  /* 1 when the split came from measured costs */
     double join_longest_ms;                          /* longest single replicate join */
     double join_busy_ms;                             /* replicate joins summed (CTA-time) */
