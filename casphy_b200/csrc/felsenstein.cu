@@ -8,9 +8,9 @@
 // power-of-two renormalisation per (node, site), the exponent carried as an
 // integer; the per-site log likelihood and its sum are binary64.
 //
-// Inside pass: internal nodes grouped by height, one launch per height, one
-// thread per (node, site).  Outside pass: the same groups of internal nodes,
-// one launch per height, highest first; for each child edge c of node p it forms
+// Inside pass: internal nodes grouped by height, one launch per height (the
+// narrow levels near the root share one), one thread per (node, site).  Outside
+// pass: the same groups of internal nodes, highest first; for each child edge c of node p it forms
 // R = U_p * M_sibling and the site term w_s (R . dM_c/dt) / (R . M_c) of
 // d log L / d t_c, then passes U_c = R P_c down.  Both ratios are invariant
 // to the scale of R, so outside vectors are renormalised freely.  Site terms
@@ -23,9 +23,10 @@
 // graph and replayed for every evaluation.
 //
 // Branch lengths are optimised over x = log t by L-BFGS in binary64 on the
-// device: the two-loop recursion and the history update run as cooperative
-// one-CTA-per-SM kernels whose grid reductions sum per-CTA partials in a
-// fixed order behind a bounded flag barrier; the host only reads back the
+// device: the two-loop recursion and the history update run on one cluster, or
+// for many edges as cooperative one-CTA-per-SM kernels whose grid reductions sum
+// per-CTA partials in a fixed order behind a bounded flag barrier, with the same
+// grouping; the host only reads back the
 // scalars the Armijo line search needs.  The "plain" variant replaces the
 // adjoint gradient by per-edge central differences of log L (2 evaluations
 // per edge) and is otherwise identical.
@@ -518,9 +519,14 @@ __global__ void __launch_bounds__(kSites) k_loglik_irr(u32 root, Tree T, IrrBuf 
 }
 
 // One (node, site) of the outside pass: both children's site terms in gsum and
-// their outside vectors stored.
+// their outside vectors stored; eds: the child edges, the second from edB() where
+// it is first needed (loaded by the caller before, it held the wide kernel at 46
+// registers and five blocks an SM: 6.65 ms an evaluation of a 200,000 x 1,024
+// tree, 6.1 with 40 and six).
+template <class EB>
 __device__ __forceinline__ void outside_irr_site(u32 root, const Tree& T, const IrrBuf& B, const Chunk& C, uint4 nf,
-                                                 u32 edB, u32 s, const double* __restrict__ w, float (&gsum)[2]) {
+                                                 EB edB, u32 s, const double* __restrict__ w, float (&gsum)[2],
+                                                 u32 (&eds)[2]) {
     const u32 v = nf.x, vi = v - T.ntip;
     const bool ok = s < C.w;
     const u32 ss = ok ? s : 0, gs = C.s0 + ss;
@@ -534,7 +540,8 @@ __device__ __forceinline__ void outside_irr_site(u32 root, const Tree& T, const 
         aY = __float_as_int(u.w);
     }
     const u32 kids[2] = {nf.y, nf.z};
-    const u32 eds[2] = {nf.w, edB};
+    eds[0] = nf.w;
+    eds[1] = edB();
     float4 l[2];
     float m0[2], qs[2];
     float2 pp[2];
@@ -597,9 +604,9 @@ __global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf
     __shared__ float2 red[kSites / 32];
     const u32 s = blockIdx.x * kSites + threadIdx.x;
     const uint4 nf = T.outInfo[off + blockIdx.y];
-    const u32 eds[2] = {nf.w, T.outEdgeB[off + blockIdx.y]};
+    u32 eds[2];
     float gsum[2];
-    outside_irr_site(root, T, B, C, nf, eds[1], s, w, gsum);
+    outside_irr_site(root, T, B, C, nf, [&] { return T.outEdgeB[off + blockIdx.y]; }, s, w, gsum, eds);
     // site terms in binary32 within the block; blocks are added in binary64
     const float2 g = block_sum2f(gsum[0], gsum[1], red);
     if (threadIdx.x == 0) {
@@ -762,7 +769,8 @@ __global__ void __launch_bounds__(32 * kTopWarps) k_outside_top_irr(u32 root, Tr
         lv, T.outInfo, T.outEdgeB, [&](uint4, u32, u32) { return In{}; },
         [&](uint4 nf, u32 eB, u32, const In&) {
             float g[2];
-            outside_irr_site(root, T, B, C, nf, eB, s, w, g);
+            u32 eds[2];
+            outside_irr_site(root, T, B, C, nf, [&] { return eB; }, s, w, g, eds);
             warp_terms(g, C, nf.w, eB, nsite32, gw);
         });
 }
