@@ -273,9 +273,12 @@ struct OpsNode {
     u32 a, b, ta, tb, ra, rb;  // children, their tips and, for tips, their ranks
 };
 __host__ __device__ inline size_t ops_smem(u32 n) { return sizeof(OpsNode) * kOpsStage + sizeof(u32) * (size_t)n; }
-__device__ void build_ops(const joinc::Args& c, const u32* __restrict__ rankOf, u32* ops, unsigned char* smem) {
-    OpsNode* stage = reinterpret_cast<OpsNode*>(smem);
-    u32* s = reinterpret_cast<u32*>(stage + kOpsStage);
+constexpr size_t kOpsMost = 231424;  // bytes of a replicate's offsets, at most: 57,856 cells
+// The offsets s: in shared memory after the stage or, for replicates beyond
+// about 53,000 cells, in memory.
+template <class S>
+__device__ __forceinline__ void build_ops(const joinc::Args& c, const u32* __restrict__ rankOf, u32* ops, OpsNode* stage,
+                                          S s) {
     const u32 n = c.ntip, root = 2 * n - 2;
     if (threadIdx.x == 0) s[root - n] = 0;
     for (u32 top = n - 1; top > 0;) {  // nodes n + top - 1 down
@@ -316,7 +319,7 @@ __device__ void build_ops(const joinc::Args& c, const u32* __restrict__ rankOf, 
 __global__ void __launch_bounds__(joinc::kThreads, 1) k_bs_join(const Rep* __restrict__ reps,
                                                                 const u32* __restrict__ order, u32 G,
                                                                 const u32* __restrict__ rankOf,
-                                                                const int* __restrict__ initErr) {
+                                                                const int* __restrict__ initErr, u32 opsShared) {
     extern __shared__ __align__(16) unsigned char smem[];
     const u32 r = order[blockIdx.x / G], rank = joinc::cluster_rank();
     if (*initErr) return;  // (an earlier kernel's: the same for all)
@@ -329,7 +332,13 @@ __global__ void __launch_bounds__(joinc::kThreads, 1) k_bs_join(const Rep* __res
     int err = 0;
     if (threadIdx.x == 0) err = *(volatile int*)c.err;
     if (__syncthreads_or(err)) return;
-    build_ops(c, rankOf + reps[r].off, reps[r].ops, smem);
+    OpsNode* stage = reinterpret_cast<OpsNode*>(smem);
+    if (opsShared) {
+        build_ops(c, rankOf + reps[r].off, reps[r].ops, stage, reinterpret_cast<u32*>(smem + sizeof(OpsNode) * kOpsStage));
+    } else {  // (the initial keys have been read)
+        build_ops(c, rankOf + reps[r].off, reps[r].ops, stage,
+                  reinterpret_cast<volatile u32*>(const_cast<unsigned long long*>(c.initKey)));
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         c.statsOut[6] = t0;
@@ -652,6 +661,12 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     std::iota(order.begin(), order.end(), 0u);
     std::stable_sort(order.begin(), order.end(), [&](u32 a, u32 b) { return repN[a] > repN[b]; });
     for (u32 r = 0; r < nrep; r++) sorted[r] = repN[order[r]];
+    if (4 * (size_t)nmax > kOpsMost) {
+        casphy_set_last_error_msg("bootstrap: replicate too large");
+        return CASPHY_ERANGE;
+    }
+    const u32 opsShared = ops_smem(nmax) <= smemLim ? 1u : 0u;
+    const size_t opsBytes = opsShared ? ops_smem(nmax) : ops_smem(0);
     u32 G = 0, fixedG = 0;
     if (const char* env = std::getenv("CASPHY_BS_GROUP"))  // a fixed size, at most 8 (the cost model is bypassed)
         for (fixedG = 1; fixedG < 8 && (int)(2 * fixedG) <= std::atoi(env);) fixedG *= 2;
@@ -661,8 +676,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         Model::Args m{};
         size_t sm = 0;
         if (!plan(nmax, g, a, m, &sm)) continue;
-        sm = std::max(sm, ops_smem(nmax));
-        if (sm > smemLim) continue;
+        sm = std::max(sm, opsBytes);
         const int slots = joinc::placeable((void*)k_bs_join, g, sm);
         if (slots < 1) continue;
         const double t = g == fixedG ? 0.0 : makespan_us(tune, sorted, g, (u32)slots);
@@ -756,7 +770,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     std::vector<RepBufs> rb(nrep);
     std::vector<u64> tileStart(nrep + 1, 0), chunkAll;
     std::vector<std::vector<u64>> chunkStarts(nrep);
-    size_t smem = ops_smem(nmax);
+    size_t smem = opsBytes;
     for (u32 r = 0; r < nrep; r++) {
         rb[r] = rep_layout(c2, repN[r]);
         const u32 n = repN[r], Sp = (n + 7u) & ~7u, nChunks = (n + kCap - 1) / kCap;
@@ -865,7 +879,8 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal)) != cudaSuccess) return e;
         if ((e = joinc::enqueue(k_bs_join, G, nrep, smem, s, (const Rep*)gl.reps, (const u32*)gl.order, G,
-                                (const u32*)gl.rankOf, (const int*)(gl.xerr + 2))) != cudaSuccess)
+                                (const u32*)gl.rankOf, (const int*)(gl.xerr + 2), opsShared)) !=
+            cudaSuccess)
             return e;
         if ((e = cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal)) != cudaSuccess) return e;
         k_bs_transfer<<<dim3((nX + kXThreads - 1) / kXThreads, nrep), kXThreads, 0, s>>>(xa);

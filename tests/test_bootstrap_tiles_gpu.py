@@ -60,3 +60,18 @@ def test_full_tree_past_one_window(gpu_lib, ntip):
     assert np.array_equal(got["ysize"][0, nodes - ntip], ysize)
     with pytest.raises(gpu_lib.CasphyError):
         gpu_lib.bootstrap_bit(words, full_edge, [0, 3], [cells[5], 7, cells[5]], w)
+
+
+def test_replicate_past_the_shared_offsets(gpu_lib):
+    """All cells with unit weights: the replicate's tree is the full tree, so
+    every clade is at distance 0."""
+    rng = np.random.default_rng(1)
+    n = 53600
+    words = synth.binary_workload(n, 64, 16, 0.03, 0.05, seed=1)
+    full_edge, _, _ = gpu_lib.join_bit(words, None, 1)
+    got = gpu_lib.bootstrap_bit(words, full_edge, [0, n], np.arange(n, dtype=np.uint32), np.ones((1, words.shape[1] * 32)))
+    assert not got["ymin"].any() and got["ysize"].all() and (got["support"] == 1).all()
+    with pytest.raises(gpu_lib.CasphyError):
+        cells = np.arange(57857, dtype=np.uint32)
+        edge = np.stack([57857 + np.arange(2 * 57856) // 2, np.arange(2 * 57856)], 1).astype(np.uint32)
+        gpu_lib.bootstrap_bit(rng.integers(0, 9, (57857, 1)).astype(np.uint32), edge, [0, 57857], cells, np.ones((1, 32)))
