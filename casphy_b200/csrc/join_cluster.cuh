@@ -18,9 +18,9 @@
 //    publishes them without the rescanned rows, whose new records every CTA
 //    forms itself from the exchanged partial bests;
 //  * one warp takes the decision and broadcasts it through shared memory;
-//  * when half of the slots are dead every CTA squeezes its own range, in the
-//    middle of a join phase; slots never move between CTAs, so a compaction
-//    needs no exchange.
+//  * when enough of the slots are dead (the model says how many) every CTA
+//    squeezes its own range, in the middle of a join phase; slots never move
+//    between CTAs, so a compaction needs no exchange.
 //
 // A Model supplies the query build, the scores of a CTA's slots and the move
 // of slot data in a compaction.  Rows of new nodes are written by CTA 0 and

@@ -1146,7 +1146,7 @@ static size_t bits_bytes(u32 ntip, u32 ncol, u32 nState) {
 // Trees of at most kClusterTips tips are joined by one cluster.  A phase on a
 // cluster costs about 4 us plus the scan of a sixteenth of the slots, on all
 // SMs about 10 us plus a scan of a 148th: at 65,000 x 1,024 the cluster takes
-// 0.93 s and all SMs 1.10 s, at 12,345 x 777 0.095 s and 0.184 s.
+// 0.89 s and all SMs 1.10 s, at 12,345 x 777 0.093 s and 0.184 s.
 constexpr u32 kClusterTips = 65536;  // (the engine's narrow keys: nodes below 2^17)
 static_assert(2 * kClusterTips <= joinc::kNarrowNodes, "narrow keys");
 // CTAs of the cluster: 16, fewer when a CTA would have no slot of its own;
@@ -1451,15 +1451,22 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
                   joinc::placeable((void*)k_cluster_join<IndelCluster<true>>, ca.G, cs);
     }
     if (scanEnv && !strcmp(scanEnv, "dense")) useBits = false;
-    lst.scan_path = useBits ? 1u : 0u;
-    Carve cv;
-    carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
-    u32* dCodesCopy = cv.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
-    u32* dOrder = cv.take<u32>(nrows);
-    u32* dState = cv.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
+    u32 *dCodesCopy, *dOrder, *dState;
     void* base = nullptr;
-    rc = ds.reserve(cv.off + 256, &base);
-    if (rc) return rc;
+    for (;;) {
+        Carve cv;
+        carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
+        dCodesCopy = cv.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
+        dOrder = cv.take<u32>(nrows);
+        dState = cv.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
+        rc = ds.reserve(cv.off + 256, &base);
+        if (!rc) break;
+        // fractional weights do without the bitsets when there is no room
+        if (!useBits || intPath) return rc;
+        cudaGetLastError();
+        useBits = false;
+    }
+    lst.scan_path = useBits ? 1u : 0u;
     Carve c2;
     c2.base = static_cast<char*>(base);
     const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
