@@ -22,8 +22,9 @@
 //    squeezes its own range, in the middle of a join phase; slots never move
 //    between CTAs, so a compaction needs no exchange.
 //
-// A Model supplies the query build, the scores of a CTA's slots and the move
-// of slot data in a compaction.  Rows of new nodes are written by CTA 0 and
+// A Model supplies the query build (and, if it likes, an early load of its
+// rows), the scores of a CTA's slots and the move of slot data in a compaction.
+// Rows of new nodes are written by CTA 0 and
 // fenced before its records are sent, so a CTA that has received them reads
 // the row from L2.
 #pragma once
@@ -193,6 +194,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
         send_lists(b, 0);
     }
     pf.mark(joinx::PROF_COMPACT);
+    typename M::Pre pre;
     for (; k < nJoin; p++) {
         const u32 buf = p & 1u;
         if (G == 1) __syncthreads();
@@ -259,6 +261,13 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             if (winner) {
                 if ((~lw) >= a.nnode || mine.partner >= a.nnode) bad = 1;
             }
+            // the rows that the decision will most likely need: their load is under
+            // way while it is taken (unconditional, so that no register is moved
+            // before the load is done)
+            if constexpr (M::kLoadsEarly) {
+                const u32 partner = __reduce_max_sync(0xFFFFFFFFu, winner ? mine.partner : 0u);
+                M::load_early(m, pre, min(~lw, a.nnode - 1u), min(partner, a.nnode - 1u));
+            }
             if (hi == 0u) bad = bad ? bad : 2u;  // two live rows always have a record
             bool stale = winner && is_dead(mine);
             if (!__any_sync(0xFFFFFFFFu, stale)) {
@@ -322,7 +331,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             break;
         }
         if (nq) {
-            const u32 nE = M::build_stale(a, m, ms, st, nq, s_rows);
+            const u32 nE = M::build_stale(a, m, ms, st, nq, s_rows, pre);
             pf.mark(joinx::PROF_SELECT);
             // best (score, node) key of every row over this CTA's live slots
             // other than its own; one thread calls row(q, ...) per slot
@@ -379,7 +388,7 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
             sz2 = size_of(j2);
         }
         const u32 own = slot1 >> 24 == rank ? slot1 & 0xFFFFFFu : joinx::kNone;
-        const u32 nE = M::build_join(a, m, ms, st, rank, j1, j2, sz1, sz2, newNode, own);
+        const u32 nE = M::build_join(a, m, ms, st, rank, j1, j2, sz1, sz2, newNode, own, pre);
         if (bookkeeper) {
             *reinterpret_cast<uint4*>(a.rawEdge + 4 * (size_t)k) = make_uint4(newNode, j1, newNode, j2);
             if (a.needSizes || a.keepSizes) a.nodeSize[newNode] = sz1 + sz2;

@@ -38,6 +38,11 @@ constexpr u32 kResidentUnits = 80000;
 
 template <bool HALF>
 struct IndelCluster {
+    // (rows of many words are loaded by all warps after the decision: loaded early
+    // by the deciding warp alone or by all, waiting for the records, 5.55 -> 5.65
+    // and 5.75 ms of a 1,024 x 256 call)
+    static constexpr bool kLoadsEarly = false;
+    struct Pre {};
     static constexpr bool kNarrow = true;  // non-negative binary16 scores; cluster_plan bounds the nodes
     struct Args {
         u32 ncol, ncolP, nState, minSize;
@@ -174,7 +179,7 @@ struct IndelCluster {
         return t;
     }
     __device__ static u32 build_stale(const joinc::Args&, const Args& m, Smem& s, const joinc::Slots&, u32 nq,
-                                      const joinc::Rec* rows) {
+                                      const joinc::Rec* rows, const Pre&) {
         s.par ^= 1u;
         u32* cnt = counts(s.par);
         for (u32 s0 = 0; s0 < m.ncolP; s0 += 2 * kThreads) {
@@ -193,7 +198,7 @@ struct IndelCluster {
     // new row; the owner of j1's slot (own: its local index) flips the slot's
     // bit in the rows where the two states differ.
     __device__ static u32 build_join(const joinc::Args& a, const Args& m, Smem& s, const joinc::Slots&, u32 rank,
-                                     u32 j1, u32 j2, u32 s1, u32 s2, u32 newNode, u32 own) {
+                                     u32 j1, u32 j2, u32 s1, u32 s2, u32 newNode, u32 own, const Pre&) {
         s.par ^= 1u;
         u32* cnt = counts(s.par);
         int mode = 3;
