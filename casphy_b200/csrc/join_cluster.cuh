@@ -149,6 +149,9 @@ __device__ __forceinline__ void cluster_join(const Args& a, const typename M::Ar
     }
     for (u32 i = tid; i < a.deathWords; i += kThreads) deathBits[i] = 0u;
     if (tid < kMaxBatch * kWarps) (&s_red[0][0])[tid] = 0ull;
+    // slot x's node is written by thread x mod 512; begin() may read it from any
+    // warp (the indel model's resident codes: warp x mod 16)
+    __syncthreads();
     M::begin(a, m, ms, rank, st);
     __syncthreads();
     if (G > 1) cluster_sync();
