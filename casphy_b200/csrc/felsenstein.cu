@@ -49,6 +49,7 @@
 
 #include "cluster.cuh"
 #include "common.cuh"
+#include "lbfgs_plan.h"
 #include "runtime.h"
 
 namespace casphy {
@@ -56,7 +57,6 @@ namespace fel {
 
 constexpr u32 kSites = 256;  // sites per block (one thread per site)
 constexpr int kWild = 0x7FFF, kNoneA = 0x7FFE;
-constexpr u32 kLbThreads = 512;
 constexpr u32 kMaxLbCTA = 256;  // CTAs of the cooperative L-BFGS kernels
 constexpr u32 kMaxHist = 16;
 
@@ -953,21 +953,19 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_accept(Lb a, u32 slot) {
     }
 }
 
-// The same steps on one cluster of kLbCluster CTAs, for problems of at most one
+// The same steps on one cluster (lbfgs_plan.h), for problems of at most one
 // element a thread of the grid kernels (n <= 512 nCTA): the direction alone, or
 // an accept, the direction and the trial point in one launch.  The grid kernels
 // spend their time in reductions behind a flag barrier of all SMs, 17 of about
 // 6 us a step, for vectors of a few KB; a cluster exchanges the partial sums
 // through distributed shared memory in under 1 us.  The sums keep the grid
-// kernels' grouping (CTA r sums the 512-element blocks r, r + 16, ... that
-// their CTAs would, and the blocks are added in order), so every bit is the
-// same.  V: blocks per CTA.
-constexpr u32 kLbCluster = 16;
-constexpr u32 kLbMaxBlocks = 160;
+// kernels' grouping (of G CTAs, CTA r sums the 512-element blocks r, r + G, ...
+// that their CTAs would, and the blocks are added in order), so every bit is the
+// same.  V: blocks per CTA, at most.
 enum { LB_ACCEPT = 1, LB_DIR = 2, LB_TRIAL = 4 };
 
 struct LbExchange {
-    u32 rank, nv, epoch, bar;
+    u32 rank, G, nv, epoch, bar;
     double* part;  // 2 x kLbMaxBlocks x 3
     double (*red)[3][kLbThreads / 32];
 };
@@ -990,13 +988,13 @@ __device__ __forceinline__ void cluster_reduce(const Lb& a, LbExchange& x, const
         }
     __syncthreads();
     if (tid < V * K) {
-        const u32 j = tid / K, k = tid % K, b = x.rank + kLbCluster * j;
+        const u32 j = tid / K, k = tid % K, b = x.rank + x.G * j;
         if (b < x.nv) {
             double s = 0.0;
             for (u32 i = 0; i < kLbThreads / 32; i++)
                 s = MAX && k == K - 1 ? fmax(s, x.red[j][k][i]) : s + x.red[j][k][i];
             const u32 to = clu::smem_u32(x.part + (buf * kLbMaxBlocks + b) * 3 + k);
-            for (u32 r = 0; r < kLbCluster; r++)
+            for (u32 r = 0; r < x.G; r++)
                 clu::st_async8(clu::mapa(to, r), (u64)__double_as_longlong(s), clu::mapa(bar, r));
         }
     }
@@ -1013,12 +1011,12 @@ __device__ __forceinline__ void cluster_reduce(const Lb& a, LbExchange& x, const
 }
 
 template <int V>
-__global__ void __launch_bounds__(kLbThreads) k_lb_cluster(Lb a, u32 what, u32 slot, u32 first, u32 count, double step) {
+__global__ void __launch_bounds__(kLbThreads) k_lb_cluster(Lb a, u32 G, u32 what, u32 slot, u32 first, u32 count, double step) {
     __shared__ double part[2 * kLbMaxBlocks * 3];
     __shared__ double red[V][3][kLbThreads / 32];
     __shared__ __align__(8) u64 bars[2];
     __shared__ double alpha[kMaxHist];
-    LbExchange x{clu::cluster_rank(), (a.n + kLbThreads - 1) / kLbThreads, 0u, clu::smem_u32(&bars[0]), part, red};
+    LbExchange x{clu::cluster_rank(), G, (a.n + kLbThreads - 1) / kLbThreads, 0u, clu::smem_u32(&bars[0]), part, red};
     if (threadIdx.x == 0) {
         clu::mbar_init(x.bar);
         clu::mbar_init(x.bar + 8);
@@ -1031,7 +1029,7 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_cluster(Lb a, u32 what, u32 s
     double g[V], d[V];
 #pragma unroll
     for (int j = 0; j < V; j++) {
-        at[j] = (x.rank + kLbCluster * j) * kLbThreads + threadIdx.x;
+        at[j] = (x.rank + G * j) * kLbThreads + threadIdx.x;
         ok[j] = at[j] < a.n;
         if (!ok[j]) at[j] = 0u;
         g[j] = ok[j] ? a.g[at[j]] : 0.0;
@@ -1377,7 +1375,7 @@ struct FelProblem {
     float *P = nullptr, *dP = nullptr;
     float2* p = nullptr;
     Lb lb{};
-    int lbCluster = -1;  // whether the L-BFGS steps run on a cluster (-1: not asked yet)
+    int lbCtas = -1;  // CTAs of the L-BFGS steps' cluster, 0: all SMs (-1: not asked yet)
     cudaGraphExec_t gFull = nullptr, gLL = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1775,17 +1773,23 @@ static int lb_coop(FelProblem& F, const void* fn, void** args) {
 // where the problem fits it, else the grid kernels.
 static int lb_step(FelProblem& F, u32 what, u32 slot, u32 first, u32 count, double step) {
     Lb& a = F.lb;
-    const u32 V = (a.n + kLbThreads * kLbCluster - 1) / (kLbThreads * kLbCluster);
-    if (F.lbCluster < 0) {
-        const bool fits = a.n <= a.nCTA * kLbThreads && a.nCTA <= kLbMaxBlocks && V <= 10;
+    const LbPlan plan = lb_plan(a.n);
+    const u32 V = plan.perCta;
+    if (F.lbCtas < 0) {
+        const char* env = std::getenv("CASPHY_LBFGS");  // grid: the kernels of all SMs
+        const bool fits = a.n <= a.nCTA * kLbThreads && plan.blocks <= kLbMaxBlocks && V <= kLbMaxPerCta &&
+                          !(env && !std::strcmp(env, "grid"));
         const void* fn = V <= 1 ? (const void*)k_lb_cluster<1> : V <= 2 ? (const void*)k_lb_cluster<2>
-                         : V <= 5 ? (const void*)k_lb_cluster<5> : (const void*)k_lb_cluster<10>;
-        F.lbCluster = fits && clu::placeable(const_cast<void*>(fn), kLbCluster, 0) > 0 ? 1 : 0;
+                         : V <= 5 ? (const void*)k_lb_cluster<5> : (const void*)k_lb_cluster<kLbMaxPerCta>;
+        F.lbCtas = fits && clu::placeable(const_cast<void*>(fn), plan.ctas, 0) > 0 ? (int)plan.ctas : 0;
     }
-    if (F.lbCluster) {
-        auto run = [&](auto fn) { return clu::enqueue(fn, kLbCluster, 1, 0, F.st, a, what, slot, first, count, step); };
-        CASPHY_CUDA_TRY(V <= 1 ? run(k_lb_cluster<1>) : V <= 2 ? run(k_lb_cluster<2>) : V <= 5 ? run(k_lb_cluster<5>)
-                                                                                      : run(k_lb_cluster<10>));
+    if (F.lbCtas) {
+        const u32 G = plan.ctas;
+        auto run = [&](auto fn) { return clu::enqueue(fn, G, 1, 0, F.st, a, G, what, slot, first, count, step); };
+        CASPHY_CUDA_TRY(V <= 1   ? run(k_lb_cluster<1>)
+                        : V <= 2 ? run(k_lb_cluster<2>)
+                        : V <= 5 ? run(k_lb_cluster<5>)
+                                 : run(k_lb_cluster<kLbMaxPerCta>));
         return CASPHY_OK;
     }
     if (what & LB_ACCEPT) {
@@ -1976,6 +1980,7 @@ extern "C" int casphy_felsenstein_optimize(uint32_t ntip, uint32_t nedge, const 
     st.site_chunks = F.nchunk;
     st.levels_inside = (u32)F.th.inOff.size() - 1;
     st.levels_outside = (u32)F.th.outOff.size() - 1;
+    st.step_ctas = (u32)std::max(F.lbCtas, 0);
     st.launches_per_eval = adj ? F.launchesFull : F.launchesLL;
     st.eval_seconds = F.graphMs / 1e3;
     if (stats) *stats = st;

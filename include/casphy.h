@@ -218,7 +218,7 @@ typedef struct {
     uint32_t site_chunks;
     uint32_t levels_inside;     /* tree height (narrow levels share a launch) */
     uint32_t levels_outside;    /* the same levels, downwards */
-    uint32_t reserved;
+    uint32_t step_ctas;         /* CTAs of the L-BFGS steps' cluster; 0: all SMs */
     double loglik_start, loglik_end;
     double seconds;             /* device time of the whole optimisation */
     uint64_t launches_per_eval; /* kernels in one evaluation graph */
