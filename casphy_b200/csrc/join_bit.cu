@@ -139,9 +139,11 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
 
 template <int PATH>
 static int launch_bit_any(joinx::Common& c, const typename BitModel<PATH>::Args& m, u32 Sp,
-                          const unsigned long long* initKey, const u32* tipSize, u32 nCTA, cudaStream_t st) {
+                          const unsigned long long* initKey, const u32* tipSize, u32 nCTA, cudaStream_t st,
+                          int* launches) {
     bool done = false;
     if (int rc = launch_bit_cluster<PATH>(c, m, Sp, initKey, st, &done)) return rc;
+    *launches += done ? 1 : 2;
     if (done) return CASPHY_OK;
     joinx::k_slot_init<<<(std::max(Sp, c.nnode) + 255) / 256, 256, 0, st>>>(
         c.ntip, Sp, c.nnode, initKey, ORD_F32_NEG1, c.lmOrd[0], c.lmIdx[0], c.slotNode[0], c.node2slot, c.nodeDeath,
@@ -304,18 +306,17 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
         if (path == PATH_UNIT) {
             BitModel<PATH_UNIT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                         {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, L.initKey, L.tip, nCTA, st);
+            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches);
         } else if (path == PATH_PLANES) {
             BitModel<PATH_PLANES>::Args m{nbin, nbinP, nplanes, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                           {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, L.initKey, L.tip, nCTA, st);
+            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches);
         } else {
             BitModel<PATH_FLOAT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                          {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, L.initKey, L.tip, nCTA, st);
+            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches);
         }
         if (rc) return rc;
-        launches += 2;
     }
     CASPHY_CUDA_TRY(cudaEventRecord(ev[3], st));
     if (ntip >= 2) {

@@ -1285,10 +1285,11 @@ static bool cluster_plan(u32 ntip, u32 ncol, u32 nState, bool unitW, joinc::Args
     return false;
 }
 
-// Launches the join on one cluster; *done says whether it could.
+// Launches the join on one cluster; *done says whether it could.  Adds the
+// kernels launched to *launches.
 template <bool HALF>
 static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, bool unitW, u32 minSize,
-                                float minRatio, cudaStream_t st, bool* done) {
+                                float minRatio, cudaStream_t st, bool* done, int* launches) {
     using M = IndelCluster<HALF>;
     joinc::Args a{};
     typename M::Args m{};
@@ -1311,10 +1312,14 @@ static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 n
     m.bits[0] = L.bits0;
     m.bits[1] = L.bits1;
     if (!joinc::placeable((void*)k_cluster_join<M>, a.G, smem)) return CASPHY_OK;
-    if (!M::resident_pitch(m, a.R))  // (else no CTA reads them)
+    if (!M::resident_pitch(m, a.R)) {  // (else no CTA reads them)
         k_split_bits<<<dim3(296, a.G), 256, 0, st>>>(L.bits0, m.rows, (ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32),
                                                  a.R / 32, L.bits1);
-    return joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
+        ++*launches;
+    }
+    const int rc = joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
+    if (*done) ++*launches;
+    return rc;
 }
 
 // Launches prep, initial scan and the persistent join.  Assumes Wsel,
@@ -1370,11 +1375,11 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
         // one cluster where it can hold the slots; a tree beyond it, or a
         // device that cannot place the cluster, runs on all SMs
         bool done = false;
-        const int rc = intPath ? launch_cluster_indel<false>(L, ntip, ncol, nState, unitW, minSize, minRatio, st, &done)
-                               : launch_cluster_indel<true>(L, ntip, ncol, nState, false, minSize, minRatio, st, &done);
+        const int rc = intPath ? launch_cluster_indel<false>(L, ntip, ncol, nState, unitW, minSize, minRatio, st, &done, &n)
+                               : launch_cluster_indel<true>(L, ntip, ncol, nState, false, minSize, minRatio, st, &done, &n);
         if (rc) return rc;
         if (done) {
-            *launches = n + 2;
+            *launches = n;
             return CASPHY_OK;
         }
         if (!intPath) return CASPHY_EINTERNAL;  // the caller asked cluster_plan() before it chose the bitsets
