@@ -108,7 +108,7 @@ constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 // Launches the join on one cluster; *done says whether it could.
 template <int PATH>
 static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PATH>::Args& bm, u32 Sp,
-                              const unsigned long long* initKey, cudaStream_t st, bool* done) {
+                              const unsigned long long* initKey, cudaStream_t st, bool* done, u32* scanPath) {
     using M = BitCluster<PATH>;
     *done = false;
     int smemMax = 0, dev = 0;
@@ -134,15 +134,18 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     size_t smem = 0;
     if (!cluster_fit<PATH>(a, m, (size_t)smemMax - 6144, &smem)) return CASPHY_OK;
     if (PATH != PATH_FLOAT && m.colWords < (size_t)m.nbin * a.R) return CASPHY_OK;
-    return joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
+    const int rc = joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
+    if (*done && m.colWords >= (size_t)m.nbin * a.R) *scanPath = 1u;
+    return rc;
 }
 
 template <int PATH>
 static int launch_bit_any(joinx::Common& c, const typename BitModel<PATH>::Args& m, u32 Sp,
                           const unsigned long long* initKey, const u32* tipSize, u32 nCTA, cudaStream_t st,
-                          int* launches) {
+                          int* launches, u32* scanPath) {
     bool done = false;
-    if (int rc = launch_bit_cluster<PATH>(c, m, Sp, initKey, st, &done)) return rc;
+    if (!joinx::grid_asked())
+        if (int rc = launch_bit_cluster<PATH>(c, m, Sp, initKey, st, &done, scanPath)) return rc;
     *launches += done ? 1 : 2;
     if (done) return CASPHY_OK;
     joinx::k_slot_init<<<(std::max(Sp, c.nnode) + 255) / 256, 256, 0, st>>>(
@@ -306,15 +309,15 @@ static int join_bit_impl(u32 ntip, u32 nbin, const u32* d_words, const u32* h_wo
         if (path == PATH_UNIT) {
             BitModel<PATH_UNIT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                         {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches);
+            rc = launch_bit_any<PATH_UNIT>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches, &lst.scan_path);
         } else if (path == PATH_PLANES) {
             BitModel<PATH_PLANES>::Args m{nbin, nbinP, nplanes, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                           {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches);
+            rc = launch_bit_any<PATH_PLANES>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches, &lst.scan_path);
         } else {
             BitModel<PATH_FLOAT>::Args m{nbin, nbinP, 0, ancType, L.planeMask, L.wf, L.nodeSeq, L.nodeBis,
                                          {L.colT0, L.colT1}};
-            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches);
+            rc = launch_bit_any<PATH_FLOAT>(c, m, Sp, L.initKey, L.tip, nCTA, st, &launches, &lst.scan_path);
         }
         if (rc) return rc;
     }

@@ -26,6 +26,7 @@
 // candidate scores is computed, and how slot data moves in a compaction.
 #pragma once
 #include <cstdlib>
+#include <cstring>
 
 #include "common.cuh"
 
@@ -818,6 +819,13 @@ inline u32 stale_batch_setting() {
     if (!e) return kMaxBatch;
     const long v = strtol(e, nullptr, 10);
     return v < 1 ? 1u : (v > (long)kMaxBatch ? kMaxBatch : (u32)v);
+}
+
+// Host: whether CASPHY_JOIN_ENGINE=grid asks for this engine where a cluster would
+// be taken (same trees; for comparisons of the two).
+inline bool grid_asked() {
+    const char* e = getenv("CASPHY_JOIN_ENGINE");
+    return e && !strcmp(e, "grid");
 }
 
 // Host: bytes of engine shared memory before the model's part.

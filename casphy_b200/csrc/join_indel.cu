@@ -1252,7 +1252,7 @@ static int launch_join_fitted(joinx::Common& c, typename M::Args& m, u32* batch,
 template <bool HALF>
 static bool cluster_plan(u32 ntip, u32 ncol, u32 nState, bool unitW, joinc::Args& a,
                          typename IndelCluster<HALF>::Args& m, size_t* smem) {
-    if (ntip < 2 || ntip > kClusterTips) return false;
+    if (ntip < 2 || ntip > kClusterTips || joinx::grid_asked()) return false;
     int smemMax = 0, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)

@@ -48,7 +48,9 @@ typedef struct {
     uint64_t kernel_launches;    /* kernels launched by this call */
     uint32_t int_path;           /* 1: exact integer accumulation was used */
     uint32_t scan_path;          /* indel: 0 column-major codes, 1 allele bitsets
-                                    (fractional weights: on one cluster only) */
+                                    (fractional weights: on one cluster only);
+                                    bit: 1 columns resident in shared memory from
+                                    the start (one cluster), 0 read through L2 */
     double init_scan_ms;         /* device time, initial all-pairs scan */
     double join_loop_ms;         /* device time, persistent join loop */
     double total_ms;             /* device time of the whole call */

@@ -46,3 +46,91 @@ def test_bit_join_counts_its_launches(gpu_lib):
     assert gpu_lib.join_bit(words, w, 0)[2]["kernel_launches"] == 5
     # one cell: no scan and no join
     assert gpu_lib.join_bit(words[:1], w, 0)[2]["kernel_launches"] == 3
+
+
+# The engine of all SMs takes trees beyond the cluster; here it is asked for at
+# sizes the oracle can follow: ranges of no slot, of one, and of several words,
+# and enough slots for its compaction (4,096).
+@pytest.mark.parametrize("weights", ["unit", "planes", "float"])
+@pytest.mark.parametrize("ncell,nsite,atype", [(2, 32, 0), (149, 96, 1), (1100, 416, 0), (5000, 64, 1)])
+def test_bit_join_on_all_sms(gpu_lib, monkeypatch, weights, ncell, nsite, atype):
+    words, w = _bit(ncell, nsite, weights, ncell + nsite)
+    want = O.join_bit(words, w, atype)
+    assert _same(gpu_lib.join_bit(words, w, atype), want)
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    got = gpu_lib.join_bit(words, w, atype)
+    assert got[2]["kernel_launches"] == 6 and got[2]["scan_path"] == 0
+    assert _same(got, want)
+
+
+@pytest.mark.parametrize("weights", ["unit", "integer", "half"])
+@pytest.mark.parametrize("ncell,nsite,nallele,min_size", [
+    (2, 1, 2, 0), (149, 33, 9, 0), (1100, 260, 30, 0), (700, 40, 8, 12), (5000, 24, 8, 0)])
+def test_indel_join_on_all_sms(gpu_lib, monkeypatch, weights, ncell, nsite, nallele, min_size):
+    """Allele bitsets for integer weights, the column scan for fractional ones."""
+    codes, ns, w = _indel(ncell, nsite, nallele, weights, ncell)
+    tip = np.random.default_rng(ncell).integers(1, 30, size=ncell) if min_size else None
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    got = gpu_lib.join_indel(codes, ns, w, tip, min_size, 1.5)
+    assert got[2]["scan_path"] == (0 if weights == "half" else 1)
+    assert got[2]["kernel_launches"] == 7
+    assert _same(got, O.join_indel(codes, ns, w, tip, min_size, 1.5))
+
+
+def _many_states(ncell, nsite, nstate, seed):
+    """Codes 0 .. nstate + 1 drawn directly, rows alike enough to share alleles."""
+    rng = np.random.default_rng(seed)
+    base = rng.integers(2, nstate + 2, size=(max(ncell // 25, 2), nsite))
+    codes = base[rng.integers(0, len(base), size=ncell)]
+    new = rng.random(codes.shape)
+    codes = np.where(new < 0.25, rng.integers(2, nstate + 2, size=codes.shape), codes)
+    return np.where(new > 0.8, rng.integers(0, 2, size=codes.shape), codes).astype(np.uint32)
+
+
+# Bitset rows copied to the stage.  More than 253 states never fit a byte; a
+# query's 2,080 entries of eight words (2,100 x 2,600) with fractional weights are
+# more than the stage holds, so the sums go on over several rounds; 4,500 x 700
+# are too many bytes at first, and a compaction makes them resident.
+@pytest.mark.parametrize("ncell,nsite,nstate,weights", [
+    (300, 70, 254, "unit"), (1500, 1024, 400, "unit"), (2100, 2000, 300, "unit"),
+    (300, 70, 254, "half"), (1500, 1024, 400, "half"), (2100, 2600, 300, "half")])
+def test_staged_bitsets_of_many_states(gpu_lib, ncell, nsite, nstate, weights):
+    codes = _many_states(ncell, nsite, nstate, ncell)
+    w = np.ones((nstate, nsite)) if weights == "unit" else \
+        np.random.default_rng(1).uniform(0.01, 4.0, size=(nstate, nsite))
+    got = gpu_lib.join_indel(codes, nstate, w)
+    assert got[2]["scan_path"] == 1 and got[2]["kernel_launches"] == (8 if weights == "half" else 7)
+    assert got[2]["stale_recomputes"] > 0 and got[2]["compactions"] == (1 if ncell > 2048 else 0)
+    assert _same(got, O.join_indel(codes, nstate, w))
+
+
+def test_staged_bitsets_then_resident_codes(gpu_lib, monkeypatch):
+    codes, ns, w = _indel(4500, 700, 8, "half", 4)
+    got = gpu_lib.join_indel(codes, ns, w)
+    assert got[2]["scan_path"] == 1 and got[2]["kernel_launches"] == 8 and got[2]["compactions"] > 0
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    assert _same(got, gpu_lib.join_indel(codes, ns, w))
+
+
+# Ordered binary32 sums with the columns in global memory: too many words for
+# shared memory throughout (1,100 x 8,192, compacted once), or until a
+# compaction (3,500 x 2,560).
+def test_bit_columns_in_global_memory(gpu_lib):
+    words, w = _bit(1100, 8192, "float", 7)
+    got = gpu_lib.join_bit(words, w, 1)
+    assert got[2]["scan_path"] == 0 and got[2]["kernel_launches"] == 5 and got[2]["compactions"] > 0
+    assert _same(got, O.join_bit(words, w, 1))
+
+
+def test_bit_columns_move_to_shared_memory(gpu_lib, monkeypatch):
+    words, w = _bit(3500, 2560, "float", 8)
+    got = gpu_lib.join_bit(words, w, 0)
+    assert got[2]["scan_path"] == 0 and got[2]["kernel_launches"] == 5 and got[2]["compactions"] > 0
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    assert _same(got, gpu_lib.join_bit(words, w, 0))
+
+
+def test_bit_columns_resident_from_the_start(gpu_lib):
+    words, w = _bit(1500, 320, "float", 9)
+    got = gpu_lib.join_bit(words, w, 0)
+    assert got[2]["scan_path"] == 1 and _same(got, O.join_bit(words, w, 0))
