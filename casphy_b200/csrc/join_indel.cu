@@ -30,6 +30,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <vector>
 
 #include "join_engine.cuh"
@@ -1143,10 +1144,20 @@ static size_t bits_bytes(u32 ntip, u32 ncol, u32 nState) {
     return 2 * (size_t)ncol * nState * Wd * sizeof(u32);
 }
 
-// Trees of at most kClusterTips tips are joined by one cluster.  A phase on a
-// cluster costs about 4 us plus the scan of a sixteenth of the slots, on all
-// SMs about 10 us plus a scan of a 148th: at 65,000 x 1,024 the cluster takes
-// 0.89 s and all SMs 1.10 s, at 12,345 x 777 0.093 s and 0.184 s.
+// One cluster or all SMs.  A phase on a cluster costs about 4 us plus the scan of
+// a sixteenth of the slots, on all SMs about 10 us plus a scan of a 148th.  With
+// integer weights the scan grows with slots x edited sites of a query, and so does
+// the choice (loop on a cluster over loop on all SMs, cells x edited sites of a
+// tip).  Unit weights: 0.52 at 12,345 x 218, 0.79 at 65,000 x 287, 0.91 at 50,000 x
+// 448, 0.96 at 65,000 x 392, 0.97 at 40,000 x 573, then 1.01 at 50,000 x 573, 1.03
+// at 65,000 x 476, 1.17 at 65,000 x 573, 1.41 at 25,000 x 1,536.  Other integers,
+// rippled bit by bit: 0.46 at 8,000 x 140, 0.73 at 20,000 x 140, 0.83 at 40,000 x
+// 72, 0.87 at 12,000 x 378, then 1.01 at 20,000 x 280, 1.05 at 65,000 x 72, 1.10 at
+// 40,000 x 140, 2.33 at 65,000 x 280.  Fractional weights are added in order, one
+// entry after the other on either engine, and the cluster is the better at every
+// size it can take (65,000 cells: 0.79 with 287 edited sites, 0.62 with 1,147;
+// 8,000: 0.25 and 0.22).
+constexpr u64 kClusterWorkUnit = 26000000, kClusterWorkInteger = 4000000;  // cells x edited sites of a tip
 constexpr u32 kClusterTips = 65536;  // (the engine's narrow keys: nodes below 2^17)
 static_assert(2 * kClusterTips <= joinc::kNarrowNodes, "narrow keys");
 // CTAs of the cluster: 16, fewer when a CTA would have no slot of its own;
@@ -1342,6 +1353,15 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
     PrepArgs pa{ntip, ncol, ncolP, nState, Sp, codes, L.Wsel, intPath ? 0x7FFFu : 0xFFFFu,
                 L.nodeRow, L.eSC, L.eW, L.eLen, L.prepErr};
     k_prep_rows<<<(ntip + 7) / 8, 256, 0, st>>>(pa);
+    // the edited sites are counted where all sites would be too many
+    bool cluster = useBits;
+    const u64 most = unitW ? kClusterWorkUnit : kClusterWorkInteger;
+    if (useBits && intPath && ntip <= kClusterTips && (u64)ntip * ncol > most) {
+        std::vector<u32> len(ntip);
+        CASPHY_CUDA_TRY(cudaMemcpyAsync(len.data(), L.eLen, sizeof(u32) * ntip, cudaMemcpyDeviceToHost, st));
+        CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+        cluster = std::accumulate(len.begin(), len.end(), u64(0)) <= most;
+    }
     if (useBits) {
         CASPHY_CUDA_TRY(cudaMemsetAsync(L.bits0, 0, sizeof(u32) * L.bitsWords, st));
         k_build_bits<<<dim3(Sp / 32, (ncol + 31) / 32), dim3(32, 8), 0, st>>>(L.nodeRow, ntip, ncol, ncolP, nState,
@@ -1371,7 +1391,7 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
     }
     n++;
     if (evInit1) CASPHY_CUDA_TRY(cudaEventRecord(evInit1, st));
-    if (useBits) {
+    if (cluster) {
         // one cluster where it can hold the slots; a tree beyond it, or a
         // device that cannot place the cluster, runs on all SMs
         bool done = false;

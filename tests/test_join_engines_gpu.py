@@ -134,3 +134,24 @@ def test_bit_columns_resident_from_the_start(gpu_lib):
     words, w = _bit(1500, 320, "float", 9)
     got = gpu_lib.join_bit(words, w, 0)
     assert got[2]["scan_path"] == 1 and _same(got, O.join_bit(words, w, 0))
+
+
+# Integer weights: a cluster up to 26,000,000 cells x edited sites, 4,000,000 when
+# the weights are not all 1, counted where cells x sites are more.  (Only the
+# engine of all SMs has refresh phases.)
+@pytest.mark.parametrize("ncell,nsite,weights,most,edited,on_cluster", [
+    (13500, 2048, "unit", 26000000, 0.90, True), (13500, 2048, "unit", 26000000, 0.97, False),
+    (5000, 1000, "integer", 4000000, 0.75, True), (5000, 1000, "integer", 4000000, 0.85, False)])
+def test_indel_engine_follows_the_edited_sites(gpu_lib, monkeypatch, ncell, nsite, weights, most, edited, on_cluster):
+    ns = 20
+    rng = np.random.default_rng(11)
+    base = rng.integers(2, ns + 2, size=(500, nsite), dtype=np.uint32)
+    codes = base[rng.integers(0, len(base), size=ncell)]
+    codes[rng.random(codes.shape) >= edited] = 1
+    assert ncell * nsite > most and (int((codes > 1).sum()) <= most) == on_cluster
+    w = np.ones((ns, nsite)) if weights == "unit" else rng.integers(1, 3, size=(ns, nsite)).astype(float)
+    got = gpu_lib.join_indel(codes, ns, w)
+    assert got[2]["scan_path"] == 1 and (got[2]["refreshes"] == 0) == on_cluster
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    other = gpu_lib.join_indel(codes, ns, w)
+    assert other[2]["refreshes"] > 0 and _same(got, other)
