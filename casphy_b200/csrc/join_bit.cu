@@ -101,8 +101,12 @@ static int launch_bit_init(const InitArgs& ia, u32 nSM, cudaStream_t st) {
 // from the start: 20,000 x 1,024 takes 3.9 us a phase against 8.6 us on all
 // SMs, but 40,000 x 1,024, whose columns are read through L2 by one GPC,
 // 13.3 us against 8.8 us.  Fractional weights are bound by their ordered adds,
-// and one cluster is the better at every size (30,000 x 1,024: 32 us a phase
-// against 83 us).
+// which take a thread of either engine the same time a (slot, set bit): 16 SMs
+// against all of them up to 90,000 cells, however many sites (loop on a cluster
+// over loop on all SMs: 0.35 at 30,000 x 1,024 and x 4,096, 0.68 at 60,000 x 512,
+// 0.80, 0.85 and 0.86 at 75,000 x 256, 1,024 and 3,072, 0.97 at 90,000 x 512 and
+// 0.98 x 1,024, then 1.11 at 100,000 x 1,024 and 1.58 at 150,000 x 512).
+constexpr u32 kFloatClusterTips = 90000;
 constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 
 // Launches the join on one cluster; *done says whether it could.
@@ -111,6 +115,7 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
                               const unsigned long long* initKey, cudaStream_t st, bool* done, u32* scanPath) {
     using M = BitCluster<PATH>;
     *done = false;
+    if (PATH == PATH_FLOAT && c.ntip > kFloatClusterTips) return CASPHY_OK;
     int smemMax = 0, dev = 0;
     CASPHY_CUDA_TRY(cudaGetDevice(&dev));
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

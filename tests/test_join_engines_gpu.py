@@ -155,3 +155,13 @@ def test_indel_engine_follows_the_edited_sites(gpu_lib, monkeypatch, ncell, nsit
     monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
     other = gpu_lib.join_indel(codes, ns, w)
     assert other[2]["refreshes"] > 0 and _same(got, other)
+
+
+# Fractional weights: a cluster up to 90,000 cells.
+@pytest.mark.parametrize("ncell,launches", [(90000, 5), (90001, 6)])
+def test_fractional_bit_engine_follows_the_cells(gpu_lib, ncell, launches):
+    rng = np.random.default_rng(2)
+    words = rng.integers(0, 1 << 31, size=(2000, 1), dtype=np.uint32)[rng.integers(0, 2000, size=ncell)]
+    words ^= np.uint32(1) << rng.integers(0, 32, size=(ncell, 1), dtype=np.uint32)
+    got = gpu_lib.join_bit(words, rng.uniform(0.01, 3.0, size=32), 1)
+    assert got[2]["kernel_launches"] == launches and got[2]["joins"] == ncell - 1
