@@ -30,7 +30,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <numeric>
 #include <vector>
 
 #include "join_engine.cuh"
@@ -168,6 +167,23 @@ __global__ void k_prep_rows(PrepArgs a) {
         n += __popc(bal);
     }
     if (lane == 0) a.eLen[warp] = n;
+}
+
+// Edited (>= 2) and unedited (1) codes of a matrix: n[0], n[1] += their numbers.
+__global__ void __launch_bounds__(256) k_count_codes(const u32* __restrict__ codes, u64 n, unsigned long long* out) {
+    u32 edited = 0, unedited = 0;
+    const u64 hop = (u64)gridDim.x * 256;
+    for (u64 i = (u64)blockIdx.x * 256 + threadIdx.x; i < n; i += hop) {
+        const u32 c = codes[i];
+        edited += c > 1u;
+        unedited += c == 1u;
+    }
+    edited = __reduce_add_sync(0xFFFFFFFFu, edited);
+    unedited = __reduce_add_sync(0xFFFFFFFFu, unedited);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(out, (unsigned long long)edited);
+        atomicAdd(out + 1, (unsigned long long)unedited);
+    }
 }
 
 // colT[s][i] = nodeRow[i][s] for tips; padding slots [ntip, Sp) get code 0.
@@ -1145,19 +1161,47 @@ static size_t bits_bytes(u32 ntip, u32 ncol, u32 nState) {
 }
 
 // One cluster or all SMs.  A phase on a cluster costs about 4 us plus the scan of
-// a sixteenth of the slots, on all SMs about 10 us plus a scan of a 148th.  With
-// integer weights the scan grows with slots x edited sites of a query, and so does
-// the choice (loop on a cluster over loop on all SMs, cells x edited sites of a
-// tip).  Unit weights: 0.52 at 12,345 x 218, 0.79 at 65,000 x 287, 0.91 at 50,000 x
-// 448, 0.96 at 65,000 x 392, 0.97 at 40,000 x 573, then 1.01 at 50,000 x 573, 1.03
-// at 65,000 x 476, 1.17 at 65,000 x 573, 1.41 at 25,000 x 1,536.  Other integers,
-// rippled bit by bit: 0.46 at 8,000 x 140, 0.73 at 20,000 x 140, 0.83 at 40,000 x
-// 72, 0.87 at 12,000 x 378, then 1.01 at 20,000 x 280, 1.05 at 65,000 x 72, 1.10 at
-// 40,000 x 140, 2.33 at 65,000 x 280.  Fractional weights are added in order, one
-// entry after the other on either engine, and the cluster is the better at every
-// size it can take (65,000 cells: 0.79 with 287 edited sites, 0.62 with 1,147;
-// 8,000: 0.25 and 0.22).
-constexpr u64 kClusterWorkUnit = 26000000, kClusterWorkInteger = 4000000;  // cells x edited sites of a tip
+// a sixteenth of the slots, on all SMs about 10 us plus a scan of a 148th, for up
+// to eight rows at once when stale rows are rescanned.  So the choice goes by
+// cells x edited sites of a tip (below: n x E) and by how much of the matrix is
+// edited: where nearly every known site is (s, edited over edited and unedited),
+// cells differ in little and most of a loop is rescans of eight rows.  Loop on a
+// cluster over loop on all SMs:
+//  * unit weights, s 0.2-0.6: 0.52 at 12,345 x 218, 0.79 at 65,000 x 287, 0.91 at
+//    50,000 x 448, 0.96 at 65,000 x 392, 0.97 at 40,000 x 573, then 1.01 at 50,000
+//    x 573, 1.03 at 65,000 x 476 and 30,000 x 1,106, 1.17 at 65,000 x 573.  s 0.88:
+//    0.94 at 20,000 x 900, 1.12 at 16,500 x 1,536.  s 0.96: 0.61 at 4,000 x 820,
+//    1.17 at 20,000 x 820, 1.50 at 12,500 x 1,680.  s 1: 0.81 at 4,000 x 850, 0.84
+//    at 20,000 x 255, 0.97 at 8,000 x 850, 1.09 at 4,000 x 1,700, 1.42 at 20,000 x
+//    850.
+//  * other integers, rippled bit by bit: 0.46 at 8,000 x 140, 0.83 at 40,000 x 72,
+//    0.87 at 12,000 x 378, then 1.01 at 20,000 x 280, 1.05 at 65,000 x 72, 2.33 at
+//    65,000 x 280.  s 1: 0.31 at 2,000 x 425, 0.65 at 12,000 x 85, 1.21 at 4,000 x
+//    425, 2.87 at 4,500 x 840.
+//  * fractional weights are added in order, one entry after the other on either
+//    engine: s to 0.64 on the cluster at every size it takes (65,000 cells: 0.76,
+//    0.62 with 1,147 edited sites, 0.86 at s 0.64); s 0.88 and more 0.53 at 30,000
+//    x 85, 0.75 at 20,000 x 850, 0.98 at 30,000 x 425, then 1.14 at 40,000 x 255,
+//    1.13 at 65,000 x 225, 2.10 at 60,000 x 255.
+struct ClusterRule {
+    double most, mostEdited;  // n x E for s up to 0.8, and at s = 1; a line between
+};
+constexpr ClusterRule kUnitRule{26e6, 6e6}, kIntegerRule{4e6, 1.2e6};
+constexpr u32 kFractionalTips = 35000;      // fractional weights: more only below kFractionalEdited
+constexpr double kFractionalWork = 18e6, kFractionalEdited = 0.7;
+// Whether the edited sites need not be counted: no matrix of this size leaves the
+// cluster.
+static bool always_cluster(u32 ntip, u32 ncol, bool intPath, bool unitW) {
+    const double all = (double)ntip * ncol;
+    if (!intPath) return ntip <= kFractionalTips && all <= kFractionalWork;
+    return all <= (unitW ? kUnitRule : kIntegerRule).mostEdited;
+}
+static bool cluster_pays(u32 ntip, bool intPath, bool unitW, double edited, double unedited) {
+    const double s = edited / std::max(edited + unedited, 1.0);
+    if (!intPath) return s <= kFractionalEdited || (ntip <= kFractionalTips && edited <= kFractionalWork);
+    const ClusterRule r = unitW ? kUnitRule : kIntegerRule;
+    return edited <= r.most + (r.mostEdited - r.most) * std::max(0.0, (s - 0.8) / 0.2);
+}
 constexpr u32 kClusterTips = 65536;  // (the engine's narrow keys: nodes below 2^17)
 static_assert(2 * kClusterTips <= joinc::kNarrowNodes, "narrow keys");
 // CTAs of the cluster: 16, fewer when a CTA would have no slot of its own;
@@ -1169,8 +1213,10 @@ static u32 cluster_size(u32 ntip) {
 }
 static u32 cluster_range(u32 ntip, u32 G) { return ((ntip + G - 1) / G + kBitsAlign - 1) / kBitsAlign * kBitsAlign; }
 
+// mayScan: fractional weights whose engine is chosen once the edited sites are
+// counted have room for the column scan too.
 static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nCTA, u32 nChunks, bool useBits,
-                                bool intPath) {
+                                bool intPath, bool mayScan) {
     const u32 nnode = 2 * ntip - 1, nedge = 2 * ntip - 2;
     // the bitset scan copies 16-byte pieces of bitset rows: slot ranges and
     // row strides are multiples of 128 slots (kBitsAlign)
@@ -1181,7 +1227,7 @@ static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nC
     l.Wsel = c.take<u16>(nw ? nw : 1);
     l.nodeRow = c.take<u16>((size_t)nnode * ncolP);
     l.colT0 = c.take<u16>(useBits && intPath ? 0 : (size_t)ncol * Sp);  // binary16 initial scan, dense join
-    l.colT1 = c.take<u16>(useBits ? 0 : (size_t)ncol * Sp);
+    l.colT1 = c.take<u16>(useBits && (intPath || !mayScan) ? 0 : (size_t)ncol * Sp);
     l.bitsWords = useBits ? (size_t)ncol * nState * (Sp / 32) : 0;
     // the cluster's layout rounds every CTA's range up
     const u32 G = cluster_size(ntip);
@@ -1337,8 +1383,8 @@ static int launch_cluster_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 n
 // tipSize and chunkStart are already on the device; clears everything the
 // kernels expect at zero.  Returns the number of kernels launched.
 static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, const u32* codes, bool intPath,
-                        bool unitW, bool useBits, u32 minSize, float minRatio, u32 nSM, u32 nChunks, u64 nTiles,
-                        cudaStream_t st, cudaEvent_t evInit0, cudaEvent_t evInit1, int* launches) {
+                        bool unitW, bool useBits, bool cluster, u32 minSize, float minRatio, u32 nSM, u32 nChunks,
+                        u64 nTiles, cudaStream_t st, cudaEvent_t evInit0, cudaEvent_t evInit1, int* launches) {
     const u32 nnode = 2 * ntip - 1;
     // slot stride: bitset words need multiples of 32 slots, the u16 column
     // scan multiples of 8 (one 16-byte load); the engine uses the same rule
@@ -1353,15 +1399,6 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
     PrepArgs pa{ntip, ncol, ncolP, nState, Sp, codes, L.Wsel, intPath ? 0x7FFFu : 0xFFFFu,
                 L.nodeRow, L.eSC, L.eW, L.eLen, L.prepErr};
     k_prep_rows<<<(ntip + 7) / 8, 256, 0, st>>>(pa);
-    // the edited sites are counted where all sites would be too many
-    bool cluster = useBits;
-    const u64 most = unitW ? kClusterWorkUnit : kClusterWorkInteger;
-    if (useBits && intPath && ntip <= kClusterTips && (u64)ntip * ncol > most) {
-        std::vector<u32> len(ntip);
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(len.data(), L.eLen, sizeof(u32) * ntip, cudaMemcpyDeviceToHost, st));
-        CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
-        cluster = std::accumulate(len.begin(), len.end(), u64(0)) <= most;
-    }
     if (useBits) {
         CASPHY_CUDA_TRY(cudaMemsetAsync(L.bits0, 0, sizeof(u32) * L.bitsWords, st));
         k_build_bits<<<dim3(Sp / 32, (ncol + 31) / 32), dim3(32, 8), 0, st>>>(L.nodeRow, ntip, ncol, ncolP, nState,
@@ -1391,9 +1428,9 @@ static int launch_indel(const IndelBuffers& L, u32 ntip, u32 ncol, u32 nState, c
     }
     n++;
     if (evInit1) CASPHY_CUDA_TRY(cudaEventRecord(evInit1, st));
-    if (cluster) {
-        // one cluster where it can hold the slots; a tree beyond it, or a
-        // device that cannot place the cluster, runs on all SMs
+    if (useBits && cluster) {
+        // a tree that one cluster cannot hold, or a device that cannot place the
+        // cluster, runs on all SMs
         bool done = false;
         const int rc = intPath ? launch_cluster_indel<false>(L, ntip, ncol, nState, unitW, minSize, minRatio, st, &done, &n)
                                : launch_cluster_indel<true>(L, ntip, ncol, nState, false, minSize, minRatio, st, &done, &n);
@@ -1476,11 +1513,12 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
                   joinc::placeable((void*)k_cluster_join<IndelCluster<true>>, ca.G, cs);
     }
     if (scanEnv && !strcmp(scanEnv, "dense")) useBits = false;
+    const bool count = useBits && ntip <= kClusterTips && !joinx::grid_asked() && !always_cluster(ntip, ncol, intPath, unitW);
     u32 *dCodesCopy, *dOrder, *dState;
     void* base = nullptr;
     for (;;) {
         Carve cv;
-        carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
+        carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath, count);
         dCodesCopy = cv.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
         dOrder = cv.take<u32>(nrows);
         dState = cv.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
@@ -1491,10 +1529,9 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
         cudaGetLastError();
         useBits = false;
     }
-    lst.scan_path = useBits ? 1u : 0u;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath);
+    const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath, count);
     dCodesCopy = c2.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
     dOrder = c2.take<u32>(nrows);
     dState = c2.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
@@ -1502,11 +1539,24 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     cudaEvent_t ev[5];
     for (auto& e : ev) CASPHY_CUDA_TRY(cudaEventCreate(&e));
     CASPHY_CUDA_TRY(cudaEventRecord(ev[0], st));
+    int launches = 0;
     const u32* codes = d_codes;
     if (h_codes) {
         if ((rc = Staged::to_device(ds, dCodesCopy, h_codes, sizeof(u32) * (size_t)ntip * ncol, st))) return rc;
         codes = dCodesCopy;
     }
+    bool cluster = useBits;
+    if (useBits && count) {
+        unsigned long long n[2] = {0, 0};
+        CASPHY_CUDA_TRY(cudaMemsetAsync(L.stats, 0, sizeof(n), st));
+        k_count_codes<<<8 * nSM, 256, 0, st>>>(codes, (u64)ntip * ncol, L.stats);
+        CASPHY_CUDA_TRY(cudaMemcpyAsync(n, L.stats, sizeof(n), cudaMemcpyDeviceToHost, st));
+        CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+        launches++;
+        cluster = cluster_pays(ntip, intPath, unitW, (double)n[0], (double)n[1]);
+        if (!intPath) useBits = cluster;
+    }
+    lst.scan_path = useBits ? 1u : 0u;
     std::vector<u64> chunkStart(nChunks + 1);
     chunk_table(ntip, nChunks, chunkStart.data());
     CASPHY_CUDA_TRY(cudaMemcpyAsync(L.Wsel, intPath ? wint.data() : hbits.data(), sizeof(u16) * hbits.size(),
@@ -1514,13 +1564,14 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     CASPHY_CUDA_TRY(cudaMemcpyAsync(L.tipSize, tipSize, sizeof(u32) * ntip, cudaMemcpyHostToDevice, st));
     CASPHY_CUDA_TRY(cudaMemcpyAsync(L.chunkStart, chunkStart.data(), sizeof(u64) * (nChunks + 1),
                                     cudaMemcpyHostToDevice, st));
-    int launches = 0;
     std::vector<u32> order(nrows, 0u);
     unsigned long long hst[8] = {0};
     if (ntip >= 2) {
-        rc = launch_indel(L, ntip, ncol, nState, codes, intPath, unitW, useBits, minSize, minRatio, (u32)nSM,
-                          nChunks, chunkStart[nChunks], st, ev[1], ev[2], &launches);
+        int n = 0;
+        rc = launch_indel(L, ntip, ncol, nState, codes, intPath, unitW, useBits, cluster, minSize, minRatio, (u32)nSM,
+                          nChunks, chunkStart[nChunks], st, ev[1], ev[2], &n);
         if (rc) return rc;
+        launches += n;
         CASPHY_CUDA_TRY(cudaEventRecord(ev[3], st));
         std::vector<u32> eLenH(ntip), raw((size_t)2 * nedge);
         int errs[2] = {0, 0};
@@ -1761,7 +1812,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev));
     const u32 nChunks = (ntip + kCap - 1) / kCap;
     Carve need;
-    carve_indel(need, ntip, ncol, nState, (u32)nSM, nChunks, false, false);
+    carve_indel(need, ntip, ncol, nState, (u32)nSM, nChunks, false, false, false);
     carve_extra(need, ntip, ncol, nState);
     const size_t bytes = need.off + 256;
     if (bytes > kScratchBytes || nChunks > 64) {
@@ -1787,7 +1838,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
     } drain{st};
     Carve c;
     c.base = static_cast<char*>(base);
-    const IndelBuffers L = carve_indel(c, ntip, ncol, nState, (u32)nSM, nChunks, false, false);
+    const IndelBuffers L = carve_indel(c, ntip, ncol, nState, (u32)nSM, nChunks, false, false, false);
     const Extra X = carve_extra(c, ntip, ncol, nState);
     const size_t nw = (size_t)nState * ncol;
 
@@ -1812,7 +1863,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
                                     st));
     CASPHY_CUDA_TRY(cudaMemsetAsync(X.dfsErr, 0, sizeof(u32), st));
     int launches = 0;
-    rc = launch_indel(L, ntip, ncol, nState, d_codes, intPath, unitW, false, minSize, minRatio, (u32)nSM, nChunks,
+    rc = launch_indel(L, ntip, ncol, nState, d_codes, intPath, unitW, false, false, minSize, minRatio, (u32)nSM, nChunks,
                       chunkStart[nChunks], st, nullptr, nullptr, &launches);
     if (rc) return rc;
     k_preorder<<<1, 32, 0, st>>>(L.rawEdge, ntip, X.relabel, X.stack, X.cursor, d_edge_out, X.order, X.dfsErr);

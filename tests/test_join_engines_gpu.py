@@ -136,22 +136,34 @@ def test_bit_columns_resident_from_the_start(gpu_lib):
     assert got[2]["scan_path"] == 1 and _same(got, O.join_bit(words, w, 0))
 
 
-# Integer weights: a cluster up to 26,000,000 cells x edited sites, 4,000,000 when
-# the weights are not all 1, counted where cells x sites are more.  (Only the
-# engine of all SMs has refresh phases.)
-@pytest.mark.parametrize("ncell,nsite,weights,most,edited,on_cluster", [
-    (13500, 2048, "unit", 26000000, 0.90, True), (13500, 2048, "unit", 26000000, 0.97, False),
-    (5000, 1000, "integer", 4000000, 0.75, True), (5000, 1000, "integer", 4000000, 0.85, False)])
-def test_indel_engine_follows_the_edited_sites(gpu_lib, monkeypatch, ncell, nsite, weights, most, edited, on_cluster):
+# The cluster's line in cells x edited sites: 26,000,000 with unit weights and
+# 4,000,000 with other integers while at most 0.8 of the known sites are edited,
+# falling to 6,000,000 and 1,200,000 where all are; fractional weights leave it
+# where more than 0.7 are edited, beyond 35,000 cells or 18,000,000.  (Only the
+# engine of all SMs has refresh phases, and only the column scan path 0.)
+@pytest.mark.parametrize("ncell,nsite,weights,edited,missing,on_cluster", [
+    (13500, 2048, "unit", 0.60, 0.0, True), (13500, 2048, "unit", 0.82, 0.0, True),
+    (13500, 2048, "unit", 0.86, 0.0, False), (13500, 2048, "unit", 0.50, 0.5, False),
+    (12000, 520, "unit", 0.94, 0.06, True),
+    (5000, 1000, "integer", 0.75, 0.0, True), (5000, 1000, "integer", 0.81, 0.0, False),
+    (5000, 1000, "integer", 0.30, 0.7, False), (2000, 601, "integer", 0.98, 0.02, True),
+    (36000, 20, "half", 0.60, 0.1, True), (36000, 20, "half", 0.80, 0.1, False),
+    (9000, 2100, "half", 0.90, 0.0, True), (9000, 2100, "half", 0.97, 0.0, False)])
+def test_indel_engine_follows_the_edited_sites(gpu_lib, monkeypatch, ncell, nsite, weights, edited, missing, on_cluster):
     ns = 20
     rng = np.random.default_rng(11)
     base = rng.integers(2, ns + 2, size=(500, nsite), dtype=np.uint32)
     codes = base[rng.integers(0, len(base), size=ncell)]
-    codes[rng.random(codes.shape) >= edited] = 1
-    assert ncell * nsite > most and (int((codes > 1).sum()) <= most) == on_cluster
-    w = np.ones((ns, nsite)) if weights == "unit" else rng.integers(1, 3, size=(ns, nsite)).astype(float)
+    u = rng.random(codes.shape)
+    codes[u >= edited] = 1
+    codes[u >= 1.0 - missing] = 0
+    w = {"unit": np.ones((ns, nsite)), "integer": rng.integers(1, 3, size=(ns, nsite)).astype(float),
+         "half": rng.uniform(0.01, 4.0, size=(ns, nsite))}[weights]
     got = gpu_lib.join_indel(codes, ns, w)
-    assert got[2]["scan_path"] == 1 and (got[2]["refreshes"] == 0) == on_cluster
+    if weights == "half":
+        assert (got[2]["scan_path"] == 1) == on_cluster
+    else:
+        assert got[2]["scan_path"] == 1 and (got[2]["refreshes"] == 0) == on_cluster
     monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
     other = gpu_lib.join_indel(codes, ns, w)
     assert other[2]["refreshes"] > 0 and _same(got, other)
