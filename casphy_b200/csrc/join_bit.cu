@@ -107,6 +107,12 @@ static int launch_bit_init(const InitArgs& ia, u32 nSM, cudaStream_t st) {
 // 0.80, 0.85 and 0.86 at 75,000 x 256, 1,024 and 3,072, 0.97 at 90,000 x 512 and
 // 0.98 x 1,024, then 1.11 at 100,000 x 1,024 and 1.58 at 150,000 x 512).
 constexpr u32 kFloatClusterTips = 90000;
+// Bit planes multiply the popcounts of a scan, by cells x planes x words (read
+// eight at a time): 0.41 at 10,000 x 512 with 3 planes, 0.77 at 20,000 x 512 with 8
+// and 10,000 x 512 with 15, 0.88 at 20,000 x 1,024 with 6 (3.8 million), then 0.94 at
+// 10,000 x 1,024 with 14 (4.5), 1.25 at 80,000 x 128 with 8 (5.1), 1.31 at 20,000 x
+// 1,024 with 14 (9.0).
+constexpr u64 kPlaneClusterWork = 4500000;
 constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 
 // Launches the join on one cluster; *done says whether it could.
@@ -116,6 +122,7 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     using M = BitCluster<PATH>;
     *done = false;
     if (PATH == PATH_FLOAT && c.ntip > kFloatClusterTips) return CASPHY_OK;
+    if (PATH == PATH_PLANES && (u64)c.ntip * bm.nplanes * ((bm.nbin + 7) / 8 * 8) > kPlaneClusterWork) return CASPHY_OK;
     int smemMax = 0, dev = 0;
     CASPHY_CUDA_TRY(cudaGetDevice(&dev));
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

@@ -177,3 +177,20 @@ def test_fractional_bit_engine_follows_the_cells(gpu_lib, ncell, launches):
     words ^= np.uint32(1) << rng.integers(0, 32, size=(ncell, 1), dtype=np.uint32)
     got = gpu_lib.join_bit(words, rng.uniform(0.01, 3.0, size=32), 1)
     assert got[2]["kernel_launches"] == launches and got[2]["joins"] == ncell - 1
+
+
+# Integer weights: a cluster up to 4,500,000 cells x planes x words, the words in
+# blocks of eight.
+@pytest.mark.parametrize("ncell,nsite,top,launches", [
+    (9375, 992, 1 << 14, 5), (9376, 992, 1 << 14, 6), (9376, 992, (1 << 14) - 1, 5), (20000, 288, 1 << 14, 6),
+    (37500, 256, 1 << 14, 5), (37501, 256, 1 << 14, 6)])
+def test_plane_bit_engine_follows_planes_and_words(gpu_lib, monkeypatch, ncell, nsite, top, launches):
+    words = synth.binary_workload(ncell, nsite, 16, 0.04, 0.05, seed=ncell)
+    w = np.zeros(nsite)
+    w[:3] = 1, 2, top
+    work = ncell * int(top).bit_length() * (-(-words.shape[1] // 8) * 8)
+    assert (work <= 4500000) == (launches == 5)
+    got = gpu_lib.join_bit(words, w, 1)
+    assert got[2]["kernel_launches"] == launches
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    assert _same(got, gpu_lib.join_bit(words, w, 1))
