@@ -617,7 +617,8 @@ __global__ void __launch_bounds__(kSites) k_outside_irr(u32 root, Tree T, IrrBuf
 
 // ------------------------------------------------------- narrow levels ---
 // The levels near the root have few nodes, and a launch each costs more than
-// their work (about 4 us against 1 us).  Sites are independent, so one CTA
+// their work (about 4 us against 1 us, for as many sites as the device holds at
+// once: narrow_levels).  Sites are independent, so one CTA
 // takes 32 sites through all narrow levels, a warp per node, with a block
 // barrier between levels; what it reads of a level's nodes was written by
 // itself (or, for the first level, by the launches before).  The arithmetic per
@@ -1285,16 +1286,30 @@ static int build_tree(u32 ntip, u32 nedge, const u32* edge, FelTreeHost& T) {
         T.outOrder.insert(T.outOrder.end(), byH[h].begin(), byH[h].end());
         T.outOff.push_back((u32)T.outOrder.size());
     }
+    return CASPHY_OK;
+}
+
+// The narrow levels of a problem whose passes take `sites` sites at a time: none
+// where the CTAs of 32 sites are more than the device holds at once, two on an SM.
+// A level near the root then waits for a wave of CTAs with most of their warps
+// idle, and a launch of its own, which fills the device, is the shorter.  An
+// evaluation (HKY85, 100 tips, 12 levels) with narrow levels and without: 55 and
+// 83 us at 3,000 sites, 82 and 91 at 9,000, 123 and 97 at 12,000, 220 and 139 at
+// 25,000, 896 and 330 at 100,000; edit model 56 and 80, 61 and 90, 102 and 94, 166
+// and 130, 666 and 340.
+constexpr u32 kTopCtasPerSm = 2;
+static void narrow_levels(FelTreeHost& T, u32 sites, u32 nsm) {
     const u32 nin = (u32)T.inOff.size() - 1, nout = (u32)T.outOff.size() - 1;
     T.inTop = nin;
+    T.outTop = 0;
+    T.topEdge.assign(T.nedge, 0);
+    if ((sites + 31) / 32 > kTopCtasPerSm * nsm) return;
     while (T.inTop > 0 && nin - T.inTop < kMaxTop && T.inOff[T.inTop] - T.inOff[T.inTop - 1] <= kNarrow) T.inTop--;
     while (T.outTop < nout && T.outTop < kMaxTop && T.outOff[T.outTop + 1] - T.outOff[T.outTop] <= kNarrow) T.outTop++;
-    T.topEdge.assign(nedge, 0);
     for (u32 i = 0; i < T.outOff[T.outTop]; i++) {
-        const u32 v = T.outOrder[i] - ntip;
+        const u32 v = T.outOrder[i] - T.ntip;
         T.topEdge[T.edgeA[v]] = T.topEdge[T.edgeB[v]] = 1;
     }
-    return CASPHY_OK;
 }
 
 // HKY85 rate matrix in nibble order A,T,C,G (transitions A<->G, T<->C),
@@ -1602,6 +1617,7 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     }
+    narrow_levels(F.th, std::min(F.W, nsite), (u32)nsm);
     const u32 nCTA = (u32)std::max(1, std::min(nsm, (int)kMaxLbCTA)), Mr = hist + 1;
     if (hist >= kMaxHist) return CASPHY_EINVAL;
     struct Bufs {
