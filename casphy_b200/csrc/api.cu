@@ -258,6 +258,24 @@ int Staged::to_host(DeviceScope& ds, void* dst, const void* src, size_t bytes, v
     return CASPHY_OK;
 }
 
+int ReadBack::run(const u32* from, void* stream) const {
+    constexpr size_t kTogether = 4096;
+    u32 all[kTogether];
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    size_t n = 0;
+    for (int i = 0; i < parts; i++) n += part[i].n;
+    const bool together = n <= kTogether;
+    if (together && n) CASPHY_CUDA_TRY(cudaMemcpyAsync(all, from, sizeof(u32) * n, cudaMemcpyDeviceToHost, st));
+    for (int i = 0; i < parts && !together; from += part[i++].n)
+        if (part[i].n)
+            CASPHY_CUDA_TRY(cudaMemcpyAsync(part[i].to, from, sizeof(u32) * part[i].n, cudaMemcpyDeviceToHost, st));
+    CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+    const u32* p = all;
+    for (int i = 0; i < parts && together; p += part[i++].n)
+        if (part[i].n) std::memcpy(part[i].to, p, sizeof(u32) * part[i].n);
+    return CASPHY_OK;
+}
+
 int require_device() {
     int n = 0;
     cudaError_t e = cudaGetDeviceCount(&n);

@@ -55,15 +55,21 @@ static u32* alloc_lists(u64 n) {
 constexpr int kThreads = 256;  // candidates per CTA
 constexpr int kQ = 32;         // query rows per CTA
 enum { SC_UNIT = 0, SC_FLOAT = 1, SC_DNA = 2 };
+// DNA searches of few row pairs x plane words go to the popcounts at once: the
+// tiles and their two extra launches take a call of 50 x 50 from 69 to 74 us, 500 x
+// 500 (16 million) from 92 to 97, 1,000 x 200 (28) from 84 to 86, 1,000 x 500 (64)
+// from 113 to 111, 2,000 x 500 from 160 to 147.
+constexpr u64 kDnaPopcounts = 16000000;
 
 // rows are column-major: word k of row t at col[k * ld + t]; DNA blocks of four
-// words lie together (uint4 at [block * ld + t]) and run only in mode 2
+// words lie together (uint4 at [block * ld + t]) and, given dnaMode, run only in
+// mode 2
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) k_mask(const u32* __restrict__ col, u32 nwords, u32 ld, u32 ntip,
                                                    u32 qBegin, u32 qEnd, const float* __restrict__ wf, float radius,
                                                    u32 uradius, u32 maskWords, u32* __restrict__ mask,
                                                    const u32* __restrict__ dnaMode) {
-    if (MODE == SC_DNA && *dnaMode != 2u) return;
+    if (MODE == SC_DNA && dnaMode && *dnaMode != 2u) return;
     extern __shared__ __align__(16) u32 qs[];  // kQ x nwords query words (query rows qBegin..qEnd-1)
     const u32 q0 = qBegin + blockIdx.y * kQ;
     const u32 t = blockIdx.x * kThreads + threadIdx.x;
@@ -163,11 +169,13 @@ __global__ void k_expand(const u32* __restrict__ mask, u32 ntip, u32 maskWords, 
 // 32b+s at bit s (the reference keeps the same low nibbles, packed eight to a
 // word, cu/radiusNeighborDNA.cu:27-53).  Behind the nblk blocks follow the N
 // positions, 128 to a uint4 (word b % 4 of block nblk + b / 4).  *mode: 1 when
-// some code is N, 2 when some code has two or three bases.
+// some code is N, 2 when some code has two or three bases.  Clears *err (null:
+// nothing to clear) for the kernel that follows.
 __global__ void k_pack_dna(const u32* __restrict__ raw, u32 ntip, u32 nbinRaw, u32 nblk, u32 ld,
-                           u32* __restrict__ col, u32* __restrict__ mode) {
+                           u32* __restrict__ col, u32* __restrict__ mode, int* err) {
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 b = blockIdx.y;
+    if (t == 0 && b == 0 && err) *err = 0;
     if (t >= ntip || b >= nblk) return;
     u32 p[4] = {0u, 0u, 0u, 0u};
     for (u32 h = 0; h < 8; h++) {
@@ -192,8 +200,10 @@ __global__ void k_pack_dna(const u32* __restrict__ raw, u32 ntip, u32 nbinRaw, u
 }
 
 // Word planes -> 128-bit chunks: uint4 at [c * ld + t] = words 4c .. 4c+3 of row t.
-__global__ void k_pack_bits(const u32* __restrict__ planes, u32 ntip, u32 nwords, uint4* __restrict__ out) {
+// Clears *err for the kernel that follows.
+__global__ void k_pack_bits(const u32* __restrict__ planes, u32 ntip, u32 nwords, uint4* __restrict__ out, int* err) {
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (t == 0 && c == 0) *err = 0;
     if (t >= ntip) return;
     u32 w[4];
 #pragma unroll
@@ -293,17 +303,19 @@ struct RadiusInput {
 // Words of the device rows: DNA rows carry their N positions behind the planes.
 static size_t row_words(const RadiusInput& in) { return in.dna ? in.nwords + 4 * ((in.nwords / 4 + 3) / 4) : in.nwords; }
 
-// Uploads the rows (ld = ntip); mode: the word k_pack_dna sets.
-static int upload_rows(DeviceScope& ds, const RadiusInput& in, Carve& c, u32** col, float** wf, u32** mode, cudaStream_t st) {
+// Uploads the rows (ld = ntip).  err: the error word of the tiles that follow, which
+// k_pack_dna clears (and mode the word that it sets); null when none do.
+static int upload_rows(DeviceScope& ds, const RadiusInput& in, Carve& c, u32** col, float** wf, u32** mode, int* err,
+                       cudaStream_t st) {
     *col = c.take<u32>(row_words(in) * in.ntip);
     *wf = c.take<float>(in.wf.size() ? in.wf.size() : 1);
-    *mode = c.take<u32>(2);  // [1]: error of a device-side wait
-    CASPHY_CUDA_TRY(cudaMemsetAsync(*mode, 0, 2 * sizeof(u32), st));
+    *mode = c.take<u32>(1);
     if (in.dna) {
+        if (err) CASPHY_CUDA_TRY(cudaMemsetAsync(*mode, 0, sizeof(u32), st));
         u32* raw = c.take<u32>((size_t)in.ntip * in.nbinRaw);
         if (int rc = Staged::to_device(ds, raw, in.hostRaw, sizeof(u32) * (size_t)in.ntip * in.nbinRaw, st)) return rc;
         k_pack_dna<<<dim3((in.ntip + 255) / 256, in.nwords / 4), 256, 0, st>>>(raw, in.ntip, in.nbinRaw, in.nwords / 4,
-                                                                               in.ntip, *col, *mode);
+                                                                               in.ntip, *col, *mode, err);
     } else {
         if (int rc = Staged::to_device(ds, *col, in.hostWordPlane, sizeof(u32) * (size_t)in.nwords * in.ntip, st))
             return rc;
@@ -365,13 +377,14 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
         casphy_set_last_error_msg("radius: rows too wide for the shared-memory query tile");
         return CASPHY_ERANGE;
     }
+    const bool tiles = in.mode == SC_UNIT || (in.dna && (u64)nq * ntip * in.nwords > kDnaPopcounts);
     DeviceScope ds;
     cudaStream_t st = 0;
     auto lay = [&](Carve& c) {
         struct B { uint4* chunks; u32* mask; u32* counts; u64* off; } b;
         b.chunks = c.take<uint4>(in.mode == SC_UNIT ? (size_t)((in.nwords + 3) / 4) * ntip : 0);
         b.mask = c.take<u32>((size_t)nq * maskWords);
-        b.counts = c.take<u32>(nq);
+        b.counts = c.take<u32>((size_t)nq + 1);  // and the error of a device-side wait, read back together
         b.off = c.take<u64>(nq);
         return b;
     };
@@ -382,26 +395,33 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     u32* dmode;
     cv.take<u32>(row_words(in) * ntip);
     cv.take<float>(in.wf.size() ? in.wf.size() : 1);
-    cv.take<u32>(2);
+    cv.take<u32>(1);
     if (in.dna) cv.take<u32>((size_t)ntip * in.nbinRaw);
+    const size_t rows0 = cv.off;
     lay(cv);
-    const size_t base0 = cv.off;
     void* base = nullptr;
-    int rc = ds.reserve(base0 + 256, &base);
+    int rc = ds.reserve(cv.off + 256, &base);
     if (rc) return rc;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    rc = upload_rows(ds, in, c2, &dcol, &dwf, &dmode, st);
+    Carve c3 = c2;
+    c3.off = rows0;  // behind the rows
+    const auto L = lay(c3);
+    int* derr = reinterpret_cast<int*>(L.counts + nq);
+    rc = upload_rows(ds, in, c2, &dcol, &dwf, &dmode, tiles ? derr : nullptr, st);
     if (rc) return rc;
-    auto L = lay(c2);
     dim3 grid((ntip + kThreads - 1) / kThreads, (nq + kQ - 1) / kQ);
     if (in.mode != SC_UNIT) {
         void* fn = in.mode == SC_DNA ? (void*)k_mask<SC_DNA> : (void*)k_mask<SC_FLOAT>;
         CASPHY_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     }
-    if (in.mode == SC_FLOAT) {
-        k_mask<SC_FLOAT><<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius, in.uradius,
-                                                        maskWords, L.mask, nullptr);
+    auto mask = [&](auto fn, const u32* mode) {
+        fn<<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius, in.uradius, maskWords,
+                                         L.mask, mode);
+    };
+    if (!tiles) {
+        if (in.dna) mask(k_mask<SC_DNA>, nullptr);
+        else mask(k_mask<SC_FLOAT>, nullptr);
     } else {
         const u32 nchunk = (in.nwords + 3) / 4;
         const bool upper = nq == ntip;
@@ -416,7 +436,7 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
         a.upper = upper ? 1u : 0u;
         a.tilesN = bitdot::tiles_n(ntip);
         a.mode = in.dna ? dmode : nullptr;
-        a.err = reinterpret_cast<int*>(dmode + 1);
+        a.err = derr;
         // (counts stay far below 2^24: the least hit as an integer)
         const u32 least = in.dna ? in.uradius : (in.radius <= 0.f ? 0u : (u32)std::min(in.radius, 268435455.f));
         RadiusTile::Params p{(int)(8u * std::min(least, 0x0FFFFFFFu)), maskWords, upper ? 1u : 0u, L.mask};
@@ -425,23 +445,22 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
             casphy_set_last_error_msg("radius: too many rows");
             return CASPHY_ERANGE;
         }
-        if (!in.dna) k_pack_bits<<<dim3((ntip + 255) / 256, nchunk), 256, 0, st>>>(dcol, ntip, in.nwords, L.chunks);
+        if (!in.dna) k_pack_bits<<<dim3((ntip + 255) / 256, nchunk), 256, 0, st>>>(dcol, ntip, in.nwords, L.chunks, derr);
         CASPHY_CUDA_TRY(cudaFuncSetAttribute((void*)bitdot::k_bitdot<RadiusTile>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitdot::kSmemBytes));
         bitdot::k_bitdot<RadiusTile><<<(u32)nt, bitdot::kThreads, bitdot::kSmemBytes, st>>>(a, p);
-        if (in.dna)
-            k_mask<SC_DNA><<<grid, kThreads, smem, st>>>(dcol, in.nwords, ntip, ntip, row0, row1, dwf, in.radius,
-                                                          in.uradius, maskWords, L.mask, dmode);
+        if (in.dna) mask(k_mask<SC_DNA>, dmode);
     }
     k_count<<<(nq + 7) / 8, 256, 0, st>>>(L.mask, nq, maskWords, L.counts);
     CASPHY_CUDA_TRY(cudaGetLastError());
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(counts, L.counts, sizeof(u32) * nq, cudaMemcpyDeviceToHost, st));
-    int werr = 0;
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(&werr, dmode + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+    u32 werr = 0;
+    ReadBack back;
+    back.add(counts, nq);
+    if (tiles) back.add(&werr, 1);
+    if ((rc = back.run(L.counts, st))) return rc;
     if (werr) {
         casphy_set_last_error_msg("radius: a device-side wait timed out");
-        return werr;
+        return (int)werr;
     }
     std::vector<u64> off(nq);
     u64 tot = 0;
@@ -480,7 +499,7 @@ static int try_impl(RadiusInput& in, u32 nrep, const u32* qidx, u32* counts) {
     Carve cv;
     cv.take<u32>(row_words(in) * in.ntip);
     cv.take<float>(in.wf.size() ? in.wf.size() : 1);
-    cv.take<u32>(2);
+    cv.take<u32>(1);
     if (in.dna) cv.take<u32>((size_t)in.ntip * in.nbinRaw);
     cv.take<u32>(nrep);
     cv.take<u32>(nrep);
@@ -492,7 +511,7 @@ static int try_impl(RadiusInput& in, u32 nrep, const u32* qidx, u32* counts) {
     u32* dcol;
     float* dwf;
     u32* dmode;
-    rc = upload_rows(ds, in, c2, &dcol, &dwf, &dmode, st);
+    rc = upload_rows(ds, in, c2, &dcol, &dwf, &dmode, nullptr, st);
     if (rc) return rc;
     u32* dq = c2.take<u32>(nrep);
     u32* dc = c2.take<u32>(nrep);

@@ -30,6 +30,21 @@ struct Staged {
     static int to_host(DeviceScope& ds, void* dst, const void* src, size_t bytes, void* stream);
 };
 
+// Results that lie one behind the other on the device, read back to the host
+// arrays they belong to.  A copy to pageable memory costs about 8 us, so a few KB
+// come in one copy.
+struct ReadBack {
+    struct Part {
+        uint32_t* to;
+        size_t n;
+    };
+    Part part[5];
+    int parts = 0;
+    void add(uint32_t* to, size_t n) { part[parts++] = Part{to, n}; }
+    // Waits for the stream; the parts are filled when it returns 0.
+    int run(const uint32_t* from, void* stream) const;
+};
+
 struct Carve {
     size_t off = 0;
     char* base = nullptr;

@@ -86,11 +86,14 @@ struct TransferTile {
     }
 };
 
-// Rows of ncol words -> 128-bit chunks, uint4 at [c * n + row], and the rows'
-// popcounts and sizes: a block takes 32 rows, a warp four of them at a time.
+// Rows of ncol words -> 128-bit chunks, uint4 at [c * n + row], the rows'
+// popcounts and sizes, and the minima's start: a block takes 32 rows, a warp four
+// of them at a time.  Clears *err for the kernel that follows.
 __global__ void __launch_bounds__(256) k_pack_rows(const u32* __restrict__ M, u32 n, u32 ncol, u32 ntip, uint4* __restrict__ out,
-                                                   u32* __restrict__ pop, u32* __restrict__ size) {
+                                                   u32* __restrict__ pop, u32* __restrict__ size, u32* __restrict__ least,
+                                                   int* err) {
     __shared__ u32 t[32][33];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * 32;
     u32 cnt[4] = {0u, 0u, 0u, 0u};  // rows r0 + warp + 8 i
     for (u32 k0 = 0; k0 < ncol; k0 += 32) {
@@ -115,13 +118,9 @@ __global__ void __launch_bounds__(256) k_pack_rows(const u32* __restrict__ M, u3
         if (lane == 0 && r < n) {
             pop[r] = c;
             size[r] = c > ntip - c ? ntip - c : c;
+            least[r] = 32u * ncol;
         }
     }
-}
-
-__global__ void k_fill_u32(u32* p, u32 n, u32 v) {
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
 }
 
 }  // namespace tdis
@@ -130,7 +129,6 @@ __global__ void k_fill_u32(u32* p, u32 n, u32 v) {
 struct TransferScratch {
     uint4 *cy, *cx;  // chunks
     u32 *py, *px;    // popcounts
-    int* err;
 };
 static TransferScratch carve_scratch(Carve& c, u32 ny, u32 nx, u32 ncol) {
     const size_t chunks = (ncol + 3) / 4;
@@ -139,23 +137,15 @@ static TransferScratch carve_scratch(Carve& c, u32 ny, u32 nx, u32 ncol) {
     s.cx = c.take<uint4>(chunks * nx);
     s.py = c.take<u32>(ny);
     s.px = c.take<u32>(nx);
-    s.err = c.take<int>(1);
     return s;
 }
 
 static int transfer_dis_device(u32 ny, u32 nx, u32 ncol, u32 ntip, const u32* dY, const u32* dX, u32* dYmin,
-                               u32* dYsize, u32* dXmin, u32* dXsize, const TransferScratch& s, cudaStream_t st) {
+                               u32* dYsize, u32* dXmin, u32* dXsize, int* err, const TransferScratch& s, cudaStream_t st) {
     using namespace tdis;
     const u32 full = 32u * ncol;
-    CASPHY_CUDA_TRY(cudaMemsetAsync(s.err, 0, sizeof(int), st));
-    if (ny) {
-        k_fill_u32<<<(ny + 255) / 256, 256, 0, st>>>(dYmin, ny, full);
-        k_pack_rows<<<(ny + 31) / 32, 256, 0, st>>>(dY, ny, ncol, ntip, s.cy, s.py, dYsize);
-    }
-    if (nx) {
-        k_fill_u32<<<(nx + 255) / 256, 256, 0, st>>>(dXmin, nx, full);
-        k_pack_rows<<<(nx + 31) / 32, 256, 0, st>>>(dX, nx, ncol, ntip, s.cx, s.px, dXsize);
-    }
+    if (ny) k_pack_rows<<<(ny + 31) / 32, 256, 0, st>>>(dY, ny, ncol, ntip, s.cy, s.py, dYsize, dYmin, err);
+    if (nx) k_pack_rows<<<(nx + 31) / 32, 256, 0, st>>>(dX, nx, ncol, ntip, s.cx, s.px, dXsize, dXmin, err);
     if (nx && ny) {
         bitdot::Args a{};
         a.A = s.cx;
@@ -164,7 +154,7 @@ static int transfer_dis_device(u32 ny, u32 nx, u32 ncol, u32 ntip, const u32* dY
         a.ldB = a.rowsB = ny;
         a.chunks = a.negFrom = (ncol + 3) / 4;
         a.tilesN = bitdot::tiles_n(ny);
-        a.err = s.err;
+        a.err = err;
         const u64 nt = bitdot::tiles(nx, ny, false);
         if (nt > 0x7FFFFFFFull) {
             casphy_set_last_error_msg("transfer: too many rows");
@@ -188,16 +178,16 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     int rc = require_device();
     if (rc) return rc;
     if (ncol == 0 || (nrow_y && (!y || !ymin || !ysize)) || (nrow_x && (!x || !xmin || !xsize))) return CASPHY_EINVAL;
+    if (!nrow_y && !nrow_x) return CASPHY_OK;
     DeviceScope ds;
     cudaStream_t st = 0;
+    // minima and sizes of both sides and the error of a device-side wait, read back together
+    const size_t nout = 2 * (size_t)nrow_y + 2 * (size_t)nrow_x + 1;
     auto lay = [&](Carve& c) {
-        struct B { u32* y; u32* x; u32* ymin; u32* ysize; u32* xmin; u32* xsize; TransferScratch s; } b;
+        struct B { u32* y; u32* x; u32* out; TransferScratch s; } b;
         b.y = c.take<u32>((size_t)nrow_y * ncol);
         b.x = c.take<u32>((size_t)nrow_x * ncol);
-        b.ymin = c.take<u32>(nrow_y);
-        b.ysize = c.take<u32>(nrow_y);
-        b.xmin = c.take<u32>(nrow_x);
-        b.xsize = c.take<u32>(nrow_x);
+        b.out = c.take<u32>(nout);
         b.s = carve_scratch(c, nrow_y, nrow_x, ncol);
         return b;
     };
@@ -211,19 +201,18 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     auto L = lay(c2);
     if (nrow_y && (rc = Staged::to_device(ds, L.y, y, sizeof(u32) * (size_t)nrow_y * ncol, st))) return rc;
     if (nrow_x && (rc = Staged::to_device(ds, L.x, x, sizeof(u32) * (size_t)nrow_x * ncol, st))) return rc;
-    rc = transfer_dis_device(nrow_y, nrow_x, ncol, ntip, L.y, L.x, L.ymin, L.ysize, L.xmin, L.xsize, L.s, st);
+    u32 *dYmin = L.out, *dYsize = dYmin + nrow_y, *dXmin = dYsize + nrow_y, *dXsize = dXmin + nrow_x;
+    rc = transfer_dis_device(nrow_y, nrow_x, ncol, ntip, L.y, L.x, dYmin, dYsize, dXmin, dXsize,
+                             reinterpret_cast<int*>(dXsize + nrow_x), L.s, st);
     if (rc) return rc;
-    int werr = 0;
-    CASPHY_CUDA_TRY(cudaMemcpyAsync(&werr, L.s.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (nrow_y) {
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(ymin, L.ymin, sizeof(u32) * nrow_y, cudaMemcpyDeviceToHost, st));
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(ysize, L.ysize, sizeof(u32) * nrow_y, cudaMemcpyDeviceToHost, st));
-    }
-    if (nrow_x) {
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(xmin, L.xmin, sizeof(u32) * nrow_x, cudaMemcpyDeviceToHost, st));
-        CASPHY_CUDA_TRY(cudaMemcpyAsync(xsize, L.xsize, sizeof(u32) * nrow_x, cudaMemcpyDeviceToHost, st));
-    }
-    CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
+    u32 werr = 0;
+    ReadBack back;
+    back.add(ymin, nrow_y);
+    back.add(ysize, nrow_y);
+    back.add(xmin, nrow_x);
+    back.add(xsize, nrow_x);
+    back.add(&werr, 1);
+    if ((rc = back.run(L.out, st))) return rc;
     if (werr) casphy_set_last_error_msg("transfer: a device-side wait timed out");
-    return werr;
+    return (int)werr;
 }
