@@ -15,7 +15,7 @@
 // epilogue forms the grouped minima from them (groups of 8 columns in a thread,
 // groups of 8 rows by shuffles), one atomicMin per row and column of the tile.
 // 9,998 x 9,998 rows of 313 words: popcounts of the XORed words took 7 ms.
-#include <vector>
+#include <algorithm>
 
 #include "bitdot.cuh"
 #include "common.cuh"
@@ -86,12 +86,13 @@ struct TransferTile {
     }
 };
 
-// Rows of ncol words -> 128-bit chunks, uint4 at [c * n + row], the rows'
-// popcounts and sizes, and the minima's start: a block takes 32 rows, a warp four
-// of them at a time.  Clears *err for the kernel that follows.
-__global__ void __launch_bounds__(256) k_pack_rows(const u32* __restrict__ M, u32 n, u32 ncol, u32 ntip, uint4* __restrict__ out,
-                                                   u32* __restrict__ pop, u32* __restrict__ size, u32* __restrict__ least,
-                                                   int* err) {
+// Rows r00 .. r00 + m - 1 of n, ncol words each (M: row r00) -> 128-bit chunks,
+// uint4 at [c * n + row], and the rows' popcounts and sizes, and the minima's start:
+// a block takes 32 rows, a warp four of them at a time.  Clears *err for the kernel
+// that follows.
+__global__ void __launch_bounds__(256) k_pack_rows(const u32* __restrict__ M, u32 r00, u32 m, u32 n, u32 ncol, u32 ntip,
+                                                   uint4* __restrict__ out, u32* __restrict__ pop, u32* __restrict__ size,
+                                                   u32* __restrict__ least, int* err) {
     __shared__ u32 t[32][33];
     if (blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * 32;
@@ -100,56 +101,64 @@ __global__ void __launch_bounds__(256) k_pack_rows(const u32* __restrict__ M, u3
 #pragma unroll
         for (u32 i = 0; i < 4; i++) {
             const u32 r = r0 + warp + 8 * i, k = k0 + lane;
-            const u32 v = r < n && k < ncol ? M[(size_t)r * ncol + k] : 0u;
+            const u32 v = r < m && k < ncol ? M[(size_t)r * ncol + k] : 0u;
             t[warp + 8 * i][lane] = v;
             cnt[i] += (u32)__popc(v);
         }
         __syncthreads();
         // warp w: chunk w of the eight, lane = row
         const u32 c = k0 / 4 + warp;
-        if (4 * c < ncol && r0 + lane < n)
-            out[(size_t)c * n + r0 + lane] =
+        if (4 * c < ncol && r0 + lane < m)
+            out[(size_t)c * n + r00 + r0 + lane] =
                 make_uint4(t[lane][4 * warp], t[lane][4 * warp + 1], t[lane][4 * warp + 2], t[lane][4 * warp + 3]);
         __syncthreads();
     }
 #pragma unroll
     for (u32 i = 0; i < 4; i++) {
         const u32 c = __reduce_add_sync(0xFFFFFFFFu, cnt[i]), r = r0 + warp + 8 * i;
-        if (lane == 0 && r < n) {
-            pop[r] = c;
-            size[r] = c > ntip - c ? ntip - c : c;
-            least[r] = 32u * ncol;
+        if (lane == 0 && r < m) {
+            pop[r00 + r] = c;
+            size[r00 + r] = c > ntip - c ? ntip - c : c;
+            least[r00 + r] = 32u * ncol;
         }
     }
 }
 
 }  // namespace tdis
 
-// Device scratch of transfer_dis_device.
-struct TransferScratch {
-    uint4 *cy, *cx;  // chunks
-    u32 *py, *px;    // popcounts
+// Rows of one side on the device.
+struct TransferSide {
+    u32 n;
+    const u32* host;
+    uint4* chunks;
+    u32* pop;
+    u32 *least, *size;  // minima and sizes
 };
-static TransferScratch carve_scratch(Carve& c, u32 ny, u32 nx, u32 ncol) {
-    const size_t chunks = (ncol + 3) / 4;
-    TransferScratch s;
-    s.cy = c.take<uint4>(chunks * ny);
-    s.cx = c.take<uint4>(chunks * nx);
-    s.py = c.take<u32>(ny);
-    s.px = c.take<u32>(nx);
-    return s;
+
+// Uploads and packs a side's rows, `per` at a time through `panel`.  The chunks are
+// all that is kept: beside the rows themselves they would take twice the memory,
+// and 600,000 clades a side (90 GB) would not fit any more.
+constexpr size_t kPanelBytes = size_t(64) << 20;
+static u32 panel_rows(u32 n, u32 ncol) {
+    return std::min(n, (u32)std::max<size_t>(kPanelBytes / (sizeof(u32) * ncol) / 32 * 32, 32));
+}
+static int pack_side(DeviceScope& ds, const TransferSide& s, u32 ncol, u32 ntip, u32* panel, int* err, cudaStream_t st) {
+    const u32 per = panel_rows(s.n, ncol);
+    for (u32 r = 0; r < s.n; r += per) {
+        const u32 m = std::min(per, s.n - r);
+        if (int rc = Staged::to_device(ds, panel, s.host + (size_t)r * ncol, sizeof(u32) * (size_t)m * ncol, st)) return rc;
+        tdis::k_pack_rows<<<(m + 31) / 32, 256, 0, st>>>(panel, r, m, s.n, ncol, ntip, s.chunks, s.pop, s.size, s.least, err);
+    }
+    return CASPHY_OK;
 }
 
-static int transfer_dis_device(u32 ny, u32 nx, u32 ncol, u32 ntip, const u32* dY, const u32* dX, u32* dYmin,
-                               u32* dYsize, u32* dXmin, u32* dXsize, int* err, const TransferScratch& s, cudaStream_t st) {
+static int transfer_tiles(const TransferSide& y, const TransferSide& x, u32 ncol, u32 ntip, int* err, cudaStream_t st) {
     using namespace tdis;
-    const u32 full = 32u * ncol;
-    if (ny) k_pack_rows<<<(ny + 31) / 32, 256, 0, st>>>(dY, ny, ncol, ntip, s.cy, s.py, dYsize, dYmin, err);
-    if (nx) k_pack_rows<<<(nx + 31) / 32, 256, 0, st>>>(dX, nx, ncol, ntip, s.cx, s.px, dXsize, dXmin, err);
+    const u32 full = 32u * ncol, nx = x.n, ny = y.n;
     if (nx && ny) {
         bitdot::Args a{};
-        a.A = s.cx;
-        a.B = s.cy;
+        a.A = x.chunks;
+        a.B = y.chunks;
         a.ldA = a.rowsA = nx;
         a.ldB = a.rowsB = ny;
         a.chunks = a.negFrom = (ncol + 3) / 4;
@@ -163,7 +172,7 @@ static int transfer_dis_device(u32 ny, u32 nx, u32 ncol, u32 ntip, const u32* dY
         CASPHY_CUDA_TRY(cudaFuncSetAttribute((void*)bitdot::k_bitdot<TransferTile>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitdot::kSmemBytes));
         bitdot::k_bitdot<TransferTile><<<(u32)nt, bitdot::kThreads, bitdot::kSmemBytes, st>>>(
-            a, TransferTile::Params{full, full - ntip, s.px, s.py, dXmin, dYmin});
+            a, TransferTile::Params{full, full - ntip, x.pop, y.pop, x.least, y.least});
     }
     CASPHY_CUDA_TRY(cudaGetLastError());
     return CASPHY_OK;
@@ -181,15 +190,19 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     if (!nrow_y && !nrow_x) return CASPHY_OK;
     DeviceScope ds;
     cudaStream_t st = 0;
-    // minima and sizes of both sides and the error of a device-side wait, read back together
-    const size_t nout = 2 * (size_t)nrow_y + 2 * (size_t)nrow_x + 1;
+    const u32 per = std::max(panel_rows(nrow_y, ncol), panel_rows(nrow_x, ncol));
+    const size_t chunks = (ncol + 3) / 4;
+    TransferSide Y{nrow_y, y, nullptr, nullptr, nullptr, nullptr}, X{nrow_x, x, nullptr, nullptr, nullptr, nullptr};
+    u32 *panel, *out;
     auto lay = [&](Carve& c) {
-        struct B { u32* y; u32* x; u32* out; TransferScratch s; } b;
-        b.y = c.take<u32>((size_t)nrow_y * ncol);
-        b.x = c.take<u32>((size_t)nrow_x * ncol);
-        b.out = c.take<u32>(nout);
-        b.s = carve_scratch(c, nrow_y, nrow_x, ncol);
-        return b;
+        panel = c.take<u32>((size_t)per * ncol);
+        for (TransferSide* s : {&Y, &X}) {
+            s->chunks = c.take<uint4>(chunks * s->n);
+            s->pop = c.take<u32>(s->n);
+        }
+        // minima and sizes of both sides and the error of a device-side wait, read
+        // back together
+        out = c.take<u32>(2 * (size_t)nrow_y + 2 * (size_t)nrow_x + 1);
     };
     Carve cv;
     lay(cv);
@@ -198,13 +211,15 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     if (rc) return rc;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    auto L = lay(c2);
-    if (nrow_y && (rc = Staged::to_device(ds, L.y, y, sizeof(u32) * (size_t)nrow_y * ncol, st))) return rc;
-    if (nrow_x && (rc = Staged::to_device(ds, L.x, x, sizeof(u32) * (size_t)nrow_x * ncol, st))) return rc;
-    u32 *dYmin = L.out, *dYsize = dYmin + nrow_y, *dXmin = dYsize + nrow_y, *dXsize = dXmin + nrow_x;
-    rc = transfer_dis_device(nrow_y, nrow_x, ncol, ntip, L.y, L.x, dYmin, dYsize, dXmin, dXsize,
-                             reinterpret_cast<int*>(dXsize + nrow_x), L.s, st);
-    if (rc) return rc;
+    lay(c2);
+    Y.least = out;
+    Y.size = Y.least + nrow_y;
+    X.least = Y.size + nrow_y;
+    X.size = X.least + nrow_x;
+    int* err = reinterpret_cast<int*>(X.size + nrow_x);
+    if ((rc = pack_side(ds, Y, ncol, ntip, panel, err, st))) return rc;
+    if ((rc = pack_side(ds, X, ncol, ntip, panel, err, st))) return rc;
+    if ((rc = transfer_tiles(Y, X, ncol, ntip, err, st))) return rc;
     u32 werr = 0;
     ReadBack back;
     back.add(ymin, nrow_y);
@@ -212,7 +227,7 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     back.add(xmin, nrow_x);
     back.add(xsize, nrow_x);
     back.add(&werr, 1);
-    if ((rc = back.run(L.out, st))) return rc;
+    if ((rc = back.run(out, st))) return rc;
     if (werr) casphy_set_last_error_msg("transfer: a device-side wait timed out");
     return (int)werr;
 }

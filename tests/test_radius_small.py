@@ -46,3 +46,17 @@ def test_transfer_of_one_side_only(gpu_lib):
     for a, b in ((y, none), (none, y), (none, none)):
         for got, want in zip(gpu_lib.transfer_dis(a, b, 90), O.transfer_dis(a, b, 90)):
             assert np.array_equal(got, want)
+
+
+def test_transfer_rows_in_panels(gpu_lib):
+    """Rows come through a 64 MiB panel: 520 rows of 32,768 words take two, the
+    other side one."""
+    rng = np.random.default_rng(3)
+    nb = 32768
+    y = rng.integers(0, 1 << 32, size=(520, nb), dtype=np.uint64).astype(np.uint32)
+    x = y[rng.integers(0, 520, size=37)].copy()
+    x[::2, :100] ^= np.uint32(1)
+    for got, want in zip(gpu_lib.transfer_dis(y, x, 32 * nb), O.transfer_dis(y, x, 32 * nb)):
+        assert np.array_equal(got, want)
+    for got, want in zip(gpu_lib.transfer_dis(x, y, 32 * nb), O.transfer_dis(x, y, 32 * nb)):
+        assert np.array_equal(got, want)
