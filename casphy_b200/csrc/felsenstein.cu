@@ -434,19 +434,17 @@ __global__ void __launch_bounds__(256) k_allele_counts(const u32* __restrict__ c
         if (at < nsite && hist[i]) atomicAdd(count + (size_t)at * qstride + i % qstride, hist[i]);
     }
 }
-// q = count / total per site, binary64 rounded to binary32; equal shares where
-// no tip has an allele.  A warp per site.
-__global__ void __launch_bounds__(256) k_allele_freq(const u32* __restrict__ count, u32 nsite, u32 qstride,
-                                                     float* __restrict__ q) {
+// The counts at q become q = count / total per site, binary64 rounded to binary32;
+// equal shares where no tip has an allele.  A warp per site.
+__global__ void __launch_bounds__(256) k_allele_freq(u32 nsite, u32 qstride, float* q) {
     const u32 lane = threadIdx.x & 31, s = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (s >= nsite) return;
+    q += (size_t)s * qstride;
     u32 t = 0;
-    for (u32 a = 1 + lane; a < qstride; a += 32) t += count[(size_t)s * qstride + a];
+    for (u32 a = lane; a < qstride; a += 32) t += __float_as_uint(q[a]);  // (index 0 counts nothing)
     t = __reduce_add_sync(0xFFFFFFFFu, t);
     for (u32 a = lane; a < qstride; a += 32)
-        q[(size_t)s * qstride + a] = a == 0 ? 0.f
-                                     : t    ? (float)((double)count[(size_t)s * qstride + a] / (double)t)
-                                            : (float)(1.0 / (qstride - 1));
+        q[a] = a == 0 ? 0.f : t ? (float)((double)__float_as_uint(q[a]) / (double)t) : (float)(1.0 / (qstride - 1));
 }
 
 // One (node, site) of the inside pass once its children's partials are in.
@@ -1624,7 +1622,6 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         u32 *kidA, *kidB, *edgeA, *edgeB, *inO, *outO, *codes, *flags, *inEB, *outEB;
         uint4 *inInfo, *outInfo;
         double *t, *w, *grad, *gpart, *part, *ll;
-        u32* alleleCount;
         int* badCode;
         float* gw;
         unsigned char* top;
@@ -1671,7 +1668,6 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         b.dP = c.take<float>(isH ? 16 * (size_t)nedge : 0);
         b.p = c.take<float2>(isH ? 0 : nedge);
         b.q = c.take<float>(isH ? 0 : (size_t)nsite * qstride);
-        b.alleleCount = c.take<u32>(isH || model->allele_freq ? 0 : (size_t)nsite * qstride);
         b.badCode = c.take<int>(1);
         b.gw = c.take<float>((size_t)nedge * ((nsite + 31) / 32));
         b.top = c.take<unsigned char>(nedge);
@@ -1731,11 +1727,12 @@ static int setup_problem(FelProblem& F, DeviceScope& ds, u32 ntip, u32 nedge, co
         const bool given = model->allele_freq != nullptr;
         const u32 useShared = !given && 32u * qstride * sizeof(u32) <= 48 * 1024 ? 1u : 0u;
         CASPHY_CUDA_TRY(cudaMemsetAsync(L.badCode, 0, sizeof(int), st));
-        if (!given) CASPHY_CUDA_TRY(cudaMemsetAsync(L.alleleCount, 0, 4ull * nsite * qstride, st));
+        u32* count = given ? nullptr : reinterpret_cast<u32*>(L.q);  // counts, then frequencies in their place
+        if (!given) CASPHY_CUDA_TRY(cudaMemsetAsync(count, 0, 4ull * nsite * qstride, st));
         k_allele_counts<<<dim3((nsite + 31) / 32, (ntip + kCountRows - 1) / kCountRows), 256,
                           useShared ? 32u * qstride * sizeof(u32) : 0u, st>>>(
-            L.codes, ntip, nsite, model->nallele, qstride, useShared, given ? nullptr : L.alleleCount, L.badCode);
-        if (!given) k_allele_freq<<<(nsite + 7) / 8, 256, 0, st>>>(L.alleleCount, nsite, qstride, L.q);
+            L.codes, ntip, nsite, model->nallele, qstride, useShared, count, L.badCode);
+        if (!given) k_allele_freq<<<(nsite + 7) / 8, 256, 0, st>>>(nsite, qstride, L.q);
         CASPHY_CUDA_TRY(cudaGetLastError());
         CASPHY_CUDA_TRY(cudaMemcpyAsync(&bad, L.badCode, sizeof(int), cudaMemcpyDeviceToHost, st));
         if (given) {
