@@ -1154,12 +1154,6 @@ struct IndelBuffers {
     unsigned long long* tileCounter; u64* chunkStart; unsigned long long* stats; u32* tipSize;
 };
 
-// Bytes of the two allele-bitset buffers for the bitset scan.
-static size_t bits_bytes(u32 ntip, u32 ncol, u32 nState) {
-    const size_t Wd = ((size_t)ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32);
-    return 2 * (size_t)ncol * nState * Wd * sizeof(u32);
-}
-
 // One cluster or all SMs.  A phase on a cluster costs about 4 us plus the scan of
 // a sixteenth of the slots, on all SMs about 10 us plus a scan of a 148th, for up
 // to eight rows at once when stale rows are rescanned.  So the choice goes by
@@ -1213,27 +1207,37 @@ static u32 cluster_size(u32 ntip) {
 }
 static u32 cluster_range(u32 ntip, u32 G) { return ((ntip + G - 1) / G + kBitsAlign - 1) / kBitsAlign * kBitsAlign; }
 
-// mayScan: fractional weights whose engine is chosen once the edited sites are
-// counted have room for the column scan too.
-static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nCTA, u32 nChunks, bool useBits,
-                                bool intPath, bool mayScan) {
+// Words of one allele-bitset buffer: rows of all slots or, for a cluster, every
+// CTA's rows of its own range, which rounds each range up.
+static size_t bits_words(u32 ntip, u32 ncol, u32 nState, bool cluster) {
+    const u32 G = cluster_size(ntip);
+    const size_t row = ((size_t)ntip + kBitsAlign - 1) / kBitsAlign * (kBitsAlign / 32);
+    const size_t split = cluster ? (size_t)cluster_range(ntip, G) / 32 * G : 0;
+    return (size_t)ncol * nState * std::max(row, split);
+}
+// What a call's buffers have room for.
+struct IndelRoom {
+    bool bits;     // allele bitsets
+    bool cluster;  // ... in a cluster's layout too
+    bool columns;  // both column matrices; else only what the initial scan needs
+};
+static IndelBuffers carve_indel(Carve& c, u32 ntip, u32 ncol, u32 nState, u32 nCTA, u32 nChunks, bool intPath,
+                                IndelRoom room) {
     const u32 nnode = 2 * ntip - 1, nedge = 2 * ntip - 2;
     // the bitset scan copies 16-byte pieces of bitset rows: slot ranges and
     // row strides are multiples of 128 slots (kBitsAlign)
-    const u32 ncolP = (ncol + 7u) & ~7u, Sp = useBits ? (ntip + kBitsAlign - 1) / kBitsAlign * kBitsAlign
-                                                      : (ntip + 31u) & ~31u;
+    const u32 ncolP = (ncol + 7u) & ~7u, Sp = room.bits ? (ntip + kBitsAlign - 1) / kBitsAlign * kBitsAlign
+                                                        : (ntip + 31u) & ~31u;
     const size_t nw = (size_t)nState * ncol;
     IndelBuffers l;
     l.Wsel = c.take<u16>(nw ? nw : 1);
     l.nodeRow = c.take<u16>((size_t)nnode * ncolP);
-    l.colT0 = c.take<u16>(useBits && intPath ? 0 : (size_t)ncol * Sp);  // binary16 initial scan, dense join
-    l.colT1 = c.take<u16>(useBits && (intPath || !mayScan) ? 0 : (size_t)ncol * Sp);
-    l.bitsWords = useBits ? (size_t)ncol * nState * (Sp / 32) : 0;
-    // the cluster's layout rounds every CTA's range up
-    const u32 G = cluster_size(ntip);
-    const size_t split = useBits && ntip <= kClusterTips ? (size_t)ncol * nState * (cluster_range(ntip, G) / 32) * G : 0;
-    l.bits0 = c.take<u32>(std::max(l.bitsWords, split));
-    l.bits1 = c.take<u32>(std::max(l.bitsWords, split));
+    l.colT0 = c.take<u16>(room.columns || !intPath ? (size_t)ncol * Sp : 0);  // binary16 initial scan, dense join
+    l.colT1 = c.take<u16>(room.columns ? (size_t)ncol * Sp : 0);
+    l.bitsWords = room.bits ? bits_words(ntip, ncol, nState, false) : 0;
+    const size_t words = room.bits ? bits_words(ntip, ncol, nState, room.cluster) : 0;
+    l.bits0 = c.take<u32>(words);
+    l.bits1 = c.take<u32>(words);
     for (int i = 0; i < 6; i++) l.lm[i] = c.take<u32>(Sp);
     l.node2slot = c.take<u32>(nnode);
     l.nodeDeath = c.take<u32>(nnode);
@@ -1501,37 +1505,43 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
     int nSM = 0;
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, ds.dev));
     const u32 nChunks = (ntip + kCap - 1) / kCap;
-    // allele-bitset scan on the integer path when the two bitset buffers fit
-    // a 48 GiB budget (CASPHY_INDEL_SCAN=dense forces the column scan)
+    // allele-bitset scan when the two bitset buffers fit a 48 GiB budget
+    // (CASPHY_INDEL_SCAN=dense forces the column scan); fractional weights: on a
+    // cluster only
     const char* scanEnv = getenv("CASPHY_INDEL_SCAN");
-    bool useBits = ntip >= 2 && bits_bytes(ntip, ncol, nState) <= (size_t(48) << 30);
-    if (useBits && !intPath) {  // ordered binary16 sums on the bitsets: the cluster engine only
+    auto fits = [&](bool cl) { return 2 * sizeof(u32) * bits_words(ntip, ncol, nState, cl) <= (size_t(48) << 30); };
+    IndelRoom room{ntip >= 2 && fits(false) && !(scanEnv && !strcmp(scanEnv, "dense")), false, false};
+    room.cluster = room.bits && ntip <= kClusterTips && !joinx::grid_asked() && fits(true);
+    if (room.cluster && !intPath) {
         joinc::Args ca{};
         IndelCluster<true>::Args cm{};
         size_t cs = 0;
-        useBits = cluster_plan<true>(ntip, ncol, nState, false, ca, cm, &cs) &&
-                  joinc::placeable((void*)k_cluster_join<IndelCluster<true>>, ca.G, cs);
+        room.cluster = cluster_plan<true>(ntip, ncol, nState, false, ca, cm, &cs) &&
+                       joinc::placeable((void*)k_cluster_join<IndelCluster<true>>, ca.G, cs);
     }
-    if (scanEnv && !strcmp(scanEnv, "dense")) useBits = false;
-    const bool count = useBits && ntip <= kClusterTips && !joinx::grid_asked() && !always_cluster(ntip, ncol, intPath, unitW);
+    if (!intPath) room.bits = room.cluster;
+    const bool count = room.cluster && !always_cluster(ntip, ncol, intPath, unitW);
+    room.columns = !room.bits || (!intPath && count);  // fractional weights may turn to the column scan
     u32 *dCodesCopy, *dOrder, *dState;
     void* base = nullptr;
     for (;;) {
         Carve cv;
-        carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath, count);
+        carve_indel(cv, ntip, ncol, nState, (u32)nSM, nChunks, intPath, room);
         dCodesCopy = cv.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
         dOrder = cv.take<u32>(nrows);
         dState = cv.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
         rc = ds.reserve(cv.off + 256, &base);
         if (!rc) break;
-        // fractional weights do without the bitsets when there is no room
-        if (!useBits || intPath) return rc;
+        // without room for the cluster's layout the call does without it:
+        // bitsets on all SMs or, for fractional weights, the column scan
+        if (!room.cluster) return rc;
         cudaGetLastError();
-        useBits = false;
+        room = IndelRoom{intPath, false, !intPath};
     }
+    bool useBits = room.bits;
     Carve c2;
     c2.base = static_cast<char*>(base);
-    const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, useBits, intPath, count);
+    const IndelBuffers L = carve_indel(c2, ntip, ncol, nState, (u32)nSM, nChunks, intPath, room);
     dCodesCopy = c2.take<u32>(h_codes ? (size_t)ntip * ncol : 0);
     dOrder = c2.take<u32>(nrows);
     dState = c2.take<u32>(h_state_out ? (size_t)nrows * ncol : 0);
@@ -1545,8 +1555,8 @@ static int join_indel_impl(u32 ntip, u32 ncol, const u32* d_codes, u32 nState, c
         if ((rc = Staged::to_device(ds, dCodesCopy, h_codes, sizeof(u32) * (size_t)ntip * ncol, st))) return rc;
         codes = dCodesCopy;
     }
-    bool cluster = useBits;
-    if (useBits && count) {
+    bool cluster = room.cluster;
+    if (cluster && count) {
         unsigned long long n[2] = {0, 0};
         CASPHY_CUDA_TRY(cudaMemsetAsync(L.stats, 0, sizeof(n), st));
         k_count_codes<<<8 * nSM, 256, 0, st>>>(codes, (u64)ntip * ncol, L.stats);
@@ -1812,7 +1822,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev));
     const u32 nChunks = (ntip + kCap - 1) / kCap;
     Carve need;
-    carve_indel(need, ntip, ncol, nState, (u32)nSM, nChunks, false, false, false);
+    carve_indel(need, ntip, ncol, nState, (u32)nSM, nChunks, false, IndelRoom{false, false, true});
     carve_extra(need, ntip, ncol, nState);
     const size_t bytes = need.off + 256;
     if (bytes > kScratchBytes || nChunks > 64) {
@@ -1838,7 +1848,7 @@ extern "C" int casphy_join_indel_noalloc(uint32_t ntip, uint32_t ncol, const uin
     } drain{st};
     Carve c;
     c.base = static_cast<char*>(base);
-    const IndelBuffers L = carve_indel(c, ntip, ncol, nState, (u32)nSM, nChunks, false, false, false);
+    const IndelBuffers L = carve_indel(c, ntip, ncol, nState, (u32)nSM, nChunks, false, IndelRoom{false, false, true});
     const Extra X = carve_extra(c, ntip, ncol, nState);
     const size_t nw = (size_t)nState * ncol;
 
