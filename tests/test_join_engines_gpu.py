@@ -179,17 +179,17 @@ def test_fractional_bit_engine_follows_the_cells(gpu_lib, ncell, launches):
     assert got[2]["kernel_launches"] == launches and got[2]["joins"] == ncell - 1
 
 
-# Integer weights: a cluster up to 4,500,000 cells x planes x words, the words in
-# blocks of eight.
+# Integer weights of several planes: a cluster up to 4,500,000 cells x planes x
+# words, the words in blocks of eight, and up to 448 words.
 @pytest.mark.parametrize("ncell,nsite,top,launches", [
     (9375, 992, 1 << 14, 5), (9376, 992, 1 << 14, 6), (9376, 992, (1 << 14) - 1, 5), (20000, 288, 1 << 14, 6),
-    (37500, 256, 1 << 14, 5), (37501, 256, 1 << 14, 6)])
+    (37500, 256, 1 << 14, 5), (37501, 256, 1 << 14, 6), (300, 14336, 4, 5), (300, 14368, 4, 6)])
 def test_plane_bit_engine_follows_planes_and_words(gpu_lib, monkeypatch, ncell, nsite, top, launches):
     words = synth.binary_workload(ncell, nsite, 16, 0.04, 0.05, seed=ncell)
     w = np.zeros(nsite)
     w[:3] = 1, 2, top
     work = ncell * int(top).bit_length() * (-(-words.shape[1] // 8) * 8)
-    assert (work <= 4500000) == (launches == 5)
+    assert (work <= 4500000 and nsite <= 14336) == (launches == 5)
     got = gpu_lib.join_bit(words, w, 1)
     assert got[2]["kernel_launches"] == launches
     monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
