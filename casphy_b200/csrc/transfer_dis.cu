@@ -14,7 +14,8 @@
 // one tensor-core contraction (bitdot.cuh) and the row popcounts; the tile's
 // epilogue forms the grouped minima from them (groups of 8 columns in a thread,
 // groups of 8 rows by shuffles), one atomicMin per row and column of the tile.
-// 9,998 x 9,998 rows of 313 words: popcounts of the XORed words took 7 ms.
+// 9,998 x 9,998 rows of 313 words: popcounts of the XORed words took 7 ms.  Calls
+// of few row pairs and words keep to those (k_cross).
 #include <algorithm>
 
 #include "bitdot.cuh"
@@ -85,6 +86,94 @@ struct TransferTile {
         if (tid < bitdot::kM && m0 + tid < a.rowsA) atomicMin(p.xmin + m0 + tid, s_x[tid]);
     }
 };
+
+// Sizes and the minima's start of both sides' rows, rows of y first: a warp a row.
+__global__ void __launch_bounds__(256) k_sizes(const u32* __restrict__ Y, u32 ny, const u32* __restrict__ X, u32 nx, u32 ncol,
+                                               u32 ntip, u32* __restrict__ ysize, u32* __restrict__ ymin,
+                                               u32* __restrict__ xsize, u32* __restrict__ xmin) {
+    const u32 i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= ny + nx) return;
+    const bool isY = i < ny;
+    const u32 r = isY ? i : i - ny;
+    const u32* row = (isY ? Y : X) + (size_t)r * ncol;
+    u32 c = 0;
+    for (u32 k = lane; k < ncol; k += 32) c += (u32)__popc(row[k]);
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if (lane == 0) {
+        (isY ? ysize : xsize)[r] = c > ntip - c ? ntip - c : c;
+        (isY ? ymin : xmin)[r] = 32u * ncol;
+    }
+}
+
+// Distances of 32 x rows (lanes) and 64 y rows (a group of eight a warp) from the
+// XORed words, 32 words of both at a time in shared memory.
+constexpr u32 kTX = 32, kTY = 64, kWords = 32;
+__global__ void __launch_bounds__(256) k_cross(const u32* __restrict__ X, const u32* __restrict__ Y, u32 nx, u32 ny, u32 ncol,
+                                               u32 ntip, u32* __restrict__ xmin, u32* __restrict__ ymin) {
+    __shared__ u32 xs[kTX][kWords + 1];
+    __shared__ u32 ys[kTY][kWords];
+    __shared__ u32 red[8][kTX];
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const u32 x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, x = x0 + lane;
+    u32 d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (u32 k0 = 0; k0 < ncol; k0 += kWords) {
+        const u32 k = k0 + lane;
+        for (u32 r = w; r < kTX; r += 8) xs[r][lane] = x0 + r < nx && k < ncol ? X[(size_t)(x0 + r) * ncol + k] : 0u;
+        for (u32 r = w; r < kTY; r += 8) ys[r][lane] = y0 + r < ny && k < ncol ? Y[(size_t)(y0 + r) * ncol + k] : 0u;
+        __syncthreads();
+        const u32 kn = min(kWords, ncol - k0);
+        for (u32 j = 0; j < kn; j++) {
+            const u32 v = xs[lane][j];
+#pragma unroll
+            for (u32 i = 0; i < 8; i++) d[i] += (u32)__popc(v ^ ys[8 * w + i][j]);
+        }
+        __syncthreads();
+    }
+    const u32 full = 32u * ncol, pad = full - ntip;
+    const bool xok = x < nx;
+    u32 A = full, B = full;
+#pragma unroll
+    for (u32 i = 0; i < 8; i++) {
+        const u32 yr = y0 + 8 * w + i;
+        if (yr < ny) {
+            A = min(A, d[i]);
+            B = min(B, full - d[i]);
+        }
+        u32 ya = xok ? d[i] : full, yb = xok ? full - d[i] : full;
+#pragma unroll
+        for (u32 o = 1; o < 8; o <<= 1) {
+            ya = min(ya, __shfl_xor_sync(0xFFFFFFFFu, ya, o));
+            yb = min(yb, __shfl_xor_sync(0xFFFFFFFFu, yb, o));
+        }
+        u32 v = (x & ~7u) < nx ? min(ya, yb - pad) : 0xFFFFFFFFu;  // groups of eight x rows
+        v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, 8));
+        v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, 16));
+        if (lane == 0 && yr < ny) atomicMin(ymin + yr, v);
+    }
+    red[w][lane] = min(A, B - pad);
+    __syncthreads();
+    if (w == 0 && xok) {
+        u32 v = red[0][lane];
+        for (u32 g = 1; g < 8 && y0 + 8 * g < ny; g++) v = min(v, red[g][lane]);
+        atomicMin(xmin + x, v);
+    }
+}
+
+// Whether the popcounts are the quicker: where row pairs x words are few, because
+// the rows are not packed and the tiles' step is long, or where the blocks are too
+// few to fill the device, because a step of theirs takes 0.12 us a word and one of the
+// tiles 0.19.  Calls by popcounts and by tiles: 5 x 5 clades x 1 word 44 and 62 us,
+// 998 x 998 x 32 (32 million) 79 and 93, 5,000 x 100 x 157 (78) 315 and 324, 1,498 x
+// 1,498 x 47 (105) 150 and 153, then 20,000 x 2,000 x 4 (160) 256 and 224, 1,998 x
+// 1,998 x 63 (251) 205 and 172, 100 x 10,000 x 313 (313) 883 and 814; of few blocks,
+// 200 x 200 x 3,000 (120 million, 28 blocks) 748 and 905, 600 x 600 x 1,000 (360, 190
+// blocks) 501 and 507, then 800 x 800 x 300 (192, 325 blocks) 231 and 223.
+constexpr u64 kPopcounts = 100000000;
+constexpr u32 kPopBlocks = 240;
+static bool popcounts_pay(u64 ny, u64 nx, u64 ncol) {
+    const u64 blocksY = (ny + kTY - 1) / kTY, blocks = (nx + kTX - 1) / kTX * blocksY;
+    return blocksY <= 65535 && (blocks <= kPopBlocks || ny * nx <= kPopcounts / ncol);
+}
 
 // Rows r00 .. r00 + m - 1 of n, ncol words each (M: row r00) -> 128-bit chunks,
 // uint4 at [c * n + row], and the rows' popcounts and sizes, and the minima's start:
@@ -178,6 +267,23 @@ static int transfer_tiles(const TransferSide& y, const TransferSide& x, u32 ncol
     return CASPHY_OK;
 }
 
+// Both sides' rows into `rows`, then sizes and distances by popcounts.
+static int transfer_popcounts(DeviceScope& ds, const TransferSide& y, const TransferSide& x, u32 ncol, u32 ntip, u32* rows,
+                              cudaStream_t st) {
+    using namespace tdis;
+    u32* dx = rows + (size_t)y.n * ncol;
+    if (y.n)
+        if (int rc = Staged::to_device(ds, rows, y.host, sizeof(u32) * (size_t)y.n * ncol, st)) return rc;
+    if (x.n)
+        if (int rc = Staged::to_device(ds, dx, x.host, sizeof(u32) * (size_t)x.n * ncol, st)) return rc;
+    k_sizes<<<(y.n + x.n + 7) / 8, 256, 0, st>>>(rows, y.n, dx, x.n, ncol, ntip, y.size, y.least, x.size, x.least);
+    if (x.n && y.n)
+        k_cross<<<dim3((x.n + kTX - 1) / kTX, (y.n + kTY - 1) / kTY), 256, 0, st>>>(dx, rows, x.n, y.n, ncol, ntip, x.least,
+                                                                                y.least);
+    CASPHY_CUDA_TRY(cudaGetLastError());
+    return CASPHY_OK;
+}
+
 }  // namespace casphy
 
 extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t ncol, uint32_t ntip, const uint32_t* y,
@@ -190,19 +296,25 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     if (!nrow_y && !nrow_x) return CASPHY_OK;
     DeviceScope ds;
     cudaStream_t st = 0;
+    const u64 nrow = (u64)nrow_y + nrow_x;
+    const bool tiles = nrow > 0xFFFFFFFFull || !tdis::popcounts_pay(nrow_y, nrow_x, ncol);
     const u32 per = std::max(panel_rows(nrow_y, ncol), panel_rows(nrow_x, ncol));
     const size_t chunks = (ncol + 3) / 4;
     TransferSide Y{nrow_y, y, nullptr, nullptr, nullptr, nullptr}, X{nrow_x, x, nullptr, nullptr, nullptr, nullptr};
     u32 *panel, *out;
     auto lay = [&](Carve& c) {
+        // minima and sizes of both sides and the error of a device-side wait, read
+        // back together
+        out = c.take<u32>(2 * (size_t)nrow + 1);
+        if (!tiles) {  // both sides' rows
+            panel = c.take<u32>((size_t)nrow * ncol);
+            return;
+        }
         panel = c.take<u32>((size_t)per * ncol);
         for (TransferSide* s : {&Y, &X}) {
             s->chunks = c.take<uint4>(chunks * s->n);
             s->pop = c.take<u32>(s->n);
         }
-        // minima and sizes of both sides and the error of a device-side wait, read
-        // back together
-        out = c.take<u32>(2 * (size_t)nrow_y + 2 * (size_t)nrow_x + 1);
     };
     Carve cv;
     lay(cv);
@@ -217,16 +329,20 @@ extern "C" int casphy_transfer_dis(uint32_t nrow_y, uint32_t nrow_x, uint32_t nc
     X.least = Y.size + nrow_y;
     X.size = X.least + nrow_x;
     int* err = reinterpret_cast<int*>(X.size + nrow_x);
-    if ((rc = pack_side(ds, Y, ncol, ntip, panel, err, st))) return rc;
-    if ((rc = pack_side(ds, X, ncol, ntip, panel, err, st))) return rc;
-    if ((rc = transfer_tiles(Y, X, ncol, ntip, err, st))) return rc;
+    if (tiles) {
+        if ((rc = pack_side(ds, Y, ncol, ntip, panel, err, st))) return rc;
+        if ((rc = pack_side(ds, X, ncol, ntip, panel, err, st))) return rc;
+        if ((rc = transfer_tiles(Y, X, ncol, ntip, err, st))) return rc;
+    } else if ((rc = transfer_popcounts(ds, Y, X, ncol, ntip, panel, st))) {
+        return rc;
+    }
     u32 werr = 0;
     ReadBack back;
     back.add(ymin, nrow_y);
     back.add(ysize, nrow_y);
     back.add(xmin, nrow_x);
     back.add(xsize, nrow_x);
-    back.add(&werr, 1);
+    if (tiles) back.add(&werr, 1);
     if ((rc = back.run(out, st))) return rc;
     if (werr) casphy_set_last_error_msg("transfer: a device-side wait timed out");
     return (int)werr;

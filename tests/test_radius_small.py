@@ -49,8 +49,8 @@ def test_transfer_of_one_side_only(gpu_lib):
 
 
 def test_transfer_rows_in_panels(gpu_lib):
-    """Rows come through a 64 MiB panel: 520 rows of 32,768 words take two, the
-    other side one."""
+    """520 rows of 32,768 words, more than the 64 MiB panel that rows for the tiles come
+    through: so few blocks take the popcounts, which need both sides whole."""
     rng = np.random.default_rng(3)
     nb = 32768
     y = rng.integers(0, 1 << 32, size=(520, nb), dtype=np.uint64).astype(np.uint32)
