@@ -111,11 +111,10 @@ constexpr u32 kFloatClusterTips = 90000;
 // eight at a time): 0.41 at 10,000 x 512 with 3 planes, 0.77 at 20,000 x 512 with 8
 // and 10,000 x 512 with 15, 0.88 at 20,000 x 1,024 with 6 (3.8 million), then 0.94 at
 // 10,000 x 1,024 with 14 (4.5), 1.25 at 80,000 x 128 with 8 (5.1), 1.31 at 20,000 x
-// 1,024 with 14 (9.0).  Rows of many words leave most warps of a CTA without a slot
-// (500 cells, 3 planes: 0.60 at 3,000 sites, 0.88 at 10,000, 1.01 at 15,000, 1.07 at
-// 20,000, 1.47 at 30,000); with one plane they still gain (0.88 at 30,000).
+// 1,024 with 14 (9.0).  Rows of many words are no reason to leave it, since a query's
+// warps share them (500 cells, 3 planes: 0.30 at 8,192 sites, 0.28 at 15,000, 0.27 at
+// 30,000).
 constexpr u64 kPlaneClusterWork = 4500000;
-constexpr u32 kPlaneClusterWords = 448;
 constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 
 // Launches the join on one cluster; *done says whether it could.
@@ -126,7 +125,7 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     *done = false;
     if (PATH == PATH_FLOAT && c.ntip > kFloatClusterTips) return CASPHY_OK;
     if (PATH == PATH_PLANES && bm.nplanes > 1 &&
-        (bm.nbin > kPlaneClusterWords || (u64)c.ntip * bm.nplanes * ((bm.nbin + 7) / 8 * 8) > kPlaneClusterWork))
+        (u64)c.ntip * bm.nplanes * ((bm.nbin + 7) / 8 * 8) > kPlaneClusterWork)
         return CASPHY_OK;
     int smemMax = 0, dev = 0;
     CASPHY_CUDA_TRY(cudaGetDevice(&dev));

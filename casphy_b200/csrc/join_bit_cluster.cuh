@@ -18,6 +18,16 @@
 namespace casphy {
 namespace bitjoin {
 
+// Rows of so many words are shared out among a query's warps where there are fewer
+// groups of 32 slots than warps; a warp that takes a group alone leaves the others
+// idle for as long as it walks the row, but shared sums cost a barrier and an atomic
+// a slot.  Loops shared and not, one plane: 4,000 cells x 48 words 15.7 and 14.2 ms,
+// x 64 16.5 and 15.6, x 96 17.5 and 17.6, x 128 18.8 and 19.9, 500 x 938 2.9 and 9.0;
+// three planes: 8,000 x 32 45.8 and 45.0, 4,000 x 48 22.4 and 23.9, x 64 24.1 and
+// 27.1, 500 x 938 5.0 and 21.2; bootstrap joins of 40 replicates of 100 to 300 cells x
+// 3,125 words 16 and 78, of 64 of 167 to 500 x 938 13 and 37.
+constexpr u32 kShareWords = 128, kShareWordsPlanes = 64;
+
 template <int PATH>
 struct BitCluster {
     static constexpr bool kNarrow = false;  // binary32 scores
@@ -69,8 +79,14 @@ struct BitCluster {
         __shared__ u32 s_ne[2];
         return s_ne + par;
     }
+    // sums of words shared out among warps, 0 between the scans
+    __device__ static u32* sums() {
+        __shared__ u32 s_sum[joinc::kThreads];
+        return s_sum;
+    }
     __device__ static void begin(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots& st) {
         s.rank = rank;
+        sums()[threadIdx.x] = 0u;
         s.col = m.colT[0] + (size_t)rank * a.R;
         s.stride = m.Sp;
         s.next = 1;
@@ -264,21 +280,26 @@ struct BitCluster {
             }
             return fa;
         }
-        const u32 P = planes(m);
+        return (float)count<RES>(m, s, c, sq, 0u, m.nbin);
+    }
+    // Integer weights: the score's words [w0, wEnd), w0 a multiple of eight.
+    template <bool RES>
+    __device__ __forceinline__ static u32 count(const Args& m, const Smem& s, const u32* c, const u32* sq, u32 w0,
+                                                u32 wEnd) {
+        const u32 stride = s.stride, P = planes(m);
         u32 acc = 0;
         if (P == 1 && RES) {
-            u32 w = 0;
+            u32 w = w0;
 #pragma unroll 4
-            for (; w + 4 <= m.nbin; w += 4) {
+            for (; w + 4 <= wEnd; w += 4) {
                 const uint4 a = *reinterpret_cast<const uint4*>(sq + w);
                 const u32 v0 = c[w * stride], v1 = c[(w + 1) * stride], v2 = c[(w + 2) * stride], v3 = c[(w + 3) * stride];
                 acc += (u32)(__popc(a.x & v0) + __popc(a.y & v1)) + (u32)(__popc(a.z & v2) + __popc(a.w & v3));
             }
-            for (; w < m.nbin; w++) acc += (u32)__popc(sq[w] & c[w * stride]);
-            return (float)acc;
+            for (; w < wEnd; w++) acc += (u32)__popc(sq[w] & c[w * stride]);
+            return acc;
         }
         // eight words of the slot at a time against every plane's
-        u32 w0 = 0;
         auto block = [&](const u32 (&v)[8]) {
             for (u32 k = 0; k < P; k++) {
                 const uint4 a = *reinterpret_cast<const uint4*>(sq + k * m.nbinP + w0);
@@ -291,20 +312,20 @@ struct BitCluster {
                            << k;
             }
         };
-        for (; w0 + 8 <= m.nbin; w0 += 8) {
+        for (; w0 + 8 <= wEnd; w0 += 8) {
             u32 v[8];
 #pragma unroll
             for (u32 j = 0; j < 8; j++) v[j] = RES ? c[(w0 + j) * stride] : ld_cg_u32(c + (size_t)(w0 + j) * stride);
             block(v);
         }
-        if (w0 < m.nbin) {  // words past the row are 0 on the slot's side
+        if (w0 < wEnd) {  // words past the row are 0 on the slot's side
             u32 v[8];
 #pragma unroll
             for (u32 j = 0; j < 8; j++)
-                v[j] = w0 + j >= m.nbin ? 0u : (RES ? c[(w0 + j) * stride] : ld_cg_u32(c + (size_t)(w0 + j) * stride));
+                v[j] = w0 + j >= wEnd ? 0u : (RES ? c[(w0 + j) * stride] : ld_cg_u32(c + (size_t)(w0 + j) * stride));
             block(v);
         }
-        return (float)acc;
+        return acc;
     }
 
     template <class F, class D>
@@ -313,9 +334,38 @@ struct BitCluster {
         const u32 lgq = nq <= 1 ? 4u : (nq <= 2 ? 3u : (nq <= 4 ? 2u : 1u));
         const u32 nwq = 1u << lgq;
         const u32 q = warp >> lgq, wi = warp & (nwq - 1u);
+        const bool resident = s.col == s.colS;
+        const u32 groups = (st.n + 31u) / 32u;
+        if (PATH != PATH_FLOAT && groups < nwq && m.nbin >= (planes(m) > 1 ? kShareWordsPlanes : kShareWords)) {
+            // a query's warps share the words of all groups of 32 slots evenly
+            u32* acc = sums() + q * nwq * 32;
+            if (q < nq) {
+                const u32* sq = s.sq + (size_t)q * planes(m) * m.nbinP;
+                const u32 blocks = (m.nbin + 7u) / 8u, total = groups * blocks;
+                for (u32 i = wi * total / nwq, end = (wi + 1u) * total / nwq; i < end;) {
+                    const u32 g = i / blocks, b = i - g * blocks, e = min(blocks, b + end - i);
+                    const u32 x = 32 * g + lane, xs = x < st.n ? x : 32 * g, w1 = min(8 * e, m.nbin);
+                    const u32 v = resident ? count<true>(m, s, s.colS + xs, sq, 8 * b, w1)
+                                           : count<false>(m, s, s.col + xs, sq, 8 * b, w1);
+                    if (x < st.n) atomicAdd(acc + x, v);
+                    i += e - b;
+                }
+            }
+            __syncthreads();
+            if (q < nq) {
+                const u32 x = 32 * wi + lane;
+                if (x < st.n) {
+                    const float v = (float)acc[x];
+                    acc[x] = 0u;
+                    f(q, x, ord_f32(v));
+                }
+                done(q);
+            }
+            if (s.prof) joinx::prof_mark(joinx::PROF_SC_ACC);
+            return;
+        }
         if (q < nq) {
             const u32* sq = s.sq + (size_t)q * planes(m) * m.nbinP;
-            const bool resident = s.col == s.colS;
             for (u32 x0 = wi * 32; x0 < st.n; x0 += nwq * 32) {
                 const u32 x = x0 + lane, xs = x < st.n ? x : x0;
                 // (two calls, so that resident columns are read as shared memory)

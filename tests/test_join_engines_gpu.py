@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+from casphy_b200 import bootstrap as B
 from casphy_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -180,17 +181,57 @@ def test_fractional_bit_engine_follows_the_cells(gpu_lib, ncell, launches):
 
 
 # Integer weights of several planes: a cluster up to 4,500,000 cells x planes x
-# words, the words in blocks of eight, and up to 448 words.
+# words, the words in blocks of eight.
 @pytest.mark.parametrize("ncell,nsite,top,launches", [
     (9375, 992, 1 << 14, 5), (9376, 992, 1 << 14, 6), (9376, 992, (1 << 14) - 1, 5), (20000, 288, 1 << 14, 6),
-    (37500, 256, 1 << 14, 5), (37501, 256, 1 << 14, 6), (300, 14336, 4, 5), (300, 14368, 4, 6)])
+    (37500, 256, 1 << 14, 5), (37501, 256, 1 << 14, 6), (300, 14368, 4, 5)])
 def test_plane_bit_engine_follows_planes_and_words(gpu_lib, monkeypatch, ncell, nsite, top, launches):
     words = synth.binary_workload(ncell, nsite, 16, 0.04, 0.05, seed=ncell)
     w = np.zeros(nsite)
     w[:3] = 1, 2, top
     work = ncell * int(top).bit_length() * (-(-words.shape[1] // 8) * 8)
-    assert (work <= 4500000 and nsite <= 14336) == (launches == 5)
+    assert (work <= 4500000) == (launches == 5)
     got = gpu_lib.join_bit(words, w, 1)
     assert got[2]["kernel_launches"] == launches
     monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
     assert _same(got, gpu_lib.join_bit(words, w, 1))
+
+
+# Wide rows are shared out among a query's warps (from 128 words, with planes from
+# 64) while there are fewer groups of 32 slots than warps: sizes on both sides of the
+# lines, rows that end within a block of eight words, groups part filled and CTAs
+# without a slot, and ranges that reach fewer groups only by a compaction.
+@pytest.mark.parametrize("weights,ncell,nsite", [
+    ("unit", 9, 4096), ("unit", 333, 4064), ("unit", 333, 4096), ("unit", 1000, 4128), ("unit", 520, 9632),
+    ("unit", 9000, 4160), ("planes", 9, 2048), ("planes", 333, 2016), ("planes", 333, 2080), ("planes", 1200, 4000),
+    ("planes", 17, 30016)])
+def test_wide_rows_on_a_cluster(gpu_lib, monkeypatch, weights, ncell, nsite):
+    words, w = _bit(ncell, nsite, weights, ncell + nsite)
+    got = gpu_lib.join_bit(words, w, 1)
+    assert got[2]["kernel_launches"] == (6 if ncell == 9000 else 5)
+    if ncell <= 1200:
+        assert _same(got, O.join_bit(words, w, 1))
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    assert _same(got, gpu_lib.join_bit(words, w, 1))
+
+
+# A replicate's columns stay in global memory at first; clusters of every size.
+@pytest.mark.parametrize("mult", [1, 3])
+@pytest.mark.parametrize("group", [1, 2, 8])
+def test_wide_rows_of_replicates(gpu_lib, monkeypatch, mult, group):
+    ncell, nsite, sizes = 1500, 12000, [2, 33, 290, 512, 700, 1500]
+    words = synth.binary_workload(ncell, nsite, 14, 0.03, 0.05, seed=2)
+    rng = np.random.default_rng(4)
+    w = np.stack([np.bincount(rng.integers(0, nsite, nsite), minlength=words.shape[1] * 32) for _ in sizes]) * float(mult)
+    cells = [np.sort(rng.permutation(ncell)[:n]) for n in sizes]
+    full = gpu_lib.join_bit(words, None, 1)[0]
+    monkeypatch.setenv("CASPHY_BS_GROUP", str(group))
+    got = gpu_lib.bootstrap_bit(words, full, np.concatenate([[0], np.cumsum(sizes)]), np.concatenate(cells), w, raw_edges=True)
+    assert got["stats"]["max_ctas_per_rep"] == group
+    monkeypatch.setenv("CASPHY_JOIN_ENGINE", "grid")
+    for r, n in enumerate(sizes):
+        edge = gpu_lib.join_bit(np.ascontiguousarray(words[cells[r]]), w[r], 1)[0]
+        ncol = (n + 31) // 32
+        a = B.clade_bits(edge, n, ncol)
+        b = B.clade_bits(got["raw_edges"][r].reshape(-1, 2), n, ncol)
+        assert np.array_equal(np.unique(a, axis=0), np.unique(b, axis=0)), n
