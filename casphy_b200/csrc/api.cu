@@ -131,16 +131,12 @@ int DeviceScope::reserve_aux(size_t bytes, void** out) {
 }
 
 // Staged copies.  The driver copies a pageable buffer through its own staging
-// on the calling thread: 17 to 20 GB/s on a B200 host whose link takes 55 GB/s.
+// on the calling thread: 20 GB/s on a B200 host whose link takes 55 GB/s.
 // kCopyThreads threads with four 1 MiB slots each reach 40 GB/s (eight were no
-// faster: starting them took what they gained).  They live for one copy, and
-// starting them takes 100 to 400 us, so buffers below kCopyMin stay with the
-// driver (a call around one upload, driver and threads: 12 MiB 0.85 and 1.05 ms,
-// 16 MiB 1.08 and 1.19, 20 MiB 1.32 and 1.35, 24 MiB 1.55 and 1.46, 32 MiB 2.03
-// and 1.71; around a download: 16 MiB 0.91 and 0.71 to 1.13, 24 MiB 1.32 and 1.15
-// to 1.29, 32 MiB 1.73 and 1.47); the slots stay with the arena, whose lock the
-// caller holds.
-constexpr size_t kCopySlot = size_t(1) << 20, kCopyMin = size_t(24) << 20;
+// faster: starting them took what they gained).  They live for one copy, so
+// buffers below kCopyMin stay with the driver; the slots stay with the arena,
+// whose lock the caller holds.
+constexpr size_t kCopySlot = size_t(1) << 20, kCopyMin = size_t(10) << 20;
 constexpr int kCopyThreads = 4, kCopyTurns = 4, kCopySlots = kCopyTurns * kCopyThreads;
 
 static bool staging_ready(Arena* a) {
