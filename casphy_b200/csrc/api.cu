@@ -131,11 +131,14 @@ int DeviceScope::reserve_aux(size_t bytes, void** out) {
 }
 
 // Staged copies.  The driver copies a pageable buffer through its own staging
-// on the calling thread: 20 GB/s on a B200 host whose link takes 55 GB/s.
-// kCopyThreads threads with four 1 MiB slots each reach 40 GB/s (eight were no
-// faster: starting them took what they gained).  They live for one copy, so
-// buffers below kCopyMin stay with the driver; the slots stay with the arena,
-// whose lock the caller holds.
+// on the calling thread: 12 GB/s on a B200 host whose link takes 55 GB/s, 20 where
+// the buffer is in the host's caches.  kCopyThreads threads with four 1 MiB slots each
+// reach 40 GB/s (eight were no faster: starting them took what they gained).  They
+// live for one copy, so buffers below kCopyMin stay with the driver (a call around one
+// upload by the driver and by threads, 10.1 MiB not in the caches 1.18 and 1.02 ms, 16
+// MiB 1.79 and 1.30, 32 MiB 3.46 and 2.01; in the caches 0.78 and 0.91, 1.12 and 1.17,
+// 2.15 and 1.72; around a download to new pages, 11 MiB 2.6 and 1.2 ms, 32 MiB 7.0
+// and 2.7); the slots stay with the arena, whose lock the caller holds.
 constexpr size_t kCopySlot = size_t(1) << 20, kCopyMin = size_t(10) << 20;
 constexpr int kCopyThreads = 4, kCopyTurns = 4, kCopySlots = kCopyTurns * kCopyThreads;
 

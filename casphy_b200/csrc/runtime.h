@@ -23,8 +23,9 @@ struct DeviceScope {
 // Copies of large pageable host buffers: kCopyMin bytes and more go through
 // pinned slots of the device's arena, filled or emptied by several host
 // threads (the driver's own staging copies on one).  to_device returns when
-// every copy is queued on the stream and src has been read; to_host when dst
-// has been written, after all work queued on the stream before.
+// every copy is queued on the stream, with a pageable src read; a page-locked one
+// may still be read until the stream has passed the copy.  to_host returns when
+// dst has been written, after all work queued on the stream before.
 struct Staged {
     static int to_device(DeviceScope& ds, void* dst, const void* src, size_t bytes, void* stream);
     static int to_host(DeviceScope& ds, void* dst, const void* src, size_t bytes, void* stream);
