@@ -60,7 +60,6 @@ namespace casphy {
 namespace boot {
 
 using namespace bitjoin;
-using Model = BitCluster<PATH_PLANES>;
 
 constexpr u32 kOpInternal = 0x80000000u, kOpRoot = 0x40000000u;
 constexpr u32 kXThreads = 128;  // clades per transfer block
@@ -69,7 +68,7 @@ constexpr u32 kOpChunk = 2048;  // ops staged in shared memory per step
 
 struct Rep {
     joinc::Args c;
-    Model::Args m;
+    BitClusterArgs m;
     InitArgs init;
     u32 off;        // first tip in the concatenated cell list
     u32* colT;
@@ -316,6 +315,7 @@ __device__ __forceinline__ void build_ops(const joinc::Args& c, const u32* __res
 }
 
 // Cluster i joins replicate order[i].
+template <class Model>
 __global__ void __launch_bounds__(joinc::kThreads, 1) k_bs_join(const Rep* __restrict__ reps,
                                                                 const u32* __restrict__ order, u32 G,
                                                                 const u32* __restrict__ rankOf,
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(joinc::kThreads, 1) k_bs_join(const Rep* __res
     const u32 r = order[blockIdx.x / G], rank = joinc::cluster_rank();
     if (*initErr) return;  // (an earlier kernel's: the same for all)
     const joinc::Args c = reps[r].c;
-    const Model::Args m = reps[r].m;
+    const BitClusterArgs m = reps[r].m;
     const u64 t0 = globaltimer_ns();
     joinc::cluster_join<Model>(c, m, rank, smem);
     __syncthreads();
@@ -646,7 +646,9 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     int maxSmem = 0;
     CASPHY_CUDA_TRY(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ds.dev));
     const size_t smemLim = (size_t)maxSmem - 6144;  // the kernel's static shared memory
-    auto plan = [&](u32 n, u32 G, joinc::Args& a, Model::Args& m, size_t* smem) {
+    const auto joinFn = wide_rows(nbin, nplanes) ? k_bs_join<BitCluster<PATH_PLANES, true>>
+                                                 : k_bs_join<BitCluster<PATH_PLANES>>;
+    auto plan = [&](u32 n, u32 G, joinc::Args& a, BitClusterArgs& m, size_t* smem) {
         a.ntip = n;
         a.nnode = 2 * n - 1;
         a.G = G;
@@ -673,11 +675,11 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     double bestUs = 0;
     for (u32 g = 1; g <= joinc::kMaxG; g *= 2) {
         joinc::Args a{};
-        Model::Args m{};
+        BitClusterArgs m{};
         size_t sm = 0;
         if (!plan(nmax, g, a, m, &sm)) continue;
         sm = std::max(sm, opsBytes);
-        const int slots = joinc::placeable((void*)k_bs_join, g, sm);
+        const int slots = joinc::placeable((void*)joinFn, g, sm);
         if (slots < 1) continue;
         const double t = g == fixedG ? 0.0 : makespan_us(tune, sorted, g, (u32)slots);
         if (G == 0 || t < bestUs) {
@@ -850,7 +852,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
     int perSM = 0;
     CASPHY_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_bs_init, kThreads, 0));
     // (the planned size may have shrunk to what the replicates need)
-    if (joinc::placeable((void*)k_bs_join, G, smem) < 1) return CASPHY_EINTERNAL;
+    if (joinc::placeable((void*)joinFn, G, smem) < 1) return CASPHY_EINTERNAL;
     XferArgs xa{nX, nrep, 32u * ((ntip + 31) / 32), gl.Xlo, gl.Xhi, gl.repN, gl.repOff, gl.repOpsOff, gl.sortedRank, gl.ops,
                 threshold, gl.ymin, gl.ysize, gl.support, gl.xerr};
     // the whole pass: prep, initial scans, the joins, transfer
@@ -878,7 +880,7 @@ extern "C" int casphy_bootstrap_bit(uint32_t ntip, uint32_t nbin, const uint32_t
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal)) != cudaSuccess) return e;
-        if ((e = joinc::enqueue(k_bs_join, G, nrep, smem, s, (const Rep*)gl.reps, (const u32*)gl.order, G,
+        if ((e = joinc::enqueue(joinFn, G, nrep, smem, s, (const Rep*)gl.reps, (const u32*)gl.order, G,
                                 (const u32*)gl.rankOf, (const int*)(gl.xerr + 2), opsShared)) !=
             cudaSuccess)
             return e;

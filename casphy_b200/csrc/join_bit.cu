@@ -121,7 +121,6 @@ constexpr u32 kClusterSlots = 32;  // ranges are multiples of a warp
 template <int PATH>
 static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PATH>::Args& bm, u32 Sp,
                               const unsigned long long* initKey, cudaStream_t st, bool* done, u32* scanPath) {
-    using M = BitCluster<PATH>;
     *done = false;
     if (PATH == PATH_FLOAT && c.ntip > kFloatClusterTips) return CASPHY_OK;
     if (PATH == PATH_PLANES && bm.nplanes > 1 &&
@@ -145,12 +144,16 @@ static int launch_bit_cluster(const joinx::Common& c, const typename BitModel<PA
     a.compactMin = 1024;
     a.bytesPerPairSite = c.bytesPerPairSite;
     a.deathWords = (c.nnode + 31) / 32;
-    typename M::Args m{bm.nbin, bm.nbinP, bm.nplanes, bm.ancType, bm.planeMask, bm.wf, bm.nodeSeq, bm.nodeBis,
-                       {bm.colT[0], bm.colT[1]}, Sp, 0, 0, 8};
+    BitClusterArgs m{bm.nbin, bm.nbinP, bm.nplanes, bm.ancType, bm.planeMask, bm.wf, bm.nodeSeq, bm.nodeBis,
+                     {bm.colT[0], bm.colT[1]}, Sp, 0, 0, 8};
     size_t smem = 0;
     if (!cluster_fit<PATH>(a, m, (size_t)smemMax - 6144, &smem)) return CASPHY_OK;
     if (PATH != PATH_FLOAT && m.colWords < (size_t)m.nbin * a.R) return CASPHY_OK;
-    const int rc = joinc::launch(k_cluster_join<M>, a.G, smem, st, done, a, m);
+    int rc;
+    if (PATH != PATH_FLOAT && wide_rows(m.nbin, m.nplanes))
+        rc = joinc::launch(k_cluster_join<BitCluster<PATH, PATH != PATH_FLOAT>>, a.G, smem, st, done, a, m);
+    else
+        rc = joinc::launch(k_cluster_join<BitCluster<PATH>>, a.G, smem, st, done, a, m);
     if (*done && m.colWords >= (size_t)m.nbin * a.R) *scanPath = 1u;
     return rc;
 }

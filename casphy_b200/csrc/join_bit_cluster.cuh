@@ -28,21 +28,28 @@ namespace bitjoin {
 // 3,125 words 16 and 78, of 64 of 167 to 500 x 938 13 and 37.
 constexpr u32 kShareWords = 128, kShareWordsPlanes = 64;
 
-template <int PATH>
+// Whether the rows of nbin words (nplanes: 0 or 1 plane) are shared so.
+inline bool wide_rows(u32 nbin, u32 nplanes) { return nbin >= (nplanes > 1 ? kShareWordsPlanes : kShareWords); }
+
+struct BitClusterArgs {
+    u32 nbin, nbinP, nplanes;
+    int ancType;
+    const u32* planeMask;  // nplanes x nbin
+    const float* wf;       // nbin x 32 (FLOAT)
+    u32* nodeSeq;
+    u32* nodeBis;
+    u32* colT[2];          // nbin x Sp
+    u32 Sp, maxBatch;
+    u32 colWords;          // shared-memory words for resident columns
+    u32 compactAt;         // sixteenths of the slots still live at a compaction
+};
+
+// WIDE: rows shared out among the warps.  A kernel of its own, because that code
+// beside the other takes the narrow rows' phases from 2.58 to 2.62 us.
+template <int PATH, bool WIDE = false>
 struct BitCluster {
     static constexpr bool kNarrow = false;  // binary32 scores
-    struct Args {
-        u32 nbin, nbinP, nplanes;
-        int ancType;
-        const u32* planeMask;  // nplanes x nbin
-        const float* wf;       // nbin x 32 (FLOAT)
-        u32* nodeSeq;
-        u32* nodeBis;
-        u32* colT[2];          // nbin x Sp
-        u32 Sp, maxBatch;
-        u32 colWords;          // shared-memory words for resident columns
-        u32 compactAt;         // sixteenths of the slots still live at a compaction
-    };
+    using Args = BitClusterArgs;
     struct Smem {
         u32* sq;       // maxBatch x planes x nbinP: (plane-masked) query words
         uint2* ent;    // FLOAT: maxBatch x nbin * 32 (column offset << 5 | bit, weight), ascending
@@ -86,7 +93,7 @@ struct BitCluster {
     }
     __device__ static void begin(const joinc::Args& a, const Args& m, Smem& s, u32 rank, const joinc::Slots& st) {
         s.rank = rank;
-        sums()[threadIdx.x] = 0u;
+        if (WIDE) sums()[threadIdx.x] = 0u;
         s.col = m.colT[0] + (size_t)rank * a.R;
         s.stride = m.Sp;
         s.next = 1;
@@ -336,7 +343,7 @@ struct BitCluster {
         const u32 q = warp >> lgq, wi = warp & (nwq - 1u);
         const bool resident = s.col == s.colS;
         const u32 groups = (st.n + 31u) / 32u;
-        if (PATH != PATH_FLOAT && groups < nwq && m.nbin >= (planes(m) > 1 ? kShareWordsPlanes : kShareWords)) {
+        if (WIDE && groups < nwq) {
             // a query's warps share the words of all groups of 32 slots evenly
             u32* acc = sums() + q * nwq * 32;
             if (q < nq) {
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(joinc::kThreads, 1) k_cluster_join(joinc::Args
 // batches of rescanned rows first, then resident columns; false when it does
 // not fit.
 template <int PATH>
-inline bool cluster_fit(joinc::Args& a, typename BitCluster<PATH>::Args& m, size_t lim, size_t* smem) {
+inline bool cluster_fit(joinc::Args& a, BitClusterArgs& m, size_t lim, size_t* smem) {
     for (a.maxBatch = joinx::stale_batch_setting(); a.maxBatch >= 1; a.maxBatch--) {
         m.maxBatch = a.maxBatch;
         m.colWords = 0;
