@@ -484,7 +484,7 @@ static int radius_impl(RadiusInput& in, u32 row0, u32 row1, u32* counts, u32* id
     CASPHY_CUDA_TRY(cudaMemcpyAsync(L.off, off.data(), sizeof(u64) * nq, cudaMemcpyHostToDevice, st));
     k_expand<<<(nq + 7) / 8, 256, 0, st>>>(L.mask, nq, maskWords, L.off, didx);
     CASPHY_CUDA_TRY(cudaGetLastError());
-    if (tot && (rc = Staged::to_host(ds, idx, didx, sizeof(u32) * tot, st))) return rc;
+    if (tot) return Staged::to_host(ds, idx, didx, sizeof(u32) * tot, st);  // (waits for the stream)
     CASPHY_CUDA_TRY(cudaStreamSynchronize(st));
     return CASPHY_OK;
 }
